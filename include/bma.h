@@ -262,6 +262,18 @@ int bma_attn_bwd_plan(const bma_attn_args* args, int32_t* backend, int32_t* q_ti
 int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec,
                  const bma_block_lists* lists, bma_stream_t stream);
 
+/* float32 inputs on the tensor core: every operand as three bf16 planes (exact), six plane products per matrix product,
+ * float32 sums -- the accuracy of FP32 FMA arithmetic.  The caller provides the workspace that holds the planes (16-byte
+ * aligned) and block lists of BMA_F32_TILE x BMA_F32_TILE blocks; everything else is as for bma_attn_fwd / bma_attn_bwd.
+ * bma_attn_f32_workspace_bytes: bytes the pass needs, or 0 when it does not cover the request (then the plain entry points
+ * do: other input types, a forced backend, backward with a head dimension above 64, L above 524288 / 131072). */
+enum { BMA_F32_TILE = 128 };
+size_t bma_attn_f32_workspace_bytes(const bma_attn_args* args, int32_t backward);
+int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
+                     void* workspace, size_t workspace_bytes, bma_stream_t stream);
+int bma_attn_bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
+                     void* workspace, size_t workspace_bytes, bma_stream_t stream);
+
 /* Backward preprocess: delta = rowsum(dO * O); when d_o_bf16 is non-NULL also writes a
  * bf16 copy of dO there (and takes delta from that rounded copy, the values the backward's
  * dO V^T product sees, so that dP - delta cancels exactly where it should) as a DENSE

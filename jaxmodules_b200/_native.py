@@ -17,6 +17,7 @@ BMA_ERR_DEVICE_CHECK = 1
 BMA_DTYPE_F32, BMA_DTYPE_BF16 = 0, 1
 BMA_MASK_CAUSAL, BMA_MASK_BAND, BMA_MASK_BLOCK_WINDOW, BMA_MASK_SEGMENT, BMA_MASK_BITMAP, BMA_MASK_TILES = 1, 2, 4, 8, 16, 32
 BMA_MASK_COMPILE_CONSERVATIVE = 256
+F32_TILE = 128   # BMA_F32_TILE
 BMA_BACKEND_AUTO, BMA_BACKEND_SIMT, BMA_BACKEND_TCGEN05 = 0, 1, 2
 
 
@@ -103,6 +104,9 @@ SIGNATURES = {
     "bma_attn_plan": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "bma_attn_bwd_plan": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "bma_attn_fwd": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p]),
+    "bma_attn_f32_workspace_bytes": (C.c_size_t, [C.POINTER(AttnArgs), C.c_int32]),
+    "bma_attn_fwd_f32": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t, C.c_void_p]),
+    "bma_attn_bwd_f32": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t, C.c_void_p]),
     "bma_attn_bwd_preprocess": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.c_void_p]),
     "bma_attn_bwd_workspace_bytes": (C.c_size_t, [C.POINTER(AttnArgs)]),
     "bma_block_lists_visited": (C.c_int, [C.POINTER(BlockLists), C.c_void_p, C.c_void_p]),

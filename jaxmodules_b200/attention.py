@@ -150,6 +150,26 @@ def plan(Q, K, V, backend=nat.BMA_BACKEND_AUTO, backward: bool = False, key_bias
     return be.value, tq.value, tk.value
 
 
+def _route(a: nat.AttnArgs, backward: bool):
+    """(backend, q_tile, kv_tile, workspace bytes) of one pass; the workspace is that of the float32 tensor-core kernels
+    (``bma_attn_fwd_f32`` / ``bma_attn_bwd_f32``) and 0 where ``plan``'s kernels run."""
+    lib = nat.lib()
+    if a.q.dtype == nat.BMA_DTYPE_F32:
+        nbytes = lib.bma_attn_f32_workspace_bytes(C.byref(a), int(backward))
+        if nbytes:
+            return nat.BMA_BACKEND_SIMT, nat.F32_TILE, nat.F32_TILE, nbytes
+    be, tq, tk = C.c_int32(), C.c_int32(), C.c_int32()
+    fn = lib.bma_attn_bwd_plan if backward else lib.bma_attn_plan
+    nat.check(fn(C.byref(a), C.byref(be), C.byref(tq), C.byref(tk)), "bma_attn_plan")
+    return be.value, tq.value, tk.value, 0
+
+
+def tiles(Q, K, V, backend=nat.BMA_BACKEND_AUTO, backward: bool = False, key_bias=None, scale=None):
+    """(q_tile, kv_tile) of the block lists that ``attention_forward`` / ``attention_backward`` consume.  They are
+    ``plan``'s, except for float32 inputs on the tensor core, whose lists have 128-blocks."""
+    return _route(_make_args(Q, K, V, backend, scale, key_bias), backward)[1:3]
+
+
 class _Span:
     """One launch group: an NVTX range named after it (visible in a timeline profiler, free otherwise) and,
     when ``sink`` is a dict, a CUDA-event bracket on the launching stream (the benchmark times single
@@ -224,10 +244,10 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
     L = K.shape[1]
     with torch.cuda.device(dev):
         a = _make_args(Q, K, V, backend, scale, key_bias)
-        be, tq, tk = plan(Q, K, V, backend, key_bias=key_bias, scale=scale)
+        be, tq, tk, f32_bytes = _route(a, False)
         dmask = _masks.to_device_mask(terms, N, L, dev)
         # when the backward pass will walk the same tile size, build its q-side lists in the same launches
-        both_sides = need_q_side and plan(Q, K, V, backend, backward=True, key_bias=key_bias, scale=scale)[1:] == (tq, tk)
+        both_sides = need_q_side and _route(a, True)[1:3] == (tq, tk)
         with _Span(_profile_sink, "mask_compile", dev):
             ready = lists_fn(tq, tk, both_sides) if lists_fn is not None else None
             lists, lt = ready if ready is not None else compile_block_lists(dmask, B, Hq, N, L, tq, tk, dev, q_side=both_sides, conservative=True)
@@ -235,7 +255,12 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
         lse = torch.empty((B, Hq, N), dtype=torch.float32, device=dev)
         a.o, a.lse = _tensor(O), lse.data_ptr()
         with _Span(_profile_sink, "fwd", dev):
-            nat.check(lib.bma_attn_fwd(C.byref(a), C.byref(dmask.spec), C.byref(lists), _stream(dev)), "bma_attn_fwd")
+            if f32_bytes:
+                ws = torch.empty((f32_bytes,), dtype=torch.uint8, device=dev)
+                nat.check(lib.bma_attn_fwd_f32(C.byref(a), C.byref(dmask.spec), C.byref(lists), ws.data_ptr(), f32_bytes, _stream(dev)),
+                          "bma_attn_fwd_f32")
+            else:
+                nat.check(lib.bma_attn_fwd(C.byref(a), C.byref(dmask.spec), C.byref(lists), _stream(dev)), "bma_attn_fwd")
         _maybe_check_status(dev, "bma_attn_fwd")
     ctx = dict(dmask=dmask, lists=lists, list_tensors=lt, backend=be, scale=scale, lists_fn=lists_fn,
                lists_tile=(tq, tk), lists_have_q_side=both_sides, key_bias=key_bias)
@@ -250,7 +275,7 @@ def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
     L = K.shape[1]
     with torch.cuda.device(dev):
         a = _make_args(Q, K, V, backend, ctx.get("scale"), ctx.get("key_bias"))
-        be, tq, tk = plan(Q, K, V, backend, backward=True, key_bias=ctx.get("key_bias"), scale=ctx.get("scale"))
+        be, tq, tk, f32_bytes = _route(a, True)
         with _Span(_profile_sink, "mask_compile_bwd", dev):
             if ctx.get("lists_have_q_side") and ctx.get("lists_tile") == (tq, tk):
                 lists, lt = ctx["lists"], ctx["list_tensors"]      # built by the forward pass
@@ -280,6 +305,13 @@ def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
                 reuse["delta"], reuse["do_bf16"] = delta, do_bf16
         if do_bf16 is not None:
             a.d_o = _tensor(do_bf16)
+        if f32_bytes:
+            ws = torch.empty((f32_bytes,), dtype=torch.uint8, device=dev)
+            with _Span(_profile_sink, "bwd", dev):
+                nat.check(lib.bma_attn_bwd_f32(C.byref(a), C.byref(ctx["dmask"].spec), C.byref(lists), ws.data_ptr(), f32_bytes, st),
+                          "bma_attn_bwd_f32")
+            _maybe_check_status(dev, "bma_attn_bwd_f32")
+            return dQ, dK, dV
         ws_bytes = lib.bma_attn_bwd_workspace_bytes(C.byref(a))
         # dS hand-over between the two backward kernels: only for lists whose two sides name the same blocks.
         # The scratch is sized by the blocks the mask visits (fetched once per mask, see masks.visited_counts).

@@ -72,23 +72,6 @@ struct DqParams {
 __device__ __forceinline__ void setmaxnreg_inc_200() { asm volatile("setmaxnreg.inc.sync.aligned.u32 200;"); }
 __device__ __forceinline__ void setmaxnreg_dec_96() { asm volatile("setmaxnreg.dec.sync.aligned.u32 96;"); }
 
-// Allowed key interval [jlo, jhi] (tile-local, inclusive) of query row q for interval-only masks.
-__device__ __forceinline__ void row_interval(const MaskView& m, int q, int k0, int& jlo, int& jhi) {
-  if (q >= m.q_valid) { jlo = 1; jhi = 0; return; }
-  const int gq = q + m.q_offset;
-  int lo = 0, hi = INT32_MAX;
-  if (m.flags & BMA_MASK_CAUSAL) hi = min(hi, gq);
-  if (m.flags & BMA_MASK_BAND) { lo = max(lo, gq - m.band_left); hi = min(hi, gq + m.band_right); }
-  if (m.flags & BMA_MASK_BLOCK_WINDOW) {
-    int wlo, whi;
-    block_window_range(m, gq, wlo, whi);
-    lo = max(lo, wlo);
-    hi = min(hi, whi - 1);
-  }
-  jlo = lo - m.k_offset - k0;
-  jhi = min(hi - m.k_offset, m.k_valid - 1) - k0;
-}
-
 template <int HD, bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,

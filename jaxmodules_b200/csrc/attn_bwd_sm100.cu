@@ -116,63 +116,6 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 __device__ __forceinline__ void setmaxnreg_inc_208() { asm volatile("setmaxnreg.inc.sync.aligned.u32 208;"); }
 __device__ __forceinline__ void setmaxnreg_dec_80() { asm volatile("setmaxnreg.dec.sync.aligned.u32 80;"); }
 
-// Allowed query interval [jlo, jhi] (tile-local columns, inclusive) of key row k for masks made of
-// interval terms.  The block window of query block i starts at s(i) = clamp(i - left, 0, nblk - total): both ends are
-// non-decreasing in i, so the query blocks whose window contains the key form one range, whatever the window's
-// block size is relative to the tile.
-__device__ __forceinline__ void col_interval(const MaskView& m, int k, int q0, int& jlo, int& jhi) {
-  jlo = 0;
-  jhi = min(BT, m.q_valid - q0) - 1;
-  if (k >= m.k_valid) { jlo = 1; jhi = 0; return; }
-  const int gk = k + m.k_offset;
-  const int base = m.q_offset + q0;  // global index of column 0
-  if (m.flags & BMA_MASK_CAUSAL) jlo = max(jlo, gk - base);
-  if (m.flags & BMA_MASK_BAND) {  // gq - left <= gk <= gq + right  <=>  gk - right <= gq <= gk + left
-    jlo = max(jlo, gk - m.band_right - base);
-    jhi = min(jhi, gk + m.band_left - base);
-  }
-  if (m.flags & BMA_MASK_BLOCK_WINDOW) {
-    const int wb = m.win_block, total = m.win_left + m.win_right, last_start = m.win_nblk - total;
-    const int kb = gk / wb;            // key block of this key
-    const int t = kb - total + 1;      // the window reaches the key iff s(i) >= t ...
-    if (t > last_start) { jlo = 1; jhi = 0; return; }
-    if (t > 0) jlo = max(jlo, (t + m.win_left) * wb - base);
-    if (kb < last_start) jhi = min(jhi, (kb + m.win_left + 1) * wb - 1 - base);   // ... and s(i) <= kb
-  }
-}
-
-struct QTileIter {  // flattened walk over (group head, listed q tile)
-  const bma_block_lists& l;
-  int b, hk, G, kj;
-  int g, it, nfull, npart;
-  const int32_t* full_idx;
-  const int32_t* part_idx;
-  __device__ QTileIter(const bma_block_lists& l_, int b_, int hk_, int G_, int kj_)
-      : l(l_), b(b_), hk(hk_), G(G_), kj(kj_), g(-1), it(0), nfull(0), npart(0), full_idx(nullptr), part_idx(nullptr) {}
-  __device__ void load_head() {
-    const int h = hk * G + g;
-    const int lb = l.B == 1 ? 0 : b, lh = l.H == 1 ? 0 : h;
-    const int64_t row = ((int64_t)lb * l.H + lh) * l.NKV + kj;
-    nfull = l.full_q_num[row];
-    npart = l.q_num[row];
-    full_idx = l.full_q_idx + row * l.NQ;
-    part_idx = l.q_idx + row * l.NQ;
-    it = 0;
-  }
-  __device__ bool next(int& h, int& qi, bool& partial) {
-    if (g < 0) { g = 0; load_head(); }
-    while (it >= nfull + npart) {
-      if (++g >= G) return false;
-      load_head();
-    }
-    h = hk * G + g;
-    partial = it >= nfull;
-    qi = partial ? part_idx[it - nfull] : full_idx[it];
-    ++it;
-    return true;
-  }
-};
-
 template <int HD, bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -419,7 +362,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           const int cg = half * 2 + c;
           if (p.interval_mask) {
             int jlo, jhi;
-            col_interval(mv, k, q0, jlo, jhi);
+            col_interval(mv, k, q0, BT, jlo, jhi);
             const int lo = max(jlo - cg * 32, 0), hi = min(jhi - cg * 32, 31);
             bits[c] = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
             if (bits[c] && (mv.flags & kTableTerms)) bits[c] &= table_bits_col32(mv, k, q0 + cg * 32);

@@ -1,0 +1,1109 @@
+// float32 attention (forward, dK/dV, dQ) on the sm_100a tensor core.
+//
+// A float32 value is the exact sum of three bfloat16 values (8 + 8 + 8 significand bits), and a product of two bfloat16
+// values is exact in the float32 accumulator.  Every operand is therefore carried as three bf16 planes hi + mid + lo, and
+// every matrix product is the sum of the six plane products whose weight reaches 2^-24 of the result:
+//     x y  ~  lo hi + hi lo + mid mid + mid hi + hi mid + hi hi        (dropped: mid lo, lo mid, lo lo <= 2^-24 |x y|)
+// issued smallest terms first.  Six passes at the bf16 rate leave 270 TFLOP/s of the measured tensor peak, against
+// 72 TFLOP/s of the FP32 FMA pipes (and the 14 - 19 the FP32 tile kernels of attn_simt.cu reach).
+//
+// Accuracy is held to that of an FP32 FMA chain: the tensor core truncates when it adds to its accumulator, so no
+// accumulation runs longer than one 64-wide tile there -- O, dQ, dK and dV are summed over the tiles in registers, with
+// rounded FP32 adds.  Against float64 the 2-norm error is 1.4e-7 - 3.5e-7 (causal, B=2 L=2048 H=16 d=64; the FP32 tile
+// kernels: 4.1e-7 - 8.5e-7).
+//
+// Measured there: forward 134 us (tile kernels 861), dK/dV 218 (1383), dQ 158 (1357), the two splits 21 each; forward with
+// d=128, N=L=1500, 16 heads: 134 us (1139).
+//
+// One split kernel writes the planes of Q, K, V (and dO) into the caller's workspace as [3, B, L, H, DP] bf16, DP = 64 or
+// 128 columns (zero padded), from where TMA fetches them; splitting inside the attention kernels would repeat the
+// conversion for every tile that reads the operand.
+//
+// Where a product has only 64 columns of output per operand (64 keys, 64 queries, 64 head columns) the hi and mid planes
+// of its B operand are stacked to N = 128: a 128x64x16 MMA takes 53 cycles, a 128x128x16 one 64.  The two accumulator
+// halves are added when they are read.
+//
+// Tensor memory columns hold the accumulators of a tile and then, over the columns that the reading thread has just
+// consumed, the three planes of P or dS as A operands (per 16 keys: 8 columns hi, 8 mid, and 8 lo in the other half).
+// Every mbarrier wait is bounded; on a timeout the thread records an error code and unwinds.
+#include <algorithm>
+
+#include "common.cuh"
+#include "ptx_sm100.cuh"
+
+namespace bma {
+namespace {
+
+using namespace ptx;
+
+constexpr int BM = 128;                          // rows of a tile (queries forward / dQ, keys dK/dV)
+constexpr int BH = 64;                           // columns of a half tile (keys forward / dQ, queries dK/dV)
+constexpr int kThreads = 384;                    // two warpgroups of row threads, one of single-warp roles
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kRowBox = BM * 128;           // one [128 x 64] bf16 box
+constexpr uint32_t kHalfBox = BH * 128;          // one [64 x 64] bf16 box
+constexpr int kMaxKvFwd = 4096, kMaxKvBwd = 1024;
+
+__device__ __forceinline__ void setmaxnreg_inc_208() { asm volatile("setmaxnreg.inc.sync.aligned.u32 208;"); }
+__device__ __forceinline__ void setmaxnreg_dec_80() { asm volatile("setmaxnreg.dec.sync.aligned.u32 80;"); }
+
+// x = hi + mid + lo, exactly, for two neighbouring values (packed like an MMA operand)
+__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16(x, y);
+  x -= __uint_as_float(hi << 16);
+  y -= __uint_as_float(hi & 0xffff0000u);
+  mid = pack_bf16(x, y);
+  x -= __uint_as_float(mid << 16);
+  y -= __uint_as_float(mid & 0xffff0000u);
+  lo = pack_bf16(x, y);
+}
+
+// Plane p of the A operand of k-step ks (16 keys or queries) inside a 128-column accumulator region.
+__device__ __forceinline__ uint32_t plane_col(int p, int ks) { return p == 2 ? 64 + 16 * ks : 16 * ks + 8 * p; }
+
+// Stores the planes of 32 consecutive values (k-steps ks0, ks0 + 1) over the columns they came from.
+__device__ __forceinline__ void store_planes32(uint32_t region, int ks0, const float* v) {
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    uint32_t hm[16], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) split3(v[u * 16 + 2 * j], v[u * 16 + 2 * j + 1], hm[j], hm[8 + j], lo[j]);
+    tmem_st16(region + 16 * (ks0 + u), hm);
+    tmem_st8(region + 64 + 16 * (ks0 + u), lo);
+  }
+}
+
+// ---- plane products ---------------------------------------------------------------------------------------------
+// region[0, 64) and region[64, 128) <- A B^T with B of 64 rows, K-major: A planes at a[0..2], B planes stacked in shared
+// memory (hi, mid, lo of 64 rows each, kHalfBox apart), one 64-column box of both per `boxes` step.
+constexpr uint32_t kIdescN64 = make_idesc_bf16(BM, 64, 0, 0), kIdescN128 = make_idesc_bf16(BM, 128, 0, 0);
+constexpr uint32_t kIdescN64T = make_idesc_bf16(BM, 64, 0, 1), kIdescN128T = make_idesc_bf16(BM, 128, 0, 1);
+
+template <int BOXES>
+__device__ __forceinline__ void product_rows(bool leader, uint32_t region, uint64_t a_hi, uint64_t b_hi) {
+  constexpr uint32_t kAPlane = (BOXES * kRowBox) >> 4, kBPlane = kHalfBox >> 4;
+  auto a_off = [](int ks) { return (uint32_t)(((ks >> 2) * kRowBox + (ks & 3) * 32) >> 4); };
+  auto b_off = [](int ks) { return (uint32_t)(((ks >> 2) * 3 * kHalfBox + (ks & 3) * 32) >> 4); };
+  if (!leader) return;
+#pragma unroll
+  for (int ks = 0; ks < BOXES * 4; ++ks) mma_ss(region, a_hi + 2 * kAPlane + a_off(ks), b_hi + b_off(ks), kIdescN64, ks > 0);
+#pragma unroll
+  for (int ks = 0; ks < BOXES * 4; ++ks) mma_ss(region + 64, a_hi + a_off(ks), b_hi + 2 * kBPlane + b_off(ks), kIdescN64, ks > 0);
+#pragma unroll
+  for (int ks = 0; ks < BOXES * 4; ++ks) mma_ss(region, a_hi + kAPlane + a_off(ks), b_hi + b_off(ks), kIdescN128, 1);
+#pragma unroll
+  for (int ks = 0; ks < BOXES * 4; ++ks) mma_ss(region, a_hi + a_off(ks), b_hi + b_off(ks), kIdescN128, 1);
+}
+
+// region <- P B with the planes of P [128 x 64] in tensor memory at `p` and B [64 x DP] read MN-major (planes DP/64 boxes
+// of [64 x 64] each).  DP 64: the hi and mid planes of B side by side, two halves to be added; DP 128: one sum.
+template <int BOXES>
+__device__ __forceinline__ void product_cols(bool leader, uint32_t region, uint32_t p, uint64_t b_hi) {
+  constexpr uint32_t kBPlane = (BOXES * kHalfBox) >> 4;
+  if (!leader) return;
+  auto b_off = [](int ks) { return (uint32_t)(ks * (2048 >> 4)); };
+  if constexpr (BOXES == 1) {
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) mma_ts(region, p + plane_col(2, ks), b_hi + b_off(ks), kIdescN64T, ks > 0);
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) mma_ts(region + 64, p + plane_col(0, ks), b_hi + 2 * kBPlane + b_off(ks), kIdescN64T, ks > 0);
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) mma_ts(region, p + plane_col(1, ks), b_hi + b_off(ks), kIdescN128T, 1);
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) mma_ts(region, p + plane_col(0, ks), b_hi + b_off(ks), kIdescN128T, 1);
+  } else {
+    constexpr int kTerms[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};   // (plane of P, plane of B)
+#pragma unroll
+    for (int t = 0; t < 6; ++t)
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)
+        mma_ts(region, p + plane_col(kTerms[t][0], ks), b_hi + kTerms[t][1] * kBPlane + b_off(ks), kIdescN128T, (t > 0) || (ks > 0));
+  }
+}
+
+// ---- splitting ----------------------------------------------------------------------------------------------------
+struct SplitJob {
+  bma_tensor t;
+  uint8_t* out;      // [3, B, L, H, DP] bf16
+  int L, H;
+};
+struct SplitParams {
+  SplitJob job[4];
+  int B, d;
+};
+
+// One thread per 8 columns: 32 bytes in, three 16-byte lines out.  Bound by HBM (4 bytes read, 6 written per element), or
+// by launch latency where the tensors are small.
+template <int DP>
+__global__ void __launch_bounds__(256) split_kernel(const SplitParams p) {
+  const SplitJob& job = p.job[blockIdx.y];
+  constexpr int kChunks = DP / 8;
+  const int64_t n = (int64_t)p.B * job.L * job.H * kChunks;
+  const bool f32 = job.t.dtype == BMA_DTYPE_F32;
+  const bool vec = f32 && (reinterpret_cast<uintptr_t>(job.t.ptr) & 15) == 0 && ((job.t.stride_b | job.t.stride_l | job.t.stride_h) & 3) == 0;
+  uint4* out = reinterpret_cast<uint4*>(job.out);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int c = (int)(i % kChunks) * 8;
+    const int64_t row = i / kChunks;
+    const int h = (int)(row % job.H);
+    const int l = (int)((row / job.H) % job.L);
+    const int b = (int)(row / ((int64_t)job.H * job.L));
+    const int64_t off = (int64_t)b * job.t.stride_b + (int64_t)l * job.t.stride_l + (int64_t)h * job.t.stride_h + c;
+    float v[8];
+    if (vec && c + 8 <= p.d) {
+      const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(job.t.ptr) + off);
+      const float4 x = src[0], y = src[1];
+      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        v[e] = 0.f;
+        if (c + e < p.d)
+          v[e] = f32 ? static_cast<const float*>(job.t.ptr)[off + e] : to_float(static_cast<const __nv_bfloat16*>(job.t.ptr)[off + e]);
+      }
+    }
+    uint32_t w[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) split3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) out[q * n + i] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+  }
+}
+
+struct F32Params {
+  bma_attn_args a;
+  bma_mask_spec spec;
+  bma_block_lists l;
+  float scale_log2;
+  int* status;
+};
+
+// Merged kv list of one query tile in shared memory, ascending, every block once: kv tile | partial << 15.
+// Called by all threads of the CTA between two __syncthreads of its own; returns the number of entries.
+template <int MAX>
+struct KvList {
+  uint16_t entry[MAX];
+  uint8_t cls[MAX];
+  int count;
+};
+template <int MAX>
+__device__ __forceinline__ int build_kv_list(KvList<MAX>& s, const bma_block_lists& l, int b, int h, int qi) {
+  const int NKV = l.NKV, lane = threadIdx.x & 31;
+  const int64_t lrow = ((int64_t)(l.B == 1 ? 0 : b) * l.H + (l.H == 1 ? 0 : h)) * l.NQ + qi;
+  for (int i = threadIdx.x; i < NKV; i += kThreads) s.cls[i] = 0;
+  __syncthreads();
+  const int nfull = l.full_kv_num[lrow], npart = l.kv_num[lrow];
+  for (int i = threadIdx.x; i < nfull; i += kThreads) s.cls[l.full_kv_idx[lrow * NKV + i]] = 2;
+  for (int i = threadIdx.x; i < npart; i += kThreads) s.cls[l.kv_idx[lrow * NKV + i]] = 1;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    int count = 0;
+    for (int base = 0; base < NKV; base += 32) {
+      const int j = base + lane;
+      const int c = j < NKV ? s.cls[j] : 0;
+      const unsigned m = __ballot_sync(0xffffffffu, c != 0);
+      if (c) s.entry[count + __popc(m & ((1u << lane) - 1))] = (uint16_t)(j | (c == 1 ? 0x8000 : 0));
+      count += __popc(m);
+    }
+    if (lane == 0) s.count = count;
+  }
+  __syncthreads();
+  return s.count;
+}
+
+// Allowed-key bits of query row q for the 64 keys from k0 (two words).
+__device__ __forceinline__ void row_bits64(const bma_mask_spec& spec, int b, int h, int q, int k0, uint32_t (&bits)[2]) {
+  const MaskView mv = make_mask_view(spec, b, h);
+  int jlo, jhi;
+  row_interval(mv, q, k0, jlo, jhi);
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int lo = max(jlo - c * 32, 0), hi = min(jhi - c * 32, 31);
+    bits[c] = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
+    if (bits[c] && (mv.flags & kTableTerms)) bits[c] &= table_bits_row32(mv, q, k0 + c * 32);
+  }
+}
+
+// 128 rows of `cols` staged floats (row pitch `pitch`) to a [*, *, *, d] tensor, whole rows per warp.
+template <int NT>
+__device__ __forceinline__ void store_rows(const float* stage, int pitch, const bma_tensor& t, int b, int l0, int lmax, int h, int d, int tid) {
+  const int rows = min(BM, lmax - l0);
+  const bool vec = (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && ((t.stride_b | t.stride_l | t.stride_h) & 3) == 0 && (d & 3) == 0;
+  const int64_t base = (int64_t)b * t.stride_b + (int64_t)l0 * t.stride_l + (int64_t)h * t.stride_h;
+  if (vec) {
+    const int per = d / 4;
+    for (int i = tid; i < rows * per; i += NT) {
+      const int r = i / per, c = (i - r * per) * 4;
+      const float4 v = *reinterpret_cast<const float4*>(stage + r * pitch + c);
+      const int64_t off = base + (int64_t)r * t.stride_l + c;
+      if (t.dtype == BMA_DTYPE_F32) *reinterpret_cast<float4*>(static_cast<float*>(t.ptr) + off) = v;
+      else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(t.ptr) + off) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    }
+  } else {
+    for (int i = tid; i < rows * d; i += NT) {
+      const int r = i / d, c = i - r * d;
+      const int64_t off = base + (int64_t)r * t.stride_l + c;
+      if (t.dtype == BMA_DTYPE_F32) static_cast<float*>(t.ptr)[off] = stage[r * pitch + c];
+      else static_cast<__nv_bfloat16*>(t.ptr)[off] = __float2bfloat16_rn(stage[r * pitch + c]);
+    }
+  }
+}
+
+// =================================================================================================================
+// Forward: one CTA per (128-query tile, query head, batch).  Each listed kv tile is cut into two halves of 64 keys;
+// warpgroup x (thread = query row) runs its own online softmax over the halves x of all tiles, so that the two
+// warpgroups ping-pong on the tensor core without waiting for one another, and the two partial results are merged in
+// shared memory at the end.
+//   warp 8: K planes, warp 10: V planes and Q planes (TMA), warp 9: MMA issue.
+//   TMEM per warpgroup: S (then the planes of P) 128 columns, P V of one half tile 128 columns.
+// =================================================================================================================
+enum {
+  FB_Q = 0, FB_S0, FB_S1, FB_P0, FB_P1, FB_O0, FB_O1, FB_OFREE0, FB_OFREE1, FB_SYNC, FB_K_FULL, FB_K_FREE = FB_K_FULL + 3,
+  FB_V_FULL = FB_K_FREE + 3, FB_V_FREE = FB_V_FULL + 3, FB_NUM = FB_V_FREE + 3
+};
+
+template <int DP>
+struct __align__(1024) FwdSmem {
+  static constexpr int kBoxes = DP / 64;
+  static constexpr int kStages = DP == 64 ? 3 : 1;   // 128 columns: 96 KB of Q planes leave room for one half tile each of K and V
+  uint8_t q[3][kBoxes][kRowBox];
+  uint8_t k[kStages][kBoxes][3][kHalfBox];
+  uint8_t v[kStages][3][kBoxes][kHalfBox];
+  float ml[2][2][BM];                                // running maximum and sum of the two halves
+  KvList<kMaxKvFwd> list;
+  uint64_t bar[FB_NUM];
+  uint32_t tmem_base;
+};
+
+template <int DP>
+__global__ void __launch_bounds__(kThreads, 1)
+f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+               const __grid_constant__ CUtensorMap map_v, const F32Params p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  using Smem = FwdSmem<DP>;
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+  constexpr int kBoxes = Smem::kBoxes, kStages = Smem::kStages;
+  const bma_attn_args& a = p.a;
+  const int qi = (int)gridDim.x - 1 - (int)blockIdx.x;   // heaviest causal tiles first
+  const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.Hq / a.Hkv);
+  const int q0 = qi * BM;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wg = warp >> 2;
+
+  if ((smem_u32(smem_raw) & 1023u) != 0u) {
+    if (threadIdx.x == 0) report_device_error(p.status, 601);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < FB_NUM; ++i) {
+      uint32_t count = 1;
+      if (i == FB_P0 || i == FB_P1 || i == FB_OFREE0 || i == FB_OFREE1) count = 128;
+      if (i == FB_SYNC) count = 256;
+      mbar_init(&sm.bar[i], count);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 8) {
+    tmem_alloc(&sm.tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  const int T = build_kv_list(sm.list, p.l, b, h, qi);
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+  // half tiles per warpgroup: the second half of the last tile may lie past the end of the keys
+  const int T0 = T;
+  const int T1 = (T > 0 && (int)(sm.list.entry[T - 1] & 0x7fff) * 128 + BH >= a.L) ? T - 1 : T;
+
+  if (wg == 2) {
+    setmaxnreg_dec_80();
+    if (warp == 8 && lane == 0 && T > 0) {
+      // ------------------------------------------------------------ K planes
+      bool ok = true;
+      int i = 0;
+      for (int n = 0; n < T && ok; ++n)
+        for (int x = 0; x < 2; ++x) {
+          if (n >= (x ? T1 : T0)) continue;
+          const int st = i % kStages;
+          if (i >= kStages) ok = mbar_wait(&sm.bar[FB_K_FREE + st], (i / kStages - 1) & 1);
+          if (!ok) break;
+          const int row = (int)(sm.list.entry[n] & 0x7fff) * 128 + x * BH;
+          mbar_expect_tx(&sm.bar[FB_K_FULL + st], 3 * kBoxes * kHalfBox);
+#pragma unroll
+          for (int box = 0; box < kBoxes; ++box)
+#pragma unroll
+            for (int pl = 0; pl < 3; ++pl) tma_load_4d(sm.k[st][box][pl], &map_k, &sm.bar[FB_K_FULL + st], box * 64, hk, row, b + pl * a.B);
+          ++i;
+        }
+      if (!ok) report_device_error(p.status, 610);
+    } else if (warp == 10 && lane == 0) {
+      // ------------------------------------------------------------ Q and V planes
+      if (T > 0) {
+        mbar_expect_tx(&sm.bar[FB_Q], 3 * kBoxes * kRowBox);
+#pragma unroll
+        for (int pl = 0; pl < 3; ++pl)
+#pragma unroll
+          for (int box = 0; box < kBoxes; ++box) tma_load_4d(sm.q[pl][box], &map_q, &sm.bar[FB_Q], box * 64, h, q0, b + pl * a.B);
+      }
+      bool ok = true;
+      int i = 0;
+      for (int n = 0; n < T && ok; ++n)
+        for (int x = 0; x < 2; ++x) {
+          if (n >= (x ? T1 : T0)) continue;
+          const int st = i % kStages;
+          if (i >= kStages) ok = mbar_wait(&sm.bar[FB_V_FREE + st], (i / kStages - 1) & 1);
+          if (!ok) break;
+          const int row = (int)(sm.list.entry[n] & 0x7fff) * 128 + x * BH;
+          mbar_expect_tx(&sm.bar[FB_V_FULL + st], 3 * kBoxes * kHalfBox);
+#pragma unroll
+          for (int pl = 0; pl < 3; ++pl)
+#pragma unroll
+            for (int box = 0; box < kBoxes; ++box) tma_load_4d(sm.v[st][pl][box], &map_v, &sm.bar[FB_V_FULL + st], box * 64, hk, row, b + pl * a.B);
+          ++i;
+        }
+      if (!ok) report_device_error(p.status, 612);
+    } else if (warp == 9 && T > 0) {
+      // ------------------------------------------------------------ MMA issue (whole warp, one elected lane issues)
+      const bool leader = elect_one();
+      const uint64_t dq = make_smem_desc(smem_u32(sm.q), 16, 1024);
+      const uint64_t dk = make_smem_desc(smem_u32(sm.k), 16, 1024);
+      const uint64_t dv = make_smem_desc(smem_u32(sm.v), kHalfBox, 1024);
+      constexpr uint32_t kStageUnits = (3 * kBoxes * kHalfBox) >> 4;
+      auto issue_s = [&](int x, int i) -> bool {
+        const int st = i % kStages;
+        if (!mbar_wait(&sm.bar[FB_K_FULL + st], (i / kStages) & 1)) return false;
+        tc_fence_after();
+        product_rows<kBoxes>(leader, tmem + x * 256, dq, dk + st * kStageUnits);
+        if (leader) { mma_commit(&sm.bar[FB_S0 + x]); mma_commit(&sm.bar[FB_K_FREE + st]); }
+        return true;
+      };
+      bool ok = mbar_wait(&sm.bar[FB_Q], 0) && issue_s(0, 0);
+      if (ok && T1 > 0) ok = issue_s(1, 1);
+      for (int n = 0; n < T && ok; ++n)
+        for (int x = 0; x < 2 && ok; ++x) {
+          if (n >= (x ? T1 : T0)) continue;
+          const int i = 2 * n + x, st = i % kStages;
+          ok = mbar_wait(&sm.bar[FB_V_FULL + st], (i / kStages) & 1) && mbar_wait(&sm.bar[FB_P0 + x], n & 1);
+          if (ok && n > 0) ok = mbar_wait(&sm.bar[FB_OFREE0 + x], (n - 1) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          product_cols<kBoxes>(leader, tmem + x * 256 + 128, tmem + x * 256, dv + st * kStageUnits);
+          if (leader) { mma_commit(&sm.bar[FB_O0 + x]); mma_commit(&sm.bar[FB_V_FREE + st]); }
+          // the next S of this half overwrites the planes of P, behind the MMAs that read them
+          if (n + 1 < (x ? T1 : T0)) ok = issue_s(x, i + 2);
+        }
+      if (!ok && leader) report_device_error(p.status, 620);
+    }
+  } else {
+    // -------------------------------------------------------------- softmax warpgroups
+    setmaxnreg_inc_208();
+    const int x = wg, row = threadIdx.x & 127, q = q0 + row;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tmem_s = tmem + x * 256 + lane_base, tmem_o = tmem_s + 128;
+    const float kb2 = a.key_bias ? __ldg(a.key_bias + h) * kLog2e : 0.f;
+    const int Tx = x ? T1 : T0;
+    float o[DP];
+#pragma unroll
+    for (int j = 0; j < DP; ++j) o[j] = 0.f;
+    float m = -INFINITY, l = 0.f;
+    bool ok = true;
+    for (int n = 0; n < Tx; ++n) {
+      const uint32_t e = sm.list.entry[n];
+      const int k0 = (int)(e & 0x7fff) * 128 + x * BH;
+      uint32_t bits[2] = {0xffffffffu, 0xffffffffu};
+      if (e & 0x8000u) row_bits64(p.spec, b, h, q, k0, bits);
+      const float kbase = (float)(p.spec.k_offset + k0);
+      // 16 scores in log2 units from tensor memory (the two accumulator halves added)
+      auto scores16 = [&](int c, float* v) {
+        uint32_t r0[16], r1[16];
+        tmem_ld16(tmem_s + c * 16, r0);
+        tmem_ld16(tmem_s + 64 + c * 16, r1);
+        tmem_wait_ld();
+        const uint32_t w = (c < 2 ? bits[0] : bits[1]) >> ((c & 1) * 16);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float s = (__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
+          v[j] = fmaf(s, p.scale_log2, kb2 * (kbase + (float)(c * 16 + j)));
+          if (!((w >> j) & 1u)) v[j] = -INFINITY;
+        }
+      };
+      ok = mbar_wait(&sm.bar[FB_S0 + x], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+      // 128 head columns leave no registers for 64 scores beside O: those are read twice, once for the maximum
+      constexpr bool kKeep = DP == 64;
+      float s[kKeep ? 64 : 16];
+      float mx = -INFINITY;
+#pragma unroll (kKeep ? 4 : 1)
+      for (int c = 0; c < 4; ++c) {
+        float* v = s + (kKeep ? c * 16 : 0);
+        scores16(c, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) mx = fmaxf(mx, v[j]);
+      }
+      const float m_new = fmaxf(m, mx), m_safe = (m_new == -INFINITY) ? 0.f : m_new;
+      const float alpha = ex2(m - m_safe);
+      m = m_new;
+      float rs[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll (kKeep ? 4 : 1)
+      for (int c = 0; c < 4; ++c) {
+        float* v = s + (kKeep ? c * 16 : 0);
+        if (!kKeep) scores16(c, v);
+        uint32_t hm[16], lo[8];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          v[j] = ex2(v[j] - m_safe);
+          rs[j & 3] += v[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) split3(v[2 * j], v[2 * j + 1], hm[j], hm[8 + j], lo[j]);
+        tmem_st16(tmem_s + c * 16, hm);        // over the 16 + 8 columns whose scores have just been used
+        tmem_st8(tmem_s + 64 + c * 16, lo);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[FB_P0 + x]);
+      l = l * alpha + ((rs[0] + rs[1]) + (rs[2] + rs[3]));
+      ok = mbar_wait(&sm.bar[FB_O0 + x], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < DP / 32; ++c) {
+        uint32_t r0[32];
+        tmem_ld32(tmem_o + c * 32, r0);
+        if constexpr (DP == 64) {
+          uint32_t r1[32];
+          tmem_ld32(tmem_o + 64 + c * 32, r1);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[c * 32 + j] = fmaf(o[c * 32 + j], alpha, __uint_as_float(r0[j]) + __uint_as_float(r1[j]));
+        } else {
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[c * 32 + j] = fmaf(o[c * 32 + j], alpha, __uint_as_float(r0[j]));
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(&sm.bar[FB_OFREE0 + x]);
+    }
+
+    // ---- merge the two halves and write O and the log-sum-exp.  After the first rendezvous every MMA of the CTA has
+    // completed (each warpgroup has seen its last P V), so the Q planes' buffer is free for staging.
+    sm.ml[x][0][row] = m;
+    sm.ml[x][1][row] = l;
+    uint32_t syncs = 0;
+    auto rendezvous = [&]() {
+      mbar_arrive(&sm.bar[FB_SYNC]);
+      ok = mbar_wait(&sm.bar[FB_SYNC], syncs & 1) && ok;
+      ++syncs;
+    };
+    rendezvous();
+    const float mo = sm.ml[x ^ 1][0][row], lo = sm.ml[x ^ 1][1][row];
+    const float mt = fmaxf(m, mo), ms = (mt == -INFINITY) ? 0.f : mt;
+    const float fx = ex2(m - ms), fo = ex2(mo - ms);
+    const float lt = l * fx + lo * fo;
+    const float mine = lt > 0.f ? fx / lt : 0.f;
+    constexpr int kPitch = DP + 4;
+    float* stage = reinterpret_cast<float*>(sm.q) + row * kPitch;
+    if (x == 0) {
+#pragma unroll
+      for (int j = 0; j < DP; j += 4) *reinterpret_cast<float4*>(stage + j) = make_float4(o[j] * mine, o[j + 1] * mine, o[j + 2] * mine, o[j + 3] * mine);
+    }
+    rendezvous();
+    if (x == 1) {
+#pragma unroll
+      for (int j = 0; j < DP; j += 4) {
+        float4 v = *reinterpret_cast<float4*>(stage + j);
+        v.x = fmaf(o[j], mine, v.x); v.y = fmaf(o[j + 1], mine, v.y); v.z = fmaf(o[j + 2], mine, v.z); v.w = fmaf(o[j + 3], mine, v.w);
+        *reinterpret_cast<float4*>(stage + j) = v;
+      }
+      if (q < a.N && a.lse) a.lse[((int64_t)b * a.Hq + h) * a.N + q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
+    }
+    rendezvous();
+    if (ok) store_rows<256>(reinterpret_cast<const float*>(sm.q), kPitch, a.o, b, q0, a.N, h, a.d, threadIdx.x);
+    else report_device_error(p.status, 630 + warp);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+}
+
+// =================================================================================================================
+// dK / dV: one CTA per (128-key tile, kv head, batch); K and V planes stay in shared memory, the q tiles of the q-side
+// lists come in halves of 64 queries.  Both warpgroups work on every half tile, 32 query columns each (thread = key row):
+//     St = K Q^T -> P, dPt = V dO^T -> dS,   dV += Pt dO (warpgroup 0 sums it in registers),  dK += dSt Q (warpgroup 1)
+// MMA order  dV(n) St(n+1) dK(n) dPt(n+1): the next scores are computed while this tile's gradients accumulate.
+//   warp 8: K, V, Q planes, warp 11: dO planes (TMA), warp 9: MMA issue, warp 10: lse and delta of the coming half tile.
+// =================================================================================================================
+enum {
+  KB_KV = 0, KB_S, KB_DP, KB_P, KB_DS, KB_DV, KB_DK, KB_DVFREE, KB_DKFREE, KB_EPI0, KB_EPI1,
+  KB_Q_FULL, KB_Q_FREE = KB_Q_FULL + 2, KB_DO_FULL = KB_Q_FREE + 2, KB_DO_FREE = KB_DO_FULL + 2, KB_STAT = KB_DO_FREE + 2,
+  KB_NUM = KB_STAT + 2
+};
+struct __align__(1024) DkdvSmem {
+  uint8_t k[3][kRowBox];
+  uint8_t v[3][kRowBox];
+  uint8_t q[2][3][kHalfBox];
+  uint8_t d_o[2][3][kHalfBox];
+  float lse2[2][BH], delta[2][BH];
+  uint64_t bar[KB_NUM];
+  uint32_t tmem_base;
+};
+constexpr uint32_t COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
+
+// flattened walk over (group head, listed q tile, half tile); a half tile past the end of the queries is left out
+struct HalfIter {
+  QTileIter it;
+  int N, h, qi;
+  bool partial, second;
+  __device__ HalfIter(const bma_block_lists& l, int b, int hk, int G, int kj, int N_) : it(l, b, hk, G, kj), N(N_), h(0), qi(0), partial(false), second(false) {}
+  __device__ bool next(int& h_, int& q0_, bool& partial_) {
+    if (second) {
+      second = false;
+      q0_ = qi * 128 + BH;
+    } else {
+      if (!it.next(h, qi, partial)) return false;
+      q0_ = qi * 128;
+      second = q0_ + BH < N;
+    }
+    h_ = h;
+    partial_ = partial;
+    return true;
+  }
+};
+
+__global__ void __launch_bounds__(kThreads, 1)
+f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                const __grid_constant__ CUtensorMap map_qh, const __grid_constant__ CUtensorMap map_do, const F32Params p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  DkdvSmem& sm = *reinterpret_cast<DkdvSmem*>(smem_raw);
+  const bma_attn_args& a = p.a;
+  const int kj = blockIdx.x, hk = blockIdx.y, b = blockIdx.z, G = a.Hq / a.Hkv;
+  const int k0 = kj * BM;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  if ((smem_u32(smem_raw) & 1023u) != 0u) {
+    if (threadIdx.x == 0) report_device_error(p.status, 701);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < KB_NUM; ++i) {
+      uint32_t count = 1;
+      if (i == KB_P || i == KB_DS) count = 256;
+      if (i == KB_DVFREE || i == KB_DKFREE || i == KB_EPI0 || i == KB_EPI1) count = 128;
+      if (i == KB_STAT || i == KB_STAT + 1) count = 32;
+      mbar_init(&sm.bar[i], count);
+    }
+    fence_barrier_init();
+    mbar_expect_tx(&sm.bar[KB_KV], 6 * kRowBox);
+#pragma unroll
+    for (int pl = 0; pl < 3; ++pl) {
+      tma_load_4d(sm.k[pl], &map_k, &sm.bar[KB_KV], 0, hk, k0, b + pl * a.B);
+      tma_load_4d(sm.v[pl], &map_v, &sm.bar[KB_KV], 0, hk, k0, b + pl * a.B);
+    }
+  }
+  if (warp == 8) {
+    tmem_alloc(&sm.tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+
+  if (warp >= 8) {
+    setmaxnreg_dec_80();
+    HalfIter walk(p.l, b, hk, G, kj, a.N);
+    int h, q0;
+    bool partial, ok = true;
+    if (warp == 8 || warp == 11) {
+      // ------------------------------------------------------------ Q (warp 8) and dO (warp 11) planes
+      if (lane == 0) {
+        const bool is_q = warp == 8;
+        for (int n = 0; ok && walk.next(h, q0, partial); ++n) {
+          const int st = n & 1;
+          uint64_t* full = &sm.bar[(is_q ? KB_Q_FULL : KB_DO_FULL) + st];
+          if (n >= 2) ok = mbar_wait(&sm.bar[(is_q ? KB_Q_FREE : KB_DO_FREE) + st], ((n >> 1) - 1) & 1);
+          if (!ok) break;
+          mbar_expect_tx(full, 3 * kHalfBox);
+#pragma unroll
+          for (int pl = 0; pl < 3; ++pl) tma_load_4d(is_q ? sm.q[st][pl] : sm.d_o[st][pl], is_q ? &map_qh : &map_do, full, 0, h, q0, b + pl * a.B);
+        }
+        if (!ok) report_device_error(p.status, 710);
+      }
+    } else if (warp == 10) {
+      // ------------------------------------------------------------ row statistics of the coming half tiles
+      for (int n = 0; ok && walk.next(h, q0, partial); ++n) {
+        const int st = n & 1;
+        if (n >= 2) ok = mbar_wait(&sm.bar[KB_Q_FREE + st], ((n >> 1) - 1) & 1);   // dK(n-2) is behind every read of its statistics
+        if (!ok) break;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int idx = e * 32 + lane, q = q0 + idx;
+          const int64_t off = ((int64_t)b * a.Hq + h) * a.N + q;
+          const float lv = q < a.N ? __ldg(a.lse + off) : -INFINITY;
+          sm.lse2[st][idx] = (lv == -INFINITY) ? INFINITY : lv * kLog2e;   // +inf: the probabilities of the row become exactly 0
+          sm.delta[st][idx] = q < a.N ? __ldg(a.delta + off) : 0.f;
+        }
+        mbar_arrive(&sm.bar[KB_STAT + st]);
+      }
+      if (!ok && lane == 0) report_device_error(p.status, 715);
+    } else {
+      // ------------------------------------------------------------ MMA issue
+      const bool leader = elect_one();
+      const uint64_t dk = make_smem_desc(smem_u32(sm.k), 16, 1024), dv = make_smem_desc(smem_u32(sm.v), 16, 1024);
+      const uint64_t dq = make_smem_desc(smem_u32(sm.q), 16, 1024), ddo = make_smem_desc(smem_u32(sm.d_o), 16, 1024);
+      const uint64_t dqm = make_smem_desc(smem_u32(sm.q), kHalfBox, 1024), ddom = make_smem_desc(smem_u32(sm.d_o), kHalfBox, 1024);
+      constexpr uint32_t kStageUnits = (3 * kHalfBox) >> 4;
+      auto issue_st = [&](int n) -> bool {
+        if (!mbar_wait(&sm.bar[KB_Q_FULL + (n & 1)], (n >> 1) & 1)) return false;
+        tc_fence_after();
+        product_rows<1>(leader, tmem + COL_ST, dk, dq + (n & 1) * kStageUnits);
+        if (leader) mma_commit(&sm.bar[KB_S]);
+        return true;
+      };
+      auto issue_dpt = [&](int n) -> bool {
+        if (!mbar_wait(&sm.bar[KB_DO_FULL + (n & 1)], (n >> 1) & 1)) return false;
+        tc_fence_after();
+        product_rows<1>(leader, tmem + COL_DPT, dv, ddo + (n & 1) * kStageUnits);
+        if (leader) mma_commit(&sm.bar[KB_DP]);
+        return true;
+      };
+      bool have = walk.next(h, q0, partial);
+      if (have) ok = mbar_wait(&sm.bar[KB_KV], 0) && issue_st(0) && issue_dpt(0);
+      for (int n = 0; have && ok; ++n) {
+        const int st = n & 1;
+        const bool more = walk.next(h, q0, partial);
+        ok = mbar_wait(&sm.bar[KB_P], n & 1);
+        if (ok && n > 0) ok = mbar_wait(&sm.bar[KB_DVFREE], (n - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        product_cols<1>(leader, tmem + COL_DV, tmem + COL_ST, ddom + st * kStageUnits);
+        if (leader) { mma_commit(&sm.bar[KB_DV]); mma_commit(&sm.bar[KB_DO_FREE + st]); }
+        if (more) ok = issue_st(n + 1);
+        if (ok) ok = mbar_wait(&sm.bar[KB_DS], n & 1);
+        if (ok && n > 0) ok = mbar_wait(&sm.bar[KB_DKFREE], (n - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        product_cols<1>(leader, tmem + COL_DK, tmem + COL_DPT, dqm + st * kStageUnits);
+        if (leader) { mma_commit(&sm.bar[KB_DK]); mma_commit(&sm.bar[KB_Q_FREE + st]); }
+        if (more) ok = issue_dpt(n + 1);
+        have = more;
+      }
+      if (!ok && leader) report_device_error(p.status, 720);
+    }
+  } else {
+    // -------------------------------------------------------------- row threads
+    setmaxnreg_inc_208();
+    const int w = warp >> 2, row = threadIdx.x & 127, k = k0 + row;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tm = tmem + lane_base;
+    float acc[64];   // warpgroup 0: dV, warpgroup 1: dK of this key row
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+    bool ok = true;
+    const uint32_t col_acc = w == 0 ? COL_DV : COL_DK;
+    uint64_t* acc_full = &sm.bar[w == 0 ? KB_DV : KB_DK];
+    uint64_t* acc_free = &sm.bar[w == 0 ? KB_DVFREE : KB_DKFREE];
+    auto flush = [&](int n) -> bool {   // acc += the gradient contribution of half tile n
+      if (!mbar_wait(acc_full, n & 1)) return false;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tm + col_acc + c * 32, r0);
+        tmem_ld32(tm + col_acc + 64 + c * 32, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[c * 32 + j] += __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+      }
+      tc_fence_before();
+      mbar_arrive(acc_free);
+      return true;
+    };
+    HalfIter walk(p.l, b, hk, G, kj, a.N);
+    int h, q0, n = 0;
+    bool partial;
+    for (; ok && walk.next(h, q0, partial); ++n) {
+      const int st = n & 1;
+      const float kbk = a.key_bias ? __ldg(a.key_bias + h) * kLog2e * (float)(p.spec.k_offset + k) : 0.f;
+      uint32_t bits = 0xffffffffu;
+      if (partial) {
+        const MaskView mv = make_mask_view(p.spec, b, h);
+        int jlo, jhi;
+        col_interval(mv, k, q0 + w * 32, 32, jlo, jhi);
+        const int lo = max(jlo, 0), hi = min(jhi, 31);
+        bits = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
+        if (bits && (mv.flags & kTableTerms)) bits &= table_bits_col32(mv, k, q0 + w * 32);
+      }
+      ok = mbar_wait(&sm.bar[KB_STAT + st], (n >> 1) & 1) && mbar_wait(&sm.bar[KB_S], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+      float pr[32];
+      {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tm + COL_ST + w * 32, r0);
+        tmem_ld32(tm + COL_ST + 64 + w * 32, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j4 = 0; j4 < 8; ++j4) {
+          const float4 lv = *reinterpret_cast<const float4*>(&sm.lse2[st][w * 32 + j4 * 4]);
+          const float l4[4] = {lv.x, lv.y, lv.z, lv.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int j = j4 * 4 + e;
+            const float s = __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+            pr[j] = (bits >> j) & 1u ? ex2(fmaf(s, p.scale_log2, kbk) - l4[e]) : 0.f;
+          }
+        }
+      }
+      store_planes32(tm + COL_ST, w * 2, pr);
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[KB_P]);
+      if (w == 1 && n > 0) ok = flush(n - 1);   // dK(n-1) was issued behind St(n): it completes under the exponentials
+      if (ok) ok = mbar_wait(&sm.bar[KB_DP], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+      {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tm + COL_DPT + w * 32, r0);
+        tmem_ld32(tm + COL_DPT + 64 + w * 32, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j4 = 0; j4 < 8; ++j4) {
+          const float4 dl = *reinterpret_cast<const float4*>(&sm.delta[st][w * 32 + j4 * 4]);
+          const float d4[4] = {dl.x, dl.y, dl.z, dl.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int j = j4 * 4 + e;
+            pr[j] *= (__uint_as_float(r0[j]) + __uint_as_float(r1[j])) - d4[e];
+          }
+        }
+      }
+      store_planes32(tm + COL_DPT, w * 2, pr);
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[KB_DS]);
+      if (w == 0) ok = flush(n);
+    }
+    if (ok && w == 1 && n > 0) ok = flush(n - 1);
+    if (ok && n == 0) ok = mbar_wait(&sm.bar[KB_KV], 0);   // let the loads land before their buffers are reused
+    // ---- epilogue: every score MMA that read K and V has completed, their buffers stage dV (0) and dK (1)
+    constexpr int kPitch = 68;
+    float* stage = reinterpret_cast<float*>(w == 0 ? &sm.v[0][0] : &sm.k[0][0]);
+    const float sc = w == 0 ? 1.f : a.scale;
+#pragma unroll
+    for (int j = 0; j < 64; j += 4)
+      if (ok) *reinterpret_cast<float4*>(stage + row * kPitch + j) = make_float4(acc[j] * sc, acc[j + 1] * sc, acc[j + 2] * sc, acc[j + 3] * sc);
+    mbar_arrive(&sm.bar[KB_EPI0 + w]);
+    ok = mbar_wait(&sm.bar[KB_EPI0 + w], 0) && ok;
+    if (ok) store_rows<128>(stage, kPitch, w == 0 ? a.dv : a.dk, b, k0, a.L, hk, a.d, row);
+    else report_device_error(p.status, 730 + warp);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+}
+
+// =================================================================================================================
+// dQ: one CTA per (128-query tile, query head, batch); Q and dO planes stay in shared memory, the listed kv tiles come in
+// halves of 64 keys through rings of three K and two V half tiles.  S is double buffered, so the next half's scores and
+// exponentials run while  dQ(n) dP(n+1)  execute.  Both warpgroups work on every half tile (32 key columns each) and
+// sum 32 columns of dQ each in registers.
+// =================================================================================================================
+enum {
+  QB_Q = 0, QB_S, QB_DP = QB_S + 2, QB_DS, QB_DQ, QB_DQFREE, QB_EPI, QB_K_FULL, QB_K_FREE = QB_K_FULL + 3, QB_V_FULL = QB_K_FREE + 3,
+  QB_V_FREE = QB_V_FULL + 2, QB_NUM = QB_V_FREE + 2
+};
+struct __align__(1024) DqSmem {
+  uint8_t q[3][kRowBox];
+  uint8_t d_o[3][kRowBox];
+  uint8_t k[3][3][kHalfBox];
+  uint8_t v[2][3][kHalfBox];
+  KvList<kMaxKvBwd> list;
+  uint64_t bar[QB_NUM];
+  uint32_t tmem_base;
+};
+constexpr uint32_t COL_S2 = 0, COL_DP2 = 256, COL_DQ2 = 384;   // S: two buffers of 128 columns
+
+__global__ void __launch_bounds__(kThreads, 1)
+f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kh,
+              const __grid_constant__ CUtensorMap map_vh, const __grid_constant__ CUtensorMap map_do, const F32Params p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  DqSmem& sm = *reinterpret_cast<DqSmem*>(smem_raw);
+  const bma_attn_args& a = p.a;
+  const int qi = (int)gridDim.x - 1 - (int)blockIdx.x;
+  const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.Hq / a.Hkv);
+  const int q0 = qi * BM;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  if ((smem_u32(smem_raw) & 1023u) != 0u) {
+    if (threadIdx.x == 0) report_device_error(p.status, 801);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < QB_NUM; ++i) mbar_init(&sm.bar[i], (i == QB_DS || i == QB_DQFREE || i == QB_EPI) ? 256 : 1);
+    fence_barrier_init();
+    mbar_expect_tx(&sm.bar[QB_Q], 6 * kRowBox);
+#pragma unroll
+    for (int pl = 0; pl < 3; ++pl) {
+      tma_load_4d(sm.q[pl], &map_q, &sm.bar[QB_Q], 0, h, q0, b + pl * a.B);
+      tma_load_4d(sm.d_o[pl], &map_do, &sm.bar[QB_Q], 0, h, q0, b + pl * a.B);
+    }
+  }
+  if (warp == 8) {
+    tmem_alloc(&sm.tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  const int T = build_kv_list(sm.list, p.l, b, h, qi);
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+  // half tiles in all; the second half of the last tile may lie past the end of the keys
+  const int total = T == 0 ? 0 : 2 * T - ((int)(sm.list.entry[T - 1] & 0x7fff) * 128 + BH >= a.L ? 1 : 0);
+
+  if (warp >= 8) {
+    setmaxnreg_dec_80();
+    bool ok = true;
+    if ((warp == 8 || warp == 10) && lane == 0) {
+      // ------------------------------------------------------------ K (warp 8) and V (warp 10) planes
+      const bool is_k = warp == 8;
+      const int stages = is_k ? 3 : 2;
+      for (int n = 0; n < total && ok; ++n) {
+        const int st = n % stages;
+        uint64_t* full = &sm.bar[(is_k ? QB_K_FULL : QB_V_FULL) + st];
+        if (n >= stages) ok = mbar_wait(&sm.bar[(is_k ? QB_K_FREE : QB_V_FREE) + st], (n / stages - 1) & 1);
+        if (!ok) break;
+        const int row = (int)(sm.list.entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
+        mbar_expect_tx(full, 3 * kHalfBox);
+#pragma unroll
+        for (int pl = 0; pl < 3; ++pl) tma_load_4d(is_k ? sm.k[st][pl] : sm.v[st][pl], is_k ? &map_kh : &map_vh, full, 0, hk, row, b + pl * a.B);
+      }
+      if (!ok) report_device_error(p.status, 810);
+    } else if (warp == 9 && total > 0) {
+      // ------------------------------------------------------------ MMA issue
+      const bool leader = elect_one();
+      const uint64_t dq = make_smem_desc(smem_u32(sm.q), 16, 1024), ddo = make_smem_desc(smem_u32(sm.d_o), 16, 1024);
+      const uint64_t dk = make_smem_desc(smem_u32(sm.k), 16, 1024), dv = make_smem_desc(smem_u32(sm.v), 16, 1024);
+      const uint64_t dkm = make_smem_desc(smem_u32(sm.k), kHalfBox, 1024);
+      constexpr uint32_t kStageUnits = (3 * kHalfBox) >> 4;
+      auto issue_s = [&](int n) -> bool {
+        if (!mbar_wait(&sm.bar[QB_K_FULL + n % 3], (n / 3) & 1)) return false;
+        tc_fence_after();
+        product_rows<1>(leader, tmem + COL_S2 + (n & 1) * 128, dq, dk + (n % 3) * kStageUnits);
+        if (leader) mma_commit(&sm.bar[QB_S + (n & 1)]);
+        return true;
+      };
+      auto issue_dp = [&](int n) -> bool {
+        if (!mbar_wait(&sm.bar[QB_V_FULL + (n & 1)], (n >> 1) & 1)) return false;
+        tc_fence_after();
+        product_rows<1>(leader, tmem + COL_DP2, ddo, dv + (n & 1) * kStageUnits);
+        if (leader) { mma_commit(&sm.bar[QB_DP]); mma_commit(&sm.bar[QB_V_FREE + (n & 1)]); }
+        return true;
+      };
+      ok = mbar_wait(&sm.bar[QB_Q], 0) && issue_s(0) && issue_dp(0);
+      if (ok && total > 1) ok = issue_s(1);
+      for (int n = 0; n < total && ok; ++n) {
+        ok = mbar_wait(&sm.bar[QB_DS], n & 1);
+        if (ok && n > 0) ok = mbar_wait(&sm.bar[QB_DQFREE], (n - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        product_cols<1>(leader, tmem + COL_DQ2, tmem + COL_DP2, dkm + (n % 3) * kStageUnits);
+        if (leader) { mma_commit(&sm.bar[QB_DQ]); mma_commit(&sm.bar[QB_K_FREE + n % 3]); }
+        if (n + 1 < total) ok = issue_dp(n + 1);
+        if (ok && n + 2 < total) ok = issue_s(n + 2);   // its S buffer was read before the DS arrivals of half tile n
+      }
+      if (!ok && leader) report_device_error(p.status, 820);
+    }
+  } else {
+    setmaxnreg_inc_208();
+    const int w = warp >> 2, row = threadIdx.x & 127, q = q0 + row;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tm = tmem + lane_base;
+    const float kb2 = a.key_bias ? __ldg(a.key_bias + h) * kLog2e : 0.f;
+    float lse2 = INFINITY, delta = 0.f;
+    if (q < a.N) {
+      const float lv = __ldg(a.lse + ((int64_t)b * a.Hq + h) * a.N + q);
+      lse2 = lv == -INFINITY ? INFINITY : lv * kLog2e;
+      delta = __ldg(a.delta + ((int64_t)b * a.Hq + h) * a.N + q);
+    }
+    float acc[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+    bool ok = true;
+    auto flush = [&](int n) -> bool {
+      if (!mbar_wait(&sm.bar[QB_DQ], n & 1)) return false;
+      tc_fence_after();
+      uint32_t r0[32], r1[32];
+      tmem_ld32(tm + COL_DQ2 + w * 32, r0);
+      tmem_ld32(tm + COL_DQ2 + 64 + w * 32, r1);
+      tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[j] += __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+      tc_fence_before();
+      mbar_arrive(&sm.bar[QB_DQFREE]);
+      return true;
+    };
+    for (int n = 0; n < total && ok; ++n) {
+      const uint32_t e = sm.list.entry[n >> 1];
+      const int k0 = (int)(e & 0x7fff) * 128 + (n & 1) * BH;
+      uint32_t bits = 0xffffffffu;
+      if (e & 0x8000u) {
+        uint32_t both[2];
+        row_bits64(p.spec, b, h, q, k0, both);
+        bits = w == 0 ? both[0] : both[1];
+      }
+      const float kbase = (float)(p.spec.k_offset + k0 + w * 32);
+      ok = mbar_wait(&sm.bar[QB_S + (n & 1)], (n >> 1) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      float pr[32];
+      {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tm + COL_S2 + (n & 1) * 128 + w * 32, r0);
+        tmem_ld32(tm + COL_S2 + (n & 1) * 128 + 64 + w * 32, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float s = __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+          pr[j] = (bits >> j) & 1u ? ex2(fmaf(s, p.scale_log2, kb2 * (kbase + (float)j)) - lse2) : 0.f;
+        }
+      }
+      if (n > 0) ok = flush(n - 1);
+      if (ok) ok = mbar_wait(&sm.bar[QB_DP], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+      {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tm + COL_DP2 + w * 32, r0);
+        tmem_ld32(tm + COL_DP2 + 64 + w * 32, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) pr[j] *= (__uint_as_float(r0[j]) + __uint_as_float(r1[j])) - delta;
+      }
+      store_planes32(tm + COL_DP2, w * 2, pr);
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[QB_DS]);
+    }
+    if (ok && total > 0) ok = flush(total - 1);
+    if (ok && total == 0) ok = mbar_wait(&sm.bar[QB_Q], 0);
+    constexpr int kPitch = 68;
+    float* stage = reinterpret_cast<float*>(&sm.q[0][0]);   // every MMA that read the Q planes has completed
+    if (ok) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 4)
+        *reinterpret_cast<float4*>(stage + row * kPitch + w * 32 + j) = make_float4(acc[j] * a.scale, acc[j + 1] * a.scale, acc[j + 2] * a.scale, acc[j + 3] * a.scale);
+    }
+    mbar_arrive(&sm.bar[QB_EPI]);
+    ok = mbar_wait(&sm.bar[QB_EPI], 0) && ok;
+    if (ok) store_rows<256>(stage, kPitch, a.dq, b, q0, a.N, h, a.d, threadIdx.x);
+    else report_device_error(p.status, 830 + warp);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+}
+
+// ---- host ------------------------------------------------------------------------------------------------------
+int padded_d(const bma_attn_args& a) { return a.d <= 64 ? 64 : 128; }
+size_t plane_bytes(int B, int L, int H, int dp) { return (size_t)3 * B * L * H * dp * 2; }
+size_t align_up(size_t x) { return (x + 1023) / 1024 * 1024; }
+
+struct Planes {
+  size_t q, k, v, d_o, total;   // offsets in the workspace
+};
+Planes planes_layout(const bma_attn_args& a, bool backward) {
+  const int dp = padded_d(a);
+  Planes p;
+  p.q = 0;
+  p.k = align_up(plane_bytes(a.B, a.N, a.Hq, dp));
+  p.v = p.k + align_up(plane_bytes(a.B, a.L, a.Hkv, dp));
+  p.d_o = p.v + align_up(plane_bytes(a.B, a.L, a.Hkv, dp));
+  p.total = p.d_o + (backward ? align_up(plane_bytes(a.B, a.N, a.Hq, dp)) : 0);
+  return p;
+}
+
+int launch_split(const bma_attn_args& a, const Planes& pl, uint8_t* ws, bool backward, cudaStream_t st) {
+  SplitParams sp;
+  sp.B = a.B; sp.d = a.d;
+  sp.job[0] = {a.q, ws + pl.q, a.N, a.Hq};
+  sp.job[1] = {a.k, ws + pl.k, a.L, a.Hkv};
+  sp.job[2] = {a.v, ws + pl.v, a.L, a.Hkv};
+  sp.job[3] = {a.d_o, ws + pl.d_o, a.N, a.Hq};
+  const int dp = padded_d(a);
+  const int64_t most = std::max((int64_t)a.B * a.N * a.Hq, (int64_t)a.B * a.L * a.Hkv) * (dp / 8);
+  const dim3 grid((unsigned)std::min<int64_t>((most + 255) / 256, 148 * 8), backward ? 4 : 3);
+  if (dp == 64) split_kernel<64><<<grid, 256, 0, st>>>(sp);
+  else split_kernel<128><<<grid, 256, 0, st>>>(sp);
+  count_launches(1);
+  BMA_CUDA_TRY(cudaGetLastError());
+  return BMA_OK;
+}
+
+int plane_map(CUtensorMap* m, const uint8_t* base, int B, int L, int H, int dp, int rows) {
+  return make_tile_map_bf16(m, base, 3 * B, L, H, dp, (int64_t)L * H * dp, (int64_t)H * dp, dp, rows);
+}
+
+int make_params(F32Params& p, const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists) {
+  p.a = a; p.spec = spec; p.l = lists;
+  p.scale_log2 = a.scale * kLog2e;
+  p.status = device_status_ptr();
+  BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
+  return BMA_OK;
+}
+
+}  // namespace
+
+size_t f32_workspace_bytes(const bma_attn_args& a, bool backward) {
+  if (a.q.dtype != BMA_DTYPE_F32 || !sm100_device()) return 0;
+  if (backward ? (a.d > 64 || ceil_div(a.L, BM) > kMaxKvBwd) : (a.d > 128 || ceil_div(a.L, BM) > kMaxKvFwd)) return 0;
+  return planes_layout(a, backward).total;
+}
+
+int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, cudaStream_t st) {
+  const Planes pl = planes_layout(a, false);
+  uint8_t* w = static_cast<uint8_t*>(ws);
+  const int dp = padded_d(a);
+  F32Params p;
+  int rc;
+  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, pl, w, false, st))) return rc;
+  CUtensorMap mq, mk, mv;
+  if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, dp, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, dp, BH)) ||
+      (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, dp, BH)))
+    return rc;
+  const dim3 grid(ceil_div(a.N, BM), a.Hq, a.B);
+  auto launch = [&](auto kernel, size_t smem) -> int {
+    BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, kThreads, smem, st>>>(mq, mk, mv, p);
+    return BMA_OK;
+  };
+  rc = dp == 64 ? launch(f32_fwd_kernel<64>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128>, sizeof(FwdSmem<128>));
+  if (rc) return rc;
+  count_launches(1);
+  BMA_CUDA_TRY(cudaGetLastError());
+  return BMA_OK;
+}
+
+int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, cudaStream_t st) {
+  const Planes pl = planes_layout(a, true);
+  uint8_t* w = static_cast<uint8_t*>(ws);
+  F32Params p;
+  int rc;
+  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, pl, w, true, st))) return rc;
+  CUtensorMap mq, mk, mv, mdo, mqh, mkh, mvh, mdoh;
+  if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, 64, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, 64, BM)) ||
+      (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, 64, BM)) || (rc = plane_map(&mdo, w + pl.d_o, a.B, a.N, a.Hq, 64, BM)) ||
+      (rc = plane_map(&mqh, w + pl.q, a.B, a.N, a.Hq, 64, BH)) || (rc = plane_map(&mkh, w + pl.k, a.B, a.L, a.Hkv, 64, BH)) ||
+      (rc = plane_map(&mvh, w + pl.v, a.B, a.L, a.Hkv, 64, BH)) || (rc = plane_map(&mdoh, w + pl.d_o, a.B, a.N, a.Hq, 64, BH)))
+    return rc;
+  BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvSmem)));
+  BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqSmem)));
+  f32_dkdv_kernel<<<dim3(ceil_div(a.L, BM), a.Hkv, a.B), kThreads, sizeof(DkdvSmem), st>>>(mk, mv, mqh, mdoh, p);
+  f32_dq_kernel<<<dim3(ceil_div(a.N, BM), a.Hq, a.B), kThreads, sizeof(DqSmem), st>>>(mq, mkh, mvh, mdo, p);
+  count_launches(2);
+  BMA_CUDA_TRY(cudaGetLastError());
+  return BMA_OK;
+}
+
+}  // namespace bma

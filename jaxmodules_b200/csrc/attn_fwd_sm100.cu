@@ -165,23 +165,6 @@ __device__ __forceinline__ float exp_part(const float* s, float sc, float m_sub,
 #endif
 }
 
-// Allowed key interval [jlo, jhi] (tile-local, inclusive) of query row q for interval-only masks.
-__device__ __forceinline__ void row_interval(const MaskView& m, int q, int k0, int& jlo, int& jhi) {
-  if (q >= m.q_valid) { jlo = 1; jhi = 0; return; }
-  const int gq = q + m.q_offset;
-  int lo = 0, hi = INT32_MAX;
-  if (m.flags & BMA_MASK_CAUSAL) hi = min(hi, gq);
-  if (m.flags & BMA_MASK_BAND) { lo = max(lo, gq - m.band_left); hi = min(hi, gq + m.band_right); }
-  if (m.flags & BMA_MASK_BLOCK_WINDOW) {
-    int wlo, whi;
-    block_window_range(m, gq, wlo, whi);
-    lo = max(lo, wlo);
-    hi = min(hi, whi - 1);
-  }
-  jlo = lo - m.k_offset - k0;
-  jhi = min(hi - m.k_offset, m.k_valid - 1) - k0;
-}
-
 // KB: the variant that folds the scale (and the per-head key bias, bma_attn_args.key_bias, when there is one)
 // into the scores BEFORE the running maximum is taken.  Compiled in only where it is needed: a key bias, or a
 // negative scale, for which max(raw score) * scale is the MINIMUM of the scaled scores and the exponentials
@@ -1176,7 +1159,7 @@ static bool fwd_persistent_enabled(const bma_mask_spec& spec) {
   return width <= 10 * BN;
 }
 
-bool sm100_supported(const bma_attn_args& a) {
+bool sm100_device() {
   static int cc_major = -1;
   if (cc_major < 0) {
     int dev = 0, v = 0;
@@ -1184,7 +1167,11 @@ bool sm100_supported(const bma_attn_args& a) {
       cc_major = v;
     else { (void)cudaGetLastError(); return false; }
   }
-  if (cc_major != 10) return false;
+  return cc_major == 10;
+}
+
+bool sm100_supported(const bma_attn_args& a) {
+  if (!sm100_device()) return false;
   return (a.d == 128 || a.d == 64) && tma_compatible(a.q) && tma_compatible(a.k) && tma_compatible(a.v) &&
          ceil_div(a.L, BN) <= kMaxKvTiles;
 }

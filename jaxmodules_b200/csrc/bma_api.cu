@@ -351,6 +351,46 @@ int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma
   return be == BMA_BACKEND_TCGEN05 ? sm100_fwd(*args, *spec, *lists, st) : simt_fwd(*args, *spec, *lists, st);
 }
 
+size_t bma_attn_f32_workspace_bytes(const bma_attn_args* args, int32_t backward) {
+  if (validate_common(args) != BMA_OK || args->backend != BMA_BACKEND_AUTO) return 0;
+  if (args->k.dtype != args->q.dtype || args->v.dtype != args->q.dtype) return 0;
+  return f32_workspace_bytes(*args, backward != 0);
+}
+
+int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+                     size_t workspace_bytes, bma_stream_t stream) {
+  const size_t need = bma_attn_f32_workspace_bytes(args, 0);
+  BMA_REQUIRE(need > 0, BMA_ERR_UNSUPPORTED);
+  BMA_REQUIRE(spec != nullptr, BMA_ERR_ARG);
+  int rc;
+  if ((rc = validate_tensor(args->q, true)) || (rc = validate_tensor(args->k, true)) ||
+      (rc = validate_tensor(args->v, true)) || (rc = validate_tensor(args->o, true)))
+    return rc;
+  if ((rc = validate_lists(args, lists, kSm100Tile, false))) return rc;
+  BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
+  BMA_REQUIRE(workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && workspace_bytes >= need, BMA_ERR_WORKSPACE);
+  return f32_fwd(*args, *spec, *lists, workspace, static_cast<cudaStream_t>(stream));
+}
+
+int bma_attn_bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+                     size_t workspace_bytes, bma_stream_t stream) {
+  const size_t need = bma_attn_f32_workspace_bytes(args, 1);
+  BMA_REQUIRE(need > 0, BMA_ERR_UNSUPPORTED);
+  BMA_REQUIRE(spec != nullptr && args->lse && args->delta, BMA_ERR_ARG);
+  int rc;
+  if ((rc = validate_tensor(args->q, true)) || (rc = validate_tensor(args->k, true)) ||
+      (rc = validate_tensor(args->v, true)) || (rc = validate_tensor(args->d_o, true)) ||
+      (rc = validate_tensor(args->dq, true)) || (rc = validate_tensor(args->dk, true)) ||
+      (rc = validate_tensor(args->dv, true)))
+    return rc;
+  BMA_REQUIRE(args->dq.dtype == args->q.dtype && args->dk.dtype == args->q.dtype && args->dv.dtype == args->q.dtype,
+              BMA_ERR_UNSUPPORTED);
+  if ((rc = validate_lists(args, lists, kSm100Tile, true))) return rc;
+  BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
+  BMA_REQUIRE(workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && workspace_bytes >= need, BMA_ERR_WORKSPACE);
+  return f32_bwd(*args, *spec, *lists, workspace, static_cast<cudaStream_t>(stream));
+}
+
 int bma_attn_bwd_preprocess(const bma_attn_args* args, void* d_o_bf16, bma_stream_t stream) {
   int rc = validate_common(args);
   if (rc != BMA_OK) return rc;

@@ -202,6 +202,80 @@ __device__ __forceinline__ uint32_t table_bits_col32(const MaskView& m, int k, i
   return w;
 }
 
+// Allowed key interval [jlo, jhi] (tile-local, inclusive) of query row q for interval-only masks.
+__device__ __forceinline__ void row_interval(const MaskView& m, int q, int k0, int& jlo, int& jhi) {
+  if (q >= m.q_valid) { jlo = 1; jhi = 0; return; }
+  const int gq = q + m.q_offset;
+  int lo = 0, hi = INT32_MAX;
+  if (m.flags & BMA_MASK_CAUSAL) hi = min(hi, gq);
+  if (m.flags & BMA_MASK_BAND) { lo = max(lo, gq - m.band_left); hi = min(hi, gq + m.band_right); }
+  if (m.flags & BMA_MASK_BLOCK_WINDOW) {
+    int wlo, whi;
+    block_window_range(m, gq, wlo, whi);
+    lo = max(lo, wlo);
+    hi = min(hi, whi - 1);
+  }
+  jlo = lo - m.k_offset - k0;
+  jhi = min(hi - m.k_offset, m.k_valid - 1) - k0;
+}
+
+// Allowed query interval [jlo, jhi] (local to the `width` columns from q0, inclusive) of key row k for masks made of
+// interval terms.  The block window of query block i starts at s(i) = clamp(i - left, 0, nblk - total): both ends are
+// non-decreasing in i, so the query blocks whose window contains the key form one range, whatever the window's
+// block size is relative to the tile.
+__device__ __forceinline__ void col_interval(const MaskView& m, int k, int q0, int width, int& jlo, int& jhi) {
+  jlo = 0;
+  jhi = min(width, m.q_valid - q0) - 1;
+  if (k >= m.k_valid) { jlo = 1; jhi = 0; return; }
+  const int gk = k + m.k_offset;
+  const int base = m.q_offset + q0;  // global index of column 0
+  if (m.flags & BMA_MASK_CAUSAL) jlo = max(jlo, gk - base);
+  if (m.flags & BMA_MASK_BAND) {  // gq - left <= gk <= gq + right  <=>  gk - right <= gq <= gk + left
+    jlo = max(jlo, gk - m.band_right - base);
+    jhi = min(jhi, gk + m.band_left - base);
+  }
+  if (m.flags & BMA_MASK_BLOCK_WINDOW) {
+    const int wb = m.win_block, total = m.win_left + m.win_right, last_start = m.win_nblk - total;
+    const int kb = gk / wb;            // key block of this key
+    const int t = kb - total + 1;      // the window reaches the key iff s(i) >= t ...
+    if (t > last_start) { jlo = 1; jhi = 0; return; }
+    if (t > 0) jlo = max(jlo, (t + m.win_left) * wb - base);
+    if (kb < last_start) jhi = min(jhi, (kb + m.win_left + 1) * wb - 1 - base);   // ... and s(i) <= kb
+  }
+}
+
+struct QTileIter {  // flattened walk over (group head, listed q tile)
+  const bma_block_lists& l;
+  int b, hk, G, kj;
+  int g, it, nfull, npart;
+  const int32_t* full_idx;
+  const int32_t* part_idx;
+  __device__ QTileIter(const bma_block_lists& l_, int b_, int hk_, int G_, int kj_)
+      : l(l_), b(b_), hk(hk_), G(G_), kj(kj_), g(-1), it(0), nfull(0), npart(0), full_idx(nullptr), part_idx(nullptr) {}
+  __device__ void load_head() {
+    const int h = hk * G + g;
+    const int lb = l.B == 1 ? 0 : b, lh = l.H == 1 ? 0 : h;
+    const int64_t row = ((int64_t)lb * l.H + lh) * l.NKV + kj;
+    nfull = l.full_q_num[row];
+    npart = l.q_num[row];
+    full_idx = l.full_q_idx + row * l.NQ;
+    part_idx = l.q_idx + row * l.NQ;
+    it = 0;
+  }
+  __device__ bool next(int& h, int& qi, bool& partial) {
+    if (g < 0) { g = 0; load_head(); }
+    while (it >= nfull + npart) {
+      if (++g >= G) return false;
+      load_head();
+    }
+    h = hk * G + g;
+    partial = it >= nfull;
+    qi = partial ? part_idx[it - nfull] : full_idx[it];
+    ++it;
+    return true;
+  }
+};
+
 // ---- numeric helpers -------------------------------------------------------------------
 __device__ __forceinline__ float to_float(float x) { return x; }
 __device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
@@ -223,6 +297,11 @@ int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
 size_t sm100_bwd_workspace_bytes(const bma_attn_args& a);
 size_t sm100_bwd_scratch_bytes(const bma_attn_args& a, const bma_block_lists& lists, const int64_t* visited_host);
 size_t sm100_bwd_scratch_min_bytes(const bma_attn_args& a, const bma_block_lists& lists, const int64_t* visited_host);
+// float32 on the tensor core (attn_f32_sm100.cu): 0 where the path does not take the request
+size_t f32_workspace_bytes(const bma_attn_args& a, bool backward);
+int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, cudaStream_t st);
+int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, cudaStream_t st);
+bool sm100_device();
 bool sm100_supported(const bma_attn_args& a);
 bool sm100_bwd_supported(const bma_attn_args& a);
 

@@ -300,9 +300,11 @@ def flex_attention(query: torch.Tensor, key: torch.Tensor, value: torch.Tensor, 
         if block_mask is None:
             terms = _masks.MaskTerms()
         else:
-            tiles = [_att.plan(Q, K, V, backend, key_bias=key_bias)[1:]]
+            if Q.dtype == torch.float32 and (block_mask.Q_BLOCK_SIZE, block_mask.KV_BLOCK_SIZE) == _att.plan(Q, K, V, backend)[1:]:
+                backend = nat.BMA_BACKEND_SIMT   # these lists can be walked as they are by the FP32 tile kernels only
+            tiles = [_att.tiles(Q, K, V, backend, key_bias=key_bias)]
             if torch.is_grad_enabled() and (query.requires_grad or key.requires_grad or value.requires_grad):
-                tiles.append(_att.plan(Q, K, V, backend, backward=True, key_bias=key_bias)[1:])
+                tiles.append(_att.tiles(Q, K, V, backend, backward=True, key_bias=key_bias))
             route = flex_route(block_mask, B, Hq, tiles, dev)
             if route == "table":
                 terms = _masks.MaskTerms(bitmap=_effective_table(block_mask, Hq // Hkv, Hq))
