@@ -65,7 +65,6 @@ struct DqParams {
   bma_mask_spec spec;
   bma_block_lists l;
   float scale_log2;
-  int interval_mask;
   int* status;
 };
 
@@ -456,7 +455,6 @@ int sm100_bwd_dq(const bma_attn_args& a, const bma_mask_spec& spec, const bma_bl
   DqParams p;
   p.a = a; p.spec = spec; p.l = lists;
   p.scale_log2 = a.scale * kLog2e;
-  p.interval_mask = (spec.flags & kTableTerms) ? 0 : 1;
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
 

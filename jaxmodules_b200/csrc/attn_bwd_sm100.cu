@@ -94,7 +94,6 @@ struct BwdParams {
   bma_mask_spec spec;
   bma_block_lists l;
   float scale_log2;
-  int interval_mask;
   int* status;
   uint8_t* ds_out;  // null, or the slots of kDsBytes: the dSt image of every visited block, addressed compactly:
                     // slot = head_base[b, h] - head_base[first head of the launch] + row_base[qi] + rank[qi][kj]
@@ -360,18 +359,11 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const int cg = half * 2 + c;
-          if (p.interval_mask) {
-            int jlo, jhi;
-            col_interval(mv, k, q0, BT, jlo, jhi);
-            const int lo = max(jlo - cg * 32, 0), hi = min(jhi - cg * 32, 31);
-            bits[c] = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
-            if (bits[c] && (mv.flags & kTableTerms)) bits[c] &= table_bits_col32(mv, k, q0 + cg * 32);
-          } else {
-            uint32_t w = 0;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) w |= (mask_allowed(mv, q0 + cg * 32 + j, k) ? 1u : 0u) << j;
-            bits[c] = w;
-          }
+          int jlo, jhi;
+          col_interval(mv, k, q0, BT, jlo, jhi);
+          const int lo = max(jlo - cg * 32, 0), hi = min(jhi - cg * 32, 31);
+          bits[c] = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
+          if (mv.flags & kTableTerms) bits[c] &= table_bits_col32(mv, k, q0 + cg * 32);
         }
       }
       if (!mbar_wait(&sm.bar[BAR_S1], n & 1)) return false;
@@ -667,7 +659,6 @@ int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   BMA_REQUIRE(lists.q_block == BT && lists.kv_block == BT && lists.q_num, BMA_ERR_ARG);
   BMA_REQUIRE(a.d_o.dtype == BMA_DTYPE_BF16, BMA_ERR_UNSUPPORTED);  // bma_attn_bwd_preprocess provides the bf16 copy
   BMA_REQUIRE(aligned16(a.d_o) && aligned16(a.dq) && aligned16(a.dk) && aligned16(a.dv), BMA_ERR_UNSUPPORTED);
-  const int interval = 1;   // every structured term has a closed per-key query interval (col_interval)
 
   CUtensorMap mq, mk, mv, mdo;
   int rc;
@@ -682,7 +673,6 @@ int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   BwdParams p;
   p.a = a; p.spec = spec; p.l = lists;
   p.scale_log2 = a.scale * kLog2e;
-  p.interval_mask = interval;
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
   p.ds_out = nullptr; p.head_base = nullptr; p.row_base = nullptr; p.rank = nullptr; p.capacity = 0;

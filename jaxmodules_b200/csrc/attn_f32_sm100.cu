@@ -733,7 +733,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         col_interval(mv, k, q0 + w * 32, 32, jlo, jhi);
         const int lo = max(jlo, 0), hi = min(jhi, 31);
         bits = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
-        if (bits && (mv.flags & kTableTerms)) bits &= table_bits_col32(mv, k, q0 + w * 32);
+        if (mv.flags & kTableTerms) bits &= table_bits_col32(mv, k, q0 + w * 32);
       }
       ok = mbar_wait(&sm.bar[KB_STAT + st], (n >> 1) & 1) && mbar_wait(&sm.bar[KB_S], n & 1);
       if (!ok) break;

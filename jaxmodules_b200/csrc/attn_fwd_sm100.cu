@@ -76,7 +76,6 @@ struct FwdParams {
   bma_mask_spec spec;
   bma_block_lists l;
   float scale_log2;
-  int interval_mask;  // 1: the mask has only interval terms (no segment ids / bit table)
   int* status;
 };
 
@@ -1196,7 +1195,6 @@ int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   FwdParams p;
   p.a = a; p.spec = spec; p.l = lists;
   p.scale_log2 = a.scale * kLog2e;
-  p.interval_mask = (spec.flags & kTableTerms) ? 0 : 1;
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
   const bool kb = a.key_bias != nullptr || a.scale < 0.f;

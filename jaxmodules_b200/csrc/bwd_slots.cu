@@ -9,8 +9,7 @@
 // head, head_base = exclusive prefix over (b, h) in row-major order of the list heads' totals.  A launch over a
 // range of (batch, head) units subtracts the head_base of its first head.
 //
-// Three small launches per backward call build the tables from the kv-side lists into the front of the caller's
-// workspace: ranks (one warp per list row), row bases (one CTA per list head), head bases (one CTA).
+// One small launch per backward call builds the tables from the kv-side lists into the front of the caller's workspace.
 #include <algorithm>
 
 #include "common.cuh"
@@ -21,13 +20,84 @@ namespace {
 
 constexpr int kMaxKvTilesBwd = 1024;  // the tensor-core backward takes L <= 131072
 
-// rank[row][kj] = number of visited kv tiles below kj, or -1 when (row, kj) is not visited; row_count[row].
-__global__ void __launch_bounds__(256) slot_rank_kernel(bma_block_lists l, int32_t* __restrict__ rank, int32_t* __restrict__ row_count) {
+__device__ __forceinline__ int row_visits(const bma_block_lists& l, int64_t row) {
+  return min(max(__ldg(l.full_kv_num + row), 0), l.NKV) + min(max(__ldg(l.kv_num + row), 0), l.NKV);
+}
+__device__ __forceinline__ long long block_sum256(long long v, long long* part) {   // the sum over 256 threads, to all of them
+  for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  long long t = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) t += part[i];
+  return t;
+}
+
+// All tables in one launch; every CTA adds up from the row counts what it needs itself, so that none waits for another
+// (three dependent launches before took 8 us; this one 3 - 5).
+//   CTA head * ceil(NQ / 8) + g: rank[row][kj] = number of visited kv tiles below kj, or -1 when (row, kj) is not
+//     visited, for eight rows (one warp each), and row_base of these rows = visits of the head's rows before them;
+//   the last CTA: head_base[i], i in [0, B * Hq] = exclusive prefix over (b, h) of the list heads' totals.
+// (A row base counts list entries; a block listed twice leaves an unused slot behind.)
+__global__ void __launch_bounds__(256) slot_tables_kernel(bma_block_lists l, int B, int Hq, int32_t* __restrict__ rank,
+                                                          int32_t* __restrict__ row_base, int64_t* __restrict__ head_total,
+                                                          int64_t* __restrict__ head_base) {
   __shared__ uint32_t bits[8][kMaxKvTilesBwd / 32];
+  __shared__ long long part[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t rows = (int64_t)l.B * l.H * l.NQ;
-  const int64_t row = (int64_t)blockIdx.x * 8 + w;
-  if (row >= rows) return;
+  const int groups = (l.NQ + 7) / 8;
+  if (blockIdx.x == gridDim.x - 1) {
+    const int LHEADS = l.B * l.H;
+    for (int i = w; i < LHEADS; i += 8) {   // one warp per list head
+      long long s = 0;
+      for (int r = lane; r < l.NQ; r += 32) s += row_visits(l, (int64_t)i * l.NQ + r);
+      for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+      if (lane == 0) head_total[i] = s;
+    }
+    __syncthreads();
+    const int64_t n = (int64_t)B * Hq;
+    long long carry = 0;
+    for (int64_t base = 0; base < n; base += 256) {
+      const int64_t i = base + threadIdx.x;
+      long long v = 0;
+      if (i < n) {
+        const int b = (int)(i / Hq), h = (int)(i % Hq);
+        v = head_total[(int64_t)(l.B == 1 ? 0 : b) * l.H + (l.H == 1 ? 0 : h)];
+      }
+      long long incl = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const long long t = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += t;
+      }
+      __syncthreads();
+      if (lane == 31) part[w] = incl;
+      __syncthreads();
+      long long before = carry, all = 0;
+      for (int j = 0; j < 8; ++j) {
+        if (j < w) before += part[j];
+        all += part[j];
+      }
+      if (i < n) head_base[i] = before + incl - v;
+      carry += all;
+    }
+    if (threadIdx.x == 0) head_base[n] = carry;
+    return;
+  }
+  const int64_t head_row = (int64_t)(blockIdx.x / groups) * l.NQ;
+  const int first = (int)(blockIdx.x % groups) * 8;
+  long long s = 0;
+  for (int r = threadIdx.x; r < first; r += 256) s += row_visits(l, head_row + r);
+  const int before = (int)block_sum256(s, part);
+  const int r = first + w;
+  if (r >= l.NQ) return;
+  const int64_t row = head_row + r;
+  if (lane == 0) {
+    int mine = before;
+    for (int i = first; i < r; ++i) mine += row_visits(l, head_row + i);
+    row_base[row] = mine;
+  }
   const int words = (l.NKV + 31) / 32;
   bits[w][lane] = 0u;
   __syncwarp();
@@ -50,96 +120,14 @@ __global__ void __launch_bounds__(256) slot_rank_kernel(bma_block_lists l, int32
     const int v = __shfl_up_sync(0xffffffffu, prefix, off);
     if (lane >= off) prefix += v;
   }
-  const int total = __shfl_sync(0xffffffffu, prefix, 31);
   const int below = prefix - __popc(mine);
-  if (lane < words) {
-    int32_t* out = rank + row * l.NKV + lane * 32;
-    for (int bit = 0; bit < 32 && lane * 32 + bit < l.NKV; ++bit)
-      out[bit] = (mine >> bit) & 1u ? below + __popc(mine & ((1u << bit) - 1u)) : -1;
+  int32_t* out = rank + row * l.NKV;
+  for (int word = 0; word < words; ++word) {   // whole words at a time, so that the stores are coalesced
+    const uint32_t bw = __shfl_sync(0xffffffffu, mine, word);
+    const int start = __shfl_sync(0xffffffffu, below, word);
+    const int j = word * 32 + lane;
+    if (j < l.NKV) out[j] = (bw >> lane) & 1u ? start + __popc(bw & ((1u << lane) - 1u)) : -1;
   }
-  if (lane == 0) row_count[row] = total;
-}
-
-// One CTA per list head: row_base = exclusive prefix of row_count over its NQ rows (in place), head_total.
-__global__ void __launch_bounds__(1024) slot_row_base_kernel(int NQ, int32_t* __restrict__ row_count_to_base, int64_t* __restrict__ head_total) {
-  __shared__ int warp_sums[32];
-  __shared__ int carry_s;
-  int32_t* rc = row_count_to_base + (int64_t)blockIdx.x * NQ;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  for (int base = 0; base < NQ; base += 1024) {
-    const int i = base + threadIdx.x;
-    const int v = i < NQ ? rc[i] : 0;
-    int incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += t;
-    }
-    if (lane == 31) warp_sums[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-      int s = warp_sums[lane];
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, s, off);
-        if (lane >= off) s += t;
-      }
-      warp_sums[lane] = s;   // inclusive over warps
-    }
-    __syncthreads();
-    const int carry = carry_s;
-    const int before = carry + (w > 0 ? warp_sums[w - 1] : 0) + incl - v;
-    if (i < NQ) rc[i] = before;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s = carry + warp_sums[31];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) head_total[blockIdx.x] = carry_s;
-}
-
-// One CTA: head_base[i] for i in [0, B*Hq] = exclusive prefix over (b, h) of head_total[b', h'].
-__global__ void __launch_bounds__(1024) slot_head_base_kernel(int B, int Hq, int LB, int LH, const int64_t* __restrict__ head_total,
-                                                              int64_t* __restrict__ head_base) {
-  __shared__ long long warp_sums[32];
-  __shared__ long long carry_s;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t n = (int64_t)B * Hq;
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  for (int64_t base = 0; base < n; base += 1024) {
-    const int64_t i = base + threadIdx.x;
-    long long v = 0;
-    if (i < n) {
-      const int b = (int)(i / Hq), h = (int)(i % Hq);
-      v = head_total[(int64_t)(LB == 1 ? 0 : b) * LH + (LH == 1 ? 0 : h)];
-    }
-    long long incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const long long t = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += t;
-    }
-    if (lane == 31) warp_sums[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-      long long s = warp_sums[lane];
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const long long t = __shfl_up_sync(0xffffffffu, s, off);
-        if (lane >= off) s += t;
-      }
-      warp_sums[lane] = s;
-    }
-    __syncthreads();
-    const long long carry = carry_s;
-    if (i < n) head_base[i] = carry + (w > 0 ? warp_sums[w - 1] : 0) + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s = carry + warp_sums[31];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) head_base[n] = carry_s;
 }
 
 // visited[b', h'] = sum over the rows of a list head of (kv_num + full_kv_num)
@@ -181,11 +169,10 @@ SlotTables slot_tables_layout(const bma_attn_args& a, const bma_block_lists& l, 
 
 int slot_tables_build(const bma_attn_args& a, const bma_block_lists& l, const SlotTables& t, cudaStream_t st) {
   BMA_REQUIRE(l.NKV <= kMaxKvTilesBwd, BMA_ERR_LIMIT);
-  const int64_t rows = (int64_t)l.B * l.H * l.NQ;
-  slot_rank_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(l, t.rank, t.row_base);
-  slot_row_base_kernel<<<(unsigned)(l.B * l.H), 1024, 0, st>>>(l.NQ, t.row_base, t.head_total);
-  slot_head_base_kernel<<<1, 1024, 0, st>>>(a.B, a.Hq, l.B, l.H, t.head_total, t.head_base);
-  count_launches(3);
+  const int64_t ctas = (int64_t)l.B * l.H * ((l.NQ + 7) / 8) + 1;
+  BMA_REQUIRE(ctas <= INT32_MAX, BMA_ERR_LIMIT);
+  slot_tables_kernel<<<(unsigned)ctas, 256, 0, st>>>(l, a.B, a.Hq, t.rank, t.row_base, t.head_total, t.head_base);
+  count_launches(1);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
 }

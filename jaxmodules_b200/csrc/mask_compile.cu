@@ -5,7 +5,8 @@
 // (jaxmodules/block_mask.py:454-498) followed by BlockMask.from_blocks (:227-275) and
 // get_sparse_{kv,q}_data_from_blocks (:411-451) returns:
 //   pass 0 (only for segment masks)  per-block min/max of the segment ids
-//   pass 1 classify                  one flag byte per block: 0 empty, 1 partial (any ^ all), 2 full (all)
+//   pass 1 classify                  one flag per block: 0 empty, 1 partial (any ^ all), 2 full (all); inside pass 2 unless
+//                                    wide rows have blocks that must be scanned
 //   pass 2 compact                   per row: count + [set indices ascending, unset indices ascending]
 //                                    (== stable argsort(-blocks)), once along kv and once along q.
 // The reference evaluates the dense B*H*Q*KV mask twice; here structured masks are classified
@@ -102,9 +103,88 @@ __device__ __forceinline__ bool interval_classify(const bma_mask_spec& s, int q0
   return true;
 }
 
-// pass 1a: one THREAD per block.  Interval terms and the per-block segment-id ranges decide almost every
-// block in closed form; flags leave as coalesced bytes.  The few blocks that stay open (a segment boundary,
-// a bit table or a change of the block window inside the block) are appended to a work list for pass 1b.
+// Flag of one block in closed form (interval terms on the block corners, segment-id ranges, stored tile classes): 0 empty,
+// 1 partial, 2 full, or 3 where only the elements can tell (a segment boundary, a bit table or a change of the block
+// window inside the block).
+constexpr int kUndecided = 3;
+__device__ __forceinline__ int block_flag(const bma_mask_spec& spec, const SegSummary& seg, int cb, int ch, int qi, int kj,
+                                          int NQ, int NKV, int QB, int KVB) {
+  bool any = false, all = false;
+  if (!interval_classify(spec, qi * QB, kj * KVB, QB, KVB, any, all)) return kUndecided;
+  if (!any) return 0;
+  bool scan = false;
+  if (spec.flags & BMA_MASK_SEGMENT) {
+    const int qmn = seg.qmin[(int64_t)cb * NQ + qi], qmx = seg.qmax[(int64_t)cb * NQ + qi];
+    const int kmn = seg.kmin[(int64_t)cb * NKV + kj], kmx = seg.kmax[(int64_t)cb * NKV + kj];
+    if (qmx < kmn || qmn > kmx) return 0;                                  // ids never meet
+    if (!(qmn == qmx && kmn == kmx && qmn == kmn)) {                       // a boundary crosses the block
+      if (spec.flags & BMA_MASK_COMPILE_CONSERVATIVE) all = false;         // "partial" without looking closer
+      else scan = true;
+    }
+  }
+  if (spec.flags & BMA_MASK_BITMAP) scan = true;
+  if (spec.flags & BMA_MASK_TILES) {
+    // a block that IS a stored tile takes the tile's class (exactly, when no other term cuts the block); any other
+    // block geometry is scanned element by element
+    const bool is_tile = QB == 128 && KVB == 128 && (spec.q_offset & 127) == 0 && (spec.k_offset & 127) == 0;
+    if (!is_tile) scan = true;
+    else {
+      const int64_t t = (((int64_t)(cb % spec.tiles_B) * spec.tiles_H + (ch % spec.tiles_H)) * spec.tiles_q +
+                         ((qi * QB + spec.q_offset) >> 7)) * spec.tiles_k + ((kj * KVB + spec.k_offset) >> 7);
+      const int tc = spec.tile_class[t];
+      if (tc == 0) return 0;
+      if (tc == 1) {
+        if (all || (spec.flags & BMA_MASK_COMPILE_CONSERVATIVE)) all = false;   // cut by the tile alone: partial
+        else scan = true;                                                        // cut by two terms: may be empty
+      }
+    }
+  }
+  return scan ? kUndecided : all ? 2 : 1;
+}
+
+// Flag of one block by its elements, by one whole warp: a lane takes a query row at a time and four words of 32 keys, so
+// that a 128 x 128 block is four batches of independent loads (stops as soon as the block is known to be partial).
+// Element by element with a row at a time, the 8 x 8 blocks of 128 x 128 of a bit table took 122 us in a launch of their own;
+// the whole build of their lists, scan included, now takes 12.
+__device__ __forceinline__ int scan_block(const bma_mask_spec& spec, int cb, int ch, int qi, int kj, int QB, int KVB) {
+  const int lane = threadIdx.x & 31;
+  const MaskView m = make_mask_view(spec, cb, ch);
+  const int q0 = qi * QB, k0 = kj * KVB;
+  const int q_end = min(q0 + QB, spec.q_valid), k_end = min(k0 + KVB, spec.k_valid);
+  bool any = false;
+  bool all = (q0 + QB <= spec.q_valid) && (k0 + KVB <= spec.k_valid);
+  for (int r = q0; r < q_end; r += 32) {
+    const int q = r + lane;
+    bool row_any = false, row_all = true;
+    if (q < q_end) {
+      int jlo, jhi;
+      row_interval(m, q, k0, jlo, jhi);
+      for (int kb = k0; kb < k_end; kb += 128) {
+        uint32_t bits[4], want[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int j0 = kb - k0 + c * 32, n = min(32, k_end - kb - c * 32);
+          want[c] = n <= 0 ? 0u : 0xffffffffu >> (32 - n);
+          const int lo = max(jlo - j0, 0), hi = min(jhi - j0, 31);
+          bits[c] = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) & want[c] : 0u;
+          if (bits[c] && (m.flags & kTableTerms)) bits[c] &= table_bits_row32(m, q, kb + c * 32);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          row_any |= bits[c] != 0u;
+          row_all &= bits[c] == want[c];
+        }
+      }
+    }
+    any |= __any_sync(0xffffffffu, row_any) != 0;
+    all &= __all_sync(0xffffffffu, row_all) != 0;
+    if (any && !all) break;
+  }
+  return all ? 2 : (any ? 1 : 0);
+}
+
+// pass 1a: one THREAD per block.  Closed forms decide almost every block; flags leave as coalesced bytes.  The blocks that
+// stay open are appended to a work list for pass 1b.
 // The list and its counter live in output arrays that pass 2 overwrites afterwards (`todo` = kv_idx, one
 // int32 per block at least; `todo_count` = kv_num[0]), so the scratch stays at one byte per block.
 struct BlockCoord { int cb, ch, qi, kj; };
@@ -129,39 +209,12 @@ __global__ void classify_kernel(bma_mask_spec spec, int CB, int CH, int NQ, int 
   // `base` is the warp's first block: uniform across the warp, so the ballot below sees all 32 lanes
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < total; base += stride) {
     const int64_t w = base + lane;
-    const bool valid = w < total;
-    bool any = false, all = false, scan = false;
-    if (valid) {
+    bool scan = false;
+    if (w < total) {
       const BlockCoord c = block_coord(w, CH, NQ, NKV);
-      const bool decided = interval_classify(spec, c.qi * QB, c.kj * KVB, QB, KVB, any, all);
-      scan = !decided;
-      if (decided && any && (spec.flags & BMA_MASK_SEGMENT)) {
-        const int qmn = seg.qmin[(int64_t)c.cb * NQ + c.qi], qmx = seg.qmax[(int64_t)c.cb * NQ + c.qi];
-        const int kmn = seg.kmin[(int64_t)c.cb * NKV + c.kj], kmx = seg.kmax[(int64_t)c.cb * NKV + c.kj];
-        if (qmx < kmn || qmn > kmx) { any = false; all = false; }          // ids never meet
-        else if (!(qmn == qmx && kmn == kmx && qmn == kmn)) {                 // a boundary crosses the block
-          if (spec.flags & BMA_MASK_COMPILE_CONSERVATIVE) all = false;        // "partial" without looking closer
-          else scan = true;
-        }
-      }
-      if (decided && any && (spec.flags & BMA_MASK_BITMAP)) scan = true;
-      if (decided && any && (spec.flags & BMA_MASK_TILES)) {
-        // a block that IS a stored tile takes the tile's class (exactly, when no other term cuts the block); any other
-        // block geometry is scanned element by element
-        const bool is_tile = QB == 128 && KVB == 128 && (spec.q_offset & 127) == 0 && (spec.k_offset & 127) == 0;
-        if (!is_tile) scan = true;
-        else {
-          const int64_t t = (((int64_t)(c.cb % spec.tiles_B) * spec.tiles_H + (c.ch % spec.tiles_H)) * spec.tiles_q +
-                             ((c.qi * QB + spec.q_offset) >> 7)) * spec.tiles_k + ((c.kj * KVB + spec.k_offset) >> 7);
-          const int tc = spec.tile_class[t];
-          if (tc == 0) { any = false; all = false; }
-          else if (tc == 1) {
-            if (all || (spec.flags & BMA_MASK_COMPILE_CONSERVATIVE)) all = false;   // cut by the tile alone: partial
-            else scan = true;                                                        // cut by two terms: may be empty
-          }
-        }
-      }
-      flags[w] = all ? 2 : (any ? 1 : 0);   // rewritten by pass 1b when `scan`
+      const int f = block_flag(spec, seg, c.cb, c.ch, c.qi, c.kj, NQ, NKV, QB, KVB);
+      scan = f == kUndecided;
+      flags[w] = (uint8_t)f;   // rewritten by pass 1b when `scan`
     }
     const unsigned m = __ballot_sync(0xffffffffu, scan);
     if (m != 0u) {  // one atomic per warp
@@ -174,8 +227,7 @@ __global__ void classify_kernel(bma_mask_spec spec, int CB, int CH, int NQ, int 
   }
 }
 
-// pass 1b: one WARP per listed block: exact any/all by evaluating the mask on every element
-// (stops as soon as the block is known to be partial).
+// pass 1b: one WARP per listed block.
 __global__ void scan_kernel(bma_mask_spec spec, int CH, int NQ, int NKV, int QB, int KVB, uint8_t* __restrict__ flags,
                             const int32_t* __restrict__ todo, const int32_t* __restrict__ todo_count) {
   const int lane = threadIdx.x & 31;
@@ -184,30 +236,24 @@ __global__ void scan_kernel(bma_mask_spec spec, int CH, int NQ, int NKV, int QB,
   for (int i = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); i < count; i += gridDim.x * warps_per_cta) {
     const int64_t w = todo[i];
     const BlockCoord c = block_coord(w, CH, NQ, NKV);
-    const MaskView m = make_mask_view(spec, c.cb, c.ch);
-    const int q0 = c.qi * QB, k0 = c.kj * KVB;
-    const int qb_end = min(q0 + QB, spec.q_valid), kb_end = min(k0 + KVB, spec.k_valid);
-    bool any = false;
-    bool all = (q0 + QB <= spec.q_valid) && (k0 + KVB <= spec.k_valid);
-    for (int q = q0; q < qb_end && !(any && !all); ++q) {
-      for (int kb = k0; kb < kb_end; kb += 32) {
-        const int k = kb + lane;
-        const bool in = k < kb_end;
-        const bool ok = in && mask_allowed(m, q, k);
-        const unsigned okb = __ballot_sync(0xffffffffu, ok);
-        const unsigned inb = __ballot_sync(0xffffffffu, in);
-        any |= (okb != 0u);
-        all &= (okb == inb);
-      }
-    }
-    if (lane == 0) flags[w] = all ? 2 : (any ? 1 : 0);
+    const int f = scan_block(spec, c.cb, c.ch, c.qi, c.kj, QB, KVB);
+    if (lane == 0) flags[w] = (uint8_t)f;
   }
 }
 
 // pass 2: one CTA per (classification row, replica chunk).  TRANSPOSED = q-side lists.
 // Shared memory: 2 index rows of `NC` int32, the row's `NC` flag bytes, + scan scratch.
-template <bool TRANSPOSED>
-__device__ __forceinline__ void compact_row(const uint8_t* __restrict__ flags, int CB, int CH, int NQ, int NKV, int out_B,
+// With `flags` null the CTA classifies its row itself, so that passes 1a and 1b, their launches and the flag bytes fall
+// away.  Each block is then classified once per list side; that is cheap in closed form, and elements are scanned here
+// only where a row is short (kInlineScanWidth).
+struct RowSource {
+  const uint8_t* flags;
+  bma_mask_spec spec;
+  SegSummary seg;
+  int QB, KVB;
+};
+template <bool TRANSPOSED, bool SCAN>
+__device__ __forceinline__ void compact_row(const RowSource& src, int CB, int CH, int NQ, int NKV, int out_B,
                                             int out_H, int32_t* __restrict__ part_num, int32_t* __restrict__ part_idx,
                                             int32_t* __restrict__ full_num, int32_t* __restrict__ full_idx) {
   extern __shared__ int32_t smem[];
@@ -221,12 +267,33 @@ __device__ __forceinline__ void compact_row(const uint8_t* __restrict__ flags, i
   const int r = blockIdx.x % NR;
   const int ch = (blockIdx.x / NR) % CH;
   const int cb = blockIdx.x / (NR * CH);
-  const uint8_t* fbase = flags + (int64_t)(cb * CH + ch) * NQ * NKV;
   // the row's flags go to shared memory first: all loads of a thread are in flight together (a column of the
   // flag grid, for the q-side lists, is one byte per 32-byte sector), and both passes below read them twice
   uint8_t* fl = reinterpret_cast<uint8_t*>(smem + 2 * NC);
-  for (int c = threadIdx.x; c < NC; c += kThreads) fl[c] = TRANSPOSED ? fbase[(int64_t)c * NKV + r] : fbase[(int64_t)r * NKV + c];
-  __syncthreads();
+  if (src.flags) {
+    const uint8_t* fbase = src.flags + (int64_t)(cb * CH + ch) * NQ * NKV;
+    for (int c = threadIdx.x; c < NC; c += kThreads) fl[c] = TRANSPOSED ? fbase[(int64_t)c * NKV + r] : fbase[(int64_t)r * NKV + c];
+    __syncthreads();
+  } else {
+    int open = 0;
+    for (int c = threadIdx.x; c < NC; c += kThreads) {
+      const int f = block_flag(src.spec, src.seg, cb, ch, TRANSPOSED ? c : r, TRANSPOSED ? r : c, NQ, NKV, src.QB, src.KVB);
+      open |= f == kUndecided;
+      fl[c] = (uint8_t)f;
+    }
+    if (!SCAN) {
+      __syncthreads();
+    } else if (__syncthreads_or(open)) {
+      for (int c = threadIdx.x >> 5; c < NC; c += kThreads / 32) {   // one warp per open block
+        const int f = fl[c];
+        __syncwarp();
+        if (f != kUndecided) continue;
+        const int g = scan_block(src.spec, cb, ch, TRANSPOSED ? c : r, TRANSPOSED ? r : c, src.QB, src.KVB);
+        if ((threadIdx.x & 31) == 0) fl[c] = (uint8_t)g;
+      }
+      __syncthreads();
+    }
+  }
   auto flag_at = [&](int c) -> int { return fl[c]; };
 
   const int per = (NC + kThreads - 1) / kThreads;
@@ -288,25 +355,25 @@ __device__ __forceinline__ void compact_row(const uint8_t* __restrict__ flags, i
   }
 }
 
-template <bool TRANSPOSED>
-__global__ void compact_kernel(const uint8_t* __restrict__ flags, int CB, int CH, int NQ, int NKV, int out_B,
-                               int out_H, int32_t* __restrict__ part_num, int32_t* __restrict__ part_idx,
-                               int32_t* __restrict__ full_num, int32_t* __restrict__ full_idx) {
-  compact_row<TRANSPOSED>(flags, CB, CH, NQ, NKV, out_B, out_H, part_num, part_idx, full_num, full_idx);
-}
-
-// Both list sides in ONE launch (blockIdx.z = 0: kv side, 1: q side): no launch gap between them, and the tail of one
-// side fills with the other's rows.  The builder is bound by the HBM writes of the index arrays.
-__global__ void compact_both_kernel(const uint8_t* __restrict__ flags, int CB, int CH, int NQ, int NKV, int out_B, int out_H,
-                                    bma_block_lists l) {
+// The kv side (blockIdx.z = 0) and, where wanted, the q side (1) in ONE launch: no launch gap between them, and the tail of
+// one side fills with the other's rows.  The builder is bound by the HBM writes of the index arrays.
+template <bool SCAN>
+__global__ void __launch_bounds__(kThreads) compact_kernel(const __grid_constant__ RowSource src, int CB, int CH, int NQ, int NKV,
+                                                           int out_B, int out_H, const __grid_constant__ bma_block_lists l) {
   if (blockIdx.z == 0) {
     if ((int)blockIdx.x < CB * CH * NQ)
-      compact_row<false>(flags, CB, CH, NQ, NKV, out_B, out_H, l.kv_num, l.kv_idx, l.full_kv_num, l.full_kv_idx);
+      compact_row<false, SCAN>(src, CB, CH, NQ, NKV, out_B, out_H, l.kv_num, l.kv_idx, l.full_kv_num, l.full_kv_idx);
   } else {
     if ((int)blockIdx.x < CB * CH * NKV)
-      compact_row<true>(flags, CB, CH, NQ, NKV, out_B, out_H, l.q_num, l.q_idx, l.full_q_num, l.full_q_idx);
+      compact_row<true, SCAN>(src, CB, CH, NQ, NKV, out_B, out_H, l.q_num, l.q_idx, l.full_q_num, l.full_q_idx);
   }
 }
+
+// Widest row whose open blocks are scanned by the CTA that compacts it: its eight warps take four blocks each then, a few
+// microseconds more than the launches of the separate passes cost; a wider row is better spread over the whole chip.
+// (In closed form the row is always classified here: 1024 x 1024 blocks, both sides, 32 heads: 93 us against 101 with the
+// flags written and read back, of which 82 us are the index arrays at the copy rate.)
+constexpr int kInlineScanWidth = 32;
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -381,58 +448,36 @@ int mask_compile_launch(const bma_mask_spec& spec, int B, int H, const bma_block
     seg_summary_kernel<<<grid, kThreads, 0, st>>>(spec, B, l.NQ, l.NKV, l.q_block, l.kv_block, seg);
     count_launches(1);
   }
-  {
+  // Blocks that closed forms cannot decide exist only with these terms (a block window whose blocks are whole multiples of
+  // the list's query blocks never changes inside one).
+  const bool window_cuts = (spec.flags & BMA_MASK_BLOCK_WINDOW) && (spec.win_block % l.q_block != 0 || spec.q_offset % l.q_block != 0);
+  const bool may_scan = (spec.flags & (BMA_MASK_BITMAP | BMA_MASK_TILES)) || window_cuts ||
+                        ((spec.flags & BMA_MASK_SEGMENT) && !(spec.flags & BMA_MASK_COMPILE_CONSERVATIVE));
+  const int width = std::max(l.NQ, l.NKV);
+  RowSource src{nullptr, spec, seg, l.q_block, l.kv_block};
+  if (may_scan && width > kInlineScanWidth) {
     const int64_t blocks = (int64_t)p.CB * p.CH * l.NQ * l.NKV;
     const int grid = (int)std::min<int64_t>((blocks + kThreads - 1) / kThreads, (int64_t)sm_count * 16);
-    // blocks that closed forms cannot decide exist only with these terms; without them pass 1b is not launched
-    const bool may_scan = (spec.flags & (BMA_MASK_BITMAP | BMA_MASK_BLOCK_WINDOW | BMA_MASK_TILES)) ||
-                          ((spec.flags & BMA_MASK_SEGMENT) && !(spec.flags & BMA_MASK_COMPILE_CONSERVATIVE));
-    if (may_scan) BMA_CUDA_TRY(cudaMemsetAsync(l.kv_num, 0, sizeof(int32_t), st));
+    BMA_CUDA_TRY(cudaMemsetAsync(l.kv_num, 0, sizeof(int32_t), st));
     classify_kernel<<<grid, kThreads, 0, st>>>(spec, p.CB, p.CH, l.NQ, l.NKV, l.q_block, l.kv_block, seg, flags, l.kv_idx, l.kv_num);
-    count_launches(1);
-    if (may_scan) {
-      scan_kernel<<<sm_count * 8, kThreads, 0, st>>>(spec, p.CH, l.NQ, l.NKV, l.q_block, l.kv_block, flags, l.kv_idx, l.kv_num);
-      count_launches(1);
-    }
+    scan_kernel<<<sm_count * 8, kThreads, 0, st>>>(spec, p.CH, l.NQ, l.NKV, l.q_block, l.kv_block, flags, l.kv_idx, l.kv_num);
+    count_launches(2);
+    src.flags = flags;
   }
-  auto launch_compact = [&](bool transposed) -> int {
-    const int NR = transposed ? l.NKV : l.NQ, NC = transposed ? l.NQ : l.NKV;
-    const int rows = p.CB * p.CH * NR;
-    const int reps = ((p.CB == l.B) ? 1 : l.B) * ((p.CH == l.H) ? 1 : l.H);
-    int gy = std::max(1, std::min(reps, (sm_count * 4 + rows - 1) / rows));
-    gy = std::min(gy, 65535);
-    const size_t smem = sizeof(int32_t) * 2 * (size_t)NC + align_up((size_t)NC, 16);
-    dim3 grid(rows, gy);
-    if (transposed) {
-      if (smem > 48 * 1024)
-        BMA_CUDA_TRY(cudaFuncSetAttribute(compact_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      compact_kernel<true><<<grid, kThreads, smem, st>>>(flags, p.CB, p.CH, l.NQ, l.NKV, l.B, l.H, l.q_num, l.q_idx,
-                                                         l.full_q_num, l.full_q_idx);
-    } else {
-      if (smem > 48 * 1024)
-        BMA_CUDA_TRY(cudaFuncSetAttribute(compact_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      compact_kernel<false><<<grid, kThreads, smem, st>>>(flags, p.CB, p.CH, l.NQ, l.NKV, l.B, l.H, l.kv_num, l.kv_idx,
-                                                          l.full_kv_num, l.full_kv_idx);
-    }
-    count_launches(1);
+  const int rows = p.CB * p.CH * (l.q_num ? width : l.NQ);
+  const int NC = l.q_num ? width : l.NKV;
+  const int reps = ((p.CB == l.B) ? 1 : l.B) * ((p.CH == l.H) ? 1 : l.H);
+  const int gy = std::min(std::max(1, std::min(reps, (sm_count * 4 + rows - 1) / rows)), 65535);
+  const size_t smem = sizeof(int32_t) * 2 * (size_t)NC + align_up((size_t)NC, 16);
+  const dim3 grid(rows, gy, l.q_num ? 2 : 1);
+  auto launch = [&](auto kernel) -> int {
+    if (smem > 48 * 1024) BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, kThreads, smem, st>>>(src, p.CB, p.CH, l.NQ, l.NKV, l.B, l.H, l);
     return BMA_OK;
   };
-  int rc = BMA_OK;
-  if (l.q_num) {   // both sides: one launch
-    const int rows = p.CB * p.CH * std::max(l.NQ, l.NKV);
-    const int reps = ((p.CB == l.B) ? 1 : l.B) * ((p.CH == l.H) ? 1 : l.H);
-    int gy = std::max(1, std::min(reps, (sm_count * 4 + rows - 1) / rows));
-    gy = std::min(gy, 65535);
-    const int NC = std::max(l.NQ, l.NKV);
-    const size_t smem = sizeof(int32_t) * 2 * (size_t)NC + align_up((size_t)NC, 16);
-    if (smem > 48 * 1024)
-      BMA_CUDA_TRY(cudaFuncSetAttribute(compact_both_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    compact_both_kernel<<<dim3(rows, gy, 2), kThreads, smem, st>>>(flags, p.CB, p.CH, l.NQ, l.NKV, l.B, l.H, l);
-    count_launches(1);
-  } else {
-    rc = launch_compact(false);
-    if (rc != BMA_OK) return rc;
-  }
+  const int rc = (may_scan && !src.flags) ? launch(compact_kernel<true>) : launch(compact_kernel<false>);
+  if (rc) return rc;
+  count_launches(1);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
 }
