@@ -262,6 +262,13 @@ int bma_attn_bwd_plan(const bma_attn_args* args, int32_t* backend, int32_t* q_ti
 int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec,
                  const bma_block_lists* lists, bma_stream_t stream);
 
+/* The same with a workspace (16-byte aligned), which lets few queries against many keys spread over the whole chip: partial
+ * results of runs of keys are combined through it.  bma_attn_fwd_workspace_bytes is 0 where none is used; with less than
+ * that bma_attn_fwd_ws runs as bma_attn_fwd does. */
+size_t bma_attn_fwd_workspace_bytes(const bma_attn_args* args, const bma_block_lists* lists);
+int bma_attn_fwd_ws(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
+                    void* workspace, size_t workspace_bytes, bma_stream_t stream);
+
 /* float32 inputs on the tensor core: every operand as three bf16 planes (exact), six plane products per matrix product,
  * float32 sums -- the accuracy of FP32 FMA arithmetic.  The caller provides the workspace that holds the planes (16-byte
  * aligned) and block lists of BMA_F32_TILE x BMA_F32_TILE blocks; everything else is as for bma_attn_fwd / bma_attn_bwd.

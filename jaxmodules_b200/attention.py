@@ -260,7 +260,10 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
                 nat.check(lib.bma_attn_fwd_f32(C.byref(a), C.byref(dmask.spec), C.byref(lists), ws.data_ptr(), f32_bytes, _stream(dev)),
                           "bma_attn_fwd_f32")
             else:
-                nat.check(lib.bma_attn_fwd(C.byref(a), C.byref(dmask.spec), C.byref(lists), _stream(dev)), "bma_attn_fwd")
+                ws_bytes = lib.bma_attn_fwd_workspace_bytes(C.byref(a), C.byref(lists))
+                ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=dev) if ws_bytes else None
+                nat.check(lib.bma_attn_fwd_ws(C.byref(a), C.byref(dmask.spec), C.byref(lists), ws.data_ptr() if ws_bytes else None, ws_bytes,
+                                              _stream(dev)), "bma_attn_fwd")
         _maybe_check_status(dev, "bma_attn_fwd")
     ctx = dict(dmask=dmask, lists=lists, list_tensors=lt, backend=be, scale=scale, lists_fn=lists_fn,
                lists_tile=(tq, tk), lists_have_q_side=both_sides, key_bias=key_bias)

@@ -20,6 +20,7 @@
 // S_x (overwrites it) needs no extra barrier.  Every mbarrier wait is bounded; on a timeout the
 // thread records an error code and unwinds to the common exit where TMEM is released.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <mutex>
 
@@ -1064,6 +1065,380 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
 }
 
+// =================================================================================================
+// Split variant for few queries (one q tile, many kv tiles): decoding and chunked prefill against long
+// cached keys.  The kernels above give every (q tile pair, query head, batch) one CTA that walks all its
+// keys: with N = 16 queries that is 16 of 256 rows in use, K and V read once per QUERY head, and one CTA
+// per head however long the keys are.  Here
+//   * a tile packs the query heads of a kv head next to one another (row = query * heads + head: one TMA
+//     box of heads x queries), so K and V are read once per kv head as long as the rows fit;
+//   * the kv list is cut into `splits` runs, one CTA each, so that the whole chip pulls on HBM;
+//   * inside a CTA the two softmax warpgroups take alternate kv tiles of the run (the same Q tile, two
+//     independent online softmaxes that ping-pong on the tensor core) and are merged in shared memory;
+//   * the runs' partial results go to a workspace, [unit, split, row] of HD floats and (max, sum), and
+//     fwd_combine_kernel weighs them together (or, with one split, the CTA writes O itself).
+// Bound by HBM: K and V once.  Measured, B = 4, 16 queries, 8192 keys, 32 / 8 heads of 128 (135 MB of
+// K and V): 33 + 4 us (4.1 TB/s) in 4 splits, against 128 us of the one-CTA-per-head kernel.
+// =================================================================================================
+enum {
+  SB_Q = 0, SB_S0, SB_S1, SB_P0, SB_P1, SB_O0, SB_O1, SB_SYNC, SB_K_FULL, SB_K_FREE = SB_K_FULL + 3, SB_V_FULL = SB_K_FREE + 3,
+  SB_V_FREE = SB_V_FULL + 2, SB_NUM = SB_V_FREE + 2
+};
+constexpr int kSplitKStages = 3, kSplitVStages = 2;
+
+template <int HD>
+struct __align__(1024) FwdSplitSmem {
+  uint8_t q[kTileBytesOf<HD>];
+  uint8_t k[kSplitKStages][kTileBytesOf<HD>];
+  uint8_t v[kSplitVStages][kTileBytesOf<HD>];
+  uint16_t merged[kMaxKvTiles];  // kv tile | partial << 15
+  uint8_t cls[kMaxKvTiles];
+  float ml[2][2][BM];            // running maximum (log2 units) and sum of the two warpgroups
+  uint64_t bar[SB_NUM];
+  uint32_t tmem_base;
+  int n_merged;
+};
+
+struct FwdSplitParams {
+  FwdParams f;
+  int heads;        // query heads packed into a tile (a divisor of the group: Hq / Hkv, or 1)
+  int tile_queries; // queries of a tile: 128 / heads rounded down
+  int q_tiles;      // tiles of one (head set, batch)
+  int splits;
+  float* part_o;    // [units, splits, 128, HD]
+  float2* part_ml;  // [units, splits, 128]
+};
+
+// Where row `row` of a unit's tile lives: unit = (b * head sets + head set) * q_tiles + tile.
+struct SplitRow { int b, h, q; bool valid; };
+__device__ __forceinline__ SplitRow split_row(const FwdSplitParams& p, int unit, int row) {
+  const int sets = p.f.a.Hq / p.heads;
+  const int tile = unit % p.q_tiles, set = (unit / p.q_tiles) % sets;
+  SplitRow r;
+  r.b = unit / (p.q_tiles * sets);
+  const int ql = row / p.heads;
+  r.h = set * p.heads + (row - ql * p.heads);
+  r.q = tile * p.tile_queries + ql;
+  r.valid = ql < p.tile_queries && r.q < p.f.a.N;
+  return r;
+}
+
+template <int HD, bool KB>
+__global__ void __launch_bounds__(kThreads, 1)
+fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                 const __grid_constant__ CUtensorMap map_v, const FwdSplitParams sp) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  constexpr uint32_t kTileBytes = kTileBytesOf<HD>;
+  FwdSplitSmem<HD>& sm = *reinterpret_cast<FwdSplitSmem<HD>*>(smem_raw);
+  const FwdParams& p = sp.f;
+  const bma_attn_args& a = p.a;
+  const int unit = blockIdx.x, split = blockIdx.y;
+  const SplitRow first = split_row(sp, unit, 0);
+  const int b = first.b, h0 = first.h, hk = h0 / (a.Hq / a.Hkv);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int wg = warp >> 2;
+  const int NKV = p.l.NKV;
+
+  if ((smem_u32(smem_raw) & 1023u) != 0u) {
+    if (threadIdx.x == 0) report_device_error(p.status, 151);
+    return;
+  }
+  // ---- kv list of the one listed q tile (head h0 stands for the set: the lists do not depend on the head where heads > 1)
+  for (int i = threadIdx.x; i < NKV; i += kThreads) sm.cls[i] = 0;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < SB_NUM; ++i) mbar_init(&sm.bar[i], (i == SB_P0 || i == SB_P1) ? 128 : (i == SB_SYNC ? 256 : 1));
+    fence_barrier_init();
+    prefetch_tensormap(&map_q);
+    mbar_expect_tx(&sm.bar[SB_Q], (uint32_t)(sp.heads * sp.tile_queries) * 128u * (HD / 64));
+#pragma unroll
+    for (int box = 0; box < HD / 64; ++box) tma_load_4d(sm.q + box * kHalfTile, &map_q, &sm.bar[SB_Q], box * 64, h0, first.q, b);
+  }
+  __syncthreads();
+  {
+    const int64_t lrow = (int64_t)(p.l.B == 1 ? 0 : b) * p.l.H + (p.l.H == 1 ? 0 : h0);   // NQ == 1
+    const int nfull = p.l.full_kv_num[lrow], npart = p.l.kv_num[lrow];
+    for (int i = threadIdx.x; i < nfull; i += kThreads) sm.cls[p.l.full_kv_idx[lrow * NKV + i]] = 2;
+    for (int i = threadIdx.x; i < npart; i += kThreads) sm.cls[p.l.kv_idx[lrow * NKV + i]] = 1;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int count = 0;
+    for (int base = 0; base < NKV; base += 32) {
+      const int j = base + lane;
+      const uint32_t c = j < NKV ? sm.cls[j] : 0;
+      const unsigned m = __ballot_sync(0xffffffffu, c != 0);
+      if (c) sm.merged[count + __popc(m & ((1u << lane) - 1))] = (uint16_t)((uint32_t)j | (c == 1 ? 0x8000u : 0u));
+      count += __popc(m);
+    }
+    if (lane == 0) sm.n_merged = count;
+  }
+  if (warp == 8) {
+    tmem_alloc(&sm.tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+  const int t0 = (int)((int64_t)sm.n_merged * split / sp.splits), T = (int)((int64_t)sm.n_merged * (split + 1) / sp.splits) - t0;
+  const uint16_t* list = sm.merged + t0;
+
+  if (wg == 2) {
+    setmaxnreg_dec_80();
+    if ((warp == 8 || warp == 10) && lane == 0) {
+      // ---------------------------------------------------------------- K (warp 8) and V (warp 10) tiles
+      const bool is_k = warp == 8;
+      const int stages = is_k ? kSplitKStages : kSplitVStages;
+      bool ok = true;
+      for (int n = 0; n < T && ok; ++n) {
+        const int st = n % stages;
+        uint64_t* full = &sm.bar[(is_k ? SB_K_FULL : SB_V_FULL) + st];
+        if (n >= stages) ok = mbar_wait(&sm.bar[(is_k ? SB_K_FREE : SB_V_FREE) + st], (n / stages - 1) & 1);
+        if (!ok) break;
+        mbar_expect_tx(full, kTileBytes);
+#pragma unroll
+        for (int box = 0; box < HD / 64; ++box)
+          tma_load_4d((is_k ? sm.k[st] : sm.v[st]) + box * kHalfTile, is_k ? &map_k : &map_v, full, box * 64, hk, (int)(list[n] & 0x7fffu) * BN, b);
+      }
+      if (!ok) report_device_error(p.status, 160);
+    } else if (warp == 9 && T > 0) {
+      // ---------------------------------------------------------------- MMA issue (whole warp, one elected lane issues)
+      const bool leader = elect_one();
+      constexpr uint32_t idesc_s = make_idesc_bf16(BM, BN, 0, 0);
+      constexpr uint32_t idesc_o = make_idesc_bf16(BM, HD, 0, 1);
+      const uint64_t dq = make_smem_desc(smem_u32(sm.q), 16, 1024), dk0 = make_smem_desc(smem_u32(sm.k), 16, 1024);
+      const uint64_t dv0 = make_smem_desc(smem_u32(sm.v), kHalfTile, 1024);
+      constexpr uint32_t kStageUnits = kTileBytes >> 4;
+      auto issue_s = [&](int n) -> bool {   // tile n of the run belongs to warpgroup n & 1
+        const int st = n % kSplitKStages;
+        if (!mbar_wait(&sm.bar[SB_K_FULL + st], (n / kSplitKStages) & 1)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t off = ((ks >> 2) * kHalfTile + (ks & 3) * 32) >> 4;
+          if (leader) mma_ss(tmem + (n & 1) * 128, dq + off, dk0 + (uint32_t)(st * kStageUnits + off), idesc_s, ks > 0);
+        }
+        if (leader) { mma_commit(&sm.bar[SB_S0 + (n & 1)]); mma_commit(&sm.bar[SB_K_FREE + st]); }
+        return true;
+      };
+      bool ok = mbar_wait(&sm.bar[SB_Q], 0) && issue_s(0);
+      if (ok && T > 1) ok = issue_s(1);
+      for (int n = 0; n < T && ok; ++n) {
+        const int x = n & 1, st = n % kSplitVStages;
+        ok = mbar_wait(&sm.bar[SB_V_FULL + st], (n / kSplitVStages) & 1) && mbar_wait(&sm.bar[SB_P0 + x], (n >> 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)
+          if (leader)
+            mma_ts(tmem + 256 + x * 128, tmem + x * 128 + ks * 8, dv0 + (uint32_t)(st * kStageUnits + ks * (2048 >> 4)), idesc_o, (n > 1) || (ks > 0));
+        if (leader) { mma_commit(&sm.bar[SB_O0 + x]); mma_commit(&sm.bar[SB_V_FREE + st]); }
+        if (n + 2 < T) ok = issue_s(n + 2);   // overwrites the P that the MMAs above read
+      }
+      if (!ok && leader) report_device_error(p.status, 161);
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax warpgroups
+    setmaxnreg_inc_208();
+    const int x = wg, row = threadIdx.x & 127;
+    const SplitRow r = split_row(sp, unit, row);
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tmem_s = tmem + x * 128 + lane_base, tmem_o = tmem + 256 + x * 128 + lane_base;
+    const float kb2 = (KB && a.key_bias) ? __ldg(a.key_bias + min(r.h, a.Hq - 1)) * kLog2e : 0.f;
+    float m_ref = -INFINITY, l = 0.f;
+    bool ok = true;
+    int cnt = 0;
+    for (int n = x; n < T; n += 2, ++cnt) {
+      const uint32_t e = list[n];
+      const int k0 = (int)(e & 0x7fffu) * BN;
+      uint32_t bits[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+      if (e & 0x8000u) {
+        const MaskView mv = make_mask_view(p.spec, b, min(r.h, a.Hq - 1));
+        int jlo, jhi;
+        row_interval(mv, r.valid ? r.q : a.N, k0, jlo, jhi);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int lo = max(jlo - c * 32, 0), hi = min(jhi - c * 32, 31);
+          bits[c] = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
+          if (bits[c] && (mv.flags & kTableTerms)) bits[c] &= table_bits_row32(mv, r.q, k0 + c * 32);
+        }
+      }
+      ok = mbar_wait(&sm.bar[SB_S0 + x], cnt & 1);
+      if (!ok) break;
+      tc_fence_after();
+      float s[BN];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t v[32];
+        tmem_ld32(tmem_s + c * 32, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) s[c * 32 + j] = __uint_as_float(v[j]);
+      }
+      const float sc = KB ? 1.f : p.scale_log2;
+      if constexpr (KB) {
+        const float base = kb2 * (float)(p.spec.k_offset + k0);
+#pragma unroll
+        for (int j = 0; j < BN; ++j) s[j] = fmaf(s[j], p.scale_log2, fmaf((float)j, kb2, base));
+      }
+      if (e & 0x8000u) {
+#pragma unroll
+        for (int j = 0; j < BN; ++j) s[j] = (bits[j >> 5] >> (j & 31)) & 1u ? s[j] : -INFINITY;
+      }
+      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < BN; j += 8) {
+        mx0 = max3(mx0, s[j], s[j + 1]);
+        mx1 = max3(mx1, s[j + 2], s[j + 3]);
+        mx2 = max3(mx2, s[j + 4], s[j + 5]);
+        mx3 = max3(mx3, s[j + 6], s[j + 7]);
+      }
+      const float m_cand = fmaxf(m_ref, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * sc);
+      const bool grow = (m_cand - m_ref) > kRescaleThreshold;
+      float alpha = 1.f;
+      if (grow) {
+        alpha = ex2(m_ref - m_cand);
+        m_ref = m_cand;
+      }
+      if (cnt > 0 && __any_sync(0xffffffffu, grow)) {
+        ok = mbar_wait(&sm.bar[SB_O0 + x], (cnt - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < HD / 32; ++c) {
+          uint32_t v[32];
+          tmem_ld32(tmem_o + c * 32, v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * alpha);
+          tmem_st32(tmem_o + c * 32, v);
+        }
+      }
+      const float m_sub = (m_ref == -INFINITY) ? 0.f : m_ref;
+      float row_sum = 0.f;
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) {
+        uint32_t pk[16];
+        row_sum += exp_part<16>(&s[ch * 32], sc, m_sub, pk);
+        tmem_st16(tmem_s + ch * 16, pk);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[SB_P0 + x]);
+      l = l * alpha + row_sum;
+    }
+    if (ok && cnt > 0) ok = mbar_wait(&sm.bar[SB_O0 + x], (cnt - 1) & 1);
+    if (ok) ok = mbar_wait(&sm.bar[SB_Q], 0);   // (a run without tiles: let the Q load land before its CTA ends)
+    tc_fence_after();
+    if (m_ref == -INFINITY) l = 0.f;            // no allowed key (the polynomial exponential of a masked score is 2^-126, not 0)
+
+    // ---- merge of the two warpgroups through shared memory (after the first rendezvous no MMA reads K or V any more)
+    sm.ml[x][0][row] = m_ref;
+    sm.ml[x][1][row] = l;
+    uint32_t syncs = 0;
+    auto rendezvous = [&]() {
+      mbar_arrive(&sm.bar[SB_SYNC]);
+      ok = mbar_wait(&sm.bar[SB_SYNC], syncs & 1) && ok;
+      ++syncs;
+    };
+    rendezvous();
+    const float mo = sm.ml[x ^ 1][0][row], lo = sm.ml[x ^ 1][1][row];
+    const float mt = fmaxf(m_ref, mo), ms = (mt == -INFINITY) ? 0.f : mt;
+    const float fx = ex2(m_ref - ms), lt = l * fx + lo * ex2(mo - ms);
+    // with several splits the partial stays unnormalised, relative to its own maximum
+    const float mine = cnt > 0 && l > 0.f ? (sp.splits == 1 ? fx / lt : fx) : 0.f;
+    constexpr int kPitch = HD + 4;
+    float* stage = reinterpret_cast<float*>(sm.k[0]) + row * kPitch;
+    for (int turn = 0; turn < 2; ++turn) {
+      if (turn == x) {
+#pragma unroll
+        for (int c = 0; c < HD / 32; ++c) {
+          uint32_t v[32];
+          if (cnt > 0) {
+            tmem_ld32(tmem_o + c * 32, v);
+            tmem_wait_ld();
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = 0u;
+          }
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            float4 o4 = turn == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<float4*>(stage + c * 32 + j);
+            o4.x = fmaf(__uint_as_float(v[j]), mine, o4.x); o4.y = fmaf(__uint_as_float(v[j + 1]), mine, o4.y);
+            o4.z = fmaf(__uint_as_float(v[j + 2]), mine, o4.z); o4.w = fmaf(__uint_as_float(v[j + 3]), mine, o4.w);
+            *reinterpret_cast<float4*>(stage + c * 32 + j) = o4;
+          }
+        }
+      }
+      rendezvous();
+    }
+    if (!ok) {
+      report_device_error(p.status, 170 + warp);
+    } else {
+      if (x == 0 && r.valid) {
+        if (sp.splits > 1) sp.part_ml[((int64_t)unit * sp.splits + split) * BM + row] = make_float2(mt, lt);
+        else if (a.lse) a.lse[((int64_t)b * a.Hq + r.h) * a.N + r.q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
+      }
+      // a warp per row: whole lines of O or of the partial
+      for (int i = warp; i < BM; i += 8) {
+        const SplitRow ri = split_row(sp, unit, i);
+        if (!ri.valid) continue;
+        const float* src = reinterpret_cast<const float*>(sm.k[0]) + i * kPitch;
+        if (sp.splits > 1) {
+          float* dst = sp.part_o + (((int64_t)unit * sp.splits + split) * BM + i) * HD;
+          if (lane < HD / 4) reinterpret_cast<float4*>(dst)[lane] = reinterpret_cast<const float4*>(src)[lane];
+        } else if (lane < HD / 4) {
+          const float4 o4 = reinterpret_cast<const float4*>(src)[lane];
+          const int64_t off = (int64_t)b * a.o.stride_b + (int64_t)ri.q * a.o.stride_l + (int64_t)ri.h * a.o.stride_h + lane * 4;
+          if (a.o.dtype == BMA_DTYPE_F32) *reinterpret_cast<float4*>(static_cast<float*>(a.o.ptr) + off) = o4;
+          else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.o.ptr) + off) = make_uint2(pack_bf16(o4.x, o4.y), pack_bf16(o4.z, o4.w));
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+}
+
+// One warp per (unit, row): O = sum over the splits of 2^(m_s - m) O_s / sum of 2^(m_s - m) l_s, and the log-sum-exp.
+template <int HD>
+__global__ void __launch_bounds__(256) fwd_combine_kernel(const FwdSplitParams sp, int units) {
+  const bma_attn_args& a = sp.f.a;
+  const int lane = threadIdx.x & 31;
+  const int rows = sp.heads * sp.tile_queries;
+  const int w = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (w >= units * rows) return;
+  const int unit = w / rows, row = w - unit * rows;
+  const SplitRow r = split_row(sp, unit, row);
+  if (!r.valid) return;
+  const float2* ml = sp.part_ml + (int64_t)unit * sp.splits * BM + row;
+  float m = -INFINITY;
+  for (int s = lane; s < sp.splits; s += 32) m = fmaxf(m, ml[s * BM].x);
+  for (int off = 16; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  const float ms = m == -INFINITY ? 0.f : m;
+  float l = 0.f;
+  for (int s = lane; s < sp.splits; s += 32) {
+    const float2 v = ml[s * BM];
+    l += v.y * ex2(v.x - ms);
+  }
+  for (int off = 16; off; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+  if (lane == 0 && a.lse) a.lse[((int64_t)r.b * a.Hq + r.h) * a.N + r.q] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
+  if (lane >= HD / 4) return;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4* src = reinterpret_cast<const float4*>(sp.part_o + ((int64_t)unit * sp.splits * BM + row) * HD) + lane;
+#pragma unroll 4
+  for (int s = 0; s < sp.splits; ++s) {
+    const float f = ex2(ml[s * BM].x - ms) * inv;
+    const float4 v = src[(int64_t)s * BM * (HD / 4)];
+    acc.x = fmaf(v.x, f, acc.x); acc.y = fmaf(v.y, f, acc.y); acc.z = fmaf(v.z, f, acc.z); acc.w = fmaf(v.w, f, acc.w);
+  }
+  const int64_t off = (int64_t)r.b * a.o.stride_b + (int64_t)r.q * a.o.stride_l + (int64_t)r.h * a.o.stride_h + lane * 4;
+  if (a.o.dtype == BMA_DTYPE_F32) *reinterpret_cast<float4*>(static_cast<float*>(a.o.ptr) + off) = acc;
+  else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.o.ptr) + off) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
+}
+
 }  // namespace
 
 // ---- host ------------------------------------------------------------------------------------
@@ -1085,12 +1460,12 @@ static EncodeTiledFn encode_fn() {
 }
 
 int make_tile_map_bf16(CUtensorMap* out, const void* base, int B, int L, int H, int d, int64_t stride_b,
-                       int64_t stride_l, int64_t stride_h, int box_rows) {
+                       int64_t stride_l, int64_t stride_h, int box_rows, int box_heads) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) { set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled entry point"); return BMA_ERR_CUDA; }
   const cuuint64_t dims[4] = {(cuuint64_t)d, (cuuint64_t)H, (cuuint64_t)L, (cuuint64_t)B};
   const cuuint64_t strides[3] = {(cuuint64_t)stride_h * 2, (cuuint64_t)stride_l * 2, (cuuint64_t)stride_b * 2};
-  const cuuint32_t box[4] = {64, 1, (cuuint32_t)box_rows, 1};
+  const cuuint32_t box[4] = {64, (cuuint32_t)box_heads, (cuuint32_t)box_rows, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1175,7 +1550,67 @@ bool sm100_supported(const bma_attn_args& a) {
          ceil_div(a.L, BN) <= kMaxKvTiles;
 }
 
-int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st) {
+// How the split kernel cuts a call, or splits == 0 where it does not take it: one listed q tile and at least two kv tiles.
+// A unit is a tile of packed rows of one (head set, batch); heads are packed when that makes fewer tiles than one per head
+// and the lists are the same for the heads of a group.  The number of splits minimises waves x (run of tiles + set-up): a
+// tile of K and V takes about 1.5 us at an SM's share of the HBM rate, set-up, merge and a workspace round trip about 5.
+struct SplitPlan { int heads, tile_queries, q_tiles, units, splits; };
+static SplitPlan split_plan(const bma_attn_args& a, const bma_block_lists& l) {
+  SplitPlan p{1, BM, 1, 0, 0};
+  if (l.NQ != 1 || l.NKV < 2 || a.N > BM) return p;
+  const int G = a.Hq / a.Hkv;
+  if (G > 1 && G <= BM && l.H == 1 && ceil_div(a.N, BM / G) < G) {
+    p.heads = G;
+    p.tile_queries = std::min(BM / G, a.N);
+    p.q_tiles = ceil_div(a.N, p.tile_queries);
+  }
+  const int64_t units = (int64_t)a.B * (a.Hq / p.heads) * p.q_tiles;
+  if (units > (1 << 20)) return p;
+  p.units = (int)units;
+  double best = 1e30;
+  for (int s = 1; s <= std::min(l.NKV / 2, 148); ++s) {
+    const double cost = std::ceil((double)units * s / 148.0) * (std::ceil((double)l.NKV / s) * 1.5 + 5.0) + (s > 1 ? 3.0 : 0.0);
+    if (cost < best) { best = cost; p.splits = s; }
+  }
+  return p;
+}
+
+size_t sm100_fwd_workspace_bytes(const bma_attn_args& a, const bma_block_lists& lists) {
+  const SplitPlan p = split_plan(a, lists);
+  return p.splits > 1 ? (size_t)p.units * p.splits * BM * (a.d + 2) * sizeof(float) : 0;
+}
+
+static int sm100_fwd_split(const bma_attn_args& a, const FwdParams& f, const SplitPlan& plan, const CUtensorMap& mk, const CUtensorMap& mv,
+                           void* ws, bool kb, cudaStream_t st) {
+  CUtensorMap mq;
+  int rc = make_tile_map_bf16(&mq, a.q.ptr, a.B, a.N, a.Hq, a.d, a.q.stride_b, a.q.stride_l, a.q.stride_h, plan.tile_queries, plan.heads);
+  if (rc) return rc;
+  FwdSplitParams p;
+  p.f = f;
+  p.heads = plan.heads; p.tile_queries = plan.tile_queries; p.q_tiles = plan.q_tiles; p.splits = plan.splits;
+  p.part_o = static_cast<float*>(ws);
+  p.part_ml = reinterpret_cast<float2*>(p.part_o + (size_t)plan.units * plan.splits * BM * a.d);
+  auto launch = [&](auto kernel, size_t smem) -> int {
+    BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<dim3(plan.units, plan.splits), kThreads, smem, st>>>(mq, mk, mv, p);
+    return BMA_OK;
+  };
+  if (a.d == 128) rc = kb ? launch(fwd_split_kernel<128, true>, sizeof(FwdSplitSmem<128>)) : launch(fwd_split_kernel<128, false>, sizeof(FwdSplitSmem<128>));
+  else rc = kb ? launch(fwd_split_kernel<64, true>, sizeof(FwdSplitSmem<64>)) : launch(fwd_split_kernel<64, false>, sizeof(FwdSplitSmem<64>));
+  if (rc) return rc;
+  count_launches(1);
+  if (plan.splits > 1) {
+    const int64_t rows = (int64_t)plan.units * plan.heads * plan.tile_queries;
+    const unsigned grid = (unsigned)((rows + 7) / 8);
+    if (a.d == 128) fwd_combine_kernel<128><<<grid, 256, 0, st>>>(p, plan.units);
+    else fwd_combine_kernel<64><<<grid, 256, 0, st>>>(p, plan.units);
+    count_launches(1);
+  }
+  BMA_CUDA_TRY(cudaGetLastError());
+  return BMA_OK;
+}
+
+int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, size_t ws_bytes, cudaStream_t st) {
   BMA_REQUIRE(lists.q_block == BM && lists.kv_block == BN, BMA_ERR_ARG);
   BMA_REQUIRE(lists.NKV <= kMaxKvTiles, BMA_ERR_LIMIT);
   BMA_REQUIRE(a.o.dtype == BMA_DTYPE_F32 || a.o.dtype == BMA_DTYPE_BF16, BMA_ERR_UNSUPPORTED);
@@ -1198,6 +1633,9 @@ int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
   const bool kb = a.key_bias != nullptr || a.scale < 0.f;
+  const SplitPlan split = split_plan(a, lists);
+  if (split.splits == 1 || (split.splits > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_bytes >= sm100_fwd_workspace_bytes(a, lists)))
+    return sm100_fwd_split(a, p, split, mk, mv, ws, kb, st);
   if (fwd_persistent_enabled(spec)) {
     // One CTA per SM for the whole launch; items are drawn from a counter that is zeroed on the stream first.
     int dev = 0, sms = 148;

@@ -333,8 +333,18 @@ int bma_attn_bwd_plan(const bma_attn_args* args, int32_t* backend, int32_t* q_ti
   return BMA_OK;
 }
 
+size_t bma_attn_fwd_workspace_bytes(const bma_attn_args* args, const bma_block_lists* lists) {
+  if (validate_common(args) != BMA_OK || !lists || pick_backend(args) != BMA_BACKEND_TCGEN05) return 0;
+  return sm100_fwd_workspace_bytes(*args, *lists);
+}
+
 int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
                  bma_stream_t stream) {
+  return bma_attn_fwd_ws(args, spec, lists, nullptr, 0, stream);
+}
+
+int bma_attn_fwd_ws(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+                    size_t workspace_bytes, bma_stream_t stream) {
   int rc = validate_common(args);
   if (rc != BMA_OK) return rc;
   BMA_REQUIRE(spec != nullptr, BMA_ERR_ARG);
@@ -348,7 +358,7 @@ int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma
   if ((rc = validate_lists(args, lists, tile, false))) return rc;
   BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return be == BMA_BACKEND_TCGEN05 ? sm100_fwd(*args, *spec, *lists, st) : simt_fwd(*args, *spec, *lists, st);
+  return be == BMA_BACKEND_TCGEN05 ? sm100_fwd(*args, *spec, *lists, workspace, workspace_bytes, st) : simt_fwd(*args, *spec, *lists, st);
 }
 
 size_t bma_attn_f32_workspace_bytes(const bma_attn_args* args, int32_t backward) {

@@ -268,8 +268,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 // ---- host side: tensor map creation through the runtime's driver entry point ---------------
 // Encodes a 4-D bf16 tensor map over a [B, L, H, d] tensor (d innermost) with a
-// (64 x 1 x rows x 1) box and 128-byte swizzle: one box is a [rows x 64] K-major operand tile.
+// (64 x heads x rows x 1) box and 128-byte swizzle: one box is a [rows * heads x 64] K-major operand tile.
 int make_tile_map_bf16(CUtensorMap* out, const void* base, int B, int L, int H, int d, int64_t stride_b,
-                       int64_t stride_l, int64_t stride_h, int box_rows);
+                       int64_t stride_l, int64_t stride_h, int box_rows, int box_heads = 1);
 
 }  // namespace bma
