@@ -9,22 +9,25 @@
 // 128x128x128 MMAs:
 //     St  = K Q^T            A = K (K-major),  B = Q  (K-major)      -> TMEM [256,384)
 //     dPt = V dO^T           A = V (K-major),  B = dO (K-major)      -> TMEM [384,512)
-//     dV += Pt dO            A = Pt (bf16 in TMEM, over dPt),  B = dO (MN-major) -> TMEM [0,128)
+//     dV += Pt dO            A = Pt (bf16 in TMEM, over St),   B = dO (MN-major) -> TMEM [0,128)
 //     dK += dSt Q            A = dSt (bf16 in TMEM, over dPt), B = Q  (MN-major) -> TMEM [128,256)
-// with Pt = exp2(St*scale*log2e - lse*log2e) and dSt = Pt * (dPt - delta) computed by eight warps
-// (thread = key row; warps w and w+4 split the 128 query columns).
+// with Pt = exp2(St*scale*log2e - lse*log2e) and dSt = Pt * (dPt - delta) computed by sixteen warps
+// (thread = key row; the four warpgroups split the 128 query columns, 32 each).
 //
-// Pipelining: the consumers pull St into registers and release its columns at once, so the next
-// tile's K Q^T runs under the element-wise math, and they compute the exponentials of tile n+1
-// while the MMAs of tile n run.  Each thread writes its Pt and dSt (bf16) over dPt columns that it
-// has itself just read — the 64 fp32 columns of its half hold 32 packed columns of Pt and 32 of dSt
-// — so the consumers never wait for one another, nor for a buffer, inside a tile; the next V dO^T
-// is issued behind the two accumulations (MMAs of one issuing thread execute in order).
-// Warp 10 stages lse*log2e and delta of the coming q tiles in shared memory.
+// Pipelining: MMA order  dV(n) St(n+1) dK(n) dPt(n+1).  Pt and dSt are handed over separately, so dV and the next St run while
+// the consumers work on dSt, and dK and the next dPt while they stage dSt and take the exponentials of tile n+1.  Each thread
+// writes its Pt and dSt (bf16) over St / dPt columns that it has itself just read, so the consumers never wait for one
+// another, nor for a buffer, inside a tile; what overwrites an operand is issued behind the MMAs that read it (MMAs of one
+// issuing thread execute in order).  One warp stages lse*log2e and delta of the coming q tiles in shared memory.
+// Sixteen warps (four per scheduler, 104 registers each) hide the latencies of tensor memory loads, exponentials and barriers
+// that eight warps of 208 registers left open.  Eight warps with one hand-over of Pt and dSt together -> eight with two ->
+// sixteen with two: packed documents (B=4 L=16384 H=16 d=128) 1960 -> 1865 -> 1730 us, lambda window 2 x 1000 48 -> 44 ->
+// 38 us, sliding window L=8192 464 -> 453 -> 437 us, causal d=64 (B=4 L=4096 H=32) 898 -> 840 -> 848 us; causal B=8 L=4096
+// H=32 d=128 is at the power limit (about 1.5 GHz) and stays at 2160 us.
 //
 // With a scratch buffer (BwdParams::ds_out) the kernel also hands every dSt tile to the dQ kernel:
-// each consumer thread stages its 64 dSt values as one 128-byte line of a 32 KB tile image laid out
-// like a 128-byte-swizzled MMA operand in shared memory, warp 11 sends the image to its slot with one
+// each consumer thread stages its 32 dSt values as half of a 128-byte line of a 32 KB tile image laid out
+// like a 128-byte-swizzled MMA operand in shared memory, one warp sends the image to its slot with one
 // bulk store, and dQ += dS K then needs no recomputation of S and dP (5 instead of 7 MMAs per block
 // for the whole backward, paid with 32 KB of HBM traffic each way).
 // Every mbarrier wait is bounded; on a timeout the thread records an error code and unwinds.
@@ -32,23 +35,6 @@
 
 #include "common.cuh"
 #include "ptx_sm100.cuh"
-
-// Element-wise math of the dK/dV kernel:
-//   0: scalar arithmetic, every exponential on the MUFU pipe
-//   1: the packed two-wide FP32 instructions of sm_100 (fma / add / mul .f32x2) for the scale-and-shift and for
-//      dS = P * (dP - delta); every exponential on the MUFU pipe
-//   2: as 1, and a quarter of the exponentials as a packed polynomial on the FMA pipe
-//   3: packed scale-and-shift with the polynomial quarter, scalar dS;  4: scalar exponentials, packed dS;  5: packed scale-and-shift only
-// Measured on config 2 / the L=8192 shape (same box): 0: 2.127 / 4.238 ms, 1: 2.233 / 4.366 ms, 2: 2.216 / 4.216 ms -- the
-// kernel is bound by shared-memory operand traffic (2 560 cycles per tile at 128 B/clk), not by instruction issue, so 0.
-#ifndef BMA_DKDV_MATH
-#define BMA_DKDV_MATH 0
-#endif
-#define BMA_DKDV_PACKED_EXP (BMA_DKDV_MATH == 1 || BMA_DKDV_MATH == 2 || BMA_DKDV_MATH == 3 || BMA_DKDV_MATH == 5)
-#define BMA_DKDV_PACKED_DS (BMA_DKDV_MATH == 1 || BMA_DKDV_MATH == 2 || BMA_DKDV_MATH == 4)
-#ifndef BMA_DKDV_POLY
-#define BMA_DKDV_POLY 0  // scalar polynomial (BMA_DKDV_MATH 0 only); measured 3.87 ms against 3.78 ms for the whole backward, so off
-#endif
 
 namespace bma {
 
@@ -62,17 +48,23 @@ namespace {
 using namespace ptx;
 
 constexpr int BT = kSm100Tile;  // the head dimension HD (64 or 128) is a template parameter
-constexpr int kConsumers = 256;
-constexpr int kThreads = kConsumers + 128;  // + one warpgroup: warp 8 TMA, warp 9 MMA issue, warp 10 row statistics, warp 11 dSt hand-over
+constexpr int kCols = 32;                     // query columns of a tile per consumer thread
+constexpr int kParts = BT / kCols;
+constexpr int kConsumers = 128 * kParts;
+constexpr int kThreads = kConsumers + 128;   // + one warpgroup of single-warp roles:
+constexpr int kWarpTma = kConsumers / 32, kWarpMma = kWarpTma + 1, kWarpStat = kWarpTma + 2, kWarpHand = kWarpTma + 3;
+// Tensor memory column (of St or dPt) of the packed Pt / dSt values of 16-query step ks: a thread packs its 32 columns into
+// the first 16 of them.
+__device__ constexpr uint32_t packed_col(int ks) { return (uint32_t)((ks >> 1) * kCols + (ks & 1) * 8); }
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kHalfTile = BT * 64 * 2;
 template <int HD> constexpr uint32_t kTileBytesOf = (HD / 64) * kHalfTile;  // a [128 x HD] operand tile
 constexpr uint32_t kDsBytes = 2 * kHalfTile;  // dSt: [128 keys x 128 queries]
-constexpr uint32_t COL_DV = 0, COL_DK = 128, COL_ST = 256, COL_DPT = 384, COL_PT = 384;
+constexpr uint32_t COL_DV = 0, COL_DK = 128, COL_ST = 256, COL_DPT = 384;
 
 enum {
   BAR_KV = 0, BAR_FULLQ0, BAR_FULLQ1, BAR_FULLDO0, BAR_FULLDO1, BAR_STAT0, BAR_STAT1,
-  BAR_S1, BAR_S2, BAR_LS, BAR_P, BAR_QF, BAR_D, BAR_SYNC2, BAR_STG, BAR_DSR,
+  BAR_S1, BAR_S2, BAR_P, BAR_DS, BAR_DK0, BAR_DK1, BAR_DV0, BAR_DV1, BAR_SYNC2, BAR_STG, BAR_DSR,
   NUM_BARS
 };
 
@@ -112,8 +104,9 @@ __device__ __forceinline__ bool consumer_sync(uint64_t* bar, uint32_t parity) {
   return mbar_wait(bar, parity);
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void setmaxnreg_inc_208() { asm volatile("setmaxnreg.inc.sync.aligned.u32 208;"); }
-__device__ __forceinline__ void setmaxnreg_dec_80() { asm volatile("setmaxnreg.dec.sync.aligned.u32 80;"); }
+// 640 threads start with 96 registers each: 512 x 104 + 128 x 64 is the same sum
+__device__ __forceinline__ void setmaxnreg_inc_consumers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 104;"); }
+__device__ __forceinline__ void setmaxnreg_dec_roles() { asm volatile("setmaxnreg.dec.sync.aligned.u32 64;"); }
 
 template <int HD, bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -139,7 +132,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (threadIdx.x == 0) {
     for (int i = 0; i < NUM_BARS; ++i) {
       uint32_t count = 1;
-      if (i == BAR_LS || i == BAR_P || i == BAR_SYNC2 || i == BAR_STG) count = kConsumers;
+      if (i == BAR_P || i == BAR_DS || i == BAR_SYNC2 || i == BAR_STG) count = kConsumers;
       if (i == BAR_STAT0 || i == BAR_STAT1) count = 32;
       mbar_init(&sm.bar[i], count);
     }
@@ -163,7 +156,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int64_t row = ((int64_t)lb * p.l.H + lh) * p.l.NKV + kj;
     total += p.l.full_q_num[row] + p.l.q_num[row];
   }
-  if (warp == 8) {
+  if (warp == kWarpTma) {
     tmem_alloc(&sm.tmem_base, kTmemCols);
     tmem_relinquish();
   }
@@ -172,9 +165,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
 
-  if (warp >= 8) {
-    setmaxnreg_dec_80();
-    if (warp == 8 && lane == 0 && total > 0) {
+  if (warp >= kWarpTma) {
+    setmaxnreg_dec_roles();
+    if (warp == kWarpTma && lane == 0 && total > 0) {
       // ---------------------------------------------------------------- TMA producer
       prefetch_tensormap(&map_q);
       prefetch_tensormap(&map_do);
@@ -188,20 +181,20 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         int h, qi; bool partial;
         loader.next(h, qi, partial);
         const int st = n & 1;
-        // The Q stage is free once dK += dSt Q of tile n-2 has completed (BAR_QF of n-2 has the parity of n), the dO
-        // stage once dV += Pt dO has (BAR_D).  dK is issued first: Q is the operand the next tile needs first (K Q^T),
-        // and its load is the one whose latency the two-stage ring barely covers.
-        if (n >= 2) ok = mbar_wait(&sm.bar[BAR_QF], n & 1);
+        // The Q stage is free once dK += dSt Q of tile n-2 has completed, the dO stage once dV += Pt dO has.  (One barrier
+        // per stage: its next phase needs the load that this thread has not issued yet, so a phase cannot be missed.)
+        // Q first: it is the operand the next tile needs first (K Q^T), and the one whose load the ring barely covers.
+        if (n >= 2) ok = mbar_wait(&sm.bar[BAR_DK0 + st], ((n >> 1) - 1) & 1);
         if (!ok) break;
         mbar_expect_tx(&sm.bar[BAR_FULLQ0 + st], kTileBytes);
         load_tile(&map_q, sm.q[st], &sm.bar[BAR_FULLQ0 + st], h, qi * BT);
-        if (n >= 2) ok = mbar_wait(&sm.bar[BAR_D], n & 1);
+        if (n >= 2) ok = mbar_wait(&sm.bar[BAR_DV0 + st], ((n >> 1) - 1) & 1);
         if (!ok) break;
         mbar_expect_tx(&sm.bar[BAR_FULLDO0 + st], kTileBytes);
         load_tile(&map_do, sm.d_o[st], &sm.bar[BAR_FULLDO0 + st], h, qi * BT);
       }
       if (!ok) report_device_error(p.status, 305);
-    } else if (warp == 9 && total > 0) {
+    } else if (warp == kWarpMma && total > 0) {
       // ---------------------------------------------------------------- MMA issuer: the whole warp runs the loop
       // (warp-uniform control flow and descriptors), one elected lane issues the tcgen05 instructions.  A loop run
       // by lane 0 alone costs ~60-70 cycles of issue per MMA under load — no slack against the 64 cycles an MMA takes.
@@ -239,29 +232,32 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       for (int n = 0; n < total && ok; ++n) {
         const int st = n & 1;
         const uint32_t ph = n & 1;
-        // St columns are free as soon as the consumers hold them in registers
-        ok = mbar_wait(&sm.bar[BAR_LS], ph);
-        if (ok && n + 1 < total) {
-          ok = mbar_wait(&sm.bar[BAR_FULLQ0 + (st ^ 1)], ((n + 1) >> 1) & 1);
-          if (ok) { tc_fence_after(); gemm_st(st ^ 1); }
-        }
-        if (ok) ok = mbar_wait(&sm.bar[BAR_P], ph);
+        ok = mbar_wait(&sm.bar[BAR_P], ph);
         if (!ok) break;
         tc_fence_after();
-        // dK += dSt Q      (A = dSt from TMEM: 8 columns per 16-query k-step, in the second 32 of the half's 64 dPt columns)
+        // dV += Pt dO      (A from TMEM, 8 columns per 16-query k-step; B = dO rows as K)
 #pragma unroll
         for (int ks = 0; ks < BT / 16; ++ks)
           if (leader)
-            mma_ts(tmem + COL_DK, tmem + COL_PT + (ks >> 2) * 64 + 32 + (ks & 3) * 8, dqm0 + (uint32_t)(st * kStageUnits + ks * (2048 >> 4)), idesc_kn, (n > 0) || (ks > 0));
-        if (leader) mma_commit(&sm.bar[BAR_QF]);  // the Q stage is free
-        // dV += Pt dO      (A from TMEM, 8 columns per 16-query k-step — the Pt of queries [64h, 64h+64) sits in the first 32
-        // of the 64 dPt columns its warps read; B = dO rows as K)
+            mma_ts(tmem + COL_DV, tmem + COL_ST + packed_col(ks), ddom0 + (uint32_t)(st * kStageUnits + ks * (2048 >> 4)), idesc_kn, (n > 0) || (ks > 0));
+        if (leader) mma_commit(&sm.bar[BAR_DV0 + st]);
+        // the next St overwrites the columns Pt was read from; it is queued behind dV += Pt dO
+        if (n + 1 < total) {
+          ok = mbar_wait(&sm.bar[BAR_FULLQ0 + (st ^ 1)], ((n + 1) >> 1) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          gemm_st(st ^ 1);
+        }
+        ok = mbar_wait(&sm.bar[BAR_DS], ph);
+        if (!ok) break;
+        tc_fence_after();
+        // dK += dSt Q
 #pragma unroll
         for (int ks = 0; ks < BT / 16; ++ks)
           if (leader)
-            mma_ts(tmem + COL_DV, tmem + COL_PT + (ks >> 2) * 64 + (ks & 3) * 8, ddom0 + (uint32_t)(st * kStageUnits + ks * (2048 >> 4)), idesc_kn, (n > 0) || (ks > 0));
-        if (leader) mma_commit(&sm.bar[BAR_D]);
-        // the next dPt overwrites the columns Pt was read from; it is queued behind dV += Pt dO
+            mma_ts(tmem + COL_DK, tmem + COL_DPT + packed_col(ks), dqm0 + (uint32_t)(st * kStageUnits + ks * (2048 >> 4)), idesc_kn, (n > 0) || (ks > 0));
+        if (leader) mma_commit(&sm.bar[BAR_DK0 + st]);
+        // the next dPt overwrites the columns dSt was read from; it is queued behind dK += dSt Q
         if (n + 1 < total) {
           ok = mbar_wait(&sm.bar[BAR_FULLDO0 + (st ^ 1)], ((n + 1) >> 1) & 1);
           if (!ok) break;
@@ -270,7 +266,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
       }
       if (!ok && leader) report_device_error(p.status, 310);
-    } else if (warp == 10 && total > 0) {
+    } else if (warp == kWarpStat && total > 0) {
       // ---------------------------------------------------------------- row statistics of the coming q tiles
       QTileIter loader(p.l, b, hk, G, kj);
       bool ok = true;
@@ -278,8 +274,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         int h, qi; bool partial;
         loader.next(h, qi, partial);
         const int st = n & 1;
-        // the stage was last read while tile n-2 was processed (BAR_D of n-2 has the parity of n)
-        if (n >= 2) ok = mbar_wait(&sm.bar[BAR_D], n & 1);
+        // the stage was last read for dSt of tile n-2, which its dK waited for
+        if (n >= 2) ok = mbar_wait(&sm.bar[BAR_DK0 + st], ((n >> 1) - 1) & 1);
         if (!ok) break;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -288,22 +284,13 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           const int64_t off = ((int64_t)b * a.Hq + h) * a.N + q;
           const float lv = q < a.N ? __ldg(a.lse + off) : -INFINITY;
           // +inf for rows that attend nothing or lie outside: their probabilities become exactly 0
-          // the packed forms add: -lse2 (and -inf for a dead row) and -delta are what is staged for them
-#if BMA_DKDV_PACKED_EXP
-          sm.lse2[st][idx] = (lv == -INFINITY) ? -INFINITY : -lv * kLog2e;
-#else
           sm.lse2[st][idx] = (lv == -INFINITY) ? INFINITY : lv * kLog2e;
-#endif
-#if BMA_DKDV_PACKED_DS
-          sm.delta[st][idx] = q < a.N ? -__ldg(a.delta + off) : 0.f;
-#else
           sm.delta[st][idx] = q < a.N ? __ldg(a.delta + off) : 0.f;
-#endif
         }
         mbar_arrive(&sm.bar[BAR_STAT0 + st]);
       }
       if (!ok && lane == 0) report_device_error(p.status, 315);
-    } else if (warp == 11 && p.ds_out != nullptr && total > 0) {
+    } else if (warp == kWarpHand && p.ds_out != nullptr && total > 0) {
       // ---------------------------------------------------------------- dSt hand-over to the dQ replay kernel
       // BAR_STG says that all consumers have staged (and fenced) the dSt image of tile n in shared memory; one
       // bulk store moves it to its slot, and BAR_DSR tells the consumers that the buffer has been read.
@@ -335,109 +322,62 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
   } else {
     // ------------------------------------------------------------------ softmax-gradient warps
-    setmaxnreg_inc_208();
-    const int quarter = warp & 3, half = warp >> 2;
+    setmaxnreg_inc_consumers();
+    const int quarter = warp & 3, part = warp >> 2;
     const int row = quarter * 32 + lane;  // TMEM lane == key row of the tile
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const uint32_t cols = lane_base + part * kCols;   // this thread's query columns of St and dPt
     const int k = k0 + row;
     bool ok = true;
     QTileIter walker(p.l, b, hk, G, kj);
     int h = 0, qi = 0;
     bool partial = false;
-    float pr[64];  // Pt of the current tile (this thread's key row, its 64 query columns)
-    uint32_t pk[32];  // ... and its bf16 pairs, packed while the exponentials keep the MUFU pipe busy
+    float pr[kCols];  // Pt of the current tile (this thread's key row, its query columns)
 
-    // exponentials of one tile: pull St out of TMEM, release its columns, Pt = exp2(St*c - lse2)
+    // exponentials of one tile: Pt = exp2(St*c - lse2), handed to the MMA warp over the St columns
     auto exp_phase = [&](int n, int h_, int qi_, bool partial_) -> bool {
       const int st = n & 1;
       const int q0 = qi_ * BT;
       // per-head key bias times this thread's global key index, in log2 units (0 without a bias)
       const float kbk = KB ? __ldg(a.key_bias + h_) * kLog2e * (float)(p.spec.k_offset + k) : 0.f;
-      uint32_t bits[2] = {0xffffffffu, 0xffffffffu};
+      uint32_t bits = 0xffffffffu;
       if (partial_) {
         const MaskView mv = make_mask_view(p.spec, b, h_);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int cg = half * 2 + c;
-          int jlo, jhi;
-          col_interval(mv, k, q0, BT, jlo, jhi);
-          const int lo = max(jlo - cg * 32, 0), hi = min(jhi - cg * 32, 31);
-          bits[c] = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
-          if (mv.flags & kTableTerms) bits[c] &= table_bits_col32(mv, k, q0 + cg * 32);
-        }
+        int jlo, jhi;
+        col_interval(mv, k, q0, BT, jlo, jhi);
+        const int lo = max(jlo - part * kCols, 0), hi = min(jhi - part * kCols, 31);
+        bits = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
+        if (mv.flags & kTableTerms) bits &= table_bits_col32(mv, k, q0 + part * kCols);
       }
+      if (!mbar_wait(&sm.bar[BAR_STAT0 + st], (n >> 1) & 1)) return false;
       if (!mbar_wait(&sm.bar[BAR_S1], n & 1)) return false;
       tc_fence_after();
-      uint32_t s0[32], s1[32];
-      tmem_ld32(tmem + COL_ST + lane_base + (half * 2) * 32, s0);
-      tmem_ld32(tmem + COL_ST + lane_base + (half * 2 + 1) * 32, s1);
+      uint32_t s[32];
+      tmem_ld32(tmem + COL_ST + cols, s);
       tmem_wait_ld();
-      tc_fence_before();
-      mbar_arrive(&sm.bar[BAR_LS]);
-      if (!mbar_wait(&sm.bar[BAR_STAT0 + st], (n >> 1) & 1)) return false;
-#if !BMA_DKDV_PACKED_EXP
 #pragma unroll
       for (int j4 = 0; j4 < 8; ++j4) {
-        const float4 la = *reinterpret_cast<const float4*>(&sm.lse2[st][(half * 2) * 32 + j4 * 4]);
-        const float4 lb = *reinterpret_cast<const float4*>(&sm.lse2[st][(half * 2 + 1) * 32 + j4 * 4]);
-        float lav[4] = {la.x, la.y, la.z, la.w}, lbv[4] = {lb.x, lb.y, lb.z, lb.w};
+        const float4 lv4 = *reinterpret_cast<const float4*>(&sm.lse2[st][part * kCols + j4 * 4]);
+        float lv[4] = {lv4.x, lv4.y, lv4.z, lv4.w};
         if constexpr (KB) {  // key bias of this thread's key row: the same shift for every query column
 #pragma unroll
-          for (int e = 0; e < 4; ++e) { lav[e] -= kbk; lbv[e] -= kbk; }
+          for (int e = 0; e < 4; ++e) lv[e] -= kbk;
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = j4 * 4 + e;
-          pr[j] = ex2(fmaf(__uint_as_float(s0[j]), p.scale_log2, -lav[e]));
-#if BMA_DKDV_POLY
-          // a quarter of the exponentials on the FMA pipe (e is a compile-time index after unrolling)
-          pr[32 + j] = (e & 1) ? exp2_fma(fmaf(__uint_as_float(s1[j]), p.scale_log2, -lbv[e]))
-                               : ex2(fmaf(__uint_as_float(s1[j]), p.scale_log2, -lbv[e]));
-#else
-          pr[32 + j] = ex2(fmaf(__uint_as_float(s1[j]), p.scale_log2, -lbv[e]));
-#endif
-        }
+        for (int e = 0; e < 4; ++e) pr[j4 * 4 + e] = ex2(fmaf(__uint_as_float(s[j4 * 4 + e]), p.scale_log2, -lv[e]));
       }
-#else
-      {
-        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-#pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          float4 la = *reinterpret_cast<const float4*>(&sm.lse2[st][(half * 2) * 32 + j4 * 4]);        // -lse2
-          float4 lb = *reinterpret_cast<const float4*>(&sm.lse2[st][(half * 2 + 1) * 32 + j4 * 4]);
-          if constexpr (KB) {  // key bias of this thread's key row: the same shift for every query column
-            la.x += kbk; la.y += kbk; la.z += kbk; la.w += kbk;
-            lb.x += kbk; lb.y += kbk; lb.z += kbk; lb.w += kbk;
-          }
-          const int j = j4 * 4;
-          const float2 xa0 = __ffma2_rn(make_float2(__uint_as_float(s0[j]), __uint_as_float(s0[j + 1])), sc2, make_float2(la.x, la.y));
-          const float2 xa1 = __ffma2_rn(make_float2(__uint_as_float(s0[j + 2]), __uint_as_float(s0[j + 3])), sc2, make_float2(la.z, la.w));
-          const float2 xb0 = __ffma2_rn(make_float2(__uint_as_float(s1[j]), __uint_as_float(s1[j + 1])), sc2, make_float2(lb.x, lb.y));
-          const float2 xb1 = __ffma2_rn(make_float2(__uint_as_float(s1[j + 2]), __uint_as_float(s1[j + 3])), sc2, make_float2(lb.z, lb.w));
-          pr[j] = ex2(xa0.x); pr[j + 1] = ex2(xa0.y);
-          pr[j + 2] = ex2(xa1.x); pr[j + 3] = ex2(xa1.y);
-          pr[32 + j] = ex2(xb0.x); pr[32 + j + 1] = ex2(xb0.y);
-#if BMA_DKDV_MATH == 2 || BMA_DKDV_MATH == 3
-          const float2 eb1 = exp2_fma2(xb1);   // two of the eight on the FMA pipe
-          pr[32 + j + 2] = eb1.x; pr[32 + j + 3] = eb1.y;
-#else
-          pr[32 + j + 2] = ex2(xb1.x); pr[32 + j + 3] = ex2(xb1.y);
-#endif
-        }
-      }
-#endif
       if (partial_) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          pr[j] = (bits[0] >> j) & 1u ? pr[j] : 0.f;
-          pr[32 + j] = (bits[1] >> j) & 1u ? pr[32 + j] : 0.f;
-        }
+        for (int j = 0; j < 32; ++j) pr[j] = (bits >> j) & 1u ? pr[j] : 0.f;
       }
+      uint32_t pk[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        pk[j] = pack_bf16(pr[2 * j], pr[2 * j + 1]);
-        pk[16 + j] = pack_bf16(pr[32 + 2 * j], pr[32 + 2 * j + 1]);
-      }
+      for (int j = 0; j < 16; ++j) pk[j] = pack_bf16(pr[2 * j], pr[2 * j + 1]);
+      // Pt takes the place of St values that this very thread has just read: no rendezvous of the consumers is needed
+      tmem_st16(tmem + COL_ST + cols, pk);
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[BAR_P]);
       return true;
     };
 
@@ -447,78 +387,44 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
     for (int n = 0; n < total && ok; ++n) {
       const int st = n & 1;
-      const uint32_t ph = n & 1;
 
       // ---- dSt = Pt * (dPt - delta)
-      ok = mbar_wait(&sm.bar[BAR_S2], ph);
+      ok = mbar_wait(&sm.bar[BAR_S2], n & 1);
       if (!ok) break;
       tc_fence_after();
-      uint32_t dsp[32];
+      uint32_t dsp[16];
       {
-        uint32_t d0[32], d1[32];
-        tmem_ld32(tmem + COL_DPT + lane_base + (half * 2) * 32, d0);
-        tmem_ld32(tmem + COL_DPT + lane_base + (half * 2 + 1) * 32, d1);
+        uint32_t d[32];
+        tmem_ld32(tmem + COL_DPT + cols, d);
         tmem_wait_ld();
-        // this thread holds its dPt values: its Pt may take their place (the store completes under the products below)
-        tmem_st32(tmem + COL_PT + lane_base + half * 64, pk);  // 64 queries = 32 packed columns, inside this half's dPt columns
-#if !BMA_DKDV_PACKED_DS
 #pragma unroll
         for (int j4 = 0; j4 < 8; ++j4) {
-          const float4 da = *reinterpret_cast<const float4*>(&sm.delta[st][(half * 2) * 32 + j4 * 4]);
-          const float4 db = *reinterpret_cast<const float4*>(&sm.delta[st][(half * 2 + 1) * 32 + j4 * 4]);
-          const float dav[4] = {da.x, da.y, da.z, da.w}, dbv[4] = {db.x, db.y, db.z, db.w};
-          float x0[4], x1[4];
+          const float4 dl4 = *reinterpret_cast<const float4*>(&sm.delta[st][part * kCols + j4 * 4]);
+          const float dl[4] = {dl4.x, dl4.y, dl4.z, dl4.w};
+          float x[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int j = j4 * 4 + e;
-            x0[e] = pr[j] * (__uint_as_float(d0[j]) - dav[e]);
-            x1[e] = pr[32 + j] * (__uint_as_float(d1[j]) - dbv[e]);
-          }
-          dsp[j4 * 2] = pack_bf16(x0[0], x0[1]);
-          dsp[j4 * 2 + 1] = pack_bf16(x0[2], x0[3]);
-          dsp[16 + j4 * 2] = pack_bf16(x1[0], x1[1]);
-          dsp[16 + j4 * 2 + 1] = pack_bf16(x1[2], x1[3]);
+          for (int e = 0; e < 4; ++e) x[e] = pr[j4 * 4 + e] * (__uint_as_float(d[j4 * 4 + e]) - dl[e]);
+          dsp[j4 * 2] = pack_bf16(x[0], x[1]);
+          dsp[j4 * 2 + 1] = pack_bf16(x[2], x[3]);
         }
-#else
-#pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          const float4 da = *reinterpret_cast<const float4*>(&sm.delta[st][(half * 2) * 32 + j4 * 4]);        // -delta
-          const float4 db = *reinterpret_cast<const float4*>(&sm.delta[st][(half * 2 + 1) * 32 + j4 * 4]);
-          const int j = j4 * 4;
-          const float2 t0 = __fadd2_rn(make_float2(__uint_as_float(d0[j]), __uint_as_float(d0[j + 1])), make_float2(da.x, da.y));
-          const float2 t1 = __fadd2_rn(make_float2(__uint_as_float(d0[j + 2]), __uint_as_float(d0[j + 3])), make_float2(da.z, da.w));
-          const float2 t2 = __fadd2_rn(make_float2(__uint_as_float(d1[j]), __uint_as_float(d1[j + 1])), make_float2(db.x, db.y));
-          const float2 t3 = __fadd2_rn(make_float2(__uint_as_float(d1[j + 2]), __uint_as_float(d1[j + 3])), make_float2(db.z, db.w));
-          const float2 x0 = __fmul2_rn(make_float2(pr[j], pr[j + 1]), t0);
-          const float2 x1 = __fmul2_rn(make_float2(pr[j + 2], pr[j + 3]), t1);
-          const float2 x2 = __fmul2_rn(make_float2(pr[32 + j], pr[32 + j + 1]), t2);
-          const float2 x3 = __fmul2_rn(make_float2(pr[32 + j + 2], pr[32 + j + 3]), t3);
-          dsp[j4 * 2] = pack_bf16(x0.x, x0.y);
-          dsp[j4 * 2 + 1] = pack_bf16(x1.x, x1.y);
-          dsp[16 + j4 * 2] = pack_bf16(x2.x, x2.y);
-          dsp[16 + j4 * 2 + 1] = pack_bf16(x3.x, x3.y);
-        }
-#endif
       }
-      // Pt and dSt go over columns of dPt that this very thread has just read (its half's 64 columns: Pt in the first 32,
-      // dSt in the second 32), so the consumers need no rendezvous and no buffer to wait for.
-      tmem_st32(tmem + COL_PT + lane_base + half * 64 + 32, dsp);
+      tmem_st16(tmem + COL_DPT + cols, dsp);   // over columns of dPt that this very thread has just read
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(&sm.bar[BAR_P]);
+      mbar_arrive(&sm.bar[BAR_DS]);
       if (p.ds_out != nullptr) {
-        // Hand-over to the dQ replay kernel, off the MMAs' critical path: the thread's 64 dSt values are one 128-byte
-        // line of the tile image (key row `row`, box `half`, 16-byte chunks swizzled like an MMA operand); the image is
-        // staged in shared memory and leaves as one bulk store (warp 11).  Global stores issued by the consumer warps
-        // themselves — a line per thread, or 512 contiguous bytes per instruction after a turn through shared memory —
+        // Hand-over to the dQ replay kernel, off the MMAs' critical path: the thread's dSt values are part of one 128-byte
+        // line of the tile image (key row `row`, box of 64 queries, 16-byte chunks swizzled like an MMA operand); the image
+        // is staged in shared memory and leaves as one bulk store (warp kWarpHand).  Global stores issued by the consumer
+        // warps themselves -- a line per thread, or 512 contiguous bytes per instruction after a turn through shared memory --
         // were measured 25 % and 9 % slower for the whole kernel: 32 KB per tile is more than the load/store path of
         // an SM absorbs without stalling the warps that issue it.
         if (n > 0) ok = mbar_wait(&sm.bar[BAR_DSR], (n - 1) & 1);  // the previous image has been read
         if (!ok) break;
-        uint8_t* ds_row = sm.ds + half * kHalfTile + row * 128;
+        uint8_t* ds_row = sm.ds + (part >> 1) * kHalfTile + row * 128;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int chunk = u ^ (row & 7);
+        for (int u = 0; u < 4; ++u) {
+          const int chunk = ((part & 1) * 4 + u) ^ (row & 7);
           *reinterpret_cast<uint4*>(ds_row + chunk * 16) = make_uint4(dsp[u * 4], dsp[u * 4 + 1], dsp[u * 4 + 2], dsp[u * 4 + 3]);
         }
         fence_proxy_async();  // the bulk store reads the image through the async proxy
@@ -533,30 +439,31 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
 
     // ---- epilogue: dK (scaled) and dV of this kv tile
-    if (ok && total > 0) ok = mbar_wait(&sm.bar[BAR_D], (total - 1) & 1);
+    if (ok && total > 0) ok = mbar_wait(&sm.bar[BAR_DK0 + ((total - 1) & 1)], ((total - 1) >> 1) & 1);  // the last MMA of all
     if (ok && total == 0) ok = mbar_wait(&sm.bar[BAR_KV], 0);  // the K/V loads must land before their buffers are reused below
     if (!ok) {
       report_device_error(p.status, 320 + warp);
     } else {
       tc_fence_after();
-      // dK (scaled) and dV go through shared memory — the K and V tiles are dead now — in the 128-byte-swizzled
+      // dK (scaled) and dV go through shared memory -- the K and V tiles are dead now -- in the 128-byte-swizzled
       // box layout and leave as TMA stores of whole lines (rows past the end of the tensor are clipped by the
-      // tensor map).  Thread (row, half) owns HD/2 columns of key row `row`.
-      uint8_t* k_row = sm.k + (HD == 128 ? half * kHalfTile : 0) + row * 128;
-      uint8_t* v_row = sm.v + (HD == 128 ? half * kHalfTile : 0) + row * 128;
+      // tensor map).  Thread (row, part) owns HD / kParts columns of key row `row`, 16 at a time.
 #pragma unroll
-      for (int c = 0; c < HD / 64; ++c) {
-        uint32_t rk[32], rv[32];
+      for (int c = 0; c < HD / kParts / 16; ++c) {
+        const int col = part * (HD / kParts) + c * 16;
+        uint32_t rk[16], rv[16];
         if (total > 0) {
-          tmem_ld32(tmem + COL_DK + lane_base + half * (HD / 2) + c * 32, rk);
-          tmem_ld32(tmem + COL_DV + lane_base + half * (HD / 2) + c * 32, rv);
+          tmem_ld16(tmem + COL_DK + lane_base + col, rk);
+          tmem_ld16(tmem + COL_DV + lane_base + col, rv);
           tmem_wait_ld();
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) { rk[j] = 0u; rv[j] = 0u; }
+          for (int j = 0; j < 16; ++j) { rk[j] = 0u; rv[j] = 0u; }
         }
+        uint8_t* k_row = sm.k + (col >> 6) * kHalfTile + row * 128;
+        uint8_t* v_row = sm.v + (col >> 6) * kHalfTile + row * 128;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 2; ++u) {
           const int j = u * 8;
           uint4 ok4, ov4;
           ok4.x = pack_bf16(__uint_as_float(rk[j]) * a.scale, __uint_as_float(rk[j + 1]) * a.scale);
@@ -567,7 +474,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           ov4.y = pack_bf16(__uint_as_float(rv[j + 2]), __uint_as_float(rv[j + 3]));
           ov4.z = pack_bf16(__uint_as_float(rv[j + 4]), __uint_as_float(rv[j + 5]));
           ov4.w = pack_bf16(__uint_as_float(rv[j + 6]), __uint_as_float(rv[j + 7]));
-          const int chunk = ((HD == 128 ? c * 4 : half * 4) + u) ^ (row & 7);
+          const int chunk = (((col & 63) >> 3) + u) ^ (row & 7);
           *reinterpret_cast<uint4*>(k_row + chunk * 16) = ok4;
           *reinterpret_cast<uint4*>(v_row + chunk * 16) = ov4;
         }
@@ -590,7 +497,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if (warp == kWarpTma) tmem_dealloc(tmem, kTmemCols);
 }
 
 bool aligned16(const bma_tensor& t) {
