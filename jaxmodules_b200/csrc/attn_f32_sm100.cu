@@ -1005,6 +1005,549 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
 }
 
+// =================================================================================================================
+// Head dimensions 65 - 128, backward.  The planes of two [128 x 128] operands (192 KB) leave no room for the streamed side, so
+// of the two resident operands one keeps its planes in shared memory (96 KB) and the other in tensor memory as the A operand
+// (192 columns).  Gradients leave through one 64-column accumulator, a chunk of 64 head columns at a time, which the row
+// threads add up in registers (warpgroup w: columns [32w, 32w + 32) of every chunk).  The streamed side comes as 64-column
+// boxes (three planes, 24 KB).  Bound by the tensor core (24 plane products per block) and the gaps around the single
+// accumulator.  Forward and backward, causal, against the FP32 tile kernels: B=2 L=2048 H=16 d=128 9811 -> 1247 us, B=1 L=4096
+// 8/2 heads 11504 -> 2279 us, B=2 L=1111 12/3 heads 3327 -> 715 us; 2-norm errors of the gradients against float64
+// 2.5e-7 - 4.1e-7 (tile kernels 4.0e-7 - 1.2e-6).
+// =================================================================================================================
+constexpr uint32_t kBoxPlanes = 3 * kHalfBox;    // one streamed box: hi, mid, lo of [64 rows x 64 columns]
+constexpr uint32_t COL_W_S = 0, COL_W_DP = 128, COL_W_ACC = 256, COL_W_A = 320;
+
+
+// The sums of product_rows<2> with the two streamed boxes wherever they are, and A in shared memory or (A_TMEM) at `a`.
+// Descriptors are passed as their low words (address, leading offset); the high word is the same for all of them, and an MMA
+// warp that keeps whole descriptors alive over the four products spills registers.
+__device__ __forceinline__ uint64_t desc_of(uint32_t low) { return make_smem_desc(0, 0, 1024) + low; }
+__device__ __forceinline__ uint32_t desc_low(const void* smem, uint32_t lbo) { return (uint32_t)make_smem_desc(smem_u32(smem), lbo, 1024); }
+template <bool A_TMEM>
+__device__ __forceinline__ void product_rows_wide(bool leader, uint32_t region, uint32_t a, uint32_t box0, uint32_t box1) {
+  asm volatile("" : "+r"(a), "+r"(box0), "+r"(box1));   // keeps the compiler from hoisting 60 sums out of the caller's loop
+  if (!leader) return;
+  constexpr uint32_t kBPlane = kHalfBox >> 4;
+  auto term = [&](int pa, int pb, uint32_t col, uint32_t idesc, bool start) {
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      const uint64_t b = desc_of((ks < 4 ? box0 : box1) + pb * kBPlane + (uint32_t)(((ks & 3) * 32) >> 4));
+      const uint32_t acc = !(start && ks == 0);
+      if constexpr (A_TMEM) mma_ts(region + col, a + pa * 64 + ks * 8, b, idesc, acc);
+      else mma_ss(region + col, desc_of(a + (uint32_t)((pa * 2 * kRowBox + (ks >> 2) * kRowBox + (ks & 3) * 32) >> 4)), b, idesc, acc);
+    }
+  };
+  term(2, 0, 0, kIdescN64, true);
+  term(0, 2, 64, kIdescN64, true);
+  term(1, 0, 0, kIdescN128, false);
+  term(0, 0, 0, kIdescN128, false);
+}
+// region[0, 64) <- P B with the planes of P [128 x 64] in tensor memory at `p` and B one box read MN-major.
+__device__ __forceinline__ void product_chunk(bool leader, uint32_t region, uint32_t p, uint32_t box) {
+  asm volatile("" : "+r"(p), "+r"(box));
+  if (!leader) return;
+  constexpr int kTerms[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};   // (plane of P, plane of B)
+#pragma unroll
+  for (int t = 0; t < 6; ++t)
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      mma_ts(region, p + plane_col(kTerms[t][0], ks), desc_of(box + (uint32_t)((kTerms[t][1] * kHalfBox + ks * 2048) >> 4)), kIdescN64T, (t > 0) || (ks > 0));
+}
+// Planes of this thread's row of an A operand (128 columns) from the workspace into tensor memory, half of the columns per
+// warpgroup; rows outside the tensor are zero.
+__device__ __forceinline__ void load_planes_tmem(uint32_t tm, int w, const uint8_t* planes, int B, int L, int H, int b, int l, int h) {
+#pragma unroll
+  for (int pl = 0; pl < 3; ++pl) {
+    uint32_t r[32];
+    const uint4* src = reinterpret_cast<const uint4*>(planes + ((((int64_t)pl * B + b) * L + l) * H + h) * 256 + w * 128);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint4 v = l < L ? __ldg(src + u) : make_uint4(0u, 0u, 0u, 0u);
+      r[4 * u] = v.x; r[4 * u + 1] = v.y; r[4 * u + 2] = v.z; r[4 * u + 3] = v.w;
+    }
+    tmem_st32(tm + COL_W_A + pl * 64 + w * 32, r);
+  }
+  tmem_wait_st();
+}
+
+struct F32WideParams {
+  F32Params f;
+  const uint8_t* a_planes;   // planes of V (dK/dV) or dO (dQ) in the workspace
+};
+
+// dK / dV, query half tiles of 64.  MMA order per half tile  dV0 dK0 dV1 St(n+1) dK1 dPt(n+1): the box of Q that dK0 frees is
+// refilled under dV1, and the exponentials of the next half tile run under its dPt.
+enum {
+  XB_K = 0, XB_A, XB_S, XB_DP, XB_P, XB_DS, XB_ACC, XB_ACCFREE, XB_EPI, XB_Q_FULL, XB_Q_FREE = XB_Q_FULL + 3, XB_DO_FULL = XB_Q_FREE + 3,
+  XB_DO_FREE = XB_DO_FULL + 2, XB_STAT = XB_DO_FREE + 2, XB_STATFREE = XB_STAT + 2, XB_NUM = XB_STATFREE + 2
+};
+struct __align__(1024) DkdvWideSmem {
+  uint8_t k[3][2][kRowBox];
+  uint8_t q[3][kBoxPlanes];
+  uint8_t d_o[2][kBoxPlanes];
+  float lse2[2][BH], delta[2][BH];
+  uint64_t bar[XB_NUM];
+  uint32_t tmem_base;
+};
+constexpr int kWidePitch = 132;
+static_assert(2 * BM * kWidePitch * sizeof(float) <= sizeof(uint8_t[3][2][kRowBox]) + 3 * kBoxPlanes, "dV and dK are staged over K and Q");
+
+__global__ void __launch_bounds__(kThreads, 1)
+f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_qh,
+                     const __grid_constant__ CUtensorMap map_do, const F32WideParams wp) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  DkdvWideSmem& sm = *reinterpret_cast<DkdvWideSmem*>(smem_raw);
+  const F32Params& p = wp.f;
+  const bma_attn_args& a = p.a;
+  const int kj = blockIdx.x, hk = blockIdx.y, b = blockIdx.z, G = a.Hq / a.Hkv;
+  const int k0 = kj * BM;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  if ((smem_u32(smem_raw) & 1023u) != 0u) {
+    if (threadIdx.x == 0) report_device_error(p.status, 751);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < XB_NUM; ++i) {
+      uint32_t count = 1;
+      if (i == XB_A || i == XB_P || i == XB_DS || i == XB_ACCFREE || i == XB_EPI) count = 256;
+      if (i == XB_STAT || i == XB_STAT + 1) count = 32;
+      mbar_init(&sm.bar[i], count);
+    }
+    fence_barrier_init();
+    mbar_expect_tx(&sm.bar[XB_K], 6 * kRowBox);
+#pragma unroll
+    for (int pl = 0; pl < 3; ++pl)
+#pragma unroll
+      for (int box = 0; box < 2; ++box) tma_load_4d(sm.k[pl][box], &map_k, &sm.bar[XB_K], box * 64, hk, k0, b + pl * a.B);
+  }
+  if (warp == 8) {
+    tmem_alloc(&sm.tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+
+  if (warp >= 8) {
+    setmaxnreg_dec_80();
+    HalfIter walk(p.l, b, hk, G, kj, a.N);
+    int h, q0;
+    bool partial, ok = true;
+    if (warp == 8 || warp == 11) {
+      // ------------------------------------------------------------ Q (warp 8, ring of three boxes) and dO (warp 11, two)
+      if (lane == 0) {
+        const bool is_q = warp == 8;
+        const int slots = is_q ? 3 : 2;
+        for (int i = 0; ok && walk.next(h, q0, partial);)
+          for (int box = 0; box < 2 && ok; ++box, ++i) {
+            const int slot = i % slots;
+            uint64_t* full = &sm.bar[(is_q ? XB_Q_FULL : XB_DO_FULL) + slot];
+            if (i >= slots) ok = mbar_wait(&sm.bar[(is_q ? XB_Q_FREE : XB_DO_FREE) + slot], (i / slots - 1) & 1);
+            if (!ok) break;
+            mbar_expect_tx(full, kBoxPlanes);
+#pragma unroll
+            for (int pl = 0; pl < 3; ++pl)
+              tma_load_4d((is_q ? sm.q[slot] : sm.d_o[slot]) + pl * kHalfBox, is_q ? &map_qh : &map_do, full, box * 64, h, q0, b + pl * a.B);
+          }
+        if (!ok) report_device_error(p.status, 760);
+      }
+    } else if (warp == 10) {
+      // ------------------------------------------------------------ row statistics of the coming half tiles
+      for (int n = 0; ok && walk.next(h, q0, partial); ++n) {
+        const int st = n & 1;
+        if (n >= 2) ok = mbar_wait(&sm.bar[XB_STATFREE + st], ((n >> 1) - 1) & 1);
+        if (!ok) break;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int idx = e * 32 + lane, q = q0 + idx;
+          const int64_t off = ((int64_t)b * a.Hq + h) * a.N + q;
+          const float lv = q < a.N ? __ldg(a.lse + off) : -INFINITY;
+          sm.lse2[st][idx] = (lv == -INFINITY) ? INFINITY : lv * kLog2e;   // +inf: the probabilities of the row become exactly 0
+          sm.delta[st][idx] = q < a.N ? __ldg(a.delta + off) : 0.f;
+        }
+        mbar_arrive(&sm.bar[XB_STAT + st]);
+      }
+      if (!ok && lane == 0) report_device_error(p.status, 765);
+    } else {
+      // ------------------------------------------------------------ MMA issue
+      const bool leader = elect_one();
+      const uint32_t dk = desc_low(sm.k, 16);
+      const uint32_t dq = desc_low(sm.q, 16), ddo = desc_low(sm.d_o, 16);
+      const uint32_t dqm = desc_low(sm.q, kHalfBox), ddom = desc_low(sm.d_o, kHalfBox);
+      constexpr uint32_t kBoxUnits = kBoxPlanes >> 4;
+      auto issue_st = [&](int n) -> bool {
+        const int i0 = 2 * n, i1 = 2 * n + 1;
+        if (!mbar_wait(&sm.bar[XB_Q_FULL + i0 % 3], (i0 / 3) & 1) || !mbar_wait(&sm.bar[XB_Q_FULL + i1 % 3], (i1 / 3) & 1)) return false;
+        tc_fence_after();
+        product_rows_wide<false>(leader, tmem + COL_W_S, dk, dq + (i0 % 3) * kBoxUnits, dq + (i1 % 3) * kBoxUnits);
+        if (leader) mma_commit(&sm.bar[XB_S]);
+        return true;
+      };
+      auto issue_dpt = [&](int n) -> bool {
+        if (!mbar_wait(&sm.bar[XB_DO_FULL], n & 1) || !mbar_wait(&sm.bar[XB_DO_FULL + 1], n & 1)) return false;
+        tc_fence_after();
+        product_rows_wide<true>(leader, tmem + COL_W_DP, tmem + COL_W_A, ddo, ddo + kBoxUnits);
+        if (leader) mma_commit(&sm.bar[XB_DP]);
+        return true;
+      };
+      int chunk = 0;   // chunks issued so far
+      auto acc_ready = [&]() -> bool {
+        const bool r = chunk == 0 || mbar_wait(&sm.bar[XB_ACCFREE], (chunk - 1) & 1);
+        ++chunk;
+        tc_fence_after();
+        return r;
+      };
+      bool have = walk.next(h, q0, partial);
+      if (have) ok = mbar_wait(&sm.bar[XB_K], 0) && issue_st(0) && mbar_wait(&sm.bar[XB_A], 0) && issue_dpt(0);
+      for (int n = 0; have && ok; ++n) {
+        const bool more = walk.next(h, q0, partial);
+        const int s0 = (2 * n) % 3, s1 = (2 * n + 1) % 3;
+        ok = mbar_wait(&sm.bar[XB_P], n & 1) && acc_ready();
+        if (!ok) break;
+        product_chunk(leader, tmem + COL_W_ACC, tmem + COL_W_S, ddom);
+        if (leader) { mma_commit(&sm.bar[XB_ACC]); mma_commit(&sm.bar[XB_DO_FREE]); }
+        ok = mbar_wait(&sm.bar[XB_DS], n & 1) && acc_ready();
+        if (!ok) break;
+        product_chunk(leader, tmem + COL_W_ACC, tmem + COL_W_DP, dqm + s0 * kBoxUnits);
+        if (leader) { mma_commit(&sm.bar[XB_ACC]); mma_commit(&sm.bar[XB_Q_FREE + s0]); mma_commit(&sm.bar[XB_STATFREE + (n & 1)]); }
+        ok = acc_ready();
+        if (!ok) break;
+        product_chunk(leader, tmem + COL_W_ACC, tmem + COL_W_S, ddom + kBoxUnits);
+        if (leader) { mma_commit(&sm.bar[XB_ACC]); mma_commit(&sm.bar[XB_DO_FREE + 1]); }
+        if (more) ok = issue_st(n + 1);
+        ok = ok && acc_ready();
+        if (!ok) break;
+        product_chunk(leader, tmem + COL_W_ACC, tmem + COL_W_DP, dqm + s1 * kBoxUnits);
+        if (leader) { mma_commit(&sm.bar[XB_ACC]); mma_commit(&sm.bar[XB_Q_FREE + s1]); }
+        if (more) ok = issue_dpt(n + 1);
+        have = more;
+      }
+      if (!ok && leader) report_device_error(p.status, 770);
+    }
+  } else {
+    // -------------------------------------------------------------- row threads
+    setmaxnreg_inc_208();
+    const int w = warp >> 2, row = threadIdx.x & 127, k = k0 + row;
+    const uint32_t tm = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    load_planes_tmem(tm, w, wp.a_planes, a.B, a.L, a.Hkv, b, k, hk);
+    tc_fence_before();
+    mbar_arrive(&sm.bar[XB_A]);
+    float acc[4][32];   // columns [32w, 32w + 32) of dV0, dK0, dV1, dK1 of this key row
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[c][j] = 0.f;
+    bool ok = true;
+    HalfIter walk(p.l, b, hk, G, kj, a.N);
+    int h, q0, n = 0;
+    bool partial;
+    for (; ok && walk.next(h, q0, partial); ++n) {
+      const int st = n & 1;
+      const float kbk = a.key_bias ? __ldg(a.key_bias + h) * kLog2e * (float)(p.spec.k_offset + k) : 0.f;
+      uint32_t bits = 0xffffffffu;
+      if (partial) {
+        const MaskView mv = make_mask_view(p.spec, b, h);
+        int jlo, jhi;
+        col_interval(mv, k, q0 + w * 32, 32, jlo, jhi);
+        const int lo = max(jlo, 0), hi = min(jhi, 31);
+        bits = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) : 0u;
+        if (mv.flags & kTableTerms) bits &= table_bits_col32(mv, k, q0 + w * 32);
+      }
+      ok = mbar_wait(&sm.bar[XB_STAT + st], (n >> 1) & 1) && mbar_wait(&sm.bar[XB_S], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+      float pr[32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r0[16], r1[16];
+        tmem_ld16(tm + COL_W_S + w * 32 + c * 16, r0);
+        tmem_ld16(tm + COL_W_S + 64 + w * 32 + c * 16, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float s = __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+          pr[c * 16 + j] = (bits >> (c * 16 + j)) & 1u ? ex2(fmaf(s, p.scale_log2, kbk) - sm.lse2[st][w * 32 + c * 16 + j]) : 0.f;
+        }
+      }
+      store_planes32(tm + COL_W_S, w * 2, pr);
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[XB_P]);
+      ok = mbar_wait(&sm.bar[XB_DP], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r0[16], r1[16];
+        tmem_ld16(tm + COL_W_DP + w * 32 + c * 16, r0);
+        tmem_ld16(tm + COL_W_DP + 64 + w * 32 + c * 16, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) pr[c * 16 + j] *= (__uint_as_float(r0[j]) + __uint_as_float(r1[j])) - sm.delta[st][w * 32 + c * 16 + j];
+      }
+      store_planes32(tm + COL_W_DP, w * 2, pr);
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[XB_DS]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {   // 4 n + c has the parity of c
+        if (ok) ok = mbar_wait(&sm.bar[XB_ACC], c & 1);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r[32];
+        tmem_ld32(tm + COL_W_ACC + w * 32, r);
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive(&sm.bar[XB_ACCFREE]);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[c][j] += __uint_as_float(r[j]);
+      }
+    }
+    if (ok && n == 0) ok = mbar_wait(&sm.bar[XB_K], 0);   // let the loads land before their buffers are reused
+    // ---- epilogue: every MMA has completed; dV and dK are staged over the K planes and the Q ring
+    mbar_arrive(&sm.bar[XB_EPI]);
+    ok = mbar_wait(&sm.bar[XB_EPI], 0) && ok;
+    float* stage = reinterpret_cast<float*>(smem_raw);
+    if (ok) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float* dst = stage + (c & 1) * BM * kWidePitch + row * kWidePitch + (c >> 1) * 64 + w * 32;
+        const float sc = (c & 1) ? a.scale : 1.f;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          *reinterpret_cast<float4*>(dst + j) = make_float4(acc[c][j] * sc, acc[c][j + 1] * sc, acc[c][j + 2] * sc, acc[c][j + 3] * sc);
+      }
+    }
+    mbar_arrive(&sm.bar[XB_EPI]);
+    ok = mbar_wait(&sm.bar[XB_EPI], 1) && ok;
+    if (ok) {
+      store_rows<256>(stage, kWidePitch, a.dv, b, k0, a.L, hk, a.d, threadIdx.x);
+      store_rows<256>(stage + BM * kWidePitch, kWidePitch, a.dk, b, k0, a.L, hk, a.d, threadIdx.x);
+    } else {
+      report_device_error(p.status, 780 + warp);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+}
+
+// dQ, key half tiles of 64: Q planes in shared memory, dO planes in tensor memory.  MMA order  dQ0 dQ1 S(n+1) dP(n+1).
+enum {
+  YB_Q = 0, YB_A, YB_S, YB_DP, YB_DS, YB_ACC, YB_ACCFREE, YB_EPI, YB_V_FULL, YB_V_FREE, YB_K_FULL, YB_K_FREE = YB_K_FULL + 3, YB_NUM = YB_K_FREE + 3
+};
+struct __align__(1024) DqWideSmem {
+  uint8_t q[3][2][kRowBox];
+  uint8_t k[3][kBoxPlanes];
+  uint8_t v[2][kBoxPlanes];
+  KvList<kMaxKvBwd> list;
+  uint64_t bar[YB_NUM];
+  uint32_t tmem_base;
+};
+
+__global__ void __launch_bounds__(kThreads, 1)
+f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kh,
+                   const __grid_constant__ CUtensorMap map_vh, const F32WideParams wp) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  DqWideSmem& sm = *reinterpret_cast<DqWideSmem*>(smem_raw);
+  const F32Params& p = wp.f;
+  const bma_attn_args& a = p.a;
+  const int qi = (int)gridDim.x - 1 - (int)blockIdx.x;
+  const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.Hq / a.Hkv);
+  const int q0 = qi * BM;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  if ((smem_u32(smem_raw) & 1023u) != 0u) {
+    if (threadIdx.x == 0) report_device_error(p.status, 851);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < YB_NUM; ++i) mbar_init(&sm.bar[i], (i == YB_A || i == YB_DS || i == YB_ACCFREE || i == YB_EPI) ? 256 : 1);
+    fence_barrier_init();
+    mbar_expect_tx(&sm.bar[YB_Q], 6 * kRowBox);
+#pragma unroll
+    for (int pl = 0; pl < 3; ++pl)
+#pragma unroll
+      for (int box = 0; box < 2; ++box) tma_load_4d(sm.q[pl][box], &map_q, &sm.bar[YB_Q], box * 64, h, q0, b + pl * a.B);
+  }
+  if (warp == 8) {
+    tmem_alloc(&sm.tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  const int T = build_kv_list(sm.list, p.l, b, h, qi);
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+  // half tiles in all; the second half of the last tile may lie past the end of the keys
+  const int total = T == 0 ? 0 : 2 * T - ((int)(sm.list.entry[T - 1] & 0x7fff) * 128 + BH >= a.L ? 1 : 0);
+
+  if (warp >= 8) {
+    setmaxnreg_dec_80();
+    bool ok = true;
+    if (warp == 8 && lane == 0) {
+      // ------------------------------------------------------------ K: ring of three boxes
+      for (int i = 0; i < 2 * total && ok; ++i) {
+        const int slot = i % 3, n = i >> 1;
+        if (i >= 3) ok = mbar_wait(&sm.bar[YB_K_FREE + slot], (i / 3 - 1) & 1);
+        if (!ok) break;
+        const int r0 = (int)(sm.list.entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
+        mbar_expect_tx(&sm.bar[YB_K_FULL + slot], kBoxPlanes);
+#pragma unroll
+        for (int pl = 0; pl < 3; ++pl)
+          tma_load_4d(sm.k[slot] + pl * kHalfBox, &map_kh, &sm.bar[YB_K_FULL + slot], (i & 1) * 64, hk, r0, b + pl * a.B);
+      }
+      if (!ok) report_device_error(p.status, 860);
+    } else if (warp == 10 && lane == 0) {
+      // ------------------------------------------------------------ V: both boxes, one stage
+      for (int n = 0; n < total && ok; ++n) {
+        if (n >= 1) ok = mbar_wait(&sm.bar[YB_V_FREE], (n - 1) & 1);
+        if (!ok) break;
+        const int r0 = (int)(sm.list.entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
+        mbar_expect_tx(&sm.bar[YB_V_FULL], 2 * kBoxPlanes);
+#pragma unroll
+        for (int box = 0; box < 2; ++box)
+#pragma unroll
+          for (int pl = 0; pl < 3; ++pl) tma_load_4d(sm.v[box] + pl * kHalfBox, &map_vh, &sm.bar[YB_V_FULL], box * 64, hk, r0, b + pl * a.B);
+      }
+      if (!ok) report_device_error(p.status, 862);
+    } else if (warp == 9 && total > 0) {
+      // ------------------------------------------------------------ MMA issue
+      const bool leader = elect_one();
+      const uint32_t dq = desc_low(sm.q, 16);
+      const uint32_t dk = desc_low(sm.k, 16), dv = desc_low(sm.v, 16);
+      const uint32_t dkm = desc_low(sm.k, kHalfBox);
+      constexpr uint32_t kBoxUnits = kBoxPlanes >> 4;
+      auto issue_s = [&](int n) -> bool {
+        const int i0 = 2 * n, i1 = 2 * n + 1;
+        if (!mbar_wait(&sm.bar[YB_K_FULL + i0 % 3], (i0 / 3) & 1) || !mbar_wait(&sm.bar[YB_K_FULL + i1 % 3], (i1 / 3) & 1)) return false;
+        tc_fence_after();
+        product_rows_wide<false>(leader, tmem + COL_W_S, dq, dk + (i0 % 3) * kBoxUnits, dk + (i1 % 3) * kBoxUnits);
+        if (leader) mma_commit(&sm.bar[YB_S]);
+        return true;
+      };
+      auto issue_dp = [&](int n) -> bool {
+        if (!mbar_wait(&sm.bar[YB_V_FULL], n & 1)) return false;
+        tc_fence_after();
+        product_rows_wide<true>(leader, tmem + COL_W_DP, tmem + COL_W_A, dv, dv + kBoxUnits);
+        if (leader) { mma_commit(&sm.bar[YB_DP]); mma_commit(&sm.bar[YB_V_FREE]); }
+        return true;
+      };
+      ok = mbar_wait(&sm.bar[YB_Q], 0) && issue_s(0) && mbar_wait(&sm.bar[YB_A], 0) && issue_dp(0);
+      for (int n = 0; n < total && ok; ++n) {
+        ok = mbar_wait(&sm.bar[YB_DS], n & 1);
+#pragma unroll
+        for (int c = 0; c < 2 && ok; ++c) {
+          if (2 * n + c > 0) ok = mbar_wait(&sm.bar[YB_ACCFREE], (2 * n + c - 1) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          const int slot = (2 * n + c) % 3;
+          product_chunk(leader, tmem + COL_W_ACC, tmem + COL_W_DP, dkm + slot * kBoxUnits);
+          if (leader) { mma_commit(&sm.bar[YB_ACC]); mma_commit(&sm.bar[YB_K_FREE + slot]); }
+        }
+        if (ok && n + 1 < total) ok = issue_s(n + 1) && issue_dp(n + 1);   // S(n) was read before the DS arrivals of half tile n
+      }
+      if (!ok && leader) report_device_error(p.status, 870);
+    }
+  } else {
+    setmaxnreg_inc_208();
+    const int w = warp >> 2, row = threadIdx.x & 127, q = q0 + row;
+    const uint32_t tm = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    load_planes_tmem(tm, w, wp.a_planes, a.B, a.N, a.Hq, b, q, h);
+    tc_fence_before();
+    mbar_arrive(&sm.bar[YB_A]);
+    const float kb2 = a.key_bias ? __ldg(a.key_bias + h) * kLog2e : 0.f;
+    float lse2 = INFINITY, delta = 0.f;
+    if (q < a.N) {
+      const float lv = __ldg(a.lse + ((int64_t)b * a.Hq + h) * a.N + q);
+      lse2 = lv == -INFINITY ? INFINITY : lv * kLog2e;
+      delta = __ldg(a.delta + ((int64_t)b * a.Hq + h) * a.N + q);
+    }
+    float acc[2][32];   // columns [32w, 32w + 32) of the two chunks of dQ of this row
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[c][j] = 0.f;
+    bool ok = true;
+    for (int n = 0; n < total && ok; ++n) {
+      const uint32_t e = sm.list.entry[n >> 1];
+      const int k0 = (int)(e & 0x7fff) * 128 + (n & 1) * BH;
+      uint32_t bits = 0xffffffffu;
+      if (e & 0x8000u) {
+        uint32_t both[2];
+        row_bits64(p.spec, b, h, q, k0, both);
+        bits = w == 0 ? both[0] : both[1];
+      }
+      const float kbase = (float)(p.spec.k_offset + k0 + w * 32);
+      ok = mbar_wait(&sm.bar[YB_S], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+      float pr[32];
+      {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tm + COL_W_S + w * 32, r0);
+        tmem_ld32(tm + COL_W_S + 64 + w * 32, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float s = __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+          pr[j] = (bits >> j) & 1u ? ex2(fmaf(s, p.scale_log2, kb2 * (kbase + (float)j)) - lse2) : 0.f;
+        }
+      }
+      ok = mbar_wait(&sm.bar[YB_DP], n & 1);
+      if (!ok) break;
+      tc_fence_after();
+      {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tm + COL_W_DP + w * 32, r0);
+        tmem_ld32(tm + COL_W_DP + 64 + w * 32, r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) pr[j] *= (__uint_as_float(r0[j]) + __uint_as_float(r1[j])) - delta;
+      }
+      store_planes32(tm + COL_W_DP, w * 2, pr);
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm.bar[YB_DS]);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (ok) ok = mbar_wait(&sm.bar[YB_ACC], c);   // chunk 2 n + c
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r[32];
+        tmem_ld32(tm + COL_W_ACC + w * 32, r);
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive(&sm.bar[YB_ACCFREE]);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[c][j] += __uint_as_float(r[j]);
+      }
+    }
+    if (ok && total == 0) ok = mbar_wait(&sm.bar[YB_Q], 0);
+    // every thread has seen the last chunk, so every MMA that read the Q planes has completed
+    mbar_arrive(&sm.bar[YB_EPI]);
+    ok = mbar_wait(&sm.bar[YB_EPI], 0) && ok;
+    float* stage = reinterpret_cast<float*>(&sm.q[0][0][0]);
+    if (ok) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          *reinterpret_cast<float4*>(stage + row * kWidePitch + c * 64 + w * 32 + j) =
+              make_float4(acc[c][j] * a.scale, acc[c][j + 1] * a.scale, acc[c][j + 2] * a.scale, acc[c][j + 3] * a.scale);
+    }
+    mbar_arrive(&sm.bar[YB_EPI]);
+    ok = mbar_wait(&sm.bar[YB_EPI], 1) && ok;
+    if (ok) store_rows<256>(stage, kWidePitch, a.dq, b, q0, a.N, h, a.d, threadIdx.x);
+    else report_device_error(p.status, 880 + warp);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+}
+
 // ---- host ------------------------------------------------------------------------------------------------------
 int padded_d(const bma_attn_args& a) { return a.d <= 64 ? 64 : 128; }
 size_t plane_bytes(int B, int L, int H, int dp) { return (size_t)3 * B * L * H * dp * 2; }
@@ -1057,7 +1600,7 @@ int make_params(F32Params& p, const bma_attn_args& a, const bma_mask_spec& spec,
 
 size_t f32_workspace_bytes(const bma_attn_args& a, bool backward) {
   if (a.q.dtype != BMA_DTYPE_F32 || !sm100_device()) return 0;
-  if (backward ? (a.d > 64 || ceil_div(a.L, BM) > kMaxKvBwd) : (a.d > 128 || ceil_div(a.L, BM) > kMaxKvFwd)) return 0;
+  if (a.d > 128 || ceil_div(a.L, BM) > (backward ? kMaxKvBwd : kMaxKvFwd)) return 0;
   return planes_layout(a, backward).total;
 }
 
@@ -1092,6 +1635,21 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   int rc;
   if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, pl, w, true, st))) return rc;
   CUtensorMap mq, mk, mv, mdo, mqh, mkh, mvh, mdoh;
+  if (a.d > 64) {
+    if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, 128, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, 128, BM)) ||
+        (rc = plane_map(&mqh, w + pl.q, a.B, a.N, a.Hq, 128, BH)) || (rc = plane_map(&mkh, w + pl.k, a.B, a.L, a.Hkv, 128, BH)) ||
+        (rc = plane_map(&mvh, w + pl.v, a.B, a.L, a.Hkv, 128, BH)) || (rc = plane_map(&mdoh, w + pl.d_o, a.B, a.N, a.Hq, 128, BH)))
+      return rc;
+    BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dkdv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvWideSmem)));
+    BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dq_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqWideSmem)));
+    F32WideParams wp{p, w + pl.v};
+    f32_dkdv_wide_kernel<<<dim3(ceil_div(a.L, BM), a.Hkv, a.B), kThreads, sizeof(DkdvWideSmem), st>>>(mk, mqh, mdoh, wp);
+    wp.a_planes = w + pl.d_o;
+    f32_dq_wide_kernel<<<dim3(ceil_div(a.N, BM), a.Hq, a.B), kThreads, sizeof(DqWideSmem), st>>>(mq, mkh, mvh, wp);
+    count_launches(2);
+    BMA_CUDA_TRY(cudaGetLastError());
+    return BMA_OK;
+  }
   if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, 64, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, 64, BM)) ||
       (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, 64, BM)) || (rc = plane_map(&mdo, w + pl.d_o, a.B, a.N, a.Hq, 64, BM)) ||
       (rc = plane_map(&mqh, w + pl.q, a.B, a.N, a.Hq, 64, BH)) || (rc = plane_map(&mkh, w + pl.k, a.B, a.L, a.Hkv, 64, BH)) ||
