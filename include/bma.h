@@ -273,7 +273,7 @@ int bma_attn_fwd_ws(const bma_attn_args* args, const bma_mask_spec* spec, const 
  * float32 sums -- the accuracy of FP32 FMA arithmetic.  The caller provides the workspace that holds the planes (16-byte
  * aligned) and block lists of BMA_F32_TILE x BMA_F32_TILE blocks; everything else is as for bma_attn_fwd / bma_attn_bwd.
  * bma_attn_f32_workspace_bytes: bytes the pass needs, or 0 when it does not cover the request (then the plain entry points
- * do: other input types, a forced backend, backward with a head dimension above 64, L above 524288 / 131072). */
+ * do: other input types, a forced backend, L above 524288 forward or 131072 backward). */
 enum { BMA_F32_TILE = 128 };
 size_t bma_attn_f32_workspace_bytes(const bma_attn_args* args, int32_t backward);
 int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,

@@ -235,7 +235,7 @@ def get_dense_from_kv_blocks(B, H, NUM_Q_BLOCKS, NUM_KV_BLOCKS, kv_num_blocks, k
 
 def compile_block_lists(dmask: "_masks.DeviceMask", B: int, H: int, N: int, L: int, q_block: int, kv_block: int,
                         device, *, out_B: Optional[int] = None, out_H: Optional[int] = None, q_side: bool = True,
-                        floor_blocks: bool = False, stream=None, conservative: bool = False):
+                        floor_blocks: bool = False, stream=None, conservative: bool = False, views: bool = True):
     """Runs ``bma_mask_compile`` and returns (lists struct, dict of tensors).
 
     ``floor_blocks`` reproduces create_block_mask's ``LEN // BLOCK`` block counts
@@ -243,7 +243,9 @@ def compile_block_lists(dmask: "_masks.DeviceMask", B: int, H: int, N: int, L: i
     are covered.  out_B/out_H default to the smallest extents the mask allows (1 where it does
     not depend on the index).  ``conservative`` sets BMA_MASK_COMPILE_CONSERVATIVE: segment-id blocks
     that the per-block id ranges cannot decide are listed as partial without an element scan — fine
-    for lists the attention kernels consume, never used for the arrays ``create_block_mask`` returns."""
+    for lists the attention kernels consume, never used for the arrays ``create_block_mask`` returns.
+    ``views=False``: the arrays lie in one buffer with the workspace and only the struct describes them (the dict keeps
+    the buffer alive): one allocation where nine cost 20 us of the host's time."""
     lib = nat.lib()
     if floor_blocks:
         NQ, NKV = N // q_block, L // kv_block
@@ -260,26 +262,38 @@ def compile_block_lists(dmask: "_masks.DeviceMask", B: int, H: int, N: int, L: i
         spec.q_valid, spec.k_valid = min(spec.q_valid, NQ * q_block), min(spec.k_valid, NKV * kv_block)
     if conservative:
         spec.flags |= nat.BMA_MASK_COMPILE_CONSERVATIVE
-    i32 = dict(dtype=torch.int32, device=device)
-    t = dict(
-        kv_num_blocks=torch.empty((LB, LH, NQ), **i32), kv_indices=torch.empty((LB, LH, NQ, NKV), **i32),
-        full_kv_num_blocks=torch.empty((LB, LH, NQ), **i32), full_kv_indices=torch.empty((LB, LH, NQ, NKV), **i32),
-        q_num_blocks=None, q_indices=None, full_q_num_blocks=None, full_q_indices=None)
-    if q_side:
-        t.update(q_num_blocks=torch.empty((LB, LH, NKV), **i32), q_indices=torch.empty((LB, LH, NKV, NQ), **i32),
-                 full_q_num_blocks=torch.empty((LB, LH, NKV), **i32), full_q_indices=torch.empty((LB, LH, NKV, NQ), **i32))
     lists = nat.BlockLists()
     lists.B, lists.H, lists.NQ, lists.NKV, lists.q_block, lists.kv_block = LB, LH, NQ, NKV, q_block, kv_block
-    lists.kv_num, lists.kv_idx = t["kv_num_blocks"].data_ptr(), t["kv_indices"].data_ptr()
-    lists.full_kv_num, lists.full_kv_idx = t["full_kv_num_blocks"].data_ptr(), t["full_kv_indices"].data_ptr()
-    if q_side:
-        lists.q_num, lists.q_idx = t["q_num_blocks"].data_ptr(), t["q_indices"].data_ptr()
-        lists.full_q_num, lists.full_q_idx = t["full_q_num_blocks"].data_ptr(), t["full_q_indices"].data_ptr()
     ws_bytes = lib.bma_mask_compile_workspace_bytes(C.byref(spec), B, H, NQ, NKV)
-    ws = torch.empty((max(ws_bytes, 1),), dtype=torch.uint8, device=device)
+    if views:
+        i32 = dict(dtype=torch.int32, device=device)
+        t = dict(
+            kv_num_blocks=torch.empty((LB, LH, NQ), **i32), kv_indices=torch.empty((LB, LH, NQ, NKV), **i32),
+            full_kv_num_blocks=torch.empty((LB, LH, NQ), **i32), full_kv_indices=torch.empty((LB, LH, NQ, NKV), **i32),
+            q_num_blocks=None, q_indices=None, full_q_num_blocks=None, full_q_indices=None)
+        if q_side:
+            t.update(q_num_blocks=torch.empty((LB, LH, NKV), **i32), q_indices=torch.empty((LB, LH, NKV, NQ), **i32),
+                     full_q_num_blocks=torch.empty((LB, LH, NKV), **i32), full_q_indices=torch.empty((LB, LH, NKV, NQ), **i32))
+        lists.kv_num, lists.kv_idx = t["kv_num_blocks"].data_ptr(), t["kv_indices"].data_ptr()
+        lists.full_kv_num, lists.full_kv_idx = t["full_kv_num_blocks"].data_ptr(), t["full_kv_indices"].data_ptr()
+        if q_side:
+            lists.q_num, lists.q_idx = t["q_num_blocks"].data_ptr(), t["q_indices"].data_ptr()
+            lists.full_q_num, lists.full_q_idx = t["full_q_num_blocks"].data_ptr(), t["full_q_indices"].data_ptr()
+        ws = t["_workspace"] = torch.empty((max(ws_bytes, 1),), dtype=torch.uint8, device=device)  # alive until the stream has consumed it
+        ws_ptr = ws.data_ptr()
+    else:
+        pad = lambda n: -(-4 * n // 256) * 256      # bytes of n int32, every array on a 256-byte boundary
+        rows, cols, cells = pad(LB * LH * NQ), pad(LB * LH * NKV), pad(LB * LH * NQ * NKV)
+        total = 2 * (rows + cells) + (2 * (cols + cells) if q_side else 0)
+        t = dict(_buffer=torch.empty((total + ws_bytes + 1,), dtype=torch.uint8, device=device))
+        ptr = t["_buffer"].data_ptr()
+        lists.kv_num, lists.kv_idx, lists.full_kv_num, lists.full_kv_idx = ptr, ptr + rows, ptr + rows + cells, ptr + 2 * rows + cells
+        if q_side:
+            at = ptr + 2 * (rows + cells)
+            lists.q_num, lists.q_idx, lists.full_q_num, lists.full_q_idx = at, at + cols, at + cols + cells, at + 2 * cols + cells
+        ws_ptr = ptr + total
     st = stream if stream is not None else torch.cuda.current_stream(device).cuda_stream
-    nat.check(lib.bma_mask_compile(C.byref(spec), B, H, C.byref(lists), ws.data_ptr(), ws_bytes, st), "bma_mask_compile")
-    t["_workspace"] = ws  # keep alive until the stream has consumed it
+    nat.check(lib.bma_mask_compile(C.byref(spec), B, H, C.byref(lists), ws_ptr, ws_bytes, st), "bma_mask_compile")
     return lists, t
 
 
