@@ -1018,7 +1018,6 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 constexpr uint32_t kBoxPlanes = 3 * kHalfBox;    // one streamed box: hi, mid, lo of [64 rows x 64 columns]
 constexpr uint32_t COL_W_S = 0, COL_W_DP = 128, COL_W_ACC = 256, COL_W_A = 320;
 
-
 // The sums of product_rows<2> with the two streamed boxes wherever they are, and A in shared memory or (A_TMEM) at `a`.
 // Descriptors are passed as their low words (address, leading offset); the high word is the same for all of them, and an MMA
 // warp that keeps whole descriptors alive over the four products spills registers.

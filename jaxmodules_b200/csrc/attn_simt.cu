@@ -1,9 +1,9 @@
 // FP32 SIMT attention kernels (forward, dK/dV, dQ) driven by the block lists.
 //
-// These cover everything the tensor-core kernels do not: float32 inputs (whose 1e-4
-// tolerance a single-pass reduced-precision MMA cannot meet), head dims other than 128,
-// and they are the exact-arithmetic cross-check for the tcgen05 path.  All arithmetic is
-// FP32 FMA; inputs may be float32 or bfloat16 and are widened when a tile is staged.
+// These cover what the tensor-core kernels do not: bfloat16 head dims other than 64 and 128, float32
+// sequences beyond the lengths of attn_f32_sm100.cu, and a forced backend -- as the exact-arithmetic
+// cross-check of the tensor-core paths.  All arithmetic is FP32 FMA; inputs may be float32 or bfloat16
+// and are widened when a tile is staged.
 //
 // Semantics follow jaxmodules/attention.py:52-105 (scores exp(q.k/sqrt(d)) times mask, rows
 // without an allowed key give 0) with a max-subtracted online softmax, which is the same
