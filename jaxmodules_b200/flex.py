@@ -253,7 +253,7 @@ def flex_attention(query: torch.Tensor, key: torch.Tensor, value: torch.Tensor, 
     ``return_lse`` raises NotImplementedError as there (:491-492).  ``score_mod``: functions of the form
     ``a * score + w[h] * k_idx + (terms constant along k_idx)`` (see ``score_mod_affine``; ``h`` is the kv-head
     index, as in the reference) run on the same kernels as a logit scale plus a per-head key bias — a
-    compile-time variant of the tcgen05 kernels for bf16, the SIMT kernels for float32; others raise
+    compile-time variant of the tcgen05 kernels for bf16, a term of the float32 ones; others raise
     NotImplementedError."""
     if return_lse:
         raise NotImplementedError("return_lse is not supported yet")
