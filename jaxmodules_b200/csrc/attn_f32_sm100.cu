@@ -30,6 +30,7 @@
 
 #include "common.cuh"
 #include "ptx_sm100.cuh"
+#include "simt_tiles.cuh"
 
 namespace bma {
 namespace {
@@ -178,6 +179,43 @@ struct F32Params {
   int* status;
 };
 
+// ---- results that are not finite ----------------------------------------------------------------------------------
+// The planes of an infinity, a NaN or a finite value above bfloat16's largest (3.39e38) are not numbers, and neither is
+// any sum that such a value, or an overflow of the products, reaches.  A CTA that finds one among its results
+// does its block row again with the FP32 tile functions, whose results these are then: two rows of 64-tiles over the same
+// lists, on the 256 row threads, in the shared memory of the CTA.  (Written behind the kernel's end so that the
+// main path pays one multiply-add per result for it; a second launch over flagged tiles cost 4 - 12 us a call.)
+__device__ __forceinline__ void note_finite(float& z, float v) { z = fmaf(v, 0.f, z); }   // NaN from the first such v
+
+struct RowSync {   // the 256 row threads
+  static __device__ __forceinline__ void sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+  static __device__ __forceinline__ bool any(bool x) {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 1, 256, p;\n selp.u32 %0, 1, 0, q;\n}" : "=r"(r) : "r"((uint32_t)x) : "memory");
+    return r != 0;
+  }
+};
+enum RedoPass { REDO_FWD, REDO_DKDV, REDO_DQ };
+template <RedoPass PASS, int DC>
+__device__ __noinline__ void redo_row(float* smem, const F32Params& fp, int tile128, int h, int b) {
+  const SimtParams p{fp.a, fp.spec, fp.l, fp.scale_log2};
+  const bool do_f32 = fp.a.d_o.dtype == BMA_DTYPE_F32;
+  for (int half = 0; half < 2; ++half) {
+    const int tile = 2 * tile128 + half;
+    if (tile * TQ >= (PASS == REDO_DKDV ? fp.a.L : fp.a.N)) return;
+    RowSync::sync();   // the shared memory is free: its last readers have arrived here
+    if constexpr (PASS == REDO_FWD) {
+      fwd_tile<float, DC, true, RowSync>(smem, p, tile, h, b);
+    } else if constexpr (PASS == REDO_DKDV) {
+      if (do_f32) dkdv_tile<float, float, DC, true, RowSync>(smem, p, tile, h, b);
+      else dkdv_tile<float, __nv_bfloat16, DC, true, RowSync>(smem, p, tile, h, b);
+    } else {
+      if (do_f32) dq_tile<float, float, DC, true, RowSync>(smem, p, tile, h, b);
+      else dq_tile<float, __nv_bfloat16, DC, true, RowSync>(smem, p, tile, h, b);
+    }
+  }
+}
+
 // Merged kv list of one query tile in shared memory, ascending, every block once: kv tile | partial << 15.
 // Called by all threads of the CTA between two __syncthreads of its own; returns the number of entries.
 template <int MAX>
@@ -273,12 +311,15 @@ struct __align__(1024) FwdSmem {
   KvList<kMaxKvFwd> list;
   uint64_t bar[FB_NUM];
   uint32_t tmem_base;
+  int not_finite;
 };
+
+static_assert(fwd_smem<4>() <= sizeof(FwdSmem<64>) && fwd_smem<8>() <= sizeof(FwdSmem<128>), "a tile is done again in the same shared memory");
 
 template <int DP>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-               const __grid_constant__ CUtensorMap map_v, const F32Params p) {
+               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ F32Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using Smem = FwdSmem<DP>;
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
@@ -300,6 +341,7 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       if (i == FB_SYNC) count = 256;
       mbar_init(&sm.bar[i], count);
     }
+    sm.not_finite = 0;
     fence_barrier_init();
   }
   if (warp == 8) {
@@ -510,12 +552,15 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
     rendezvous();
     if (x == 1) {
+      float z = 0.f;
 #pragma unroll
       for (int j = 0; j < DP; j += 4) {
         float4 v = *reinterpret_cast<float4*>(stage + j);
         v.x = fmaf(o[j], mine, v.x); v.y = fmaf(o[j + 1], mine, v.y); v.z = fmaf(o[j + 2], mine, v.z); v.w = fmaf(o[j + 3], mine, v.w);
         *reinterpret_cast<float4*>(stage + j) = v;
+        note_finite(z, (v.x + v.y) + (v.z + v.w));
       }
+      if (z != 0.f) sm.not_finite = 1;
       if (q < a.N && a.lse) a.lse[((int64_t)b * a.Hq + h) * a.N + q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
     }
     rendezvous();
@@ -525,6 +570,7 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if (warp < 8 && sm.not_finite) redo_row<REDO_FWD, DP / 16>(reinterpret_cast<float*>(smem_raw), p, qi, h, b);
 }
 
 // =================================================================================================================
@@ -547,7 +593,9 @@ struct __align__(1024) DkdvSmem {
   float lse2[2][BH], delta[2][BH];
   uint64_t bar[KB_NUM];
   uint32_t tmem_base;
+  int not_finite;
 };
+static_assert(dkdv_smem<4>() <= sizeof(DkdvSmem), "a tile is done again in the same shared memory");
 constexpr uint32_t COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
 
 // flattened walk over (group head, listed q tile, half tile); a half tile past the end of the queries is left out
@@ -573,7 +621,7 @@ struct HalfIter {
 
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                const __grid_constant__ CUtensorMap map_qh, const __grid_constant__ CUtensorMap map_do, const F32Params p) {
+                const __grid_constant__ CUtensorMap map_qh, const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DkdvSmem& sm = *reinterpret_cast<DkdvSmem*>(smem_raw);
   const bma_attn_args& a = p.a;
@@ -593,6 +641,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
       if (i == KB_STAT || i == KB_STAT + 1) count = 32;
       mbar_init(&sm.bar[i], count);
     }
+    sm.not_finite = 0;
     fence_barrier_init();
     mbar_expect_tx(&sm.bar[KB_KV], 6 * kRowBox);
 #pragma unroll
@@ -792,6 +841,10 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
     constexpr int kPitch = 68;
     float* stage = reinterpret_cast<float*>(w == 0 ? &sm.v[0][0] : &sm.k[0][0]);
     const float sc = w == 0 ? 1.f : a.scale;
+    float z = 0.f;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) note_finite(z, acc[j] * sc);
+    if (z != 0.f) sm.not_finite = 1;
 #pragma unroll
     for (int j = 0; j < 64; j += 4)
       if (ok) *reinterpret_cast<float4*>(stage + row * kPitch + j) = make_float4(acc[j] * sc, acc[j + 1] * sc, acc[j + 2] * sc, acc[j + 3] * sc);
@@ -803,6 +856,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if (warp < 8 && sm.not_finite) redo_row<REDO_DKDV, 4>(reinterpret_cast<float*>(smem_raw), p, kj, hk, b);
 }
 
 // =================================================================================================================
@@ -823,12 +877,14 @@ struct __align__(1024) DqSmem {
   KvList<kMaxKvBwd> list;
   uint64_t bar[QB_NUM];
   uint32_t tmem_base;
+  int not_finite;
 };
+static_assert(dq_smem<4>() <= sizeof(DqSmem), "as above");
 constexpr uint32_t COL_S2 = 0, COL_DP2 = 256, COL_DQ2 = 384;   // S: two buffers of 128 columns
 
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kh,
-              const __grid_constant__ CUtensorMap map_vh, const __grid_constant__ CUtensorMap map_do, const F32Params p) {
+              const __grid_constant__ CUtensorMap map_vh, const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DqSmem& sm = *reinterpret_cast<DqSmem*>(smem_raw);
   const bma_attn_args& a = p.a;
@@ -843,6 +899,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   }
   if (threadIdx.x == 0) {
     for (int i = 0; i < QB_NUM; ++i) mbar_init(&sm.bar[i], (i == QB_DS || i == QB_DQFREE || i == QB_EPI) ? 256 : 1);
+    sm.not_finite = 0;
     fence_barrier_init();
     mbar_expect_tx(&sm.bar[QB_Q], 6 * kRowBox);
 #pragma unroll
@@ -988,6 +1045,10 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
     if (ok && total > 0) ok = flush(total - 1);
     if (ok && total == 0) ok = mbar_wait(&sm.bar[QB_Q], 0);
+    float z = 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) note_finite(z, acc[j] * a.scale);
+    if (z != 0.f) sm.not_finite = 1;
     constexpr int kPitch = 68;
     float* stage = reinterpret_cast<float*>(&sm.q[0][0]);   // every MMA that read the Q planes has completed
     if (ok) {
@@ -1003,6 +1064,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if (warp < 8 && sm.not_finite) redo_row<REDO_DQ, 4>(reinterpret_cast<float*>(smem_raw), p, qi, h, b);
 }
 
 // =================================================================================================================
@@ -1088,13 +1150,15 @@ struct __align__(1024) DkdvWideSmem {
   float lse2[2][BH], delta[2][BH];
   uint64_t bar[XB_NUM];
   uint32_t tmem_base;
+  int not_finite;
 };
+static_assert(dkdv_smem<8>() <= sizeof(DkdvWideSmem), "as above");
 constexpr int kWidePitch = 132;
 static_assert(2 * BM * kWidePitch * sizeof(float) <= sizeof(uint8_t[3][2][kRowBox]) + 3 * kBoxPlanes, "dV and dK are staged over K and Q");
 
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_qh,
-                     const __grid_constant__ CUtensorMap map_do, const F32WideParams wp) {
+                     const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32WideParams wp) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DkdvWideSmem& sm = *reinterpret_cast<DkdvWideSmem*>(smem_raw);
   const F32Params& p = wp.f;
@@ -1114,6 +1178,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
       if (i == XB_STAT || i == XB_STAT + 1) count = 32;
       mbar_init(&sm.bar[i], count);
     }
+    sm.not_finite = 0;
     fence_barrier_init();
     mbar_expect_tx(&sm.bar[XB_K], 6 * kRowBox);
 #pragma unroll
@@ -1306,6 +1371,12 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
       }
     }
     if (ok && n == 0) ok = mbar_wait(&sm.bar[XB_K], 0);   // let the loads land before their buffers are reused
+    float z = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int j = 0; j < 32; ++j) note_finite(z, (c & 1) ? acc[c][j] * a.scale : acc[c][j]);
+    if (z != 0.f) sm.not_finite = 1;
     // ---- epilogue: every MMA has completed; dV and dK are staged over the K planes and the Q ring
     mbar_arrive(&sm.bar[XB_EPI]);
     ok = mbar_wait(&sm.bar[XB_EPI], 0) && ok;
@@ -1332,6 +1403,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   tc_fence_before();
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if (warp < 8 && sm.not_finite) redo_row<REDO_DKDV, 8>(reinterpret_cast<float*>(smem_raw), p, kj, hk, b);
 }
 
 // dQ, key half tiles of 64: Q planes in shared memory, dO planes in tensor memory.  MMA order  dQ0 dQ1 S(n+1) dP(n+1).
@@ -1345,11 +1417,14 @@ struct __align__(1024) DqWideSmem {
   KvList<kMaxKvBwd> list;
   uint64_t bar[YB_NUM];
   uint32_t tmem_base;
+  int not_finite;
 };
+
+static_assert(dq_smem<8>() <= sizeof(DqWideSmem), "as above");
 
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kh,
-                   const __grid_constant__ CUtensorMap map_vh, const F32WideParams wp) {
+                   const __grid_constant__ CUtensorMap map_vh, const __grid_constant__ F32WideParams wp) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DqWideSmem& sm = *reinterpret_cast<DqWideSmem*>(smem_raw);
   const F32Params& p = wp.f;
@@ -1365,6 +1440,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   }
   if (threadIdx.x == 0) {
     for (int i = 0; i < YB_NUM; ++i) mbar_init(&sm.bar[i], (i == YB_A || i == YB_DS || i == YB_ACCFREE || i == YB_EPI) ? 256 : 1);
+    sm.not_finite = 0;
     fence_barrier_init();
     mbar_expect_tx(&sm.bar[YB_Q], 6 * kRowBox);
 #pragma unroll
@@ -1525,6 +1601,12 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       }
     }
     if (ok && total == 0) ok = mbar_wait(&sm.bar[YB_Q], 0);
+    float z = 0.f;
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int j = 0; j < 32; ++j) note_finite(z, acc[c][j] * a.scale);
+    if (z != 0.f) sm.not_finite = 1;
     // every thread has seen the last chunk, so every MMA that read the Q planes has completed
     mbar_arrive(&sm.bar[YB_EPI]);
     ok = mbar_wait(&sm.bar[YB_EPI], 0) && ok;
@@ -1545,6 +1627,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   tc_fence_before();
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if (warp < 8 && sm.not_finite) redo_row<REDO_DQ, 8>(reinterpret_cast<float*>(smem_raw), p, qi, h, b);
 }
 
 // ---- host ------------------------------------------------------------------------------------------------------
