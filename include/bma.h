@@ -269,11 +269,16 @@ size_t bma_attn_fwd_workspace_bytes(const bma_attn_args* args, const bma_block_l
 int bma_attn_fwd_ws(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
                     void* workspace, size_t workspace_bytes, bma_stream_t stream);
 
-/* float32 inputs on the tensor core: every operand as three bf16 planes (exact), six plane products per matrix product,
- * float32 sums -- the accuracy of FP32 FMA arithmetic.  The caller provides the workspace that holds the planes (16-byte
- * aligned) and block lists of BMA_F32_TILE x BMA_F32_TILE blocks; everything else is as for bma_attn_fwd / bma_attn_bwd.
- * bma_attn_f32_workspace_bytes: bytes the pass needs, or 0 when it does not cover the request (then the plain entry points
- * do: other input types, a forced backend, L above 524288 forward or 131072 backward). */
+/* float32 inputs on the tensor core: every operand as three bf16 planes, six plane products per matrix product, float32
+ * sums -- the accuracy of FP32 FMA arithmetic.  Three planes hold a value exactly from 2^-110 up to 3.38e38 in magnitude;
+ * below that its error is at most 2^-133.  Tiles whose result is not finite -- an infinity, a NaN or a larger value reaches
+ * them, or a sum overflows -- are done again with FP32 FMA arithmetic, so that such values have the effect they have there.
+ * The caller provides the workspace that holds the planes (16-byte aligned) and block lists of BMA_F32_TILE x BMA_F32_TILE
+ * blocks; everything else is as for bma_attn_fwd / bma_attn_bwd.
+ * bma_attn_f32_workspace_bytes: bytes the pass needs (6 per value of Q, K, V and, backward, dO, the head dimension padded to
+ * 64 or 128), or 0 when it does not cover the request (then the plain entry points do: other input types, a forced backend,
+ * L above 524288 forward or 131072 backward).  With less workspace than that (NULL, 0 included) the whole pass runs with FP32
+ * FMA arithmetic over the same lists, which needs none. */
 enum { BMA_F32_TILE = 128 };
 size_t bma_attn_f32_workspace_bytes(const bma_attn_args* args, int32_t backward);
 int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,

@@ -265,9 +265,9 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
         a.o, a.lse = _tensor(O), lse.data_ptr()
         with _Span(_profile_sink, "fwd", dev):
             if f32_bytes:
-                ws = torch.empty((f32_bytes,), dtype=torch.uint8, device=dev)
-                nat.check(lib.bma_attn_fwd_f32(C.byref(a), C.byref(dmask.spec), C.byref(lists), ws.data_ptr(), f32_bytes, st),
-                          "bma_attn_fwd_f32")
+                ws = _float32_planes(dev, f32_bytes)
+                nat.check(lib.bma_attn_fwd_f32(C.byref(a), C.byref(dmask.spec), C.byref(lists), ws.data_ptr() if ws is not None else None,
+                                               f32_bytes if ws is not None else 0, st), "bma_attn_fwd_f32")
             else:
                 ws_bytes = lib.bma_attn_fwd_workspace_bytes(C.byref(a), C.byref(lists))
                 ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=dev) if ws_bytes else None
@@ -319,10 +319,10 @@ def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
         if do_bf16 is not None:
             a.d_o = _tensor(do_bf16)
         if f32_bytes:
-            ws = torch.empty((f32_bytes,), dtype=torch.uint8, device=dev)
+            ws = _float32_planes(dev, f32_bytes)
             with _Span(_profile_sink, "bwd", dev):
-                nat.check(lib.bma_attn_bwd_f32(C.byref(a), C.byref(ctx["dmask"].spec), C.byref(lists), ws.data_ptr(), f32_bytes, st),
-                          "bma_attn_bwd_f32")
+                nat.check(lib.bma_attn_bwd_f32(C.byref(a), C.byref(ctx["dmask"].spec), C.byref(lists), ws.data_ptr() if ws is not None else None,
+                                               f32_bytes if ws is not None else 0, st), "bma_attn_bwd_f32")
             _maybe_check_status(dev, "bma_attn_bwd_f32")
             return dQ, dK, dV
         ws_bytes = lib.bma_attn_bwd_workspace_bytes(C.byref(a))
@@ -385,6 +385,23 @@ def set_backward_scratch_limit(nbytes: int, fraction: float = 1.0) -> None:
 def release_backward_scratch() -> None:
     """Frees every scratch buffer (they come back at the next backward call that wants one)."""
     _scratch_buffers.clear()
+
+
+# Most that the bf16 planes of one float32 pass may take: 1.5 x 64 or 128 / d times its inputs (d = 128, 131072 tokens of 32
+# heads: 9.7 GB forward, 12.9 GB backward).  Above it, and where the device has no such room, the FP32 tile kernels
+# run, which need none and take 2 - 9 times as long (d = 1: 240 against 96 us for 2 x 2048 tokens of 8 heads, d = 64: 515
+# against 98; there is no head dimension for which they are the faster ones).
+_F32_PLANES_LIMIT = 16 << 30
+
+
+def _float32_planes(dev: torch.device, nbytes: int) -> Optional[torch.Tensor]:
+    """Workspace of one float32 pass, or None where it exceeds the limit or the free memory of the device."""
+    if nbytes > _F32_PLANES_LIMIT:
+        return None
+    try:
+        return torch.empty((nbytes,), dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def _backward_scratch(dev: torch.device, nbytes: int) -> torch.Tensor:

@@ -19,20 +19,20 @@
 namespace bma {
 namespace {
 
-template <typename T, int DC>
+template <typename T, int DC, bool WIDE>
 __global__ void __launch_bounds__(NT) simt_fwd_kernel(const SimtParams p) {
   extern __shared__ __align__(16) float sm[];
-  fwd_tile<T, DC, false, CtaSync>(sm, p, blockIdx.x, blockIdx.y, blockIdx.z);
+  fwd_tile<T, DC, WIDE, CtaSync>(sm, p, blockIdx.x, blockIdx.y, blockIdx.z);
 }
-template <typename T, typename TDO, int DC>
+template <typename T, typename TDO, int DC, bool WIDE>
 __global__ void __launch_bounds__(NT) simt_bwd_dkdv_kernel(const SimtParams p) {
   extern __shared__ __align__(16) float sm[];
-  dkdv_tile<T, TDO, DC, false, CtaSync>(sm, p, blockIdx.x, blockIdx.y, blockIdx.z);
+  dkdv_tile<T, TDO, DC, WIDE, CtaSync>(sm, p, blockIdx.x, blockIdx.y, blockIdx.z);
 }
-template <typename T, typename TDO, int DC>
+template <typename T, typename TDO, int DC, bool WIDE>
 __global__ void __launch_bounds__(NT) simt_bwd_dq_kernel(const SimtParams p) {
   extern __shared__ __align__(16) float sm[];
-  dq_tile<T, TDO, DC, false, CtaSync>(sm, p, blockIdx.x, blockIdx.y, blockIdx.z);
+  dq_tile<T, TDO, DC, WIDE, CtaSync>(sm, p, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 template <typename K>
@@ -41,48 +41,48 @@ int set_smem(K kernel, size_t bytes) {
   return BMA_OK;
 }
 
-template <typename T, int DC>
+template <typename T, int DC, bool WIDE>
 int launch_fwd(const SimtParams& p, cudaStream_t st) {
-  int rc = set_smem(simt_fwd_kernel<T, DC>, fwd_smem<DC>());
+  int rc = set_smem(simt_fwd_kernel<T, DC, WIDE>, fwd_smem<DC>());
   if (rc) return rc;
   dim3 grid(ceil_div(p.a.N, TQ), p.a.Hq, p.a.B);
-  simt_fwd_kernel<T, DC><<<grid, NT, fwd_smem<DC>(), st>>>(p);
+  simt_fwd_kernel<T, DC, WIDE><<<grid, NT, fwd_smem<DC>(), st>>>(p);
   count_launches(1);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
 }
 
-template <typename T, typename TDO, int DC>
+template <typename T, typename TDO, int DC, bool WIDE>
 int launch_bwd(const SimtParams& p, cudaStream_t st) {
-  int rc = set_smem(simt_bwd_dkdv_kernel<T, TDO, DC>, dkdv_smem<DC>());
+  int rc = set_smem(simt_bwd_dkdv_kernel<T, TDO, DC, WIDE>, dkdv_smem<DC>());
   if (rc) return rc;
-  rc = set_smem(simt_bwd_dq_kernel<T, TDO, DC>, dq_smem<DC>());
+  rc = set_smem(simt_bwd_dq_kernel<T, TDO, DC, WIDE>, dq_smem<DC>());
   if (rc) return rc;
   dim3 gkv(ceil_div(p.a.L, TK), p.a.Hkv, p.a.B);
-  simt_bwd_dkdv_kernel<T, TDO, DC><<<gkv, NT, dkdv_smem<DC>(), st>>>(p);
+  simt_bwd_dkdv_kernel<T, TDO, DC, WIDE><<<gkv, NT, dkdv_smem<DC>(), st>>>(p);
   dim3 gq(ceil_div(p.a.N, TQ), p.a.Hq, p.a.B);
-  simt_bwd_dq_kernel<T, TDO, DC><<<gq, NT, dq_smem<DC>(), st>>>(p);
+  simt_bwd_dq_kernel<T, TDO, DC, WIDE><<<gq, NT, dq_smem<DC>(), st>>>(p);
   count_launches(2);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
 }
 
-template <typename T>
+template <typename T, bool WIDE>
 int dispatch_fwd(const SimtParams& p, cudaStream_t st) {
   const int d = p.a.d;
-  if (d <= 16) return launch_fwd<T, 1>(p, st);
-  if (d <= 32) return launch_fwd<T, 2>(p, st);
-  if (d <= 64) return launch_fwd<T, 4>(p, st);
-  if (d <= 128) return launch_fwd<T, 8>(p, st);
+  if (d <= 16) return launch_fwd<T, 1, WIDE>(p, st);
+  if (d <= 32) return launch_fwd<T, 2, WIDE>(p, st);
+  if (d <= 64) return launch_fwd<T, 4, WIDE>(p, st);
+  if (d <= 128) return launch_fwd<T, 8, WIDE>(p, st);
   return BMA_ERR_UNSUPPORTED;
 }
-template <typename T, typename TDO>
+template <typename T, typename TDO, bool WIDE>
 int dispatch_bwd(const SimtParams& p, cudaStream_t st) {
   const int d = p.a.d;
-  if (d <= 16) return launch_bwd<T, TDO, 1>(p, st);
-  if (d <= 32) return launch_bwd<T, TDO, 2>(p, st);
-  if (d <= 64) return launch_bwd<T, TDO, 4>(p, st);
-  if (d <= 128) return launch_bwd<T, TDO, 8>(p, st);
+  if (d <= 16) return launch_bwd<T, TDO, 1, WIDE>(p, st);
+  if (d <= 32) return launch_bwd<T, TDO, 2, WIDE>(p, st);
+  if (d <= 64) return launch_bwd<T, TDO, 4, WIDE>(p, st);
+  if (d <= 128) return launch_bwd<T, TDO, 8, WIDE>(p, st);
   return BMA_ERR_UNSUPPORTED;
 }
 
@@ -91,18 +91,27 @@ int dispatch_bwd(const SimtParams& p, cudaStream_t st) {
 int simt_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st) {
   BMA_REQUIRE(lists.q_block == TQ && lists.kv_block == TK, BMA_ERR_ARG);
   const SimtParams p = simt_params(a, spec, lists);
-  if (a.q.dtype == BMA_DTYPE_F32) return dispatch_fwd<float>(p, st);
-  return dispatch_fwd<__nv_bfloat16>(p, st);
+  if (a.q.dtype == BMA_DTYPE_F32) return dispatch_fwd<float, false>(p, st);
+  return dispatch_fwd<__nv_bfloat16, false>(p, st);
 }
 
 int simt_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st) {
   BMA_REQUIRE(lists.q_block == TQ && lists.kv_block == TK && lists.q_num, BMA_ERR_ARG);
   const SimtParams p = simt_params(a, spec, lists);
   const bool f32 = a.q.dtype == BMA_DTYPE_F32, do_f32 = a.d_o.dtype == BMA_DTYPE_F32;
-  if (f32 && do_f32) return dispatch_bwd<float, float>(p, st);
-  if (f32) return dispatch_bwd<float, __nv_bfloat16>(p, st);
-  if (do_f32) return dispatch_bwd<__nv_bfloat16, float>(p, st);
-  return dispatch_bwd<__nv_bfloat16, __nv_bfloat16>(p, st);
+  if (f32 && do_f32) return dispatch_bwd<float, float, false>(p, st);
+  if (f32) return dispatch_bwd<float, __nv_bfloat16, false>(p, st);
+  if (do_f32) return dispatch_bwd<__nv_bfloat16, float, false>(p, st);
+  return dispatch_bwd<__nv_bfloat16, __nv_bfloat16, false>(p, st);
+}
+
+int simt_wide_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st) {
+  return dispatch_fwd<float, true>(simt_params(a, spec, lists), st);
+}
+
+int simt_wide_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st) {
+  const SimtParams p = simt_params(a, spec, lists);
+  return a.d_o.dtype == BMA_DTYPE_F32 ? dispatch_bwd<float, float, true>(p, st) : dispatch_bwd<float, __nv_bfloat16, true>(p, st);
 }
 
 }  // namespace bma

@@ -378,7 +378,8 @@ int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const
     return rc;
   if ((rc = validate_lists(args, lists, kSm100Tile, false))) return rc;
   BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
-  BMA_REQUIRE(workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && workspace_bytes >= need, BMA_ERR_WORKSPACE);
+  if (!workspace || workspace_bytes < need) return simt_wide_fwd(*args, *spec, *lists, static_cast<cudaStream_t>(stream));
+  BMA_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15) == 0, BMA_ERR_WORKSPACE);
   return f32_fwd(*args, *spec, *lists, workspace, static_cast<cudaStream_t>(stream));
 }
 
@@ -397,7 +398,8 @@ int bma_attn_bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const
               BMA_ERR_UNSUPPORTED);
   if ((rc = validate_lists(args, lists, kSm100Tile, true))) return rc;
   BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
-  BMA_REQUIRE(workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && workspace_bytes >= need, BMA_ERR_WORKSPACE);
+  if (!workspace || workspace_bytes < need) return simt_wide_bwd(*args, *spec, *lists, static_cast<cudaStream_t>(stream));
+  BMA_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15) == 0, BMA_ERR_WORKSPACE);
   return f32_bwd(*args, *spec, *lists, workspace, static_cast<cudaStream_t>(stream));
 }
 

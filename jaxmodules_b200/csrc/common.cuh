@@ -303,6 +303,9 @@ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // Host-side dispatchers implemented in the individual .cu files.
 int simt_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st);
 int simt_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st);
+// float32 over lists of BMA_F32_TILE blocks
+int simt_wide_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st);
+int simt_wide_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, cudaStream_t st);
 int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, size_t ws_bytes,
               cudaStream_t st);
 size_t sm100_fwd_workspace_bytes(const bma_attn_args& a, const bma_block_lists& lists);
