@@ -131,7 +131,29 @@ struct SplitJob {
 struct SplitParams {
   SplitJob job[4];
   int B, d;
+  const uint8_t* used;   // null, or one byte per kv block [used_B, NKV] (jobs 1 and 2, K and V): 0 = no list names it
+  int used_B, NKV;
 };
+
+// used[b', kj] = 1 where a list of batch entry b' names kv block kj (a kv-side list; backward: or a q-side list of kj has an
+// entry), else 0.  One CTA per batch entry of the lists.
+__global__ void __launch_bounds__(256) used_blocks_kernel(bma_block_lists l, bool backward, uint8_t* __restrict__ used) {
+  __shared__ uint8_t mark[kMaxKvFwd];
+  for (int i = threadIdx.x; i < l.NKV; i += 256) mark[i] = 0;
+  __syncthreads();
+  const int rows = l.H * l.NQ, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = warp; r < rows; r += 8) {
+    const int64_t row = (int64_t)blockIdx.x * rows + r;
+    const int nfull = l.full_kv_num[row], npart = l.kv_num[row];
+    for (int i = lane; i < nfull; i += 32) mark[l.full_kv_idx[row * l.NKV + i]] = 1;
+    for (int i = lane; i < npart; i += 32) mark[l.kv_idx[row * l.NKV + i]] = 1;
+  }
+  if (backward)
+    for (int i = threadIdx.x; i < l.H * l.NKV; i += 256)
+      if (l.q_num[(int64_t)blockIdx.x * l.H * l.NKV + i] + l.full_q_num[(int64_t)blockIdx.x * l.H * l.NKV + i] > 0) mark[i % l.NKV] = 1;
+  __syncthreads();
+  for (int i = threadIdx.x; i < l.NKV; i += 256) used[(int64_t)blockIdx.x * l.NKV + i] = mark[i];
+}
 
 // One thread per 8 columns: 32 bytes in, three 16-byte lines out.  Bound by HBM (4 bytes read, 6 written per element), or
 // by launch latency where the tensors are small.
@@ -143,7 +165,7 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitParams p) {
   const bool f32 = job.t.dtype == BMA_DTYPE_F32;
   const bool vec = f32 && (reinterpret_cast<uintptr_t>(job.t.ptr) & 15) == 0 && ((job.t.stride_b | job.t.stride_l | job.t.stride_h) & 3) == 0;
   uint4* out = reinterpret_cast<uint4*>(job.out);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  auto split8 = [&](int64_t i) {
     const int c = (int)(i % kChunks) * 8;
     const int64_t row = i / kChunks;
     const int h = (int)(row % job.H);
@@ -168,6 +190,21 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitParams p) {
     for (int e = 0; e < 4; ++e) split3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
 #pragma unroll
     for (int q = 0; q < 3; ++q) out[q * n + i] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+  };
+  if (!p.used || blockIdx.y == 0 || blockIdx.y == 3) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) split8(i);
+    return;
+  }
+  // K and V: a kv block at a time, in pieces of 1024 lines so that a few blocks fill the chip as well
+  constexpr int kPiece = 1024;
+  const int parts = (BM * job.H * kChunks + kPiece - 1) / kPiece;
+  for (int64_t w = blockIdx.x; w < (int64_t)p.B * p.NKV * parts; w += gridDim.x) {
+    const int64_t blk = w / parts;
+    const int b = (int)(blk / p.NKV), l0 = (int)(blk % p.NKV) * BM, at = (int)(w % parts) * kPiece;
+    if (!__ldg(p.used + (int64_t)(p.used_B == 1 ? 0 : b) * p.NKV + l0 / BM)) continue;
+    const int64_t first = ((int64_t)b * job.L + l0) * job.H * kChunks;
+    const int end = min(at + kPiece, min(BM, job.L - l0) * job.H * kChunks);
+    for (int i = at + (int)threadIdx.x; i < end; i += blockDim.x) split8(first + i);
   }
 }
 
@@ -1636,8 +1673,16 @@ size_t plane_bytes(int B, int L, int H, int dp) { return (size_t)3 * B * L * H *
 size_t align_up(size_t x) { return (x + 1023) / 1024 * 1024; }
 
 struct Planes {
-  size_t q, k, v, d_o, total;   // offsets in the workspace
+  size_t q, k, v, d_o, used, total;   // offsets in the workspace
 };
+// Few queries against many keys may see a small part of them: then only the planes of listed kv blocks are made.  (What the
+// other blocks' planes hold is read by the dK / dV kernel alone, as the resident operand of a CTA that has no query tile.)
+// Marking takes a launch (2 us), the planes of 4M values of K and V as much; with more query tiles than a quarter of the kv
+// blocks, the other kernels take far longer than the planes.  (16 queries that see 512 of 65536 keys, B = 4, 16/4 heads of 64,
+// the whole call: 247 us with all planes, 64 with the listed ones.)
+bool used_blocks(const bma_attn_args& a) {
+  return 4 * ceil_div(a.N, BM) <= ceil_div(a.L, BM) && (int64_t)a.B * a.L * a.Hkv * a.d >= (1 << 22);
+}
 Planes planes_layout(const bma_attn_args& a, bool backward) {
   const int dp = padded_d(a);
   Planes p;
@@ -1645,13 +1690,20 @@ Planes planes_layout(const bma_attn_args& a, bool backward) {
   p.k = align_up(plane_bytes(a.B, a.N, a.Hq, dp));
   p.v = p.k + align_up(plane_bytes(a.B, a.L, a.Hkv, dp));
   p.d_o = p.v + align_up(plane_bytes(a.B, a.L, a.Hkv, dp));
-  p.total = p.d_o + (backward ? align_up(plane_bytes(a.B, a.N, a.Hq, dp)) : 0);
+  p.used = p.d_o + (backward ? align_up(plane_bytes(a.B, a.N, a.Hq, dp)) : 0);
+  p.total = p.used + (used_blocks(a) ? align_up((size_t)a.B * ceil_div(a.L, BM)) : 0);
   return p;
 }
 
-int launch_split(const bma_attn_args& a, const Planes& pl, uint8_t* ws, bool backward, cudaStream_t st) {
+int launch_split(const bma_attn_args& a, const bma_block_lists& l, const Planes& pl, uint8_t* ws, bool backward, cudaStream_t st) {
   SplitParams sp;
   sp.B = a.B; sp.d = a.d;
+  sp.used = nullptr; sp.used_B = l.B; sp.NKV = l.NKV;
+  if (used_blocks(a)) {
+    used_blocks_kernel<<<(unsigned)l.B, 256, 0, st>>>(l, backward, ws + pl.used);
+    count_launches(1);
+    sp.used = ws + pl.used;
+  }
   sp.job[0] = {a.q, ws + pl.q, a.N, a.Hq};
   sp.job[1] = {a.k, ws + pl.k, a.L, a.Hkv};
   sp.job[2] = {a.v, ws + pl.v, a.L, a.Hkv};
@@ -1692,7 +1744,7 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   const int dp = padded_d(a);
   F32Params p;
   int rc;
-  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, pl, w, false, st))) return rc;
+  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, lists, pl, w, false, st))) return rc;
   CUtensorMap mq, mk, mv;
   if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, dp, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, dp, BH)) ||
       (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, dp, BH)))
@@ -1715,7 +1767,7 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   uint8_t* w = static_cast<uint8_t*>(ws);
   F32Params p;
   int rc;
-  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, pl, w, true, st))) return rc;
+  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, lists, pl, w, true, st))) return rc;
   CUtensorMap mq, mk, mv, mdo, mqh, mkh, mvh, mdoh;
   if (a.d > 64) {
     if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, 128, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, 128, BM)) ||
