@@ -309,7 +309,7 @@ int bma_block_lists_visited(const bma_block_lists* lists, int64_t* visited, bma_
 /* Optional scratch of bma_attn_bwd (0 when the backend has no use for it).  Given a workspace of
  * at least this size, the tensor-core backward hands every bf16 dS tile (32 KB per VISITED
  * 128x128 block; the slots are addressed compactly -- a prefix over the block lists, built into
- * the front of the workspace by one small launch per call) from the dK/dV kernel to the dQ
+ * the front of the workspace by one or two small launches per call) from the dK/dV kernel to the dQ
  * kernel through that buffer instead of recomputing S and dP there: 5 instead of 7 MMAs per
  * block, for 32 KB of HBM traffic each way.
  *   visited_host: HOST array [lists->B * lists->H] of visited-block counts per list head (from

@@ -9,7 +9,7 @@
 // head, head_base = exclusive prefix over (b, h) in row-major order of the list heads' totals.  A launch over a
 // range of (batch, head) units subtracts the head_base of its first head.
 //
-// One small launch per backward call builds the tables from the kv-side lists into the front of the caller's workspace.
+// One small launch per backward call (two with many list heads) builds the tables from the kv-side lists into the front of the caller's workspace.
 #include <algorithm>
 
 #include "common.cuh"
@@ -19,6 +19,9 @@ namespace bma {
 namespace {
 
 constexpr int kMaxKvTilesBwd = 1024;  // the tensor-core backward takes L <= 131072
+// List heads up to which one launch builds all tables: eight warps take four heads each then, about as long as a second
+// launch.  (2048 heads of two rows, B = 32, H = 64, N = 256, forward and backward: 775 us with one launch, 689 with two.)
+constexpr int kHeadsInOneLaunch = 32;
 
 __device__ __forceinline__ int row_visits(const bma_block_lists& l, int64_t row) {
   return min(max(__ldg(l.full_kv_num + row), 0), l.NKV) + min(max(__ldg(l.kv_num + row), 0), l.NKV);
@@ -35,20 +38,23 @@ __device__ __forceinline__ long long block_sum256(long long v, long long* part) 
 }
 
 // All tables in one launch; every CTA adds up from the row counts what it needs itself, so that none waits for another
-// (three dependent launches before took 8 us; this one 3 - 5).
+// (three dependent launches before took 8 us; this one 3 - 5).  The last CTA alone reads the rows of all list heads: with
+// many heads that would be a chain of dependent reads on one SM, so there (kHeadsInOneLaunch) the CTAs of a head's last rows
+// write its total and a second launch (HEADS) adds the totals up.
 //   CTA head * ceil(NQ / 8) + g: rank[row][kj] = number of visited kv tiles below kj, or -1 when (row, kj) is not
 //     visited, for eight rows (one warp each), and row_base of these rows = visits of the head's rows before them;
 //   the last CTA: head_base[i], i in [0, B * Hq] = exclusive prefix over (b, h) of the list heads' totals.
 // (A row base counts list entries; a block listed twice leaves an unused slot behind.)
-__global__ void __launch_bounds__(256) slot_tables_kernel(bma_block_lists l, int B, int Hq, int32_t* __restrict__ rank,
+enum SlotPhase { ALL, ROWS, HEADS };
+__global__ void __launch_bounds__(256) slot_tables_kernel(SlotPhase phase, bma_block_lists l, int B, int Hq, int32_t* __restrict__ rank,
                                                           int32_t* __restrict__ row_base, int64_t* __restrict__ head_total,
                                                           int64_t* __restrict__ head_base) {
   __shared__ uint32_t bits[8][kMaxKvTilesBwd / 32];
   __shared__ long long part[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int groups = (l.NQ + 7) / 8;
-  if (blockIdx.x == gridDim.x - 1) {
-    const int LHEADS = l.B * l.H;
+  if (phase == HEADS || (phase == ALL && blockIdx.x == gridDim.x - 1)) {
+    const int LHEADS = phase == HEADS ? 0 : l.B * l.H;
     for (int i = w; i < LHEADS; i += 8) {   // one warp per list head
       long long s = 0;
       for (int r = lane; r < l.NQ; r += 32) s += row_visits(l, (int64_t)i * l.NQ + r);
@@ -97,6 +103,7 @@ __global__ void __launch_bounds__(256) slot_tables_kernel(bma_block_lists l, int
     int mine = before;
     for (int i = first; i < r; ++i) mine += row_visits(l, head_row + i);
     row_base[row] = mine;
+    if (phase == ROWS && r == l.NQ - 1) head_total[blockIdx.x / groups] = mine + row_visits(l, row);
   }
   const int words = (l.NKV + 31) / 32;
   bits[w][lane] = 0u;
@@ -171,8 +178,10 @@ int slot_tables_build(const bma_attn_args& a, const bma_block_lists& l, const Sl
   BMA_REQUIRE(l.NKV <= kMaxKvTilesBwd, BMA_ERR_LIMIT);
   const int64_t ctas = (int64_t)l.B * l.H * ((l.NQ + 7) / 8) + 1;
   BMA_REQUIRE(ctas <= INT32_MAX, BMA_ERR_LIMIT);
-  slot_tables_kernel<<<(unsigned)ctas, 256, 0, st>>>(l, a.B, a.Hq, t.rank, t.row_base, t.head_total, t.head_base);
-  count_launches(1);
+  const bool one = (int64_t)l.B * l.H <= kHeadsInOneLaunch;
+  slot_tables_kernel<<<(unsigned)(one ? ctas : ctas - 1), 256, 0, st>>>(one ? ALL : ROWS, l, a.B, a.Hq, t.rank, t.row_base, t.head_total, t.head_base);
+  if (!one) slot_tables_kernel<<<1, 256, 0, st>>>(HEADS, l, a.B, a.Hq, t.rank, t.row_base, t.head_total, t.head_base);
+  count_launches(one ? 1 : 2);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
 }
