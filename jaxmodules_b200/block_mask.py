@@ -313,8 +313,30 @@ def create_block_mask(mask_mod, B: int, H: int, Q_LEN: int, KV_LEN: int, BLOCK_S
         _, t = compile_block_lists(dmask, B, H, Q_LEN, KV_LEN, QB, KVB, device, out_B=B, out_H=H, q_side=True,
                                    floor_blocks=True)
     NQ, NKV = Q_LEN // QB, KV_LEN // KVB
-    return BlockMask(B=B, H=H, Q_LEN=NQ * QB, KV_LEN=NKV * KVB, Q_BLOCK_SIZE=QB, KV_BLOCK_SIZE=KVB,
+    bm = BlockMask(B=B, H=H, Q_LEN=NQ * QB, KV_LEN=NKV * KVB, Q_BLOCK_SIZE=QB, KV_BLOCK_SIZE=KVB,
                      kv_num_blocks=t["kv_num_blocks"], kv_indices=t["kv_indices"],
                      q_num_blocks=t["q_num_blocks"], q_indices=t["q_indices"],
                      full_kv_num_blocks=t["full_kv_num_blocks"], full_kv_indices=t["full_kv_indices"],
                      full_q_num_blocks=t["full_q_num_blocks"], full_q_indices=t["full_q_indices"], mask_mod=mask_mod)
+    del t["_workspace"]
+    bm._made = (mask_mod, terms, _versions(terms), (B, H, NQ * QB, NKV * KVB, QB, KVB), t)
+    return bm
+
+
+def _versions(terms):
+    """How often the arrays of a mask have been written to; None where that is not counted (inference mode)."""
+    arrays = [x for x in (terms.seg_q, terms.seg_k) if x is not None]
+    return None if any(x.is_inference() for x in arrays) else [x._version for x in arrays]
+
+
+def is_as_made(bm: BlockMask) -> bool:
+    """True for a BlockMask that ``create_block_mask`` returned and whose sizes, mask and arrays nobody has replaced or written to
+    since: its lists are the blocks of its mask, every one once and alike on both sides.  (The arrays are held, so that
+    their identity means something; they were new then, at version 0.)"""
+    made = getattr(bm, "_made", None)
+    if made is None:
+        return False
+    mask_mod, terms, versions, sizes, arrays = made
+    return (bm.mask_mod is mask_mod and getattr(mask_mod, "terms", None) is terms and versions is not None and versions == _versions(terms)
+            and sizes == (bm.B, bm.H, bm.Q_LEN, bm.KV_LEN, bm.Q_BLOCK_SIZE, bm.KV_BLOCK_SIZE)
+            and all(getattr(bm, n) is x and not x.is_inference() and x._version == 0 for n, x in arrays.items()))
