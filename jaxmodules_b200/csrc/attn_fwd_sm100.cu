@@ -1554,6 +1554,9 @@ bool sm100_supported(const bma_attn_args& a) {
 // A unit is a tile of packed rows of one (head set, batch); heads are packed when that makes fewer tiles than one per head
 // and the lists are the same for the heads of a group.  The number of splits minimises waves x (run of tiles + set-up): a
 // tile of K and V takes about 1.5 us at an SM's share of the HBM rate, set-up, merge and a workspace round trip about 5.
+// (Measured with heads of 128, 16 queries on 8192 keys.)  Splitting fills a chip that units alone leave partly idle: with 32
+// and more CTAs for every SM there is no such gap, and the partials (66 KB a CTA, 315 MB at this bound) would only grow.
+constexpr int kMaxSplitWaves = 32;
 struct SplitPlan { int heads, tile_queries, q_tiles, units, splits; };
 static SplitPlan split_plan(const bma_attn_args& a, const bma_block_lists& l) {
   SplitPlan p{1, BM, 1, 0, 0};
@@ -1567,9 +1570,14 @@ static SplitPlan split_plan(const bma_attn_args& a, const bma_block_lists& l) {
   const int64_t units = (int64_t)a.B * (a.Hq / p.heads) * p.q_tiles;
   if (units > (1 << 20)) return p;
   p.units = (int)units;
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? std::max(n, 1) : 148;
+  }();
   double best = 1e30;
-  for (int s = 1; s <= std::min(l.NKV / 2, 148); ++s) {
-    const double cost = std::ceil((double)units * s / 148.0) * (std::ceil((double)l.NKV / s) * 1.5 + 5.0) + (s > 1 ? 3.0 : 0.0);
+  for (int s = 1; s <= std::min(l.NKV / 2, sms); ++s) {
+    if (s > 1 && units * s > (int64_t)kMaxSplitWaves * sms) break;
+    const double cost = std::ceil((double)units * s / sms) * (std::ceil((double)l.NKV / s) * 1.5 + 5.0) + (s > 1 ? 3.0 : 0.0);
     if (cost < best) { best = cost; p.splits = s; }
   }
   return p;

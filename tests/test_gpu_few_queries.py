@@ -43,3 +43,21 @@ def test_few_queries(B, N, L, Hq, Hkv, d, mask, out):
     got, want = lse.cpu().numpy(), ref["lse"]
     dead = np.isinf(want)
     assert np.array_equal(np.isinf(got), dead) and np.abs(got - want)[~dead].max() <= 1e-3
+
+
+def test_split_workspace_is_bounded():
+    """The partial results of the runs stay below 32 waves of CTAs whatever the sizes (nothing is launched here)."""
+    import ctypes as C
+    from jaxmodules_b200 import _native as nat
+    from jaxmodules_b200 import attention as A
+    q, k = (torch.zeros(1, n, 1, 128, dtype=torch.bfloat16, device="cuda") for n in (16, 256))
+    a, lists = A._make_args(q, k, k), nat.BlockLists()
+    cta = 128 * (128 + 2) * 4
+    most = 32 * torch.cuda.get_device_properties(0).multi_processor_count * cta
+    asked = []
+    for B, N, Hq, Hkv, L in ((4, 16, 32, 8, 8192), (16, 127, 64, 64, 65536), (250, 127, 16, 4, 524288), (312, 127, 64, 16, 524288), (4000, 1, 2, 2, 524288)):
+        a.B, a.N, a.Hq, a.Hkv, a.L = B, N, Hq, Hkv, L
+        lists.B = lists.H = lists.NQ = 1
+        lists.NKV = L // 128
+        asked.append(nat.lib().bma_attn_fwd_workspace_bytes(C.byref(a), C.byref(lists)))
+    assert asked[0] > 0 and max(asked) <= most, asked
