@@ -330,6 +330,11 @@ def _traced_causal(b, h, q, k):
     return k <= q
 
 
+def backend_name(be, tile):
+    """bma_attn_plan's backend; float32 on the tensor core is not its choice but shows in the tile."""
+    return "tcgen05, float32 as three bf16 planes" if be == 1 and tile == 128 else {1: "simt", 2: "tcgen05"}.get(be, str(be))
+
+
 def measure_config(name, dev, steps=5, warmup=3, seed=100, traced=False):
     """One side workload, device-timed: forward + backward through masked_attention_via_map on inputs generated
     on the device; the launch groups are timed separately with CUDA events on the launching stream.  ``traced``:
@@ -349,7 +354,7 @@ def measure_config(name, dev, steps=5, warmup=3, seed=100, traced=False):
     if traced:
         assert w["mask"] == "causal"
         kw = dict(mask_fn=_traced_causal, block_size=w["bs"])
-    be, tq, tk = A.plan(Q, K, V)
+    be, (tq, tk) = A.plan(Q, K, V)[0], A.tiles(Q, K, V)
     terms = M.MaskTerms(causal=True) if kw.get("is_causal") else M.terms_from_mask_fn(kw["mask_fn"], B, H, L, L, device=dev)
     if kw.get("window_size") is not None:
         bs = w["bs"]
@@ -389,7 +394,7 @@ def measure_config(name, dev, steps=5, warmup=3, seed=100, traced=False):
     in_bytes = 3 * B * L * H * d * Q.element_size() + dO.numel() * 4
     out = {"l2": ("inputs (%.0f MB) exceed the 126 MB L2; no flush needed" % (in_bytes / 1e6)) if in_bytes > 126e6 else
                  ("inputs (%.2f MB) fit in L2 and are not flushed: a latency figure, not a bandwidth one" % (in_bytes / 1e6)),
-           "workload": w["desc"], "backend": {1: "simt", 2: "tcgen05"}.get(be, str(be)), "steps": steps, "warmup": warmup,
+           "workload": w["desc"], "backend": backend_name(be, tq), "steps": steps, "warmup": warmup,
            "nonempty_blocks": blocks, "ms_per_step": ms, "value": tf(step_flops, ms), "fwd_tflops": tf(fwd_flops, per.get("fwd")),
            "bwd_tflops": tf(step_flops - fwd_flops, per.get("bwd")), "kernel_ms": per, "status": A.device_status(dev)}
     if be == 2:
@@ -430,7 +435,7 @@ def block_mask_build_entry(w, dev, steps, warmup):
     torch.cuda.empty_cache()
     return {"workload": "create_block_mask, " + w["desc"], "ms": ms, "list_bytes_per_build": out_bytes, "GB/s": gbs,
             "frac_of_hbm": gbs / hbm, "peak": hbm, "peak_kind": peak_kind,
-            "kernels": "classify_kernel + compact_both_kernel"}
+            "kernels": "compact_kernel (classifies its rows itself)"}
 
 
 def c5_head_shards(rank, world, dev, dist, steps=3, warmup=2):
@@ -716,7 +721,8 @@ def main():
         torch.cuda.synchronize(dev)
 
     # FLOP count from the block lists the kernels actually walk
-    be, tq, tk = A.plan(*((x.transpose(1, 2) for x in (Q, K, V)) if flex else (Q, K, V)))
+    qkv = [x.transpose(1, 2) for x in (Q, K, V)] if flex else (Q, K, V)
+    be, (tq, tk) = A.plan(*qkv)[0], A.tiles(*qkv)
     terms = M.MaskTerms(causal=True) if kw.get("is_causal") else M.terms_from_mask_fn(kw["mask_fn"], B, H, L, L)
     if kw.get("window_size") is not None:
         bs = w["bs"]
@@ -888,7 +894,7 @@ def main():
             "config": {"workload": w["desc"], "api": "flex_attention [B,H,L,d] + BlockMask(128)" if flex else "masked_attention_via_map [B,L,H,d]",
                        "per_gpu_batch": B, "global_batch": B * world,
                        "parallelism": f"batch x head shards, {world} GPU(s), no collective",
-                       "backend": {1: "simt", 2: "tcgen05"}.get(be, str(be)), "tile": tq, "nonempty_blocks_per_gpu": blocks,
+                       "backend": backend_name(be, tq), "tile": tq, "nonempty_blocks_per_gpu": blocks,
                        "l2": "inputs (Q,K,V,dO > 1 GB) exceed the 126 MB L2; no flush needed",
                        "flop_model": "fwd 4*bq*bk*d per non-empty block, bwd 2.5x fwd"},
             "fwd_tflops": fwd_tf, "bwd_tflops": bwd_tf,

@@ -149,6 +149,9 @@ def _device_guard(device):
 
 
 def plan(Q, K, V, backend=nat.BMA_BACKEND_AUTO, backward: bool = False, key_bias=None, scale=None):
+    """(backend, q_tile, kv_tile) of ``bma_attn_fwd`` / ``bma_attn_bwd`` for these tensors.  float32 calls do not go through these
+    two unless a backend is forced (here it is the FP32 tile kernels), but through ``bma_attn_fwd_f32`` / ``bma_attn_bwd_f32``:
+    ``tiles`` says what the attention passes really walk."""
     """(backend, q_tile, kv_tile) the library will use for the forward (or backward) pass."""
     a = _make_args(Q, K, V, backend, scale, key_bias)
     be, tq, tk = C.c_int32(), C.c_int32(), C.c_int32()
@@ -463,6 +466,9 @@ def masked_attention_via_map(
     number of ``block_size`` blocks, clamped at the sequence ends, applied on top of the mask
     (jaxmodules/attention.py:161-167, 199-204); without ``window_size`` the result does not
     depend on ``block_size``.  Rows without any allowed key return 0.
+
+    float32 inputs keep float32 accuracy (2e-6 in the 2-norm) and the effect that infinities and NaN have in float32
+    arithmetic, block-sparse: what lies in a key block that a query block does not visit does not reach it.
 
     Extras (keyword-only, defaulting to the reference's behaviour): ``out_dtype`` — the
     reference returns float32 for every input dtype, pass ``torch.bfloat16`` to halve the

@@ -1,4 +1,4 @@
-// Backward dK / dV for bf16, head dim 128, on the sm_100a tensor core (tcgen05 + TMEM + TMA).
+// Backward dK / dV for bf16, head dims 64 and 128, on the sm_100a tensor core (tcgen05 + TMEM + TMA).
 // (dQ is produced by a query-major kernel — attn_bwd_dq_replay_sm100.cu from the dS tiles this
 // kernel stores, or attn_bwd_dq_sm100.cu by recomputation; splitting the backward in two keeps every
 // accumulator in tensor memory: no global reductions, no float32 workspace, and a fixed summation order.)
@@ -23,7 +23,7 @@
 // that eight warps of 208 registers left open.  Eight warps with one hand-over of Pt and dSt together -> eight with two ->
 // sixteen with two: packed documents (B=4 L=16384 H=16 d=128) 1960 -> 1865 -> 1730 us, lambda window 2 x 1000 48 -> 44 ->
 // 38 us, sliding window L=8192 464 -> 453 -> 437 us, causal d=64 (B=4 L=4096 H=32) 898 -> 840 -> 848 us; causal B=8 L=4096
-// H=32 d=128 is at the power limit (about 1.5 GHz) and stays at 2160 us.
+// H=32 d=128 stays at 2160 us (3200 cycles per tile, at about 1.5 GHz).
 //
 // With a scratch buffer (BwdParams::ds_out) the kernel also hands every dSt tile to the dQ kernel:
 // each consumer thread stages its 32 dSt values as half of a 128-byte line of a 32 KB tile image laid out
@@ -97,7 +97,7 @@ struct BwdParams {
   int nhk;          // than the whole problem), and the number of kv heads in the range
 };
 
-// Rendezvous of the 256 consumer threads on an mbarrier: arrive, then a bounded wait (a plain
+// Rendezvous of the kConsumers (512) consumer threads on an mbarrier: arrive, then a bounded wait (a plain
 // bar.sync would wait forever for a thread that gave up on an earlier wait).
 __device__ __forceinline__ bool consumer_sync(uint64_t* bar, uint32_t parity) {
   mbar_arrive(bar);

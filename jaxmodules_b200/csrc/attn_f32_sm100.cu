@@ -1,15 +1,15 @@
 // float32 attention (forward, dK/dV, dQ) on the sm_100a tensor core.
 //
-// A float32 value is the exact sum of three bfloat16 values (8 + 8 + 8 significand bits), and a product of two bfloat16
-// values is exact in the float32 accumulator.  Every operand is therefore carried as three bf16 planes hi + mid + lo, and
+// A float32 value between 2^-110 and 3.38e38 in magnitude is the exact sum of three bfloat16 values (8 + 8 + 8 significand bits),
+// and a product of two bfloat16 values is exact in the float32 accumulator.  Every operand is therefore carried as three bf16 planes hi + mid + lo, and
 // every matrix product is the sum of the six plane products whose weight reaches 2^-24 of the result:
 //     x y  ~  lo hi + hi lo + mid mid + mid hi + hi mid + hi hi        (dropped: mid lo, lo mid, lo lo <= 2^-24 |x y|)
 // issued smallest terms first.  Six passes at the bf16 rate leave 270 TFLOP/s of the measured tensor peak, against
 // 72 TFLOP/s of the FP32 FMA pipes (and the 14 - 19 the FP32 tile kernels of attn_simt.cu reach).
 //
-// Accuracy is held to that of an FP32 FMA chain: the tensor core truncates when it adds to its accumulator, so no
-// accumulation runs longer than one 64-wide tile there -- O, dQ, dK and dV are summed over the tiles in registers, with
-// rounded FP32 adds.  Against float64 the 2-norm error is 1.4e-7 - 3.5e-7 (causal, B=2 L=2048 H=16 d=64; the FP32 tile
+// Accuracy is held to that of an FP32 FMA chain: the tensor core truncates when it adds to its accumulator, so accumulations
+// are short there -- the plane products of one 64-wide tile (of the padded head dimension, 64 or 128, for S and dP) -- and O,
+// dQ, dK and dV are summed over the tiles in registers, with rounded FP32 adds.  Against float64 the 2-norm error is 1.4e-7 - 3.5e-7 (causal, B=2 L=2048 H=16 d=64; the FP32 tile
 // kernels: 4.1e-7 - 8.5e-7).
 //
 // Measured there: forward 134 us (tile kernels 861), dK/dV 218 (1383), dQ 158 (1357), the two splits 21 each; forward with
@@ -22,6 +22,14 @@
 // Where a product has only 64 columns of output per operand (64 keys, 64 queries, 64 head columns) the hi and mid planes
 // of its B operand are stacked to N = 128: a 128x64x16 MMA takes 53 cycles, a 128x128x16 one 64.  The two accumulator
 // halves are added when they are read.
+//
+// Order: such a sum is a chain of 64- and 128-column MMAs into the same columns, issued by one thread with nothing between
+// them, and the first of a region overwrites it.  PTX promises the order of tcgen05.mma pairs of one accumulator and one
+// shape; that pairs of different shapes run in the order of issue too is how the tensor core of an SM works through the
+// MMAs of a CTA, not a written rule.  A swap would lose whole products (2^-8 of the result or more, and not the same twice):
+// every float32 test would see it, and tests/test_gpu_kernel_variants.py repeats calls for it.  One shape throughout would cost
+// 256 cycles per 16-deep step with 128 columns (and a zero plane behind every lo plane, a third more shared memory for the
+// operand), 318 with 64, instead of 234.
 //
 // Tensor memory columns hold the accumulators of a tile and then, over the columns that the reading thread has just
 // consumed, the three planes of P or dS as A operands (per 16 keys: 8 columns hi, 8 mid, and 8 lo in the other half).

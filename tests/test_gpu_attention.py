@@ -489,12 +489,15 @@ def test_tensor_core_backend_is_selected():
     Q32 = torch.zeros(1, 256, 2, 32, dtype=torch.bfloat16, device="cuda")
     assert A.plan(Q32, Q32, Q32)[0] == nat.BMA_BACKEND_SIMT
     Qf = torch.zeros(1, 256, 2, 64, dtype=torch.float32, device="cuda")
-    assert A.plan(Qf, Qf, Qf)[0] == nat.BMA_BACKEND_SIMT
+    assert A.plan(Qf, Qf, Qf)[0] == nat.BMA_BACKEND_SIMT     # bma_attn_fwd's answer; the attention passes go elsewhere:
+    for backward in (False, True):
+        assert A.tiles(Qf, Qf, Qf, backward=backward) == (128, 128)
+        assert A.tiles(Qf, Qf, Qf, nat.BMA_BACKEND_SIMT, backward=backward) == (64, 64)
     rc = C.c_int32()
     assert nat.lib().bma_device_status(torch.cuda.current_stream().cuda_stream, C.byref(rc)) == nat.BMA_OK and rc.value == 0
 
 
-@pytest.mark.parametrize("dtype,d", [(torch.float32, 16), (torch.bfloat16, 128)], ids=["f32_simt", "bf16_tcgen05"])
+@pytest.mark.parametrize("dtype,d", [(torch.float32, 16), (torch.bfloat16, 128)], ids=["f32", "bf16_tcgen05"])
 def test_kernel_fn_family(dtype, d):
     """kernel_fn = exp(a*q.k + b): threshold_kernel (jaxmodules/attention.py:18-36) and the custom
     kernel of the reference's tests/test_mapped_attention.py:1122-1142; forward, lse and gradients."""

@@ -169,6 +169,8 @@ def test_grad_reference_shapes():
 
 
 def routes_for(q, k, v, bm, grads=True):
+    """The route over the tiles that plan() names: for float32 those of the FP32 tile kernels (test_gpu_flex_f32_routes.py has the
+    routes that float32 calls take by themselves)."""
     Q, K, V = (t.transpose(1, 2) for t in (q, k, v))
     tiles = [A.plan(Q, K, V)[1:]] + ([A.plan(Q, K, V, backward=True)[1:]] if grads else [])
     return flex_route(bm, q.shape[0], q.shape[1], tiles, q.device)
