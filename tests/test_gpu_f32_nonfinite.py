@@ -79,3 +79,21 @@ def test_expected_values(d):
     s = torch.einsum("nhd,lhd->hnl", t["q"][0, :, :1].double().cpu(), t["k"][0, :, :1].double().cpu()) / d ** 0.5
     ref = torch.einsum("hnl,lhd->nhd", torch.softmax(s, -1), t["v"][0, :, :1].double().cpu())
     assert (O[0, :, :1] - ref).abs().max() <= 1e-5
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_bf16_output_and_cotangent(d):
+    """float32 inputs with a bfloat16 output, so that the cotangent is bfloat16 too.  delta is taken from the rounded O (2^-9), which
+    bounds how far dQ and dK of the two sides may differ; O itself by a rounding."""
+    t = _inputs(d, 200, "do_inf")
+    t["do"] = t["do"].bfloat16()
+    kw = dict(is_causal=True, out_dtype=torch.bfloat16)
+    out = []
+    for backend in (nat.BMA_BACKEND_AUTO, nat.BMA_BACKEND_SIMT):
+        q, k, v = (t[n].clone().requires_grad_(True) for n in "qkv")
+        O = jm.masked_attention_via_map(q, k, v, backend=backend, **kw)
+        out.append([x.detach().float() for x in (O, *torch.autograd.grad(O, (q, k, v), t["do"]))])
+    for name, g, w in zip(("O", "dQ", "dK", "dV"), *out):
+        assert torch.equal(torch.isnan(g), torch.isnan(w)) and torch.equal(torch.isinf(g), torch.isinf(w)), name
+        fin = torch.isfinite(w)
+        assert (g[fin] - w[fin]).norm() <= (2e-6 if name == "dV" else 4e-3) * w[fin].norm(), name
