@@ -318,8 +318,9 @@ def create_block_mask(mask_mod, B: int, H: int, Q_LEN: int, KV_LEN: int, BLOCK_S
                      q_num_blocks=t["q_num_blocks"], q_indices=t["q_indices"],
                      full_kv_num_blocks=t["full_kv_num_blocks"], full_kv_indices=t["full_kv_indices"],
                      full_q_num_blocks=t["full_q_num_blocks"], full_q_indices=t["full_q_indices"], mask_mod=mask_mod)
-    del t["_workspace"]
-    bm._made = (mask_mod, terms, _versions(terms), (B, H, NQ * QB, NKV * KVB, QB, KVB), t)
+    if isinstance(mask_mod, _masks.StructuredMask):
+        del t["_workspace"]
+        bm._made = (mask_mod, terms, terms.seg_q is not None and _versions(terms), (B, H, NQ * QB, NKV * KVB, QB, KVB), t)
     return bm
 
 
@@ -337,6 +338,7 @@ def is_as_made(bm: BlockMask) -> bool:
     if made is None:
         return False
     mask_mod, terms, versions, sizes, arrays = made
-    return (bm.mask_mod is mask_mod and getattr(mask_mod, "terms", None) is terms and versions is not None and versions == _versions(terms)
+    return (bm.mask_mod is mask_mod and mask_mod.terms is terms
+            and (terms.seg_q is None or (versions is not None and versions == _versions(terms)))
             and sizes == (bm.B, bm.H, bm.Q_LEN, bm.KV_LEN, bm.Q_BLOCK_SIZE, bm.KV_BLOCK_SIZE)
             and all(getattr(bm, n) is x and not x.is_inference() and x._version == 0 for n, x in arrays.items()))
