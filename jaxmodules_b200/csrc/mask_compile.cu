@@ -146,6 +146,9 @@ __device__ __forceinline__ int block_flag(const bma_mask_spec& spec, const SegSu
 // that a 128 x 128 block is four batches of independent loads (stops as soon as the block is known to be partial).
 // Element by element with a row at a time, the 8 x 8 blocks of 128 x 128 of a bit table took 122 us in a launch of their own;
 // the whole build of their lists, scan included, now takes 12.
+// The first 32 x 32 elements come first by themselves: most blocks that a segment edge crosses are known to be partial then, and
+// a batch of 32 x 128 segment ids costs four times as many comparisons (documents of 77 tokens, 16 x 4096, whole build
+// with blocks of 64: element by element 63 us, batches alone 76, now 66; blocks of 128: 75, 68, 61).
 __device__ __forceinline__ int scan_block(const bma_mask_spec& spec, int cb, int ch, int qi, int kj, int QB, int KVB) {
   const int lane = threadIdx.x & 31;
   const MaskView m = make_mask_view(spec, cb, ch);
@@ -153,17 +156,19 @@ __device__ __forceinline__ int scan_block(const bma_mask_spec& spec, int cb, int
   const int q_end = min(q0 + QB, spec.q_valid), k_end = min(k0 + KVB, spec.k_valid);
   bool any = false;
   bool all = (q0 + QB <= spec.q_valid) && (k0 + KVB <= spec.k_valid);
-  for (int r = q0; r < q_end; r += 32) {
+  for (int step = 0; !(any && !all); ++step) {
+    const int r = q0 + max(step - 1, 0) * 32, k_to = step == 0 ? min(k0 + 32, k_end) : k_end;
+    if (r >= q_end) break;
     const int q = r + lane;
     bool row_any = false, row_all = true;
     if (q < q_end) {
       int jlo, jhi;
       row_interval(m, q, k0, jlo, jhi);
-      for (int kb = k0; kb < k_end; kb += 128) {
+      for (int kb = k0; kb < k_to; kb += 128) {
         uint32_t bits[4], want[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const int j0 = kb - k0 + c * 32, n = min(32, k_end - kb - c * 32);
+          const int j0 = kb - k0 + c * 32, n = min(32, k_to - kb - c * 32);
           want[c] = n <= 0 ? 0u : 0xffffffffu >> (32 - n);
           const int lo = max(jlo - j0, 0), hi = min(jhi - j0, 31);
           bits[c] = (lo <= hi) ? ((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) & want[c] : 0u;
@@ -178,7 +183,7 @@ __device__ __forceinline__ int scan_block(const bma_mask_spec& spec, int cb, int
     }
     any |= __any_sync(0xffffffffu, row_any) != 0;
     all &= __all_sync(0xffffffffu, row_all) != 0;
-    if (any && !all) break;
+    if (r + 32 >= q_end && k_to == k_end) break;   // (a block of 32 x 32 is done after the first look)
   }
   return all ? 2 : (any ? 1 : 0);
 }
@@ -374,6 +379,10 @@ __global__ void __launch_bounds__(kThreads) compact_kernel(const __grid_constant
 // (In closed form the row is always classified here: 1024 x 1024 blocks, both sides, 32 heads: 93 us against 101 with the
 // flags written and read back, of which 82 us are the index arrays at the copy rate.)
 constexpr int kInlineScanWidth = 32;
+// ... and most blocks of such rows: each is scanned once per list side there, which costs more than two launches once the chip is
+// full.  (32 x 32 blocks of 128 of a bit table per head, whole build: 32 heads 64 us in separate passes, 62 here; 512 heads 125
+// and 133.)
+constexpr int64_t kInlineScanBlocks = 1 << 15;
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -455,8 +464,8 @@ int mask_compile_launch(const bma_mask_spec& spec, int B, int H, const bma_block
                         ((spec.flags & BMA_MASK_SEGMENT) && !(spec.flags & BMA_MASK_COMPILE_CONSERVATIVE));
   const int width = std::max(l.NQ, l.NKV);
   RowSource src{nullptr, spec, seg, l.q_block, l.kv_block};
-  if (may_scan && width > kInlineScanWidth) {
-    const int64_t blocks = (int64_t)p.CB * p.CH * l.NQ * l.NKV;
+  const int64_t blocks = (int64_t)p.CB * p.CH * l.NQ * l.NKV;
+  if (may_scan && (width > kInlineScanWidth || blocks > kInlineScanBlocks)) {
     const int grid = (int)std::min<int64_t>((blocks + kThreads - 1) / kThreads, (int64_t)sm_count * 16);
     BMA_CUDA_TRY(cudaMemsetAsync(l.kv_num, 0, sizeof(int32_t), st));
     classify_kernel<<<grid, kThreads, 0, st>>>(spec, p.CB, p.CH, l.NQ, l.NKV, l.q_block, l.kv_block, seg, flags, l.kv_idx, l.kv_num);
