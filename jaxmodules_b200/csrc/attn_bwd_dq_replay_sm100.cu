@@ -61,6 +61,8 @@ struct ReplayParams {
   const int32_t* row_base;
   int64_t capacity;
   int b0, h0, nh;
+  int pairs;       // ceil(query tiles / 2), one CTA each
+  bool by_rank;    // order of the CTAs, see cta_of
   int* status;
 };
 
@@ -72,8 +74,11 @@ bwd_dq_replay_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   ReplaySmem<HD>& sm = *reinterpret_cast<ReplaySmem<HD>*>(smem_raw);
 
   const bma_attn_args& a = p.a;
-  const int pair = (int)gridDim.x - 1 - (int)blockIdx.x;  // heaviest causal tiles first
-  const int h = blockIdx.y + p.h0, b = blockIdx.z + p.b0;
+  int pair, h, b;
+  cta_of(p.by_rank, pair, h, b);
+  pair = p.pairs - 1 - pair;   // the last pair of a causal mask has the longest walk
+  h += p.h0;
+  b += p.b0;
   const int hk = h / (a.Hq / a.Hkv);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int wg = warp >> 2;
@@ -282,7 +287,9 @@ int sm100_bwd_dq_from_ds(const bma_attn_args& a, const bma_block_lists& lists, c
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
 
-  dim3 grid(ceil_div(ceil_div(a.N, BM), 2), p.nh, nb);
+  p.pairs = ceil_div(ceil_div(a.N, BM), 2);
+  p.by_rank = longest_first(p.pairs, p.nh, nb, (int64_t)2 * a.L * a.d / G);
+  const dim3 grid = cta_grid(p.by_rank, p.pairs, p.nh, nb);
   auto launch = [&](auto kernel, size_t smem) -> int {
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<grid, kThreads, smem, st>>>(mk, mdq, p);

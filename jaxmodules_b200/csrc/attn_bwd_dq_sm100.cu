@@ -64,6 +64,8 @@ struct DqParams {
   bma_attn_args a;
   bma_mask_spec spec;
   bma_block_lists l;
+  int pairs;       // ceil(query tiles / 2), one CTA each
+  bool by_rank;    // order of the CTAs, see cta_of
   float scale_log2;
   int* status;
 };
@@ -81,8 +83,9 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   DqSmem<HD>& sm = *reinterpret_cast<DqSmem<HD>*>(smem_raw);
 
   const bma_attn_args& a = p.a;
-  const int pair = (int)gridDim.x - 1 - (int)blockIdx.x;  // heaviest causal tiles first
-  const int h = blockIdx.y, b = blockIdx.z;
+  int pair, h, b;
+  cta_of(p.by_rank, pair, h, b);
+  pair = p.pairs - 1 - pair;   // the last pair of a causal mask has the longest walk
   const int hk = h / (a.Hq / a.Hkv);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // provably warp-uniform
   const int wg = warp >> 2;
@@ -458,7 +461,9 @@ int sm100_bwd_dq(const bma_attn_args& a, const bma_mask_spec& spec, const bma_bl
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
 
-  dim3 grid(ceil_div(ceil_div(a.N, BM), 2), a.Hq, a.B);
+  p.pairs = ceil_div(ceil_div(a.N, BM), 2);
+  p.by_rank = longest_first(p.pairs, a.Hq, a.B, (int64_t)4 * a.L * a.d * a.Hkv / a.Hq);
+  const dim3 grid = cta_grid(p.by_rank, p.pairs, a.Hq, a.B);
   auto launch = [&](auto kernel, size_t smem) -> int {
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<grid, kThreads, smem, st>>>(mq, mk, mv, mdo, mdq, p);

@@ -95,6 +95,7 @@ struct BwdParams {
   int64_t capacity; // slots the buffer holds (a slot index beyond it is reported, never written)
   int b0, hk0;      // first batch / kv head of this launch (the grid covers a range when the scratch is smaller
   int nhk;          // than the whole problem), and the number of kv heads in the range
+  bool by_rank;     // order of the CTAs, see cta_of
 };
 
 // Rendezvous of the kConsumers (512) consumer threads on an mbarrier: arrive, then a bounded wait (a plain
@@ -118,8 +119,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   BwdSmem<HD>& sm = *reinterpret_cast<BwdSmem<HD>*>(smem_raw);
 
   const bma_attn_args& a = p.a;
-  const int kj = blockIdx.x;  // causal: kv tile 0 sees the most q tiles, so launch order is already heavy-first
-  const int hk = blockIdx.y + p.hk0, b = blockIdx.z + p.b0;
+  int kj, hk, b;   // (under a causal mask kv tile 0 sees the most q tiles)
+  cta_of(p.by_rank, kj, hk, b);
+  hk += p.hk0;
+  b += p.b0;
   const int G = a.Hq / a.Hkv;
   const int k0 = kj * BT;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // provably warp-uniform
@@ -518,7 +521,8 @@ template <typename P>
 static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
                        const CUtensorMap& mdk, const CUtensorMap& mdv, P& p, int b0, int nb, int hk0, int nhk, cudaStream_t st) {
   p.b0 = b0; p.hk0 = hk0; p.nhk = nhk;
-  dim3 grid(ceil_div(a.L, BT), nhk, nb);
+  p.by_rank = longest_first(ceil_div(a.L, BT), nhk, nb, (int64_t)4 * a.N * a.d * (a.Hq / a.Hkv));
+  const dim3 grid = cta_grid(p.by_rank, ceil_div(a.L, BT), nhk, nb);
   int rc;
   auto launch = [&](auto kernel, size_t smem) -> int {
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

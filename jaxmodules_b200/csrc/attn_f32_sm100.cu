@@ -222,6 +222,7 @@ struct F32Params {
   bma_block_lists l;
   float scale_log2;
   int* status;
+  LaunchOrder order;
 };
 
 // ---- results that are not finite ----------------------------------------------------------------------------------
@@ -370,8 +371,12 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   constexpr int kBoxes = Smem::kBoxes, kStages = Smem::kStages;
   const bma_attn_args& a = p.a;
-  const int qi = (int)gridDim.x - 1 - (int)blockIdx.x;   // heaviest causal tiles first
-  const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.Hq / a.Hkv);
+  int qi, h;
+  cta_of(p.order, qi, h);
+  qi = p.order.tiles - 1 - qi;
+  const int b = h / a.Hq;
+  h -= b * a.Hq;
+  const int hk = h / (a.Hq / a.Hkv);
   const int q0 = qi * BM;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wg = warp >> 2;
 
@@ -670,7 +675,10 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DkdvSmem& sm = *reinterpret_cast<DkdvSmem*>(smem_raw);
   const bma_attn_args& a = p.a;
-  const int kj = blockIdx.x, hk = blockIdx.y, b = blockIdx.z, G = a.Hq / a.Hkv;
+  int kj, hk;
+  cta_of(p.order, kj, hk);
+  const int b = hk / a.Hkv, G = a.Hq / a.Hkv;
+  hk -= b * a.Hkv;
   const int k0 = kj * BM;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
@@ -933,8 +941,12 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DqSmem& sm = *reinterpret_cast<DqSmem*>(smem_raw);
   const bma_attn_args& a = p.a;
-  const int qi = (int)gridDim.x - 1 - (int)blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.Hq / a.Hkv);
+  int qi, h;
+  cta_of(p.order, qi, h);
+  qi = p.order.tiles - 1 - qi;
+  const int b = h / a.Hq;
+  h -= b * a.Hq;
+  const int hk = h / (a.Hq / a.Hkv);
   const int q0 = qi * BM;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
@@ -1208,7 +1220,10 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   DkdvWideSmem& sm = *reinterpret_cast<DkdvWideSmem*>(smem_raw);
   const F32Params& p = wp.f;
   const bma_attn_args& a = p.a;
-  const int kj = blockIdx.x, hk = blockIdx.y, b = blockIdx.z, G = a.Hq / a.Hkv;
+  int kj, hk;
+  cta_of(p.order, kj, hk);
+  const int b = hk / a.Hkv, G = a.Hq / a.Hkv;
+  hk -= b * a.Hkv;
   const int k0 = kj * BM;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
@@ -1474,8 +1489,12 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   DqWideSmem& sm = *reinterpret_cast<DqWideSmem*>(smem_raw);
   const F32Params& p = wp.f;
   const bma_attn_args& a = p.a;
-  const int qi = (int)gridDim.x - 1 - (int)blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.Hq / a.Hkv);
+  int qi, h;
+  cta_of(p.order, qi, h);
+  qi = p.order.tiles - 1 - qi;
+  const int b = h / a.Hq;
+  h -= b * a.Hq;
+  const int hk = h / (a.Hq / a.Hkv);
   const int q0 = qi * BM;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
@@ -1730,6 +1749,10 @@ int plane_map(CUtensorMap* m, const uint8_t* base, int B, int L, int H, int dp, 
   return make_tile_map_bf16(m, base, 3 * B, L, H, dp, (int64_t)L * H * dp, (int64_t)H * dp, dp, rows);
 }
 
+// CTAs by query tile (streaming the planes of K and V), by key tile (those of Q and dO of a head group)
+LaunchOrder q_order(const bma_attn_args& a, int dp) { return launch_order(ceil_div(a.N, BM), (int64_t)a.B * a.Hq, (int64_t)12 * a.L * dp * a.Hkv / a.Hq); }
+LaunchOrder k_order(const bma_attn_args& a, int dp) { return launch_order(ceil_div(a.L, BM), (int64_t)a.B * a.Hkv, (int64_t)12 * a.N * dp * (a.Hq / a.Hkv)); }
+
 int make_params(F32Params& p, const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists) {
   p.a = a; p.spec = spec; p.l = lists;
   p.scale_log2 = a.scale * kLog2e;
@@ -1757,10 +1780,10 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, dp, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, dp, BH)) ||
       (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, dp, BH)))
     return rc;
-  const dim3 grid(ceil_div(a.N, BM), a.Hq, a.B);
+  p.order = q_order(a, dp);
   auto launch = [&](auto kernel, size_t smem) -> int {
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, kThreads, smem, st>>>(mq, mk, mv, p);
+    kernel<<<launch_ctas(p.order), kThreads, smem, st>>>(mq, mk, mv, p);
     return BMA_OK;
   };
   rc = dp == 64 ? launch(f32_fwd_kernel<64>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128>, sizeof(FwdSmem<128>));
@@ -1785,9 +1808,11 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dkdv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvWideSmem)));
     BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dq_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqWideSmem)));
     F32WideParams wp{p, w + pl.v};
-    f32_dkdv_wide_kernel<<<dim3(ceil_div(a.L, BM), a.Hkv, a.B), kThreads, sizeof(DkdvWideSmem), st>>>(mk, mqh, mdoh, wp);
+    wp.f.order = k_order(a, 128);
+    f32_dkdv_wide_kernel<<<launch_ctas(wp.f.order), kThreads, sizeof(DkdvWideSmem), st>>>(mk, mqh, mdoh, wp);
     wp.a_planes = w + pl.d_o;
-    f32_dq_wide_kernel<<<dim3(ceil_div(a.N, BM), a.Hq, a.B), kThreads, sizeof(DqWideSmem), st>>>(mq, mkh, mvh, wp);
+    wp.f.order = q_order(a, 128);
+    f32_dq_wide_kernel<<<launch_ctas(wp.f.order), kThreads, sizeof(DqWideSmem), st>>>(mq, mkh, mvh, wp);
     count_launches(2);
     BMA_CUDA_TRY(cudaGetLastError());
     return BMA_OK;
@@ -1799,8 +1824,10 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     return rc;
   BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvSmem)));
   BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqSmem)));
-  f32_dkdv_kernel<<<dim3(ceil_div(a.L, BM), a.Hkv, a.B), kThreads, sizeof(DkdvSmem), st>>>(mk, mv, mqh, mdoh, p);
-  f32_dq_kernel<<<dim3(ceil_div(a.N, BM), a.Hq, a.B), kThreads, sizeof(DqSmem), st>>>(mq, mkh, mvh, mdo, p);
+  p.order = k_order(a, 64);
+  f32_dkdv_kernel<<<launch_ctas(p.order), kThreads, sizeof(DkdvSmem), st>>>(mk, mv, mqh, mdoh, p);
+  p.order = q_order(a, 64);
+  f32_dq_kernel<<<launch_ctas(p.order), kThreads, sizeof(DqSmem), st>>>(mq, mkh, mvh, mdo, p);
   count_launches(2);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;

@@ -37,6 +37,46 @@ void count_launches(int n);
 
 __device__ __forceinline__ void report_device_error(int* status, int code) { atomicCAS(status, 0, code); }
 
+// ---- order of a launch's CTAs -------------------------------------------------------------
+// One CTA per (tile, head, batch).  CTAs start in the order of their linear index: one head after another, the longest walk of each
+// (under a causal mask) first, or the longest walks of all heads first.  In the first order a launch ends with the longest walks of its last
+// heads on an idle chip: 512 CTAs of 16 causal tiles take 1.29 of the even span, 1.05 in the second (float32, 2 x 2048 tokens, 16
+// heads of 64: kernels 570 -> 480 us, the call 600 -> 545; bf16, forward and backward: 1 x 4096, 16 heads of 128 366 -> 304 us, 4 x 1024, 32/8
+// heads of 128 281 -> 250, 1 x 8192, 16/8 heads of 64 912 -> 791, packed documents 2 x 4096, 16 heads 562 -> 470).  The second is for
+// launches whose end counts, at most 4 waves, and whose heads together stream (K and V forward) no more than L2 holds: in a
+// longer launch the end is a few per cent, less than what heads side by side cost there (dQ replay of 7 waves, 8 x 2048, 16 heads: the
+// call 690 -> 713 us; causal B=8 L=4096 H=32 d=128, 28 and 55 waves: 4800 -> 4950).
+constexpr int kSms = 148;
+constexpr int64_t kStreamInL2 = 64 << 20;   // of 126 MB, of which a line may take two (one per die)
+inline bool longest_first(int64_t tiles, int64_t heads, int64_t batches, int64_t stream_bytes_per_head) {
+  return tiles * heads * batches <= 4 * kSms && heads <= 65535 && heads * batches * stream_bytes_per_head <= kStreamInL2;
+}
+inline dim3 cta_grid(bool by_rank, int tiles, int heads, int batches) { return by_rank ? dim3(heads, batches, tiles) : dim3(tiles, heads, batches); }
+// rank: 0 for the first tile to start of its head
+__device__ __forceinline__ void cta_of(bool by_rank, int& rank, int& head, int& batch) {
+  rank = by_rank ? blockIdx.z : blockIdx.x;
+  head = by_rank ? blockIdx.x : blockIdx.y;
+  batch = by_rank ? blockIdx.y : blockIdx.z;
+}
+// The same in groups, for the float32 kernels, which run 6 - 12 times as long on a byte, so that no launch is too long for it:
+// one-dimensional grid, rank 0 of every head of a group, then rank 1, and so on; `head` counts the (batch, head) pairs.
+struct LaunchOrder {
+  int tiles, heads, group;
+};
+__device__ __forceinline__ void cta_of(const LaunchOrder& o, int& rank, int& head) {
+  const int per = o.group * o.tiles, g = (int)blockIdx.x / per, r = (int)blockIdx.x - g * per;
+  const int in_group = min(o.group, o.heads - g * o.group);   // (the last group may be smaller)
+  rank = __shfl_sync(0xffffffffu, r / in_group, 0);           // (warp-uniform, which the compiler does not see through divisions)
+  head = __shfl_sync(0xffffffffu, g * o.group + r % in_group, 0);
+}
+inline LaunchOrder launch_order(int tiles, int64_t heads, int64_t stream_bytes_per_head) {
+  int64_t group = kStreamInL2 / (stream_bytes_per_head > 0 ? stream_bytes_per_head : 1);
+  if (group < 1) group = 1;
+  const int64_t groups = heads > group ? (heads + group - 1) / group : 1;
+  return {tiles, (int)heads, (int)((heads + groups - 1) / groups)};   // groups of one size: a small last one would end the launch alone
+}
+inline unsigned launch_ctas(const LaunchOrder& o) { return (unsigned)(o.tiles * o.heads); }
+
 // Terms of the mask that are looked up (segment ids, bit table, tile bits) rather than computed from the indices.
 constexpr int kTableTerms = BMA_MASK_SEGMENT | BMA_MASK_BITMAP | BMA_MASK_TILES;
 

@@ -1,0 +1,57 @@
+"""The order in which CTAs start (csrc/common.cuh, longest_first and LaunchOrder).  Every (tile, head, batch) has to be done exactly once
+in either order, and in groups of heads that do and do not divide them: a call over all heads equals, bit for bit, calls over one
+head at a time."""
+import numpy as np
+import pytest
+import torch
+
+import jaxmodules_b200 as jm
+from jaxmodules_b200 import attention as A, masks as M
+
+pytestmark = pytest.mark.gpu
+
+
+def _docs(B, L, step):
+    return np.minimum(np.arange(L, dtype=np.int32) // step, 10 ** 6)[None, :].repeat(B, 0)
+
+
+CASES = [
+    # dtype, B, L, Hq, Hkv, d, recompute dQ
+    (torch.bfloat16, 1, 300, 5, 5, 64, False),       # longest walks of all heads first
+    (torch.bfloat16, 3, 1000, 6, 2, 128, True),      # likewise, grouped heads
+    (torch.bfloat16, 3, 4100, 7, 7, 128, False),     # forward 21 x 17 CTAs and K, V of 44 MB: likewise; dK/dV 21 x 33, the other order
+    (torch.bfloat16, 1, 16300, 9, 9, 128, False),    # K and V of 75 MB: one head after another
+    (torch.bfloat16, 4, 16384, 32, 32, 64, False),   # more than 4 waves: one head after another
+    (torch.float32, 1, 8200, 11, 11, 64, False),     # groups of at most 10 heads: 6 + 5
+    (torch.float32, 2, 700, 6, 2, 128, False),       # one group
+]
+
+
+@pytest.mark.parametrize("dtype,B,L,Hq,Hkv,d,recompute", CASES)
+def test_all_heads_equal_one_head_at_a_time(dtype, B, L, Hq, Hkv, d, recompute):
+    G = Hq // Hkv
+    g = torch.Generator(device="cuda").manual_seed(L + Hq)
+    q, do = (torch.randn((B, L, Hq, d), device="cuda", generator=g).to(dtype) for _ in range(2))
+    k, v = (torch.randn((B, L, Hkv, d), device="cuda", generator=g).to(dtype) for _ in range(2))
+    ids = _docs(B, L, 333)
+
+    def call(q, k, v, do, ids):
+        q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
+        O = jm.masked_attention_via_map(q, k, v, mask_fn=M.document_mask(ids, causal=True), out_dtype=dtype)
+        return (O.detach(), *torch.autograd.grad(O, (q, k, v), do))
+
+    limit = A._scratch_limit
+    try:
+        if recompute:
+            A.set_backward_scratch_limit(0)
+        whole = call(q, k, v, do, ids)
+        for b in range(B):
+            for hk in range(0, Hkv, max(1, Hkv // 8)):      # (every head of the small cases, eight of the large one)
+                s = slice(hk * G, hk * G + G)
+                one = call(q[b:b + 1, :, s], k[b:b + 1, :, hk:hk + 1], v[b:b + 1, :, hk:hk + 1], do[b:b + 1, :, s], ids[b:b + 1])
+                for name, x, y in zip(("O", "dQ", "dK", "dV"), whole, one):
+                    part = x[b:b + 1, :, s] if name in ("O", "dQ") else x[b:b + 1, :, hk:hk + 1]
+                    assert torch.equal(part, y), (name, b, hk)
+    finally:
+        A.set_backward_scratch_limit(limit)
+    assert A.device_status() == 0
