@@ -5,9 +5,12 @@ every compute entry point needs a CUDA device.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import os
 from pathlib import Path
+
+import torch
 
 _LIB_PATH = Path(__file__).resolve().parent / "libbma.so"
 
@@ -156,3 +159,33 @@ def lib():
 def check(status: int, where: str):
     if status != BMA_OK:
         raise BmaError(status, where)
+
+
+_host = None
+
+
+def host():
+    """The extension module _host.so (csrc/host.cc), bound to the loaded library; raises if it was not built."""
+    global _host
+    if _host is None:
+        handle = lib()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError(f"jaxmodules_b200/_host.so cannot be loaded ({e}): build it with `python -m jaxmodules_b200.build`") from e
+        module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in SIGNATURES}, BmaError)
+        _host = module
+    return _host
+
+
+def stream(device) -> int:
+    """Handle of the current stream (without the Stream object that torch.cuda.current_stream builds: 0.3 against 2.5 us)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def device_guard(device):
+    """``torch.cuda.device(device)``, or nothing where that device is current already (the usual case, 3 us less)."""
+    return _NO_GUARD if device.index is None or device.index == torch.cuda.current_device() else torch.cuda.device(device)

@@ -8,7 +8,6 @@ recomputing the forward.  There is no CPU or eager-PyTorch path.
 """
 from __future__ import annotations
 
-import contextlib
 import ctypes as C
 import math
 import os
@@ -135,19 +134,6 @@ def _make_args(Q, K, V, backend=nat.BMA_BACKEND_AUTO, scale=None, key_bias=None)
     return a
 
 
-def _stream(device) -> int:
-    """Handle of the current stream (without the Stream object that torch.cuda.current_stream builds: 0.3 against 2.5 us)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
-
-
-_NO_GUARD = contextlib.nullcontext()
-
-
-def _device_guard(device):
-    """``torch.cuda.device(device)``, or nothing where that device is current already (the usual case, 3 us less)."""
-    return _NO_GUARD if device.index == torch.cuda.current_device() else torch.cuda.device(device)
-
-
 def plan(Q, K, V, backend=nat.BMA_BACKEND_AUTO, backward: bool = False, key_bias=None, scale=None):
     """(backend, q_tile, kv_tile) of ``bma_attn_fwd`` / ``bma_attn_bwd`` for these tensors.  float32 calls do not go through these
     two unless a backend is forced (here it is the FP32 tile kernels), but through ``bma_attn_fwd_f32`` / ``bma_attn_bwd_f32``:
@@ -161,8 +147,8 @@ def plan(Q, K, V, backend=nat.BMA_BACKEND_AUTO, backward: bool = False, key_bias
 
 
 def _route(a: nat.AttnArgs, backward: bool):
-    """(backend, q_tile, kv_tile, workspace bytes) of one pass; the workspace is that of the float32 tensor-core kernels
-    (``bma_attn_fwd_f32`` / ``bma_attn_bwd_f32``) and 0 where ``plan``'s kernels run."""
+    """(backend, q_tile, kv_tile, workspace bytes) of one pass for an argument structure; the workspace is that of the float32
+    tensor-core kernels (``bma_attn_fwd_f32`` / ``bma_attn_bwd_f32``) and 0 where ``plan``'s kernels run."""
     lib = nat.lib()
     if a.q.dtype == nat.BMA_DTYPE_F32:
         nbytes = lib.bma_attn_f32_workspace_bytes(C.byref(a), int(backward))
@@ -177,30 +163,29 @@ def _route(a: nat.AttnArgs, backward: bool):
 def tiles(Q, K, V, backend=nat.BMA_BACKEND_AUTO, backward: bool = False, key_bias=None, scale=None):
     """(q_tile, kv_tile) of the block lists that ``attention_forward`` / ``attention_backward`` consume.  They are
     ``plan``'s, except for float32 inputs on the tensor core, whose lists have 128-blocks."""
-    return _route(_make_args(Q, K, V, backend, scale, key_bias), backward)[1:3]
+    return nat.host().routes(Q, K, V, key_bias, scale, backend, not backward, backward)[int(backward)][1:3]
+
+
+def _span(key, device):
+    return nat._NO_GUARD if _profile_sink is None else _Span(_profile_sink, key, device)
 
 
 class _Span:
-    """One launch group: an NVTX range named after it (visible in a timeline profiler, free otherwise) and,
-    when ``sink`` is a dict, a CUDA-event bracket on the launching stream (the benchmark times single
-    kernels with it)."""
+    """A CUDA-event bracket around one launch group on the launching stream (the benchmark times single kernels with it).
+    The NVTX range of the group is inside the native call."""
 
     def __init__(self, sink, key, device):
         self.sink, self.key, self.device = sink, key, device
 
     def __enter__(self):
-        torch.cuda.nvtx.range_push("bma." + self.key)
-        if self.sink is not None:
-            self.t0 = torch.cuda.Event(enable_timing=True)
-            self.t1 = torch.cuda.Event(enable_timing=True)
-            self.t0.record(torch.cuda.current_stream(self.device))
+        self.t0 = torch.cuda.Event(enable_timing=True)
+        self.t1 = torch.cuda.Event(enable_timing=True)
+        self.t0.record(torch.cuda.current_stream(self.device))
         return self
 
     def __exit__(self, *exc):
-        if self.sink is not None:
-            self.t1.record(torch.cuda.current_stream(self.device))
-            self.sink.setdefault(self.key, []).append((self.t0, self.t1))
-        torch.cuda.nvtx.range_pop()
+        self.t1.record(torch.cuda.current_stream(self.device))
+        self.sink.setdefault(self.key, []).append((self.t0, self.t1))
         return False
 
 
@@ -219,7 +204,7 @@ def device_status(device=None) -> int:
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     with torch.cuda.device(dev):
         code = C.c_int32()
-        rc = nat.lib().bma_device_status(_stream(dev), C.byref(code))
+        rc = nat.lib().bma_device_status(nat.stream(dev), C.byref(code))
         if rc not in (nat.BMA_OK, nat.BMA_ERR_DEVICE_CHECK):
             nat.check(rc, "bma_device_status")
         return int(code.value)
@@ -248,34 +233,24 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
     block lists (struct, tensors) instead of compiling them from the mask terms; it returns
     None when it has none for that tile size.  ``key_bias``: float32 ``[Hq]`` on the device, the
     logits get ``+ key_bias[h] * k`` (see ``bma_attn_args.key_bias``)."""
-    lib = nat.lib()
+    host = nat.host()
     dev = Q.device
-    B, N, Hq, d = Q.shape
+    B, N, Hq, _ = Q.shape
     L = K.shape[1]
-    with _device_guard(dev):
-        a = _make_args(Q, K, V, backend, scale, key_bias)
-        st = _stream(dev)
-        be, tq, tk, f32_bytes = _route(a, False)
+    with nat.device_guard(dev):
+        st = nat.stream(dev)
+        (be, tq, tk, f32_bytes), backward = host.routes(Q, K, V, key_bias, scale, backend, True, need_q_side)
         dmask = _masks.to_device_mask(terms, N, L, dev)
         # when the backward pass will walk the same tile size, build its q-side lists in the same launches
-        both_sides = need_q_side and _route(a, True)[1:3] == (tq, tk)
-        with _Span(_profile_sink, "mask_compile", dev):
+        both_sides = need_q_side and backward[1:3] == (tq, tk)
+        with _span("mask_compile", dev):
             ready = lists_fn(tq, tk, both_sides) if lists_fn is not None else None
             lists, lt = ready if ready is not None else compile_block_lists(
                 dmask, B, Hq, N, L, tq, tk, dev, q_side=both_sides, stream=st, conservative=True, views=False)
-        O = torch.empty((B, N, Hq, d), dtype=out_dtype, device=dev)
-        lse = torch.empty((B, Hq, N), dtype=torch.float32, device=dev)
-        a.o, a.lse = _tensor(O), lse.data_ptr()
-        with _Span(_profile_sink, "fwd", dev):
-            if f32_bytes:
-                ws = _float32_planes(dev, f32_bytes)
-                nat.check(lib.bma_attn_fwd_f32(C.byref(a), C.byref(dmask.spec), C.byref(lists), ws.data_ptr() if ws is not None else None,
-                                               f32_bytes if ws is not None else 0, st), "bma_attn_fwd_f32")
-            else:
-                ws_bytes = lib.bma_attn_fwd_workspace_bytes(C.byref(a), C.byref(lists))
-                ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=dev) if ws_bytes else None
-                nat.check(lib.bma_attn_fwd_ws(C.byref(a), C.byref(dmask.spec), C.byref(lists), ws.data_ptr() if ws_bytes else None, ws_bytes, st),
-                          "bma_attn_fwd")
+        with _span("fwd", dev):
+            planes = _float32_planes(dev, f32_bytes) if f32_bytes else None
+            O, lse = host.forward(Q, K, V, key_bias, scale, backend, C.addressof(dmask.spec), C.addressof(lists), f32_bytes, planes,
+                                  _DTYPES[out_dtype] == nat.BMA_DTYPE_BF16, st)
         _maybe_check_status(dev, "bma_attn_fwd")
     ctx = dict(dmask=dmask, lists=lists, list_tensors=lt, backend=be, scale=scale, lists_fn=lists_fn,
                lists_tile=(tq, tk), lists_have_q_side=both_sides, key_bias=key_bias)
@@ -284,84 +259,70 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
 
 def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
     """dQ, dK, dV through ``bma_attn_bwd_preprocess`` + ``bma_attn_bwd``."""
-    lib = nat.lib()
+    host = nat.host()
     dev = Q.device
-    B, N, Hq, d = Q.shape
+    B, N, Hq, _ = Q.shape
     L = K.shape[1]
-    with _device_guard(dev):
-        a = _make_args(Q, K, V, backend, ctx.get("scale"), ctx.get("key_bias"))
-        st = _stream(dev)
-        be, tq, tk, f32_bytes = _route(a, True)
-        with _Span(_profile_sink, "mask_compile_bwd", dev):
+    scale, key_bias = ctx.get("scale"), ctx.get("key_bias")
+    with nat.device_guard(dev):
+        st = nat.stream(dev)
+        be, tq, tk, f32_bytes = host.routes(Q, K, V, key_bias, scale, backend, False, True)[1]
+        lists_fn = ctx.get("lists_fn")
+        with _span("mask_compile_bwd", dev):
             if ctx.get("lists_have_q_side") and ctx.get("lists_tile") == (tq, tk):
                 lists, lt = ctx["lists"], ctx["list_tensors"]      # built by the forward pass
             else:
-                lists_fn = ctx.get("lists_fn")
                 ready = lists_fn(tq, tk, True) if lists_fn is not None else None
                 lists, lt = ready if ready is not None else compile_block_lists(
                     ctx["dmask"], B, Hq, N, L, tq, tk, dev, q_side=True, stream=st, conservative=True, views=False)
+        spec_at, lists_at = C.addressof(ctx["dmask"].spec), C.addressof(lists)
         if dO.stride(-1) != 1:
             dO = dO.contiguous()
-        delta = torch.empty((B, Hq, N), dtype=torch.float32, device=dev)
-        dQ, dK, dV = torch.empty_like(Q), torch.empty_like(K), torch.empty_like(V)
-        a.o, a.lse, a.d_o, a.delta = _tensor(O), lse.data_ptr(), _tensor(dO), delta.data_ptr()
-        a.dq, a.dk, a.dv = _tensor(dQ), _tensor(dK), _tensor(dV)
-        do_bf16 = None
-        if be == nat.BMA_BACKEND_TCGEN05 and dO.dtype != torch.bfloat16:
-            do_bf16 = torch.empty((B, N, Hq, d), dtype=torch.bfloat16, device=dev)
+        bf16_copy = be == nat.BMA_BACKEND_TCGEN05 and dO.dtype != torch.bfloat16
         reuse = ctx.get("reuse")       # a dict the caller keeps for one (O, dO): delta and the bf16 cotangent are taken once
-        if reuse is not None and "delta" in reuse and (do_bf16 is None or reuse["do_bf16"] is not None):
-            delta, do_bf16 = reuse["delta"], (reuse["do_bf16"] if do_bf16 is not None else None)
-            a.delta = delta.data_ptr()
+        if reuse is not None and "delta" in reuse and (not bf16_copy or reuse["do_bf16"] is not None):
+            delta, do_bf16 = reuse["delta"], (reuse["do_bf16"] if bf16_copy else None)
         else:
-            with _Span(_profile_sink, "bwd_preprocess", dev):
-                nat.check(lib.bma_attn_bwd_preprocess(C.byref(a), do_bf16.data_ptr() if do_bf16 is not None else None, st),
-                          "bma_attn_bwd_preprocess")
+            with _span("bwd_preprocess", dev):
+                delta, do_bf16 = host.preprocess(Q, K, V, O, dO, key_bias, scale, backend, bf16_copy, st)
             if reuse is not None:
                 reuse["delta"], reuse["do_bf16"] = delta, do_bf16
         if do_bf16 is not None:
-            a.d_o = _tensor(do_bf16)
+            dO = do_bf16
         if f32_bytes:
-            ws = _float32_planes(dev, f32_bytes)
-            with _Span(_profile_sink, "bwd", dev):
-                nat.check(lib.bma_attn_bwd_f32(C.byref(a), C.byref(ctx["dmask"].spec), C.byref(lists), ws.data_ptr() if ws is not None else None,
-                                               f32_bytes if ws is not None else 0, st), "bma_attn_bwd_f32")
+            planes = _float32_planes(dev, f32_bytes)
+            with _span("bwd", dev):
+                grads = host.backward(Q, K, V, O, lse, dO, delta, key_bias, scale, backend, spec_at, lists_at, f32_bytes, planes, 0, 0, 0, st)
             _maybe_check_status(dev, "bma_attn_bwd_f32")
-            return dQ, dK, dV
-        ws_bytes = lib.bma_attn_bwd_workspace_bytes(C.byref(a))
+            return grads
         # dS hand-over between the two backward kernels: only for lists whose two sides name the same blocks.
         # The scratch is sized by the blocks the mask visits (fetched once per mask, see masks.visited_counts).
-        lists_fn = ctx.get("lists_fn")
-        visited = scratch = 0
+        visited = 0
         if be == nat.BMA_BACKEND_TCGEN05 and _scratch_limit > 0 and (lists_fn is None or getattr(lists_fn, "consistent", False)):
-            if lists_fn is None:
-                counts = _masks.visited_counts(ctx["dmask"], lists, dev)
-            else:
-                counts = lists_fn.visited_counts(lists, dev)
-            visited = (C.c_int64 * len(counts))(*[int(c) for c in counts])
-            scratch = lib.bma_attn_bwd_scratch_bytes(C.byref(a), C.byref(lists), visited)
+            counts = _masks.visited_counts(ctx["dmask"], lists, dev) if lists_fn is None else lists_fn.visited_counts(lists, dev)
+            visited = counts.__array_interface__["data"][0]       # int64, alive with `counts`
+        ws_bytes, scratch, scratch_min = host.backward_bytes(Q, K, V, key_bias, scale, backend, lists_at, visited)
         given = min(scratch, _scratch_limit, int(scratch * _scratch_fraction) if _scratch_fraction < 1.0 else scratch)
-        if 0 < given < scratch and given < lib.bma_attn_bwd_scratch_min_bytes(C.byref(a), C.byref(lists), visited):
+        if 0 < given < scratch and given < scratch_min:
             given = 0          # not even the largest (batch, kv head) unit fits: the dQ kernel recomputes, no buffer is needed
+        ws = None
         if given > 0:
-            ws, ws_bytes = _backward_scratch(dev, max(given, ws_bytes)), max(given, ws_bytes)
-        else:
-            ws = torch.empty((max(ws_bytes, 1),), dtype=torch.uint8, device=dev)
-        last_backward_info.update(scratch_bytes=int(scratch), workspace_bytes=int(ws_bytes), whole=bool(scratch and given >= scratch))
+            ws_bytes = max(given, ws_bytes)
+            ws = _backward_scratch(dev, ws_bytes)
+        last_backward_info.update(scratch_bytes=scratch, workspace_bytes=ws_bytes, whole=bool(scratch and given >= scratch))
         mid = None
         if _profile_sink is not None and be == nat.BMA_BACKEND_TCGEN05 and (given == 0 or given >= scratch):
             # the library records this event between its dK/dV pass and its dQ pass (only when it runs as one range)
             mid = torch.cuda.Event(enable_timing=True)
             mid.record(torch.cuda.current_stream(dev))
-        with _Span(_profile_sink, "bwd", dev) as span:
-            nat.check(lib.bma_attn_bwd(C.byref(a), C.byref(ctx["dmask"].spec), C.byref(lists), ws.data_ptr(), ws_bytes,
-                                       visited if visited else None, mid.cuda_event if mid is not None else None, st),
-                      "bma_attn_bwd")
+        with _span("bwd", dev) as span:
+            grads = host.backward(Q, K, V, O, lse, dO, delta, key_bias, scale, backend, spec_at, lists_at, 0, ws, ws_bytes, visited,
+                                  mid.cuda_event if mid is not None else 0, st)
         _maybe_check_status(dev, "bma_attn_bwd")
         if mid is not None:
             _profile_sink.setdefault("bwd_dkdv", []).append((span.t0, mid))
             _profile_sink.setdefault("bwd_dq_replay" if given >= scratch > 0 else "bwd_dq_recompute", []).append((mid, span.t1))
-    return dQ, dK, dV
+    return grads
 
 
 # Scratch of the tensor-core backward (the dS tiles handed from the dK/dV kernel to the dQ kernel): 32 KB per block the
@@ -409,7 +370,7 @@ def _float32_planes(dev: torch.device, nbytes: int) -> Optional[torch.Tensor]:
 
 def _backward_scratch(dev: torch.device, nbytes: int) -> torch.Tensor:
     # keyed by stream too: two backward passes in flight on different streams must not share slots
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(), _stream(dev))
+    key = (dev.index if dev.index is not None else torch.cuda.current_device(), nat.stream(dev))
     buf = _scratch_buffers.get(key)
     if buf is None or buf.numel() < nbytes:
         _scratch_buffers.pop(key, None)   # drop the old buffer before asking for the larger one
@@ -497,7 +458,7 @@ def masked_attention_via_map(
     assert d == dq and Lv == L and dv == d, f"shape mismatch in K {tuple(K.shape)}, Q {tuple(Q.shape)} and V {tuple(V.shape)}"
     assert Hq % Hk == 0, "Hq must be divisible by Hk"
     assert Hv == Hk, "Hv must be equal to Hk"
-    block_window(N, L, block_size, window_size)      # argument errors first, wherever the tensors live
+    window = block_window(N, L, block_size, window_size)      # argument errors first, wherever the tensors live
     if not (Q.is_cuda and K.is_cuda and V.is_cuda):
         raise RuntimeError("masked_attention_via_map needs CUDA tensors; there is no CPU path")
     if Q.dtype not in _DTYPES or K.dtype != Q.dtype or V.dtype != Q.dtype:
@@ -508,7 +469,6 @@ def masked_attention_via_map(
     else:
         terms = _masks.terms_from_mask_fn(mask_fn, B, Hq, N, L, device=Q.device)
 
-    window = block_window(N, L, block_size, window_size)
     if window is not None:
         terms = terms.merged(_masks.MaskTerms(window=window))
 

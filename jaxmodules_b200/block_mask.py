@@ -246,7 +246,6 @@ def compile_block_lists(dmask: "_masks.DeviceMask", B: int, H: int, N: int, L: i
     for lists the attention kernels consume, never used for the arrays ``create_block_mask`` returns.
     ``views=False``: the arrays lie in one buffer with the workspace and only the struct describes them (the dict keeps
     the buffer alive): one allocation where nine cost 20 us of the host's time."""
-    lib = nat.lib()
     if floor_blocks:
         NQ, NKV = N // q_block, L // kv_block
     else:
@@ -255,46 +254,22 @@ def compile_block_lists(dmask: "_masks.DeviceMask", B: int, H: int, N: int, L: i
         raise ValueError("sequence shorter than one block")
     LB = out_B if out_B is not None else (B if dmask.depends_b else 1)
     LH = out_H if out_H is not None else (H if dmask.depends_h else 1)
-    spec = dmask.spec
-    if floor_blocks or conservative:
-        spec = nat.MaskSpec.from_buffer_copy(spec)
-    if floor_blocks:
-        spec.q_valid, spec.k_valid = min(spec.q_valid, NQ * q_block), min(spec.k_valid, NKV * kv_block)
-    if conservative:
-        spec.flags |= nat.BMA_MASK_COMPILE_CONSERVATIVE
-    lists = nat.BlockLists()
-    lists.B, lists.H, lists.NQ, lists.NKV, lists.q_block, lists.kv_block = LB, LH, NQ, NKV, q_block, kv_block
-    ws_bytes = lib.bma_mask_compile_workspace_bytes(C.byref(spec), B, H, NQ, NKV)
-    if views:
-        i32 = dict(dtype=torch.int32, device=device)
-        t = dict(
-            kv_num_blocks=torch.empty((LB, LH, NQ), **i32), kv_indices=torch.empty((LB, LH, NQ, NKV), **i32),
-            full_kv_num_blocks=torch.empty((LB, LH, NQ), **i32), full_kv_indices=torch.empty((LB, LH, NQ, NKV), **i32),
-            q_num_blocks=None, q_indices=None, full_q_num_blocks=None, full_q_indices=None)
-        if q_side:
-            t.update(q_num_blocks=torch.empty((LB, LH, NKV), **i32), q_indices=torch.empty((LB, LH, NKV, NQ), **i32),
-                     full_q_num_blocks=torch.empty((LB, LH, NKV), **i32), full_q_indices=torch.empty((LB, LH, NKV, NQ), **i32))
-        lists.kv_num, lists.kv_idx = t["kv_num_blocks"].data_ptr(), t["kv_indices"].data_ptr()
-        lists.full_kv_num, lists.full_kv_idx = t["full_kv_num_blocks"].data_ptr(), t["full_kv_indices"].data_ptr()
-        if q_side:
-            lists.q_num, lists.q_idx = t["q_num_blocks"].data_ptr(), t["q_indices"].data_ptr()
-            lists.full_q_num, lists.full_q_idx = t["full_q_num_blocks"].data_ptr(), t["full_q_indices"].data_ptr()
-        ws = t["_workspace"] = torch.empty((max(ws_bytes, 1),), dtype=torch.uint8, device=device)  # alive until the stream has consumed it
-        ws_ptr = ws.data_ptr()
-    else:
-        pad = lambda n: -(-4 * n // 256) * 256      # bytes of n int32, every array on a 256-byte boundary
-        rows, cols, cells = pad(LB * LH * NQ), pad(LB * LH * NKV), pad(LB * LH * NQ * NKV)
-        total = 2 * (rows + cells) + (2 * (cols + cells) if q_side else 0)
-        t = dict(_buffer=torch.empty((total + ws_bytes + 1,), dtype=torch.uint8, device=device))
-        ptr = t["_buffer"].data_ptr()
-        lists.kv_num, lists.kv_idx, lists.full_kv_num, lists.full_kv_idx = ptr, ptr + rows, ptr + rows + cells, ptr + 2 * rows + cells
-        if q_side:
-            at = ptr + 2 * (rows + cells)
-            lists.q_num, lists.q_idx, lists.full_q_num, lists.full_q_idx = at, at + cols, at + cols + cells, at + 2 * cols + cells
-        ws_ptr = ptr + total
-    st = stream if stream is not None else torch.cuda.current_stream(device).cuda_stream
-    nat.check(lib.bma_mask_compile(C.byref(spec), B, H, C.byref(lists), ws_ptr, ws_bytes, st), "bma_mask_compile")
-    return lists, t
+    device = torch.device(device)
+    lists = nat.BlockLists(LB, LH, NQ, NKV, q_block, kv_block)
+    arrays = nat.host().compile_lists(
+        C.addressof(dmask.spec), C.addressof(lists), B, H, q_side, views, nat.BMA_MASK_COMPILE_CONSERVATIVE if conservative else 0,
+        NQ * q_block if floor_blocks else _ANY, NKV * kv_block if floor_blocks else _ANY,
+        torch.cuda.current_device() if device.index is None else device.index, nat.stream(device) if stream is None else stream)
+    if not views:
+        return lists, dict(_buffer=arrays[0])
+    if not q_side:
+        arrays[4:4] = [None] * 4
+    return lists, dict(zip(_ARRAYS, arrays))
+
+
+_ANY = (1 << 31) - 1
+_ARRAYS = ("kv_num_blocks", "kv_indices", "full_kv_num_blocks", "full_kv_indices", "q_num_blocks", "q_indices", "full_q_num_blocks",
+           "full_q_indices", "_workspace")      # (the workspace: alive until the stream has consumed it)
 
 
 def create_block_mask(mask_mod, B: int, H: int, Q_LEN: int, KV_LEN: int, BLOCK_SIZE, device=None) -> BlockMask:
@@ -307,7 +282,7 @@ def create_block_mask(mask_mod, B: int, H: int, Q_LEN: int, KV_LEN: int, BLOCK_S
         raise RuntimeError("create_block_mask runs on a CUDA device; none is available")
     device = torch.device(device if device is not None else "cuda")
     QB, KVB = extract_block_size(BLOCK_SIZE)
-    with torch.cuda.device(device):
+    with nat.device_guard(device):
         terms = _masks.terms_from_mask_fn(mask_mod, B, H, Q_LEN, KV_LEN, device=device)
         dmask = _masks.to_device_mask(terms, Q_LEN, KV_LEN, device)
         _, t = compile_block_lists(dmask, B, H, Q_LEN, KV_LEN, QB, KVB, device, out_B=B, out_H=H, q_side=True,

@@ -1,4 +1,4 @@
-"""Builds libbma.so (the C-ABI library with every CUDA kernel) in-tree with nvcc for sm_100a.
+"""Builds libbma.so (the C-ABI library with every CUDA kernel) in-tree with nvcc for sm_100a, and _host.so (the host side of a call, csrc/host.cc).
 
     python -m jaxmodules_b200.build [--force] [--verbose]
 
@@ -18,6 +18,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = CSRC / "build"
 LIB = PKG / "libbma.so"
+HOST = PKG / "_host.so"
 
 SOURCES = ["bma_api.cu", "mask_compile.cu", "mask_program.cu", "attn_simt.cu", "attn_fwd_sm100.cu", "attn_bwd_sm100.cu", "attn_bwd_dq_sm100.cu", "attn_bwd_dq_replay_sm100.cu", "attn_f32_sm100.cu", "bwd_slots.cu"]
 
@@ -58,8 +59,10 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             raise RuntimeError(f"nvcc failed for {src}:\n{r.stdout}\n{r.stderr}")
         return o, r.stderr
 
-    with ThreadPoolExecutor(max_workers=min(8, len(SOURCES))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, len(SOURCES)) + 1) as ex:
+        host = ex.submit(_build_host, force)
         results = list(ex.map(compile_one, SOURCES))
+        host.result()
     objs = [str(o) for o, _ in results]
     if verbose:
         for _, log in results:
@@ -72,6 +75,24 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
     _build_jax_adapter(force)
     return LIB
+
+
+def _build_host(force: bool) -> None:
+    """_host.so: the extension module between torch tensors and the entry points of the library."""
+    src = CSRC / "host.cc"
+    if not force and not _stale(HOST, [src, PKG.parent / "include" / "bma.h", Path(__file__)]):
+        return
+    import sysconfig
+    import torch
+    inc = Path(torch.__file__).parent / "include"
+    dirs = [sysconfig.get_paths()["include"], inc, inc / "torch" / "csrc" / "api" / "include", Path(_nvcc()).resolve().parent.parent / "include"]
+    cmd = [os.environ.get("CXX", "g++"), "-shared", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    for d in dirs:
+        cmd += ["-isystem", str(d)]
+    cmd += [str(src), "-o", str(HOST), "-L", str(Path(torch.__file__).parent / "lib"), "-lc10", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-ldl"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building the host module failed:\n{r.stdout}\n{r.stderr}")
 
 
 def _build_jax_adapter(force: bool) -> None:

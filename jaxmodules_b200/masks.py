@@ -341,10 +341,8 @@ def visited_counts(dmask: DeviceMask, lists: "nat.BlockLists", device, extra_key
     """Host int64 array [lists.B * lists.H] of visited (full + partial) blocks per list head for the lists just
     compiled from ``dmask``; cached per mask, shape and tile size."""
     import ctypes as C
-    s = dmask.spec
-    key = (s.flags, s.q_valid, s.k_valid, s.q_offset, s.k_offset, s.band_left, s.band_right, s.win_block, s.win_left,
-           s.win_right, s.win_nblk, tuple((id(t), t._version, tuple(t.shape)) for t in dmask.keep),
-           lists.B, lists.H, lists.NQ, lists.NKV, lists.q_block, lists.kv_block, str(torch.device(device))) + tuple(extra_key)
+    key = (bytes(dmask.spec), tuple((id(t), t._version, tuple(t.shape)) for t in dmask.keep),
+           lists.B, lists.H, lists.NQ, lists.NKV, lists.q_block, lists.kv_block, torch.device(device)) + tuple(extra_key)
     hit = _visited_counts.get(key)
     if hit is not None and all(r() is t for r, t in zip(hit[0], dmask.keep)):
         return hit[1]
