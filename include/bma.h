@@ -262,9 +262,16 @@ int bma_attn_bwd_plan(const bma_attn_args* args, int32_t* backend, int32_t* q_ti
 int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec,
                  const bma_block_lists* lists, bma_stream_t stream);
 
+/* 1 where the forward pass (bma_attn_fwd_f32 where bma_attn_f32_workspace_bytes covers the request, else bma_attn_fwd_ws) is best
+ * given lists without arrays: sizes and block sizes as ever, B = H = 1, kv_num, kv_idx, full_kv_num and full_kv_idx NULL.  The mask then
+ * has interval terms only (no segment ids, bit table or tiles), and the kernels know its blocks from their indices; such lists
+ * are accepted for every such mask on the tensor-core kernels. */
+int32_t bma_attn_fwd_implies_lists(const bma_attn_args* args, const bma_mask_spec* spec);
+
 /* The same with a workspace (16-byte aligned), which lets few queries against many keys spread over the whole chip: partial
  * results of runs of keys are combined through it.  bma_attn_fwd_workspace_bytes is 0 where none is used; with less than
- * that bma_attn_fwd_ws runs as bma_attn_fwd does. */
+ * that bma_attn_fwd_ws runs as bma_attn_fwd does.  (Up to eight runs meet in the shared memory of a cluster of CTAs instead, on
+ * a device that has room for the clusters.) */
 size_t bma_attn_fwd_workspace_bytes(const bma_attn_args* args, const bma_block_lists* lists);
 int bma_attn_fwd_ws(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
                     void* workspace, size_t workspace_bytes, bma_stream_t stream);

@@ -245,8 +245,12 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
         both_sides = need_q_side and backward[1:3] == (tq, tk)
         with _span("mask_compile", dev):
             ready = lists_fn(tq, tk, both_sides) if lists_fn is not None else None
-            lists, lt = ready if ready is not None else compile_block_lists(
-                dmask, B, Hq, N, L, tq, tk, dev, q_side=both_sides, stream=st, conservative=True, views=False)
+            if ready is not None:
+                lists, lt = ready
+            elif not both_sides and host.implies_lists(Q, K, V, key_bias, scale, backend, C.addressof(dmask.spec)):
+                lists, lt = nat.BlockLists(1, 1, -(-N // tq), -(-L // tk), tq, tk), None     # no arrays: the kernels know the blocks
+            else:
+                lists, lt = compile_block_lists(dmask, B, Hq, N, L, tq, tk, dev, q_side=both_sides, stream=st, conservative=True, views=False)
         with _span("fwd", dev):
             planes = _float32_planes(dev, f32_bytes) if f32_bytes else None
             O, lse = host.forward(Q, K, V, key_bias, scale, backend, C.addressof(dmask.spec), C.addressof(lists), f32_bytes, planes,

@@ -145,12 +145,15 @@ struct SplitParams {
 
 // used[b', kj] = 1 where a list of batch entry b' names kv block kj (a kv-side list; backward: or a q-side list of kj has an
 // entry), else 0.  One CTA per batch entry of the lists.
-__global__ void __launch_bounds__(256) used_blocks_kernel(bma_block_lists l, bool backward, uint8_t* __restrict__ used) {
+__global__ void __launch_bounds__(256) used_blocks_kernel(bma_block_lists l, bma_mask_spec spec, bool backward, uint8_t* __restrict__ used) {
   __shared__ uint8_t mark[kMaxKvFwd];
   for (int i = threadIdx.x; i < l.NKV; i += 256) mark[i] = 0;
   __syncthreads();
   const int rows = l.H * l.NQ, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int r = warp; r < rows; r += 8) {
+  if (!l.kv_num)
+    for (int i = threadIdx.x; i < l.NKV; i += 256)
+      for (int qi = 0; qi < l.NQ; ++qi) mark[i] |= interval_class(spec, qi, i, BM, BM) != 0;
+  for (int r = warp; r < rows && l.kv_num; r += 8) {
     const int64_t row = (int64_t)blockIdx.x * rows + r;
     const int nfull = l.full_kv_num[row], npart = l.kv_num[row];
     for (int i = lane; i < nfull; i += 32) mark[l.full_kv_idx[row * l.NKV + i]] = 1;
@@ -271,14 +274,18 @@ struct KvList {
   int count;
 };
 template <int MAX>
-__device__ __forceinline__ int build_kv_list(KvList<MAX>& s, const bma_block_lists& l, int b, int h, int qi) {
+__device__ __forceinline__ int build_kv_list(KvList<MAX>& s, const bma_block_lists& l, const bma_mask_spec& spec, int b, int h, int qi) {
   const int NKV = l.NKV, lane = threadIdx.x & 31;
   const int64_t lrow = ((int64_t)(l.B == 1 ? 0 : b) * l.H + (l.H == 1 ? 0 : h)) * l.NQ + qi;
-  for (int i = threadIdx.x; i < NKV; i += kThreads) s.cls[i] = 0;
-  __syncthreads();
-  const int nfull = l.full_kv_num[lrow], npart = l.kv_num[lrow];
-  for (int i = threadIdx.x; i < nfull; i += kThreads) s.cls[l.full_kv_idx[lrow * NKV + i]] = 2;
-  for (int i = threadIdx.x; i < npart; i += kThreads) s.cls[l.kv_idx[lrow * NKV + i]] = 1;
+  if (l.kv_num) {
+    for (int i = threadIdx.x; i < NKV; i += kThreads) s.cls[i] = 0;
+    __syncthreads();
+    const int nfull = l.full_kv_num[lrow], npart = l.kv_num[lrow];
+    for (int i = threadIdx.x; i < nfull; i += kThreads) s.cls[l.full_kv_idx[lrow * NKV + i]] = 2;
+    for (int i = threadIdx.x; i < npart; i += kThreads) s.cls[l.kv_idx[lrow * NKV + i]] = 1;
+  } else {   // no lists: a mask of interval terms, whose blocks are known from the indices
+    for (int i = threadIdx.x; i < NKV; i += kThreads) s.cls[i] = (uint8_t)interval_class(spec, qi, i, BM, BM);
+  }
   __syncthreads();
   if (threadIdx.x < 32) {
     int count = 0;
@@ -399,7 +406,7 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     tmem_relinquish();
   }
   tc_fence_before();
-  const int T = build_kv_list(sm.list, p.l, b, h, qi);
+  const int T = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   // half tiles per warpgroup: the second half of the last tile may lie past the end of the keys
@@ -970,7 +977,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     tmem_relinquish();
   }
   tc_fence_before();
-  const int T = build_kv_list(sm.list, p.l, b, h, qi);
+  const int T = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   // half tiles in all; the second half of the last tile may lie past the end of the keys
@@ -1517,7 +1524,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     tmem_relinquish();
   }
   tc_fence_before();
-  const int T = build_kv_list(sm.list, p.l, b, h, qi);
+  const int T = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   // half tiles in all; the second half of the last tile may lie past the end of the keys
@@ -1722,12 +1729,12 @@ Planes planes_layout(const bma_attn_args& a, bool backward) {
   return p;
 }
 
-int launch_split(const bma_attn_args& a, const bma_block_lists& l, const Planes& pl, uint8_t* ws, bool backward, cudaStream_t st) {
+int launch_split(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& l, const Planes& pl, uint8_t* ws, bool backward, cudaStream_t st) {
   SplitParams sp;
   sp.B = a.B; sp.d = a.d;
   sp.used = nullptr; sp.used_B = l.B; sp.NKV = l.NKV;
   if (used_blocks(a)) {
-    used_blocks_kernel<<<(unsigned)l.B, 256, 0, st>>>(l, backward, ws + pl.used);
+    used_blocks_kernel<<<(unsigned)l.B, 256, 0, st>>>(l, spec, backward, ws + pl.used);
     count_launches(1);
     sp.used = ws + pl.used;
   }
@@ -1775,7 +1782,7 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   const int dp = padded_d(a);
   F32Params p;
   int rc;
-  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, lists, pl, w, false, st))) return rc;
+  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, spec, lists, pl, w, false, st))) return rc;
   CUtensorMap mq, mk, mv;
   if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, dp, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, dp, BH)) ||
       (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, dp, BH)))
@@ -1798,7 +1805,7 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   uint8_t* w = static_cast<uint8_t*>(ws);
   F32Params p;
   int rc;
-  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, lists, pl, w, true, st))) return rc;
+  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, spec, lists, pl, w, true, st))) return rc;
   CUtensorMap mq, mk, mv, mdo, mqh, mkh, mvh, mdoh;
   if (a.d > 64) {
     if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, 128, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, 128, BM)) ||

@@ -20,6 +20,7 @@
 // S_x (overwrites it) needs no extra barrier.  Every mbarrier wait is bounded; on a timeout the
 // thread records an error code and unwinds to the common exit where TMEM is released.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -217,6 +218,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
   for (int x = 0; x < 2; ++x) {
     const int qi = pair * 2 + x;
     if (qi >= NQ) break;
+    if (!p.l.kv_num) {   // no lists: a mask of interval terms, whose blocks are known from the indices
+      for (int i = threadIdx.x; i < NKV; i += kThreads) sm.cls[x][i] = (uint8_t)interval_class(p.spec, qi, i, BM, BN);
+      continue;
+    }
     const int64_t lrow = ((int64_t)lb * p.l.H + lh) * NQ + qi;
     const int nfull = p.l.full_kv_num[lrow], npart = p.l.kv_num[lrow];
     const int32_t* full_idx = p.l.full_kv_idx + lrow * NKV;
@@ -1078,16 +1083,18 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 //   * the kv list is cut into `splits` runs, one CTA each, so that the whole chip pulls on HBM;
 //   * inside a CTA the two softmax warpgroups take alternate kv tiles of the run (the same Q tile, two
 //     independent online softmaxes that ping-pong on the tensor core) and are merged in shared memory;
-//   * the runs' partial results go to a workspace, [unit, split, row] of HD floats and (max, sum), and
-//     fwd_combine_kernel weighs them together (or, with one split, the CTA writes O itself).
+//   * up to eight runs are a cluster and add their partial results up through one another's shared memory; more go to
+//     a workspace, [unit, split, row] of HD floats and (max, sum), and fwd_combine_kernel weighs them together.
 // Bound by HBM: K and V once.  Measured, B = 4, 16 queries, 8192 keys, 32 / 8 heads of 128 (135 MB of
-// K and V): 33 + 4 us (4.1 TB/s) in 4 splits, against 128 us of the one-CTA-per-head kernel.
+// K and V): 32 us in 4 splits (33 + 4 with the workspace, 128 as one CTA per head).  Of these the stream of K and V takes 19 (7 TB/s);
+// 5 go by until its first tiles are there, 3 in the staging and 4 in the sum of the partials.
 // =================================================================================================
 enum {
   SB_Q = 0, SB_S0, SB_S1, SB_P0, SB_P1, SB_O0, SB_O1, SB_SYNC, SB_K_FULL, SB_K_FREE = SB_K_FULL + 3, SB_V_FULL = SB_K_FREE + 3,
   SB_V_FREE = SB_V_FULL + 2, SB_NUM = SB_V_FREE + 2
 };
 constexpr int kSplitKStages = 3, kSplitVStages = 2;
+constexpr int kMaxCluster = 8;   // runs that meet in shared memory
 
 template <int HD>
 struct __align__(1024) FwdSplitSmem {
@@ -1108,6 +1115,7 @@ struct FwdSplitParams {
   int tile_queries; // queries of a tile: 128 / heads rounded down
   int q_tiles;      // tiles of one (head set, batch)
   int splits;
+  int cluster;      // CTAs of a unit that add their partials up through one another's shared memory: `splits`, or 1
   float* part_o;    // [units, splits, 128, HD]
   float2* part_ml;  // [units, splits, 128]
 };
@@ -1136,6 +1144,8 @@ fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   const FwdParams& p = sp.f;
   const bma_attn_args& a = p.a;
   const int unit = blockIdx.x, split = blockIdx.y;
+  constexpr int kPitch = HD + 4;
+  static_assert(2 * BM * kPitch * sizeof(float) <= sizeof(sm.k) + sizeof(sm.v), "the partials are staged over K and V");
   const SplitRow first = split_row(sp, unit, 0);
   const int b = first.b, h0 = first.h, hk = h0 / (a.Hq / a.Hkv);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -1147,7 +1157,7 @@ fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     return;
   }
   // ---- kv list of the one listed q tile (head h0 stands for the set: the lists do not depend on the head where heads > 1)
-  for (int i = threadIdx.x; i < NKV; i += kThreads) sm.cls[i] = 0;
+  for (int i = threadIdx.x; i < NKV; i += kThreads) sm.cls[i] = p.l.kv_num ? 0 : (uint8_t)interval_class(p.spec, 0, i, BM, BN);
   if (threadIdx.x == 0) {
     for (int i = 0; i < SB_NUM; ++i) mbar_init(&sm.bar[i], (i == SB_P0 || i == SB_P1) ? 128 : (i == SB_SYNC ? 256 : 1));
     fence_barrier_init();
@@ -1157,7 +1167,7 @@ fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     for (int box = 0; box < HD / 64; ++box) tma_load_4d(sm.q + box * kHalfTile, &map_q, &sm.bar[SB_Q], box * 64, h0, first.q, b);
   }
   __syncthreads();
-  {
+  if (p.l.kv_num) {
     const int64_t lrow = (int64_t)(p.l.B == 1 ? 0 : b) * p.l.H + (p.l.H == 1 ? 0 : h0);   // NQ == 1
     const int nfull = p.l.full_kv_num[lrow], npart = p.l.kv_num[lrow];
     for (int i = threadIdx.x; i < nfull; i += kThreads) sm.cls[p.l.full_kv_idx[lrow * NKV + i]] = 2;
@@ -1335,73 +1345,95 @@ fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     tc_fence_after();
     if (m_ref == -INFINITY) l = 0.f;            // no allowed key (the polynomial exponential of a masked score is 2^-126, not 0)
 
-    // ---- merge of the two warpgroups through shared memory (after the first rendezvous no MMA reads K or V any more)
+    // ---- the partial results of the two warpgroups to shared memory (after the rendezvous no MMA reads K or V any more)
     sm.ml[x][0][row] = m_ref;
     sm.ml[x][1][row] = l;
-    uint32_t syncs = 0;
-    auto rendezvous = [&]() {
-      mbar_arrive(&sm.bar[SB_SYNC]);
-      ok = mbar_wait(&sm.bar[SB_SYNC], syncs & 1) && ok;
-      ++syncs;
-    };
-    rendezvous();
-    const float mo = sm.ml[x ^ 1][0][row], lo = sm.ml[x ^ 1][1][row];
-    const float mt = fmaxf(m_ref, mo), ms = (mt == -INFINITY) ? 0.f : mt;
-    const float fx = ex2(m_ref - ms), lt = l * fx + lo * ex2(mo - ms);
-    // with several splits the partial stays unnormalised, relative to its own maximum
-    const float mine = cnt > 0 && l > 0.f ? (sp.splits == 1 ? fx / lt : fx) : 0.f;
-    constexpr int kPitch = HD + 4;
-    float* stage = reinterpret_cast<float*>(sm.k[0]) + row * kPitch;
-    for (int turn = 0; turn < 2; ++turn) {
-      if (turn == x) {
-#pragma unroll
-        for (int c = 0; c < HD / 32; ++c) {
-          uint32_t v[32];
-          if (cnt > 0) {
-            tmem_ld32(tmem_o + c * 32, v);
-            tmem_wait_ld();
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = 0u;
-          }
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            float4 o4 = turn == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<float4*>(stage + c * 32 + j);
-            o4.x = fmaf(__uint_as_float(v[j]), mine, o4.x); o4.y = fmaf(__uint_as_float(v[j + 1]), mine, o4.y);
-            o4.z = fmaf(__uint_as_float(v[j + 2]), mine, o4.z); o4.w = fmaf(__uint_as_float(v[j + 3]), mine, o4.w);
-            *reinterpret_cast<float4*>(stage + c * 32 + j) = o4;
-          }
-        }
-      }
-      rendezvous();
-    }
+    mbar_arrive(&sm.bar[SB_SYNC]);
+    ok = mbar_wait(&sm.bar[SB_SYNC], 0) && ok;
     if (!ok) {
       report_device_error(p.status, 170 + warp);
-    } else {
-      if (x == 0 && r.valid) {
-        if (sp.splits > 1) sp.part_ml[((int64_t)unit * sp.splits + split) * BM + row] = make_float2(mt, lt);
-        else if (a.lse) a.lse[((int64_t)b * a.Hq + r.h) * a.N + r.q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
-      }
-      // a warp per row: whole lines of O or of the partial
-      for (int i = warp; i < BM; i += 8) {
-        const SplitRow ri = split_row(sp, unit, i);
-        if (!ri.valid) continue;
-        const float* src = reinterpret_cast<const float*>(sm.k[0]) + i * kPitch;
-        if (sp.splits > 1) {
-          float* dst = sp.part_o + (((int64_t)unit * sp.splits + split) * BM + i) * HD;
-          if (lane < HD / 4) reinterpret_cast<float4*>(dst)[lane] = reinterpret_cast<const float4*>(src)[lane];
-        } else if (lane < HD / 4) {
-          const float4 o4 = reinterpret_cast<const float4*>(src)[lane];
-          const int64_t off = (int64_t)b * a.o.stride_b + (int64_t)ri.q * a.o.stride_l + (int64_t)ri.h * a.o.stride_h + lane * 4;
-          if (a.o.dtype == BMA_DTYPE_F32) *reinterpret_cast<float4*>(static_cast<float*>(a.o.ptr) + off) = o4;
-          else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.o.ptr) + off) = make_uint2(pack_bf16(o4.x, o4.y), pack_bf16(o4.z, o4.w));
+    } else if (__any_sync(0xffffffffu, r.valid)) {
+      float* stage = reinterpret_cast<float*>(sm.k[0]) + (x * BM + row) * kPitch;
+#pragma unroll
+      for (int c = 0; c < HD / 32; ++c) {
+        uint32_t v[32];
+        if (cnt > 0) {
+          tmem_ld32(tmem_o + c * 32, v);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0u;
         }
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          *reinterpret_cast<float4*>(stage + c * 32 + j) =
+              make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
       }
     }
   }
   tc_fence_before();
-  __syncthreads();
+  if (sp.cluster > 1) cluster_sync();
+  else __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+
+  // ---- every row: the weighted sum of its partials (two per CTA), relative to their common maximum; half a warp per row, the rows dealt
+  // out over the CTAs of the cluster.  (A round of loads from another CTA takes 0.5 us: all rows go through the three rounds
+  // at once.  The code is short rather than unrolled: it runs once, from a cold instruction cache.)
+  if (warp < 8) {
+    const int rows = sp.heads * sp.tile_queries, sources = 2 * sp.cluster, rank = sp.cluster > 1 ? (int)cluster_rank() : 0;
+    const int c = lane & 15;
+#pragma unroll 1
+    for (int i0 = warp * 2; i0 * sp.cluster < rows; i0 += 16) {
+      const int i = rank + sp.cluster * (i0 + (lane >> 4));
+      const int ql = i / sp.heads, q = first.q + ql, h = h0 + i - ql * sp.heads;
+      const bool valid = i < rows && q < a.N;
+      float m = -INFINITY, l = 0.f;
+      if (valid && c < sources) {
+        const uint32_t at = cluster_addr(&sm.ml[c & 1][0][i], (uint32_t)(c >> 1));
+        m = cluster_ld(at);
+        l = cluster_ld(at + BM * (uint32_t)sizeof(float));
+      }
+      float mt = l > 0.f ? m : -INFINITY;
+#pragma unroll
+      for (int off = 8; off; off >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, off));
+      const float f = l > 0.f ? ex2(m - mt) : 0.f;
+      float lt = l * f;
+#pragma unroll
+      for (int off = 8; off; off >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, off);
+      float4 acc[HD / 64];
+#pragma unroll
+      for (int u = 0; u < HD / 64; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float* part = reinterpret_cast<const float*>(sm.k[0]) + (valid ? i : 0) * kPitch + c * 4;
+#pragma unroll 4
+      for (int src = 0; src < sources; ++src) {
+        const uint32_t at = cluster_addr(part + (src & 1) * BM * kPitch, (uint32_t)(src >> 1));
+        const float w = __shfl_sync(0xffffffffu, f, src, 16);
+#pragma unroll
+        for (int u = 0; u < HD / 64; ++u) {
+          const float4 v = cluster_ld4(at + u * 256);
+          acc[u].x = fmaf(v.x, w, acc[u].x); acc[u].y = fmaf(v.y, w, acc[u].y); acc[u].z = fmaf(v.z, w, acc[u].z); acc[u].w = fmaf(v.w, w, acc[u].w);
+        }
+      }
+      if (!valid) continue;
+      if (sp.splits > sp.cluster) {   // the runs meet in the workspace: unnormalised, relative to the maximum of this one
+        const int64_t at = ((int64_t)unit * sp.splits + split) * BM + i;
+        if (c == 0) sp.part_ml[at] = make_float2(mt, lt);
+#pragma unroll
+        for (int u = 0; u < HD / 64; ++u) reinterpret_cast<float4*>(sp.part_o + at * HD)[u * 16 + c] = acc[u];
+        continue;
+      }
+      if (c == 0 && a.lse) a.lse[((int64_t)b * a.Hq + h) * a.N + q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
+      const float inv = lt > 0.f ? 1.f / lt : 0.f;
+#pragma unroll
+      for (int u = 0; u < HD / 64; ++u) {
+        const float4 o4 = make_float4(acc[u].x * inv, acc[u].y * inv, acc[u].z * inv, acc[u].w * inv);
+        const int64_t off = (int64_t)b * a.o.stride_b + (int64_t)q * a.o.stride_l + (int64_t)h * a.o.stride_h + u * 64 + c * 4;
+        if (a.o.dtype == BMA_DTYPE_F32) *reinterpret_cast<float4*>(static_cast<float*>(a.o.ptr) + off) = o4;
+        else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.o.ptr) + off) = make_uint2(pack_bf16(o4.x, o4.y), pack_bf16(o4.z, o4.w));
+      }
+    }
+  }
+  if (sp.cluster > 1) cluster_sync();   // shared memory stays until the others have read it
 }
 
 // One warp per (unit, row): O = sum over the splits of 2^(m_s - m) O_s / sum of 2^(m_s - m) l_s, and the log-sum-exp.
@@ -1586,9 +1618,59 @@ static SplitPlan split_plan(const bma_attn_args& a, const bma_block_lists& l) {
   return p;
 }
 
+// The persistent kernel draws its items' lists ahead, from memory; the other two build theirs at their start, and know the blocks of
+// interval terms without lists: a launch less,
+// 3 us of the device and 8 - 10 of the host (1 x 1500 float32 tokens, 16/4 heads of 128: the call 139 -> 131 us).
+bool sm100_fwd_wants_lists(const bma_attn_args& a, const bma_mask_spec& spec) {
+  const bma_block_lists one{1, 1, ceil_div(a.N, BM), ceil_div(a.L, BN), BM, BN};
+  return split_plan(a, one).splits == 0 && fwd_persistent_enabled(spec);
+}
+
 size_t sm100_fwd_workspace_bytes(const bma_attn_args& a, const bma_block_lists& lists) {
   const SplitPlan p = split_plan(a, lists);
   return p.splits > 1 ? (size_t)p.units * p.splits * BM * (a.d + 2) * sizeof(float) : 0;
+}
+
+// CTAs of a cluster: the runs of a unit, where up to eight of them run at the same time on the SMs of a GPC without making more waves
+// of the launch; else 1, and the runs meet in the workspace.  (4 runs of 32 units, 16 queries on 8192 keys: 32 us against
+// 33 + 4 in two launches.)
+static cudaLaunchAttribute cluster_of(int n) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1; attr.val.clusterDim.y = n; attr.val.clusterDim.z = 1;
+  return attr;
+}
+static cudaLaunchConfig_t split_config(const SplitPlan& plan, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(plan.units, plan.splits);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  return cfg;
+}
+static int split_cluster(int d, const SplitPlan& plan) {
+  if (plan.splits < 2 || plan.splits > kMaxCluster) return 1;
+  static std::atomic<int> at_once[2][kMaxCluster + 1];   // clusters of a size that the device runs at the same time, plus one
+  std::atomic<int>& known = at_once[d == 128][plan.splits];
+  int n = known.load(std::memory_order_relaxed);
+  if (!n) {
+    auto ask = [&](auto kernel, size_t smem) {
+      cudaLaunchConfig_t cfg = split_config(plan, smem, nullptr);
+      cudaLaunchAttribute attr = cluster_of(plan.splits);
+      cfg.attrs = &attr; cfg.numAttrs = 1;
+      int most = 0;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        most = 0;
+      }
+      return most;
+    };
+    n = 1 + (d == 128 ? ask(fwd_split_kernel<128, false>, sizeof(FwdSplitSmem<128>)) : ask(fwd_split_kernel<64, false>, sizeof(FwdSplitSmem<64>)));
+    known.store(n, std::memory_order_relaxed);
+  }
+  const int clusters = n - 1;
+  return clusters > 0 && ceil_div(plan.units, clusters) <= ceil_div(plan.units * plan.splits, kSms) ? plan.splits : 1;
 }
 
 static int sm100_fwd_split(const bma_attn_args& a, const FwdParams& f, const SplitPlan& plan, const CUtensorMap& mk, const CUtensorMap& mv,
@@ -1601,16 +1683,20 @@ static int sm100_fwd_split(const bma_attn_args& a, const FwdParams& f, const Spl
   p.heads = plan.heads; p.tile_queries = plan.tile_queries; p.q_tiles = plan.q_tiles; p.splits = plan.splits;
   p.part_o = static_cast<float*>(ws);
   p.part_ml = reinterpret_cast<float2*>(p.part_o + (size_t)plan.units * plan.splits * BM * a.d);
+  p.cluster = split_cluster(a.d, plan);
   auto launch = [&](auto kernel, size_t smem) -> int {
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<dim3(plan.units, plan.splits), kThreads, smem, st>>>(mq, mk, mv, p);
+    cudaLaunchConfig_t cfg = split_config(plan, smem, st);
+    cudaLaunchAttribute attr = cluster_of(p.cluster);
+    if (p.cluster > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
+    BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p));
     return BMA_OK;
   };
   if (a.d == 128) rc = kb ? launch(fwd_split_kernel<128, true>, sizeof(FwdSplitSmem<128>)) : launch(fwd_split_kernel<128, false>, sizeof(FwdSplitSmem<128>));
   else rc = kb ? launch(fwd_split_kernel<64, true>, sizeof(FwdSplitSmem<64>)) : launch(fwd_split_kernel<64, false>, sizeof(FwdSplitSmem<64>));
   if (rc) return rc;
   count_launches(1);
-  if (plan.splits > 1) {
+  if (plan.splits > p.cluster) {
     const int64_t rows = (int64_t)plan.units * plan.heads * plan.tile_queries;
     const unsigned grid = (unsigned)((rows + 7) / 8);
     if (a.d == 128) fwd_combine_kernel<128><<<grid, 256, 0, st>>>(p, plan.units);
@@ -1645,9 +1731,9 @@ int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
   const bool kb = a.key_bias != nullptr || a.scale < 0.f;
   const SplitPlan split = split_plan(a, lists);
-  if (split.splits == 1 || (split.splits > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_bytes >= sm100_fwd_workspace_bytes(a, lists)))
+  if (split.splits == 1 || split_cluster(a.d, split) > 1 || (split.splits > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_bytes >= sm100_fwd_workspace_bytes(a, lists)))
     return sm100_fwd_split(a, p, split, mk, mv, ws, kb, st);
-  if (fwd_persistent_enabled(spec)) {
+  if (lists.kv_num && fwd_persistent_enabled(spec)) {
     // One CTA per SM for the whole launch; items are drawn from a counter that is zeroed on the stream first.
     int dev = 0, sms = 148;
     BMA_CUDA_TRY(cudaGetDevice(&dev));

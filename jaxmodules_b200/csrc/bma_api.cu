@@ -232,9 +232,11 @@ int validate_common(const bma_attn_args* a) {
   return BMA_OK;
 }
 
-int validate_lists(const bma_attn_args* a, const bma_block_lists* l, int tile, bool need_q_side) {
+// `implied`: the mask if the pass knows the blocks of interval terms by itself, so that all four arrays of the kv side may be NULL
+int validate_lists(const bma_attn_args* a, const bma_block_lists* l, int tile, bool need_q_side, const bma_mask_spec* implied = nullptr) {
   BMA_REQUIRE(l != nullptr, BMA_ERR_ARG);
-  BMA_REQUIRE(l->kv_num && l->kv_idx && l->full_kv_num && l->full_kv_idx, BMA_ERR_ARG);
+  const bool none = !l->kv_num && !l->kv_idx && !l->full_kv_num && !l->full_kv_idx;
+  BMA_REQUIRE((l->kv_num && l->kv_idx && l->full_kv_num && l->full_kv_idx) || (none && implied && !(implied->flags & kTableTerms)), BMA_ERR_ARG);
   BMA_REQUIRE(!need_q_side || (l->q_num && l->q_idx && l->full_q_num && l->full_q_idx), BMA_ERR_ARG);
   BMA_REQUIRE(l->q_block == tile && l->kv_block == tile, BMA_ERR_ARG);
   BMA_REQUIRE(l->NQ == ceil_div(a->N, tile) && l->NKV == ceil_div(a->L, tile), BMA_ERR_ARG);
@@ -338,6 +340,12 @@ size_t bma_attn_fwd_workspace_bytes(const bma_attn_args* args, const bma_block_l
   return sm100_fwd_workspace_bytes(*args, *lists);
 }
 
+int32_t bma_attn_fwd_implies_lists(const bma_attn_args* args, const bma_mask_spec* spec) {
+  if (validate_common(args) != BMA_OK || !spec || (spec->flags & kTableTerms)) return 0;
+  if (bma_attn_f32_workspace_bytes(args, 0)) return 1;
+  return pick_backend(args) == BMA_BACKEND_TCGEN05 && !sm100_fwd_wants_lists(*args, *spec);
+}
+
 int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
                  bma_stream_t stream) {
   return bma_attn_fwd_ws(args, spec, lists, nullptr, 0, stream);
@@ -355,7 +363,7 @@ int bma_attn_fwd_ws(const bma_attn_args* args, const bma_mask_spec* spec, const 
   const int be = pick_backend(args);
   BMA_REQUIRE(be > 0, BMA_ERR_UNSUPPORTED);
   const int tile = be == BMA_BACKEND_TCGEN05 ? kSm100Tile : kSimtTile;
-  if ((rc = validate_lists(args, lists, tile, false))) return rc;
+  if ((rc = validate_lists(args, lists, tile, false, be == BMA_BACKEND_TCGEN05 ? spec : nullptr))) return rc;
   BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return be == BMA_BACKEND_TCGEN05 ? sm100_fwd(*args, *spec, *lists, workspace, workspace_bytes, st) : simt_fwd(*args, *spec, *lists, st);
@@ -376,7 +384,7 @@ int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const
   if ((rc = validate_tensor(args->q, true)) || (rc = validate_tensor(args->k, true)) ||
       (rc = validate_tensor(args->v, true)) || (rc = validate_tensor(args->o, true)))
     return rc;
-  if ((rc = validate_lists(args, lists, kSm100Tile, false))) return rc;
+  if ((rc = validate_lists(args, lists, kSm100Tile, false, spec))) return rc;
   BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
   if (!workspace || workspace_bytes < need) return simt_wide_fwd(*args, *spec, *lists, static_cast<cudaStream_t>(stream));
   BMA_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15) == 0, BMA_ERR_WORKSPACE);

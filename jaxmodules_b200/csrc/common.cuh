@@ -296,6 +296,47 @@ __device__ __forceinline__ void col_interval(const MaskView& m, int k, int q0, i
   }
 }
 
+// Exact any/all of the interval terms (valid box, causal, band, block window) on one block.
+// Returns false when the block window changes inside the q block, in which case the caller
+// has to scan.  any/all are only meaningful when true is returned.
+__device__ __forceinline__ bool interval_classify(const bma_mask_spec& s, int q0, int k0, int QB, int KVB,
+                                                  bool& any, bool& all) {
+  const int qa = q0, qb = min(q0 + QB, s.q_valid) - 1;
+  const int ka = k0, kb = min(k0 + KVB, s.k_valid) - 1;
+  any = false; all = false;
+  if (qb < qa || kb < ka) return true;
+  const bool whole = (q0 + QB <= s.q_valid) && (k0 + KVB <= s.k_valid);
+  const int64_t gqa = (int64_t)qa + s.q_offset, gqb = (int64_t)qb + s.q_offset;
+  int64_t gka = (int64_t)ka + s.k_offset, gkb = (int64_t)kb + s.k_offset;
+  int64_t lo = INT64_MIN / 4, hi = INT64_MAX / 4;
+  if (s.flags & BMA_MASK_CAUSAL) hi = min(hi, (int64_t)0);
+  if (s.flags & BMA_MASK_BAND) { lo = max(lo, -(int64_t)s.band_left); hi = min(hi, (int64_t)s.band_right); }
+  bool window_covers = true;
+  int64_t aka = gka, akb = gkb;  // key range after intersecting with the window (for "any")
+  if (s.flags & BMA_MASK_BLOCK_WINDOW) {
+    if (gqa / s.win_block != gqb / s.win_block) return false;
+    const int total = s.win_left + s.win_right;
+    int64_t st = max((int64_t)0, gqa / s.win_block - s.win_left);
+    st = min(st, (int64_t)s.win_nblk - total);
+    const int64_t wlo = st * s.win_block, whi = (st + total) * s.win_block;
+    window_covers = (gka >= wlo) && (gkb < whi);
+    aka = max(gka, wlo);
+    akb = min(gkb, whi - 1);
+  }
+  // k - q takes every integer value in [aka - gqb, akb - gqa] on the box
+  any = (aka <= akb) && (max(lo, aka - gqb) <= min(hi, akb - gqa));
+  all = whole && window_covers && (gka - gqb >= lo) && (gkb - gqa <= hi);
+  return true;
+}
+
+// Class of one block of a mask of interval terms alone: 0 empty, 1 partial, 2 full.  Where the block window changes inside the q block the
+// block counts as partial: the kernels look at the elements of those.
+__device__ __forceinline__ int interval_class(const bma_mask_spec& s, int qi, int kj, int QB, int KVB) {
+  bool any, all;
+  if (!interval_classify(s, qi * QB, kj * KVB, QB, KVB, any, all)) return 1;
+  return all ? 2 : any ? 1 : 0;
+}
+
 struct QTileIter {  // flattened walk over (group head, listed q tile)
   const bma_block_lists& l;
   int b, hk, G, kj;
@@ -349,6 +390,7 @@ int simt_wide_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_b
 int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, size_t ws_bytes,
               cudaStream_t st);
 size_t sm100_fwd_workspace_bytes(const bma_attn_args& a, const bma_block_lists& lists);
+bool sm100_fwd_wants_lists(const bma_attn_args& a, const bma_mask_spec& spec);
 int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws,
               size_t ws_bytes, const int64_t* visited_host, cudaEvent_t mark, cudaStream_t st);
 size_t sm100_bwd_workspace_bytes(const bma_attn_args& a);

@@ -26,7 +26,7 @@ using OptTensor = std::optional<Tensor>;
 
 // ---- the library ------------------------------------------------------------------------------------------------
 #define BMA_FUNCTIONS(X)                                                                                                      \
-  X(bma_mask_compile_workspace_bytes) X(bma_mask_compile) X(bma_attn_plan) X(bma_attn_bwd_plan) X(bma_attn_fwd_workspace_bytes) \
+  X(bma_mask_compile_workspace_bytes) X(bma_mask_compile) X(bma_attn_plan) X(bma_attn_bwd_plan) X(bma_attn_fwd_implies_lists) X(bma_attn_fwd_workspace_bytes) \
   X(bma_attn_fwd_ws) X(bma_attn_f32_workspace_bytes) X(bma_attn_fwd_f32) X(bma_attn_bwd_f32) X(bma_attn_bwd_preprocess)       \
   X(bma_attn_bwd_workspace_bytes) X(bma_attn_bwd_scratch_bytes) X(bma_attn_bwd_scratch_min_bytes) X(bma_attn_bwd)
 struct Library {
@@ -111,6 +111,11 @@ py::tuple routes(const Tensor& q, const Tensor& k, const Tensor& v, const OptTen
     return py::make_tuple(r.backend, r.q_tile, r.kv_tile, r.f32_bytes);
   };
   return py::make_tuple(one(forward, false), one(backward, true));
+}
+
+bool implies_lists(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& key_bias, std::optional<double> scale, int backend, uintptr_t spec_at) {
+  const bma_attn_args a = arguments(q, k, v, key_bias, scale, backend);
+  return lib.bma_attn_fwd_implies_lists(&a, at_address<bma_mask_spec>(spec_at));
 }
 
 // ---- block lists ------------------------------------------------------------------------------------------------
@@ -256,6 +261,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q, const Tensor& k, co
 PYBIND11_MODULE(_host, m) {
   m.def("bind", &bind);
   m.def("routes", torch::wrap_pybind_function(routes));
+  m.def("implies_lists", torch::wrap_pybind_function(implies_lists));
   m.def("compile_lists", torch::wrap_pybind_function(compile_lists));
   m.def("forward", torch::wrap_pybind_function(forward));
   m.def("preprocess", torch::wrap_pybind_function(preprocess));

@@ -108,16 +108,31 @@ __device__ __forceinline__ ListRow list_row(const bma_block_lists& l, int b, int
 // (kF32Tile); a block gives the two tiles of the walked side that lie inside the sequence.
 template <bool QSIDE, bool WIDE>
 struct TileWalk {
+  static constexpr bool kNoLists = WIDE && !QSIDE;   // may come without lists (a mask of interval terms): the blocks in order of their index
   ListRow lr;
-  int it, n, extent;
-  __device__ __forceinline__ TileWalk(const bma_block_lists& l, int b, int h, int tile, int extent_)
-      : lr(list_row<QSIDE>(l, b, h, WIDE ? tile >> 1 : tile)), it(0), extent(extent_) {
+  const bma_mask_spec* spec;
+  int it, n, extent, row;
+  __device__ __forceinline__ TileWalk(const bma_block_lists& l, const bma_mask_spec& s, int b, int h, int tile, int extent_)
+      : spec(&s), it(0), extent(extent_), row(WIDE ? tile >> 1 : tile) {
+    if (kNoLists && !l.kv_num) {
+      lr.full_idx = nullptr;
+      n = 2 * l.NKV;
+      return;
+    }
+    lr = list_row<QSIDE>(l, b, h, row);
     n = (lr.nfull + lr.npart) * (WIDE ? 2 : 1);
   }
   __device__ __forceinline__ bool next(int& tile, bool& partial) {
     for (; it < n;) {
       const int e = WIDE ? it >> 1 : it, half = it & 1;
       ++it;
+      if (kNoLists && !lr.full_idx) {
+        const int c = interval_class(*spec, row, e, 2 * TQ, 2 * TK);
+        partial = c == 1;
+        tile = 2 * e + half;
+        if (c && tile * TK < extent) return true;
+        continue;
+      }
       partial = e >= lr.nfull;
       const int blk = partial ? lr.part_idx[e - lr.nfull] : lr.full_idx[e];
       tile = WIDE ? 2 * blk + half : blk;
@@ -155,7 +170,7 @@ __device__ __forceinline__ void fwd_tile(float* sm, const SimtParams& p, int qi,
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const MaskView mv = make_mask_view(p.spec, b, h);
   const float kb2 = p.a.key_bias ? __ldg(p.a.key_bias + h) * kLog2e : 0.f;  // per-head key bias in log2 units
-  TileWalk<false, WIDE> walk(p.l, b, h, qi, a.L);
+  TileWalk<false, WIDE> walk(p.l, p.spec, b, h, qi, a.L);
 
   stage_natural<T, DP>(Qs, a.q, b, q0, h, a.N, a.d);
 
@@ -314,7 +329,7 @@ __device__ __forceinline__ void dkdv_tile(float* sm, const SimtParams& p, int kj
     const int h = hk * G + g;
     const MaskView mv = make_mask_view(p.spec, b, h);
     const float kb2 = p.a.key_bias ? __ldg(p.a.key_bias + h) * kLog2e : 0.f;  // per-head key bias in log2 units
-    TileWalk<true, WIDE> walk(p.l, b, h, kj, a.N);
+    TileWalk<true, WIDE> walk(p.l, p.spec, b, h, kj, a.N);
     int qi;
     bool partial;
     while (walk.next(qi, partial)) {
@@ -388,7 +403,7 @@ __device__ __forceinline__ void dq_tile(float* sm, const SimtParams& p, int qi, 
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const MaskView mv = make_mask_view(p.spec, b, h);
   const float kb2 = p.a.key_bias ? __ldg(p.a.key_bias + h) * kLog2e : 0.f;  // per-head key bias in log2 units
-  TileWalk<false, WIDE> walk(p.l, b, h, qi, a.L);
+  TileWalk<false, WIDE> walk(p.l, p.spec, b, h, qi, a.L);
 
   stage_natural<T, DP>(Qs, a.q, b, q0, h, a.N, a.d);
   stage_natural<TDO, DP>(dOs, a.d_o, b, q0, h, a.N, a.d);
