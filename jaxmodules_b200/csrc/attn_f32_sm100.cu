@@ -56,27 +56,35 @@ constexpr int kMaxKvFwd = 4096, kMaxKvBwd = 1024;
 __device__ __forceinline__ void setmaxnreg_inc_208() { asm volatile("setmaxnreg.inc.sync.aligned.u32 208;"); }
 __device__ __forceinline__ void setmaxnreg_dec_80() { asm volatile("setmaxnreg.dec.sync.aligned.u32 80;"); }
 
-// x = hi + mid + lo, exactly, for two neighbouring values (packed like an MMA operand)
-__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = pack_bf16(x, y);
-  x -= __uint_as_float(hi << 16);
-  y -= __uint_as_float(hi & 0xffff0000u);
-  mid = pack_bf16(x, y);
-  x -= __uint_as_float(mid << 16);
-  y -= __uint_as_float(mid & 0xffff0000u);
-  lo = pack_bf16(x, y);
+// x = hi + mid + lo, exactly, for two neighbouring values (packed like an MMA operand).  The row threads work on pairs throughout: the
+// packed FP32 instructions round like the scalar ones and take one issue slot for two.
+__device__ __forceinline__ float2 minus_hi(float2 x, uint32_t hi) {
+  return __ffma2_rn(make_float2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u)), make_float2(-1.f, -1.f), x);
 }
+__device__ __forceinline__ void split3(float2 x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16(x.x, x.y);
+  x = minus_hi(x, hi);
+  mid = pack_bf16(x.x, x.y);
+  x = minus_hi(x, mid);
+  lo = pack_bf16(x.x, x.y);
+}
+// Sum of the two halves of an accumulator region, columns 2j and 2j + 1.
+__device__ __forceinline__ float2 halves(const uint32_t* r0, const uint32_t* r1, int j) {
+  return __fadd2_rn(make_float2(__uint_as_float(r0[2 * j]), __uint_as_float(r0[2 * j + 1])),
+                    make_float2(__uint_as_float(r1[2 * j]), __uint_as_float(r1[2 * j + 1])));
+}
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
 
 // Plane p of the A operand of k-step ks (16 keys or queries) inside a 128-column accumulator region.
 __device__ __forceinline__ uint32_t plane_col(int p, int ks) { return p == 2 ? 64 + 16 * ks : 16 * ks + 8 * p; }
 
 // Stores the planes of 32 consecutive values (k-steps ks0, ks0 + 1) over the columns they came from.
-__device__ __forceinline__ void store_planes32(uint32_t region, int ks0, const float* v) {
+__device__ __forceinline__ void store_planes32(uint32_t region, int ks0, const float2* v) {
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     uint32_t hm[16], lo[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) split3(v[u * 16 + 2 * j], v[u * 16 + 2 * j + 1], hm[j], hm[8 + j], lo[j]);
+    for (int j = 0; j < 8; ++j) split3(v[u * 8 + j], hm[j], hm[8 + j], lo[j]);
     tmem_st16(region + 16 * (ks0 + u), hm);
     tmem_st8(region + 64 + 16 * (ks0 + u), lo);
   }
@@ -198,7 +206,7 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitParams p) {
     }
     uint32_t w[3][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) split3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+    for (int e = 0; e < 4; ++e) split3(make_float2(v[2 * e], v[2 * e + 1]), w[0][e], w[1][e], w[2][e]);
 #pragma unroll
     for (int q = 0; q < 3; ++q) out[q * n + i] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
   };
@@ -217,6 +225,12 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitParams p) {
     const int end = min(at + kPiece, min(BM, job.L - l0) * job.H * kChunks);
     for (int i = at + (int)threadIdx.x; i < end; i += blockDim.x) split8(first + i);
   }
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
 struct F32Params {
@@ -315,6 +329,15 @@ __device__ __forceinline__ void row_bits64(const bma_mask_spec& spec, int b, int
   }
 }
 
+// Probabilities of 32 columns: those that `bits` does not allow become 0.
+__device__ __forceinline__ void keep_allowed(float2* pr, uint32_t bits) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (!((bits >> (2 * j)) & 1u)) pr[j].x = 0.f;
+    if (!((bits >> (2 * j + 1)) & 1u)) pr[j].y = 0.f;
+  }
+}
+
 // 128 rows of `cols` staged floats (row pitch `pitch`) to a [*, *, *, d] tensor, whole rows per warp.
 template <int NT>
 __device__ __forceinline__ void store_rows(const float* stage, int pitch, const bma_tensor& t, int b, int l0, int lmax, int h, int d, int tid) {
@@ -369,7 +392,8 @@ struct __align__(1024) FwdSmem {
 
 static_assert(fwd_smem<4>() <= sizeof(FwdSmem<64>) && fwd_smem<8>() <= sizeof(FwdSmem<128>), "a tile is done again in the same shared memory");
 
-template <int DP>
+// KB: with a key bias, or a negative scale (for which the maximum of the scores is not that of the scaled ones).
+template <int DP, bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ F32Params p) {
@@ -500,9 +524,9 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const uint32_t tmem_s = tmem + x * 256 + lane_base, tmem_o = tmem_s + 128;
     const float kb2 = a.key_bias ? __ldg(a.key_bias + h) * kLog2e : 0.f;
     const int Tx = x ? T1 : T0;
-    float o[DP];
+    float2 o[DP / 2];
 #pragma unroll
-    for (int j = 0; j < DP; ++j) o[j] = 0.f;
+    for (int j = 0; j < DP / 2; ++j) o[j] = both(0.f);
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int n = 0; n < Tx; ++n) {
@@ -510,19 +534,27 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       const int k0 = (int)(e & 0x7fff) * 128 + x * BH;
       uint32_t bits[2] = {0xffffffffu, 0xffffffffu};
       if (e & 0x8000u) row_bits64(p.spec, b, h, q, k0, bits);
+      const bool cut = (e & 0x8000u) != 0;
       const float kbase = (float)(p.spec.k_offset + k0);
-      // 16 scores in log2 units from tensor memory (the two accumulator halves added)
-      auto scores16 = [&](int c, float* v) {
+      // 16 scores from tensor memory (KB: in log2 units)
+      auto scores16 = [&](int c, float2* v) {
         uint32_t r0[16], r1[16];
         tmem_ld16(tmem_s + c * 16, r0);
         tmem_ld16(tmem_s + 64 + c * 16, r1);
         tmem_wait_ld();
-        const uint32_t w = (c < 2 ? bits[0] : bits[1]) >> ((c & 1) * 16);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float s = (__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
-          v[j] = fmaf(s, p.scale_log2, kb2 * (kbase + (float)(c * 16 + j)));
-          if (!((w >> j) & 1u)) v[j] = -INFINITY;
+        for (int j = 0; j < 8; ++j) {
+          v[j] = halves(r0, r1, j);
+          if constexpr (KB)
+            v[j] = __ffma2_rn(v[j], both(p.scale_log2), make_float2(kb2 * (kbase + (float)(c * 16 + 2 * j)), kb2 * (kbase + (float)(c * 16 + 2 * j + 1))));
+        }
+        if (cut) {
+          const uint32_t w = (c < 2 ? bits[0] : bits[1]) >> ((c & 1) * 16);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (!((w >> (2 * j)) & 1u)) v[j].x = -INFINITY;
+            if (!((w >> (2 * j + 1)) & 1u)) v[j].y = -INFINITY;
+          }
         }
       };
       ok = mbar_wait(&sm.bar[FB_S0 + x], n & 1);
@@ -530,38 +562,43 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       tc_fence_after();
       // 128 head columns leave no registers for 64 scores beside O: those are read twice, once for the maximum
       constexpr bool kKeep = DP == 64;
-      float s[kKeep ? 64 : 16];
-      float mx = -INFINITY;
+      float2 s[kKeep ? 32 : 8];
+      float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll (kKeep ? 4 : 1)
       for (int c = 0; c < 4; ++c) {
-        float* v = s + (kKeep ? c * 16 : 0);
+        float2* v = s + (kKeep ? c * 8 : 0);
         scores16(c, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) mx = fmaxf(mx, v[j]);
+        for (int j = 0; j < 8; j += 2) {
+          mx0 = max3(mx0, v[j].x, v[j].y);
+          mx1 = max3(mx1, v[j + 1].x, v[j + 1].y);
+        }
       }
-      const float m_new = fmaxf(m, mx), m_safe = (m_new == -INFINITY) ? 0.f : m_new;
+      const float mx = fmaxf(mx0, mx1);
+      const float m_new = fmaxf(m, KB || mx == -INFINITY ? mx : mx * p.scale_log2), m_safe = (m_new == -INFINITY) ? 0.f : m_new;
       const float alpha = ex2(m - m_safe);
       m = m_new;
-      float rs[4] = {0.f, 0.f, 0.f, 0.f};
+      const float2 sc = both(KB ? 1.f : p.scale_log2);
+      float2 rs[2] = {both(0.f), both(0.f)};
 #pragma unroll (kKeep ? 4 : 1)
       for (int c = 0; c < 4; ++c) {
-        float* v = s + (kKeep ? c * 16 : 0);
+        float2* v = s + (kKeep ? c * 8 : 0);
         if (!kKeep) scores16(c, v);
         uint32_t hm[16], lo[8];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          v[j] = ex2(v[j] - m_safe);
-          rs[j & 3] += v[j];
+        for (int j = 0; j < 8; ++j) {
+          const float2 t = __ffma2_rn(v[j], sc, both(-m_safe));
+          const float2 pr = make_float2(ex2(t.x), ex2(t.y));
+          rs[j & 1] = __fadd2_rn(rs[j & 1], pr);
+          split3(pr, hm[j], hm[8 + j], lo[j]);
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) split3(v[2 * j], v[2 * j + 1], hm[j], hm[8 + j], lo[j]);
         tmem_st16(tmem_s + c * 16, hm);        // over the 16 + 8 columns whose scores have just been used
         tmem_st8(tmem_s + 64 + c * 16, lo);
       }
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(&sm.bar[FB_P0 + x]);
-      l = l * alpha + ((rs[0] + rs[1]) + (rs[2] + rs[3]));
+      l = l * alpha + ((rs[0].x + rs[0].y) + (rs[1].x + rs[1].y));
       ok = mbar_wait(&sm.bar[FB_O0 + x], n & 1);
       if (!ok) break;
       tc_fence_after();
@@ -574,11 +611,12 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           tmem_ld32(tmem_o + 64 + c * 32, r1);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) o[c * 32 + j] = fmaf(o[c * 32 + j], alpha, __uint_as_float(r0[j]) + __uint_as_float(r1[j]));
+          for (int j = 0; j < 16; ++j) o[c * 16 + j] = __ffma2_rn(o[c * 16 + j], both(alpha), halves(r0, r1, j));
         } else {
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) o[c * 32 + j] = fmaf(o[c * 32 + j], alpha, __uint_as_float(r0[j]));
+          for (int j = 0; j < 16; ++j)
+            o[c * 16 + j] = __ffma2_rn(o[c * 16 + j], both(alpha), make_float2(__uint_as_float(r0[2 * j]), __uint_as_float(r0[2 * j + 1])));
         }
       }
       tc_fence_before();
@@ -605,7 +643,7 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     float* stage = reinterpret_cast<float*>(sm.q) + row * kPitch;
     if (x == 0) {
 #pragma unroll
-      for (int j = 0; j < DP; j += 4) *reinterpret_cast<float4*>(stage + j) = make_float4(o[j] * mine, o[j + 1] * mine, o[j + 2] * mine, o[j + 3] * mine);
+      for (int j = 0; j < DP; j += 4) *reinterpret_cast<float4*>(stage + j) = make_float4(o[j / 2].x * mine, o[j / 2].y * mine, o[j / 2 + 1].x * mine, o[j / 2 + 1].y * mine);
     }
     rendezvous();
     if (x == 1) {
@@ -613,7 +651,7 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
       for (int j = 0; j < DP; j += 4) {
         float4 v = *reinterpret_cast<float4*>(stage + j);
-        v.x = fmaf(o[j], mine, v.x); v.y = fmaf(o[j + 1], mine, v.y); v.z = fmaf(o[j + 2], mine, v.z); v.w = fmaf(o[j + 3], mine, v.w);
+        v.x = fmaf(o[j / 2].x, mine, v.x); v.y = fmaf(o[j / 2].y, mine, v.y); v.z = fmaf(o[j / 2 + 1].x, mine, v.z); v.w = fmaf(o[j / 2 + 1].y, mine, v.w);
         *reinterpret_cast<float4*>(stage + j) = v;
         note_finite(z, (v.x + v.y) + (v.z + v.w));
       }
@@ -647,7 +685,7 @@ struct __align__(1024) DkdvSmem {
   uint8_t v[3][kRowBox];
   uint8_t q[2][3][kHalfBox];
   uint8_t d_o[2][3][kHalfBox];
-  float lse2[2][BH], delta[2][BH];
+  float nlse2[2][BH], ndelta[2][BH];   // minus the log-sum-exp (log2 units) and delta
   uint64_t bar[KB_NUM];
   uint32_t tmem_base;
   int not_finite;
@@ -676,6 +714,7 @@ struct HalfIter {
   }
 };
 
+template <bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                 const __grid_constant__ CUtensorMap map_qh, const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32Params p) {
@@ -750,8 +789,8 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
           const int idx = e * 32 + lane, q = q0 + idx;
           const int64_t off = ((int64_t)b * a.Hq + h) * a.N + q;
           const float lv = q < a.N ? __ldg(a.lse + off) : -INFINITY;
-          sm.lse2[st][idx] = (lv == -INFINITY) ? INFINITY : lv * kLog2e;   // +inf: the probabilities of the row become exactly 0
-          sm.delta[st][idx] = q < a.N ? __ldg(a.delta + off) : 0.f;
+          sm.nlse2[st][idx] = (lv == -INFINITY) ? -INFINITY : -lv * kLog2e;   // -inf: the probabilities of the row become exactly 0
+          sm.ndelta[st][idx] = q < a.N ? -__ldg(a.delta + off) : 0.f;
         }
         mbar_arrive(&sm.bar[KB_STAT + st]);
       }
@@ -806,9 +845,9 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
     const int w = warp >> 2, row = threadIdx.x & 127, k = k0 + row;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tm = tmem + lane_base;
-    float acc[64];   // warpgroup 0: dV, warpgroup 1: dK of this key row
+    float2 acc[32];   // warpgroup 0: dV, warpgroup 1: dK of this key row
 #pragma unroll
-    for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+    for (int j = 0; j < 32; ++j) acc[j] = both(0.f);
     bool ok = true;
     const uint32_t col_acc = w == 0 ? COL_DV : COL_DK;
     uint64_t* acc_full = &sm.bar[w == 0 ? KB_DV : KB_DK];
@@ -823,7 +862,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         tmem_ld32(tm + col_acc + 64 + c * 32, r1);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[c * 32 + j] += __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+        for (int j = 0; j < 16; ++j) acc[c * 16 + j] = __fadd2_rn(acc[c * 16 + j], halves(r0, r1, j));
       }
       tc_fence_before();
       mbar_arrive(acc_free);
@@ -834,7 +873,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
     bool partial;
     for (; ok && walk.next(h, q0, partial); ++n) {
       const int st = n & 1;
-      const float kbk = a.key_bias ? __ldg(a.key_bias + h) * kLog2e * (float)(p.spec.k_offset + k) : 0.f;
+      const float kbk = KB ? __ldg(a.key_bias + h) * kLog2e * (float)(p.spec.k_offset + k) : 0.f;
       uint32_t bits = 0xffffffffu;
       if (partial) {
         const MaskView mv = make_mask_view(p.spec, b, h);
@@ -847,7 +886,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
       ok = mbar_wait(&sm.bar[KB_STAT + st], (n >> 1) & 1) && mbar_wait(&sm.bar[KB_S], n & 1);
       if (!ok) break;
       tc_fence_after();
-      float pr[32];
+      float2 pr[16];
       {
         uint32_t r0[32], r1[32];
         tmem_ld32(tm + COL_ST + w * 32, r0);
@@ -855,15 +894,16 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         tmem_wait_ld();
 #pragma unroll
         for (int j4 = 0; j4 < 8; ++j4) {
-          const float4 lv = *reinterpret_cast<const float4*>(&sm.lse2[st][w * 32 + j4 * 4]);
-          const float l4[4] = {lv.x, lv.y, lv.z, lv.w};
+          const float4 lv = *reinterpret_cast<const float4*>(&sm.nlse2[st][w * 32 + j4 * 4]);
+          float2 l2[2] = {make_float2(lv.x, lv.y), make_float2(lv.z, lv.w)};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int j = j4 * 4 + e;
-            const float s = __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
-            pr[j] = (bits >> j) & 1u ? ex2(fmaf(s, p.scale_log2, kbk) - l4[e]) : 0.f;
+          for (int e = 0; e < 2; ++e) {
+            if constexpr (KB) l2[e] = __fadd2_rn(l2[e], both(kbk));
+            const float2 t = __ffma2_rn(halves(r0, r1, j4 * 2 + e), both(p.scale_log2), l2[e]);
+            pr[j4 * 2 + e] = make_float2(ex2(t.x), ex2(t.y));
           }
         }
+        if (partial) keep_allowed(pr, bits);
       }
       store_planes32(tm + COL_ST, w * 2, pr);
       tmem_wait_st();
@@ -880,13 +920,9 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         tmem_wait_ld();
 #pragma unroll
         for (int j4 = 0; j4 < 8; ++j4) {
-          const float4 dl = *reinterpret_cast<const float4*>(&sm.delta[st][w * 32 + j4 * 4]);
-          const float d4[4] = {dl.x, dl.y, dl.z, dl.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int j = j4 * 4 + e;
-            pr[j] *= (__uint_as_float(r0[j]) + __uint_as_float(r1[j])) - d4[e];
-          }
+          const float4 dl = *reinterpret_cast<const float4*>(&sm.ndelta[st][w * 32 + j4 * 4]);
+          pr[j4 * 2] = __fmul2_rn(pr[j4 * 2], __fadd2_rn(halves(r0, r1, j4 * 2), make_float2(dl.x, dl.y)));
+          pr[j4 * 2 + 1] = __fmul2_rn(pr[j4 * 2 + 1], __fadd2_rn(halves(r0, r1, j4 * 2 + 1), make_float2(dl.z, dl.w)));
         }
       }
       store_planes32(tm + COL_DPT, w * 2, pr);
@@ -903,11 +939,15 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
     const float sc = w == 0 ? 1.f : a.scale;
     float z = 0.f;
 #pragma unroll
-    for (int j = 0; j < 64; ++j) note_finite(z, acc[j] * sc);
+    for (int j = 0; j < 32; ++j) {
+      acc[j] = __fmul2_rn(acc[j], both(sc));
+      note_finite(z, acc[j].x);
+      note_finite(z, acc[j].y);
+    }
     if (z != 0.f) sm.not_finite = 1;
 #pragma unroll
     for (int j = 0; j < 64; j += 4)
-      if (ok) *reinterpret_cast<float4*>(stage + row * kPitch + j) = make_float4(acc[j] * sc, acc[j + 1] * sc, acc[j + 2] * sc, acc[j + 3] * sc);
+      if (ok) *reinterpret_cast<float4*>(stage + row * kPitch + j) = make_float4(acc[j / 2].x, acc[j / 2].y, acc[j / 2 + 1].x, acc[j / 2 + 1].y);
     mbar_arrive(&sm.bar[KB_EPI0 + w]);
     ok = mbar_wait(&sm.bar[KB_EPI0 + w], 0) && ok;
     if (ok) store_rows<128>(stage, kPitch, w == 0 ? a.dv : a.dk, b, k0, a.L, hk, a.d, row);
@@ -942,6 +982,7 @@ struct __align__(1024) DqSmem {
 static_assert(dq_smem<4>() <= sizeof(DqSmem), "as above");
 constexpr uint32_t COL_S2 = 0, COL_DP2 = 256, COL_DQ2 = 384;   // S: two buffers of 128 columns
 
+template <bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kh,
               const __grid_constant__ CUtensorMap map_vh, const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32Params p) {
@@ -1042,15 +1083,15 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tm = tmem + lane_base;
     const float kb2 = a.key_bias ? __ldg(a.key_bias + h) * kLog2e : 0.f;
-    float lse2 = INFINITY, delta = 0.f;
+    float nlse2 = -INFINITY, ndelta = 0.f;   // minus the log-sum-exp (log2 units) and delta
     if (q < a.N) {
       const float lv = __ldg(a.lse + ((int64_t)b * a.Hq + h) * a.N + q);
-      lse2 = lv == -INFINITY ? INFINITY : lv * kLog2e;
-      delta = __ldg(a.delta + ((int64_t)b * a.Hq + h) * a.N + q);
+      nlse2 = lv == -INFINITY ? -INFINITY : -lv * kLog2e;
+      ndelta = -__ldg(a.delta + ((int64_t)b * a.Hq + h) * a.N + q);
     }
-    float acc[32];
+    float2 acc[16];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+    for (int j = 0; j < 16; ++j) acc[j] = both(0.f);
     bool ok = true;
     auto flush = [&](int n) -> bool {
       if (!mbar_wait(&sm.bar[QB_DQ], n & 1)) return false;
@@ -1060,7 +1101,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       tmem_ld32(tm + COL_DQ2 + 64 + w * 32, r1);
       tmem_wait_ld();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] += __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+      for (int j = 0; j < 16; ++j) acc[j] = __fadd2_rn(acc[j], halves(r0, r1, j));
       tc_fence_before();
       mbar_arrive(&sm.bar[QB_DQFREE]);
       return true;
@@ -1078,17 +1119,20 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       ok = mbar_wait(&sm.bar[QB_S + (n & 1)], (n >> 1) & 1);
       if (!ok) break;
       tc_fence_after();
-      float pr[32];
+      float2 pr[16];
       {
         uint32_t r0[32], r1[32];
         tmem_ld32(tm + COL_S2 + (n & 1) * 128 + w * 32, r0);
         tmem_ld32(tm + COL_S2 + (n & 1) * 128 + 64 + w * 32, r1);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float s = __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
-          pr[j] = (bits >> j) & 1u ? ex2(fmaf(s, p.scale_log2, kb2 * (kbase + (float)j)) - lse2) : 0.f;
+        for (int j = 0; j < 16; ++j) {
+          float2 l2 = both(nlse2);
+          if constexpr (KB) l2 = __fadd2_rn(l2, make_float2(kb2 * (kbase + (float)(2 * j)), kb2 * (kbase + (float)(2 * j + 1))));
+          const float2 t = __ffma2_rn(halves(r0, r1, j), both(p.scale_log2), l2);
+          pr[j] = make_float2(ex2(t.x), ex2(t.y));
         }
+        if (e & 0x8000u) keep_allowed(pr, bits);
       }
       if (n > 0) ok = flush(n - 1);
       if (ok) ok = mbar_wait(&sm.bar[QB_DP], n & 1);
@@ -1100,7 +1144,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         tmem_ld32(tm + COL_DP2 + 64 + w * 32, r1);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) pr[j] *= (__uint_as_float(r0[j]) + __uint_as_float(r1[j])) - delta;
+        for (int j = 0; j < 16; ++j) pr[j] = __fmul2_rn(pr[j], __fadd2_rn(halves(r0, r1, j), both(ndelta)));
       }
       store_planes32(tm + COL_DP2, w * 2, pr);
       tmem_wait_st();
@@ -1111,14 +1155,18 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     if (ok && total == 0) ok = mbar_wait(&sm.bar[QB_Q], 0);
     float z = 0.f;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) note_finite(z, acc[j] * a.scale);
+    for (int j = 0; j < 16; ++j) {
+      acc[j] = __fmul2_rn(acc[j], both(a.scale));
+      note_finite(z, acc[j].x);
+      note_finite(z, acc[j].y);
+    }
     if (z != 0.f) sm.not_finite = 1;
     constexpr int kPitch = 68;
     float* stage = reinterpret_cast<float*>(&sm.q[0][0]);   // every MMA that read the Q planes has completed
     if (ok) {
 #pragma unroll
       for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<float4*>(stage + row * kPitch + w * 32 + j) = make_float4(acc[j] * a.scale, acc[j + 1] * a.scale, acc[j + 2] * a.scale, acc[j + 3] * a.scale);
+        *reinterpret_cast<float4*>(stage + row * kPitch + w * 32 + j) = make_float4(acc[j / 2].x, acc[j / 2].y, acc[j / 2 + 1].x, acc[j / 2 + 1].y);
     }
     mbar_arrive(&sm.bar[QB_EPI]);
     ok = mbar_wait(&sm.bar[QB_EPI], 0) && ok;
@@ -1211,7 +1259,7 @@ struct __align__(1024) DkdvWideSmem {
   uint8_t k[3][2][kRowBox];
   uint8_t q[3][kBoxPlanes];
   uint8_t d_o[2][kBoxPlanes];
-  float lse2[2][BH], delta[2][BH];
+  float nlse2[2][BH], ndelta[2][BH];   // minus the log-sum-exp (log2 units) and delta
   uint64_t bar[XB_NUM];
   uint32_t tmem_base;
   int not_finite;
@@ -1220,6 +1268,7 @@ static_assert(dkdv_smem<8>() <= sizeof(DkdvWideSmem), "as above");
 constexpr int kWidePitch = 132;
 static_assert(2 * BM * kWidePitch * sizeof(float) <= sizeof(uint8_t[3][2][kRowBox]) + 3 * kBoxPlanes, "dV and dK are staged over K and Q");
 
+template <bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_qh,
                      const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32WideParams wp) {
@@ -1296,8 +1345,8 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
           const int idx = e * 32 + lane, q = q0 + idx;
           const int64_t off = ((int64_t)b * a.Hq + h) * a.N + q;
           const float lv = q < a.N ? __ldg(a.lse + off) : -INFINITY;
-          sm.lse2[st][idx] = (lv == -INFINITY) ? INFINITY : lv * kLog2e;   // +inf: the probabilities of the row become exactly 0
-          sm.delta[st][idx] = q < a.N ? __ldg(a.delta + off) : 0.f;
+          sm.nlse2[st][idx] = (lv == -INFINITY) ? -INFINITY : -lv * kLog2e;   // -inf: the probabilities of the row become exactly 0
+          sm.ndelta[st][idx] = q < a.N ? -__ldg(a.delta + off) : 0.f;
         }
         mbar_arrive(&sm.bar[XB_STAT + st]);
       }
@@ -1366,18 +1415,18 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     load_planes_tmem(tm, w, wp.a_planes, a.B, a.L, a.Hkv, b, k, hk);
     tc_fence_before();
     mbar_arrive(&sm.bar[XB_A]);
-    float acc[4][32];   // columns [32w, 32w + 32) of dV0, dK0, dV1, dK1 of this key row
+    float2 acc[4][16];   // columns [32w, 32w + 32) of dV0, dK0, dV1, dK1 of this key row
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[c][j] = 0.f;
+      for (int j = 0; j < 16; ++j) acc[c][j] = both(0.f);
     bool ok = true;
     HalfIter walk(p.l, b, hk, G, kj, a.N);
     int h, q0, n = 0;
     bool partial;
     for (; ok && walk.next(h, q0, partial); ++n) {
       const int st = n & 1;
-      const float kbk = a.key_bias ? __ldg(a.key_bias + h) * kLog2e * (float)(p.spec.k_offset + k) : 0.f;
+      const float kbk = KB ? __ldg(a.key_bias + h) * kLog2e * (float)(p.spec.k_offset + k) : 0.f;
       uint32_t bits = 0xffffffffu;
       if (partial) {
         const MaskView mv = make_mask_view(p.spec, b, h);
@@ -1390,7 +1439,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
       ok = mbar_wait(&sm.bar[XB_STAT + st], (n >> 1) & 1) && mbar_wait(&sm.bar[XB_S], n & 1);
       if (!ok) break;
       tc_fence_after();
-      float pr[32];
+      float2 pr[16];
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t r0[16], r1[16];
@@ -1398,11 +1447,14 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         tmem_ld16(tm + COL_W_S + 64 + w * 32 + c * 16, r1);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float s = __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
-          pr[c * 16 + j] = (bits >> (c * 16 + j)) & 1u ? ex2(fmaf(s, p.scale_log2, kbk) - sm.lse2[st][w * 32 + c * 16 + j]) : 0.f;
+        for (int j = 0; j < 8; ++j) {
+          float2 l2 = *reinterpret_cast<const float2*>(&sm.nlse2[st][w * 32 + c * 16 + 2 * j]);
+          if constexpr (KB) l2 = __fadd2_rn(l2, both(kbk));
+          const float2 t = __ffma2_rn(halves(r0, r1, j), both(p.scale_log2), l2);
+          pr[c * 8 + j] = make_float2(ex2(t.x), ex2(t.y));
         }
       }
+      if (partial) keep_allowed(pr, bits);
       store_planes32(tm + COL_W_S, w * 2, pr);
       tmem_wait_st();
       tc_fence_before();
@@ -1417,7 +1469,8 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         tmem_ld16(tm + COL_W_DP + 64 + w * 32 + c * 16, r1);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) pr[c * 16 + j] *= (__uint_as_float(r0[j]) + __uint_as_float(r1[j])) - sm.delta[st][w * 32 + c * 16 + j];
+        for (int j = 0; j < 8; ++j)
+          pr[c * 8 + j] = __fmul2_rn(pr[c * 8 + j], __fadd2_rn(halves(r0, r1, j), *reinterpret_cast<const float2*>(&sm.ndelta[st][w * 32 + c * 16 + 2 * j])));
       }
       store_planes32(tm + COL_W_DP, w * 2, pr);
       tmem_wait_st();
@@ -1434,7 +1487,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         tc_fence_before();
         mbar_arrive(&sm.bar[XB_ACCFREE]);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[c][j] += __uint_as_float(r[j]);
+        for (int j = 0; j < 16; ++j) acc[c][j] = __fadd2_rn(acc[c][j], make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])));
       }
     }
     if (ok && n == 0) ok = mbar_wait(&sm.bar[XB_K], 0);   // let the loads land before their buffers are reused
@@ -1442,7 +1495,11 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-      for (int j = 0; j < 32; ++j) note_finite(z, (c & 1) ? acc[c][j] * a.scale : acc[c][j]);
+      for (int j = 0; j < 16; ++j) {
+        if (c & 1) acc[c][j] = __fmul2_rn(acc[c][j], both(a.scale));
+        note_finite(z, acc[c][j].x);
+        note_finite(z, acc[c][j].y);
+      }
     if (z != 0.f) sm.not_finite = 1;
     // ---- epilogue: every MMA has completed; dV and dK are staged over the K planes and the Q ring
     mbar_arrive(&sm.bar[XB_EPI]);
@@ -1452,10 +1509,9 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         float* dst = stage + (c & 1) * BM * kWidePitch + row * kWidePitch + (c >> 1) * 64 + w * 32;
-        const float sc = (c & 1) ? a.scale : 1.f;
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(acc[c][j] * sc, acc[c][j + 1] * sc, acc[c][j + 2] * sc, acc[c][j + 3] * sc);
+          *reinterpret_cast<float4*>(dst + j) = make_float4(acc[c][j / 2].x, acc[c][j / 2].y, acc[c][j / 2 + 1].x, acc[c][j / 2 + 1].y);
       }
     }
     mbar_arrive(&sm.bar[XB_EPI]);
@@ -1489,6 +1545,7 @@ struct __align__(1024) DqWideSmem {
 
 static_assert(dq_smem<8>() <= sizeof(DqWideSmem), "as above");
 
+template <bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kh,
                    const __grid_constant__ CUtensorMap map_vh, const __grid_constant__ F32WideParams wp) {
@@ -1605,17 +1662,17 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     tc_fence_before();
     mbar_arrive(&sm.bar[YB_A]);
     const float kb2 = a.key_bias ? __ldg(a.key_bias + h) * kLog2e : 0.f;
-    float lse2 = INFINITY, delta = 0.f;
+    float nlse2 = -INFINITY, ndelta = 0.f;   // minus the log-sum-exp (log2 units) and delta
     if (q < a.N) {
       const float lv = __ldg(a.lse + ((int64_t)b * a.Hq + h) * a.N + q);
-      lse2 = lv == -INFINITY ? INFINITY : lv * kLog2e;
-      delta = __ldg(a.delta + ((int64_t)b * a.Hq + h) * a.N + q);
+      nlse2 = lv == -INFINITY ? -INFINITY : -lv * kLog2e;
+      ndelta = -__ldg(a.delta + ((int64_t)b * a.Hq + h) * a.N + q);
     }
-    float acc[2][32];   // columns [32w, 32w + 32) of the two chunks of dQ of this row
+    float2 acc[2][16];   // columns [32w, 32w + 32) of the two chunks of dQ of this row
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[c][j] = 0.f;
+      for (int j = 0; j < 16; ++j) acc[c][j] = both(0.f);
     bool ok = true;
     for (int n = 0; n < total && ok; ++n) {
       const uint32_t e = sm.list.entry[n >> 1];
@@ -1630,17 +1687,20 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       ok = mbar_wait(&sm.bar[YB_S], n & 1);
       if (!ok) break;
       tc_fence_after();
-      float pr[32];
+      float2 pr[16];
       {
         uint32_t r0[32], r1[32];
         tmem_ld32(tm + COL_W_S + w * 32, r0);
         tmem_ld32(tm + COL_W_S + 64 + w * 32, r1);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float s = __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
-          pr[j] = (bits >> j) & 1u ? ex2(fmaf(s, p.scale_log2, kb2 * (kbase + (float)j)) - lse2) : 0.f;
+        for (int j = 0; j < 16; ++j) {
+          float2 l2 = both(nlse2);
+          if constexpr (KB) l2 = __fadd2_rn(l2, make_float2(kb2 * (kbase + (float)(2 * j)), kb2 * (kbase + (float)(2 * j + 1))));
+          const float2 t = __ffma2_rn(halves(r0, r1, j), both(p.scale_log2), l2);
+          pr[j] = make_float2(ex2(t.x), ex2(t.y));
         }
+        if (e & 0x8000u) keep_allowed(pr, bits);
       }
       ok = mbar_wait(&sm.bar[YB_DP], n & 1);
       if (!ok) break;
@@ -1651,7 +1711,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tmem_ld32(tm + COL_W_DP + 64 + w * 32, r1);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) pr[j] *= (__uint_as_float(r0[j]) + __uint_as_float(r1[j])) - delta;
+        for (int j = 0; j < 16; ++j) pr[j] = __fmul2_rn(pr[j], __fadd2_rn(halves(r0, r1, j), both(ndelta)));
       }
       store_planes32(tm + COL_W_DP, w * 2, pr);
       tmem_wait_st();
@@ -1668,7 +1728,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tc_fence_before();
         mbar_arrive(&sm.bar[YB_ACCFREE]);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[c][j] += __uint_as_float(r[j]);
+        for (int j = 0; j < 16; ++j) acc[c][j] = __fadd2_rn(acc[c][j], make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])));
       }
     }
     if (ok && total == 0) ok = mbar_wait(&sm.bar[YB_Q], 0);
@@ -1676,7 +1736,11 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int j = 0; j < 32; ++j) note_finite(z, acc[c][j] * a.scale);
+      for (int j = 0; j < 16; ++j) {
+        acc[c][j] = __fmul2_rn(acc[c][j], both(a.scale));
+        note_finite(z, acc[c][j].x);
+        note_finite(z, acc[c][j].y);
+      }
     if (z != 0.f) sm.not_finite = 1;
     // every thread has seen the last chunk, so every MMA that read the Q planes has completed
     mbar_arrive(&sm.bar[YB_EPI]);
@@ -1688,7 +1752,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
           *reinterpret_cast<float4*>(stage + row * kWidePitch + c * 64 + w * 32 + j) =
-              make_float4(acc[c][j] * a.scale, acc[c][j + 1] * a.scale, acc[c][j + 2] * a.scale, acc[c][j + 3] * a.scale);
+              make_float4(acc[c][j / 2].x, acc[c][j / 2].y, acc[c][j / 2 + 1].x, acc[c][j / 2 + 1].y);
     }
     mbar_arrive(&sm.bar[YB_EPI]);
     ok = mbar_wait(&sm.bar[YB_EPI], 1) && ok;
@@ -1793,7 +1857,8 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     kernel<<<launch_ctas(p.order), kThreads, smem, st>>>(mq, mk, mv, p);
     return BMA_OK;
   };
-  rc = dp == 64 ? launch(f32_fwd_kernel<64>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128>, sizeof(FwdSmem<128>));
+  if (a.key_bias || a.scale < 0.f) rc = dp == 64 ? launch(f32_fwd_kernel<64, true>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, true>, sizeof(FwdSmem<128>));
+  else rc = dp == 64 ? launch(f32_fwd_kernel<64, false>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, false>, sizeof(FwdSmem<128>));
   if (rc) return rc;
   count_launches(1);
   BMA_CUDA_TRY(cudaGetLastError());
@@ -1812,14 +1877,16 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
         (rc = plane_map(&mqh, w + pl.q, a.B, a.N, a.Hq, 128, BH)) || (rc = plane_map(&mkh, w + pl.k, a.B, a.L, a.Hkv, 128, BH)) ||
         (rc = plane_map(&mvh, w + pl.v, a.B, a.L, a.Hkv, 128, BH)) || (rc = plane_map(&mdoh, w + pl.d_o, a.B, a.N, a.Hq, 128, BH)))
       return rc;
-    BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dkdv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvWideSmem)));
-    BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dq_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqWideSmem)));
+    auto dkdv = a.key_bias ? f32_dkdv_wide_kernel<true> : f32_dkdv_wide_kernel<false>;
+    auto dq = a.key_bias ? f32_dq_wide_kernel<true> : f32_dq_wide_kernel<false>;
+    BMA_CUDA_TRY(cudaFuncSetAttribute(dkdv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvWideSmem)));
+    BMA_CUDA_TRY(cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqWideSmem)));
     F32WideParams wp{p, w + pl.v};
     wp.f.order = k_order(a, 128);
-    f32_dkdv_wide_kernel<<<launch_ctas(wp.f.order), kThreads, sizeof(DkdvWideSmem), st>>>(mk, mqh, mdoh, wp);
+    dkdv<<<launch_ctas(wp.f.order), kThreads, sizeof(DkdvWideSmem), st>>>(mk, mqh, mdoh, wp);
     wp.a_planes = w + pl.d_o;
     wp.f.order = q_order(a, 128);
-    f32_dq_wide_kernel<<<launch_ctas(wp.f.order), kThreads, sizeof(DqWideSmem), st>>>(mq, mkh, mvh, wp);
+    dq<<<launch_ctas(wp.f.order), kThreads, sizeof(DqWideSmem), st>>>(mq, mkh, mvh, wp);
     count_launches(2);
     BMA_CUDA_TRY(cudaGetLastError());
     return BMA_OK;
@@ -1829,12 +1896,14 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
       (rc = plane_map(&mqh, w + pl.q, a.B, a.N, a.Hq, 64, BH)) || (rc = plane_map(&mkh, w + pl.k, a.B, a.L, a.Hkv, 64, BH)) ||
       (rc = plane_map(&mvh, w + pl.v, a.B, a.L, a.Hkv, 64, BH)) || (rc = plane_map(&mdoh, w + pl.d_o, a.B, a.N, a.Hq, 64, BH)))
     return rc;
-  BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvSmem)));
-  BMA_CUDA_TRY(cudaFuncSetAttribute(f32_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqSmem)));
+  auto dkdv = a.key_bias ? f32_dkdv_kernel<true> : f32_dkdv_kernel<false>;
+  auto dq = a.key_bias ? f32_dq_kernel<true> : f32_dq_kernel<false>;
+  BMA_CUDA_TRY(cudaFuncSetAttribute(dkdv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvSmem)));
+  BMA_CUDA_TRY(cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqSmem)));
   p.order = k_order(a, 64);
-  f32_dkdv_kernel<<<launch_ctas(p.order), kThreads, sizeof(DkdvSmem), st>>>(mk, mv, mqh, mdoh, p);
+  dkdv<<<launch_ctas(p.order), kThreads, sizeof(DkdvSmem), st>>>(mk, mv, mqh, mdoh, p);
   p.order = q_order(a, 64);
-  f32_dq_kernel<<<launch_ctas(p.order), kThreads, sizeof(DqSmem), st>>>(mq, mkh, mvh, mdo, p);
+  dq<<<launch_ctas(p.order), kThreads, sizeof(DqSmem), st>>>(mq, mkh, mvh, mdo, p);
   count_launches(2);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
