@@ -35,6 +35,7 @@
 // consumed, the three planes of P or dS as A operands (per 16 keys: 8 columns hi, 8 mid, and 8 lo in the other half).
 // Every mbarrier wait is bounded; on a timeout the thread records an error code and unwinds.
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "ptx_sm100.cuh"
@@ -363,6 +364,72 @@ __device__ __forceinline__ void store_rows(const float* stage, int pitch, const 
   }
 }
 
+// Rows of a tile whose key list is shared out over the CTAs of a cluster: the weighted sum of their partials (two per CTA: [2][BM] rows
+// of DP + 4 floats at `stage`, maximum and sum at `ml`) relative to their common maximum.  Half a warp per row, eight warps, the rows
+// dealt out over the CTAs; a result that is not finite is noted in the first CTA.
+template <int DP>
+__device__ __noinline__ void sum_parts(const float* stage, const float* ml, int* not_finite, const F32Params& p, int parts, int part, int q0, int h, int b) {
+  const bma_attn_args& a = p.a;
+  const int lane = threadIdx.x & 31, c = lane & 15, warp = threadIdx.x >> 5, sources = 2 * parts;
+  constexpr int kPitch = DP + 4;
+  const bool vec = (reinterpret_cast<uintptr_t>(a.o.ptr) & 15) == 0 && ((a.o.stride_b | a.o.stride_l | a.o.stride_h) & 3) == 0 && (a.d & 3) == 0;
+  float z = 0.f;
+#pragma unroll 1
+  for (int i0 = warp * 2; i0 * parts < BM; i0 += 16) {
+    const int i = part + parts * (i0 + (lane >> 4)), q = q0 + i;
+    const bool valid = i < BM && q < a.N;
+    float m = -INFINITY, l = 0.f;
+    if (valid && c < sources) {
+      const uint32_t at = cluster_addr(ml + (c & 1) * 2 * BM + i, (uint32_t)(c >> 1));
+      m = cluster_ld(at);
+      l = cluster_ld(at + BM * (uint32_t)sizeof(float));
+    }
+    float mt = m;
+#pragma unroll
+    for (int off = 8; off; off >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, off));
+    const float f = ex2(m - (mt == -INFINITY ? 0.f : mt));
+    float lt = l * f;
+#pragma unroll
+    for (int off = 8; off; off >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, off);
+    float4 acc[DP / 64];
+#pragma unroll
+    for (int u = 0; u < DP / 64; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* mine = stage + (valid ? i : 0) * kPitch + c * 4;
+#pragma unroll 4
+    for (int src = 0; src < sources; ++src) {
+      const uint32_t at = cluster_addr(mine + (src & 1) * BM * kPitch, (uint32_t)(src >> 1));
+      const float w = __shfl_sync(0xffffffffu, f, src, 16);
+#pragma unroll
+      for (int u = 0; u < DP / 64; ++u) {
+        const float4 v = cluster_ld4(at + u * 256);
+        acc[u].x = fmaf(v.x, w, acc[u].x); acc[u].y = fmaf(v.y, w, acc[u].y); acc[u].z = fmaf(v.z, w, acc[u].z); acc[u].w = fmaf(v.w, w, acc[u].w);
+      }
+    }
+    if (!valid) continue;
+    if (c == 0 && a.lse) a.lse[((int64_t)b * a.Hq + h) * a.N + q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
+    const float inv = lt > 0.f ? 1.f / lt : 0.f;   // (0 for a NaN as well: then a sum below is not finite)
+#pragma unroll
+    for (int u = 0; u < DP / 64; ++u) {
+      float o4[4] = {acc[u].x * inv, acc[u].y * inv, acc[u].z * inv, acc[u].w * inv};
+      note_finite(z, (o4[0] + o4[1]) + (o4[2] + o4[3]));
+      const int col = u * 64 + c * 4;
+      const int64_t off = (int64_t)b * a.o.stride_b + (int64_t)q * a.o.stride_l + (int64_t)h * a.o.stride_h + col;
+      if (vec && col < a.d) {
+        if (a.o.dtype == BMA_DTYPE_F32) *reinterpret_cast<float4*>(static_cast<float*>(a.o.ptr) + off) = make_float4(o4[0], o4[1], o4[2], o4[3]);
+        else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.o.ptr) + off) = make_uint2(pack_bf16(o4[0], o4[1]), pack_bf16(o4[2], o4[3]));
+      } else if (!vec) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (col + e >= a.d) break;
+          if (a.o.dtype == BMA_DTYPE_F32) static_cast<float*>(a.o.ptr)[off + e] = o4[e];
+          else static_cast<__nv_bfloat16*>(a.o.ptr)[off + e] = __float2bfloat16_rn(o4[e]);
+        }
+      }
+    }
+  }
+  if (!(z == 0.f)) cluster_st(cluster_addr(not_finite, 0), 1);
+}
+
 // =================================================================================================================
 // Forward: one CTA per (128-query tile, query head, batch).  Each listed kv tile is cut into two halves of 64 keys;
 // warpgroup x (thread = query row) runs its own online softmax over the halves x of all tiles, so that the two
@@ -396,14 +463,14 @@ static_assert(fwd_smem<4>() <= sizeof(FwdSmem<64>) && fwd_smem<8>() <= sizeof(Fw
 template <int DP, bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ F32Params p) {
+               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ F32Params p, const int parts, const int first) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using Smem = FwdSmem<DP>;
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   constexpr int kBoxes = Smem::kBoxes, kStages = Smem::kStages;
   const bma_attn_args& a = p.a;
   int qi, h;
-  cta_of(p.order, qi, h);
+  cta_of(p.order, first + (int)blockIdx.x / parts, qi, h);
   qi = p.order.tiles - 1 - qi;
   const int b = h / a.Hq;
   h -= b * a.Hq;
@@ -430,12 +497,15 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     tmem_relinquish();
   }
   tc_fence_before();
-  const int T = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
+  const int listed = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
+  // this CTA's part of the list
+  const int part = (int)blockIdx.x % parts, t0 = listed * part / parts, T = listed * (part + 1) / parts - t0;
+  const uint16_t* entry = sm.list.entry + t0;
   // half tiles per warpgroup: the second half of the last tile may lie past the end of the keys
   const int T0 = T;
-  const int T1 = (T > 0 && (int)(sm.list.entry[T - 1] & 0x7fff) * 128 + BH >= a.L) ? T - 1 : T;
+  const int T1 = (T > 0 && (int)(entry[T - 1] & 0x7fff) * 128 + BH >= a.L) ? T - 1 : T;
 
   if (wg == 2) {
     setmaxnreg_dec_80();
@@ -449,7 +519,7 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           const int st = i % kStages;
           if (i >= kStages) ok = mbar_wait(&sm.bar[FB_K_FREE + st], (i / kStages - 1) & 1);
           if (!ok) break;
-          const int row = (int)(sm.list.entry[n] & 0x7fff) * 128 + x * BH;
+          const int row = (int)(entry[n] & 0x7fff) * 128 + x * BH;
           mbar_expect_tx(&sm.bar[FB_K_FULL + st], 3 * kBoxes * kHalfBox);
 #pragma unroll
           for (int box = 0; box < kBoxes; ++box)
@@ -475,7 +545,7 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           const int st = i % kStages;
           if (i >= kStages) ok = mbar_wait(&sm.bar[FB_V_FREE + st], (i / kStages - 1) & 1);
           if (!ok) break;
-          const int row = (int)(sm.list.entry[n] & 0x7fff) * 128 + x * BH;
+          const int row = (int)(entry[n] & 0x7fff) * 128 + x * BH;
           mbar_expect_tx(&sm.bar[FB_V_FULL + st], 3 * kBoxes * kHalfBox);
 #pragma unroll
           for (int pl = 0; pl < 3; ++pl)
@@ -530,7 +600,7 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int n = 0; n < Tx; ++n) {
-      const uint32_t e = sm.list.entry[n];
+      const uint32_t e = entry[n];
       const int k0 = (int)(e & 0x7fff) * 128 + x * BH;
       uint32_t bits[2] = {0xffffffffu, 0xffffffffu};
       if (e & 0x8000u) row_bits64(p.spec, b, h, q, k0, bits);
@@ -634,6 +704,12 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ++syncs;
     };
     rendezvous();
+    if (parts > 1) {   // both partial results as they are; the cluster adds them up below
+      float* stage = reinterpret_cast<float*>(sm.q) + (x * BM + row) * (DP + 4);
+#pragma unroll
+      for (int j = 0; j < DP; j += 4) *reinterpret_cast<float4*>(stage + j) = make_float4(o[j / 2].x, o[j / 2].y, o[j / 2 + 1].x, o[j / 2 + 1].y);
+      if (!ok) report_device_error(p.status, 630 + warp);
+    } else {
     const float mo = sm.ml[x ^ 1][0][row], lo = sm.ml[x ^ 1][1][row];
     const float mt = fmaxf(m, mo), ms = (mt == -INFINITY) ? 0.f : mt;
     const float fx = ex2(m - ms), fo = ex2(mo - ms);
@@ -661,10 +737,17 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     rendezvous();
     if (ok) store_rows<256>(reinterpret_cast<const float*>(sm.q), kPitch, a.o, b, q0, a.N, h, a.d, threadIdx.x);
     else report_device_error(p.status, 630 + warp);
+    }
   }
   tc_fence_before();
-  __syncthreads();
+  if (parts > 1) cluster_sync();
+  else __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if (parts > 1) {
+    if (warp < 8) sum_parts<DP>(reinterpret_cast<const float*>(sm.q), &sm.ml[0][0][0], &sm.not_finite, p, parts, part, q0, h, b);
+    cluster_sync();   // shared memory stays until the others have read it
+    if (part > 0) return;
+  }
   if (warp < 8 && sm.not_finite) redo_row<REDO_FWD, DP / 16>(reinterpret_cast<float*>(smem_raw), p, qi, h, b);
 }
 
@@ -722,7 +805,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
   DkdvSmem& sm = *reinterpret_cast<DkdvSmem*>(smem_raw);
   const bma_attn_args& a = p.a;
   int kj, hk;
-  cta_of(p.order, kj, hk);
+  cta_of(p.order, (int)blockIdx.x, kj, hk);
   const int b = hk / a.Hkv, G = a.Hq / a.Hkv;
   hk -= b * a.Hkv;
   const int k0 = kj * BM;
@@ -990,7 +1073,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   DqSmem& sm = *reinterpret_cast<DqSmem*>(smem_raw);
   const bma_attn_args& a = p.a;
   int qi, h;
-  cta_of(p.order, qi, h);
+  cta_of(p.order, (int)blockIdx.x, qi, h);
   qi = p.order.tiles - 1 - qi;
   const int b = h / a.Hq;
   h -= b * a.Hq;
@@ -1277,7 +1360,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   const F32Params& p = wp.f;
   const bma_attn_args& a = p.a;
   int kj, hk;
-  cta_of(p.order, kj, hk);
+  cta_of(p.order, (int)blockIdx.x, kj, hk);
   const int b = hk / a.Hkv, G = a.Hq / a.Hkv;
   hk -= b * a.Hkv;
   const int k0 = kj * BM;
@@ -1554,7 +1637,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const F32Params& p = wp.f;
   const bma_attn_args& a = p.a;
   int qi, h;
-  cta_of(p.order, qi, h);
+  cta_of(p.order, (int)blockIdx.x, qi, h);
   qi = p.order.tiles - 1 - qi;
   const int b = h / a.Hq;
   h -= b * a.Hq;
@@ -1832,6 +1915,98 @@ int make_params(F32Params& p, const bma_attn_args& a, const bma_mask_spec& spec,
   return BMA_OK;
 }
 
+cudaLaunchConfig_t f32_fwd_config(int tiles, int parts, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(tiles * parts));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  return cfg;
+}
+cudaLaunchAttribute row_cluster(int n) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = n; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  return attr;
+}
+// Clusters of `parts` CTAs of the forward kernel that the device runs at the same time.
+constexpr int kMaxParts = 8;
+int f32_fwd_clusters(int dp, int parts) {
+  if (parts == 1) return kSms;
+  static std::atomic<int> known[2][kMaxParts + 1];   // that, plus one
+  std::atomic<int>& k = known[dp == 128][parts];
+  int n = k.load(std::memory_order_relaxed);
+  if (!n) {
+    auto ask = [&](auto kernel, size_t smem) {
+      cudaLaunchConfig_t cfg = f32_fwd_config(kSms, parts, smem, nullptr);
+      cudaLaunchAttribute attr = row_cluster(parts);
+      cfg.attrs = &attr; cfg.numAttrs = 1;
+      int most = 0;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        most = 0;
+      }
+      return most;
+    };
+    n = 1 + (dp == 128 ? ask(f32_fwd_kernel<128, false>, sizeof(FwdSmem<128>)) : ask(f32_fwd_kernel<64, false>, sizeof(FwdSmem<64>)));
+    k.store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+
+// How many CTAs share a tile's key list: `parts` in one launch of all tiles, or, where every tile takes as long, 1 for whole waves of
+// tiles and `last_parts` for the `last` ones, in a launch of their own.  Launches of up to four waves leave SMs without work: too
+// few tiles, a last wave of a few, or a causal mask whose longest walk takes longer than the average SM's share.  The model counts key tiles:
+// a walk of w tiles takes w / parts + 3, the three for set-up, merge and the partials' way through shared memory (a CTA takes 8 - 14 us
+// besides its tiles of 3.1 us at 64 head columns, 4.8 at 128).  Calls: 1 x 1500 tokens, 16/4 heads of 128, no mask, 148 + 44 tiles in 3
+// parts 147 -> 116 us; causal 1 x 1000, 8 heads of 64 76 -> 44, 1 x 4096,
+// 4 heads of 128 169 -> 116 (of which about 30 and 15 are the lists' launch and the host path).
+struct FwdShare {
+  int parts, last, last_parts;
+};
+FwdShare f32_fwd_share(const bma_attn_args& a, const bma_mask_spec& spec, int dp, int NQ, int NKV) {
+  FwdShare best{1, 0, 1};
+  const int heads = a.B * a.Hq;
+  const int64_t tiles64 = (int64_t)NQ * heads;
+  if (tiles64 > 4 * kSms || NKV < 2) return best;
+  const int tiles = (int)tiles64;
+  const double o = 3.;
+  double longest = NKV, sum = (double)tiles * NKV;
+  const bool causal = (spec.flags & BMA_MASK_CAUSAL) != 0;
+  if (causal) {
+    longest = sum = 0.;
+    for (int qi = 0; qi < NQ; ++qi) {
+      const int64_t keys = std::min<int64_t>((int64_t)(qi + 1) * BM, a.N) + spec.q_offset - spec.k_offset;
+      const double w = (double)std::min<int64_t>(std::max<int64_t>((keys + BM - 1) / BM, 0), NKV);
+      longest = std::max(longest, w);
+      sum += w * heads;
+    }
+  }
+  if (spec.flags & BMA_MASK_BAND) {   // the walks of a band are about as long as it is wide
+    const double w = std::min(longest, ((double)spec.band_left + spec.band_right) / BM + 2.);
+    sum = std::min(sum, w * tiles);
+    longest = w;
+  }
+  auto even = [&](int count, int parts, int clusters) { return (double)ceil_div(count, clusters) * (longest / parts + o); };
+  double cost = 1e30;
+  for (int parts = 1; parts <= std::min(kMaxParts, NKV); ++parts) {
+    const int clusters = f32_fwd_clusters(dp, parts);
+    if (clusters < 1) continue;
+    const double c = causal ? std::max(longest / parts + o, (sum / parts + tiles * o) / clusters * 1.05) : even(tiles, parts, clusters);
+    if (c < 0.95 * cost) { cost = c; best = {parts, 0, 1}; }
+  }
+  const int last = tiles % kSms;
+  if (!causal && tiles > kSms && last > 0)
+    for (int parts = 2; parts <= std::min(kMaxParts, NKV); ++parts) {
+      const int clusters = f32_fwd_clusters(dp, parts);
+      if (clusters < last) continue;
+      const double c = even(tiles - last, 1, kSms) + even(last, parts, clusters);
+      if (c < 0.95 * cost) { cost = c; best = {1, last, parts}; }
+    }
+  return best;
+}
+
 }  // namespace
 
 size_t f32_workspace_bytes(const bma_attn_args& a, bool backward) {
@@ -1854,13 +2029,22 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   p.order = q_order(a, dp);
   auto launch = [&](auto kernel, size_t smem) -> int {
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<launch_ctas(p.order), kThreads, smem, st>>>(mq, mk, mv, p);
-    return BMA_OK;
+    const int items = (int)launch_ctas(p.order);
+    auto run = [&](int first, int count, int parts) -> int {
+      cudaLaunchConfig_t cfg = f32_fwd_config(count, parts, smem, st);
+      cudaLaunchAttribute attr = row_cluster(parts);
+      if (parts > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
+      BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p, parts, first));
+      count_launches(1);
+      return BMA_OK;
+    };
+    const FwdShare share = f32_fwd_share(a, spec, dp, lists.NQ, lists.NKV);
+    const int r = run(0, items - share.last, share.parts);
+    return r || !share.last ? r : run(items - share.last, share.last, share.last_parts);
   };
   if (a.key_bias || a.scale < 0.f) rc = dp == 64 ? launch(f32_fwd_kernel<64, true>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, true>, sizeof(FwdSmem<128>));
   else rc = dp == 64 ? launch(f32_fwd_kernel<64, false>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, false>, sizeof(FwdSmem<128>));
   if (rc) return rc;
-  count_launches(1);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
 }

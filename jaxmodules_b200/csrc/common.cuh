@@ -63,8 +63,8 @@ __device__ __forceinline__ void cta_of(bool by_rank, int& rank, int& head, int& 
 struct LaunchOrder {
   int tiles, heads, group;
 };
-__device__ __forceinline__ void cta_of(const LaunchOrder& o, int& rank, int& head) {
-  const int per = o.group * o.tiles, g = (int)blockIdx.x / per, r = (int)blockIdx.x - g * per;
+__device__ __forceinline__ void cta_of(const LaunchOrder& o, int index, int& rank, int& head) {
+  const int per = o.group * o.tiles, g = index / per, r = index - g * per;
   const int in_group = min(o.group, o.heads - g * o.group);   // (the last group may be smaller)
   rank = __shfl_sync(0xffffffffu, r / in_group, 0);           // (warp-uniform, which the compiler does not see through divisions)
   head = __shfl_sync(0xffffffffu, g * o.group + r % in_group, 0);

@@ -1,6 +1,6 @@
 """The order in which CTAs start (csrc/common.cuh, longest_first and LaunchOrder).  Every (tile, head, batch) has to be done exactly once
-in either order, and in groups of heads that do and do not divide them: a call over all heads equals, bit for bit, calls over one
-head at a time."""
+in either order, and in groups of heads that do and do not divide them: a call over all heads equals (bfloat16: bit for bit) calls over
+one head at a time."""
 import numpy as np
 import pytest
 import torch
@@ -51,7 +51,9 @@ def test_all_heads_equal_one_head_at_a_time(dtype, B, L, Hq, Hkv, d, recompute):
                 one = call(q[b:b + 1, :, s], k[b:b + 1, :, hk:hk + 1], v[b:b + 1, :, hk:hk + 1], do[b:b + 1, :, s], ids[b:b + 1])
                 for name, x, y in zip(("O", "dQ", "dK", "dV"), whole, one):
                     part = x[b:b + 1, :, s] if name in ("O", "dQ") else x[b:b + 1, :, hk:hk + 1]
-                    assert torch.equal(part, y), (name, b, hk)
+                    # (a float32 forward pass over few tiles shares their keys out over CTAs: each evaluation is within 2e-6 of the
+                    # exact result in the 2-norm, tests/test_gpu_f32.py)
+                    assert torch.equal(part, y) or (dtype == torch.float32 and (part.double() - y.double()).norm() <= 4e-6 * y.double().norm()), (name, b, hk)
     finally:
         A.set_backward_scratch_limit(limit)
     assert A.device_status() == 0
