@@ -96,6 +96,7 @@ struct BwdParams {
   int b0, hk0;      // first batch / kv head of this launch (the grid covers a range when the scratch is smaller
   int nhk;          // than the whole problem), and the number of kv heads in the range
   bool by_rank;     // order of the CTAs, see cta_of
+  int parts;        // CTAs of a cluster that share a kv tile's walk
 };
 
 // Rendezvous of the kConsumers (512) consumer threads on an mbarrier: arrive, then a bounded wait (a plain
@@ -109,18 +110,44 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 __device__ __forceinline__ void setmaxnreg_inc_consumers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 104;"); }
 __device__ __forceinline__ void setmaxnreg_dec_roles() { asm volatile("setmaxnreg.dec.sync.aligned.u32 64;"); }
 
+// dK and dV of a kv tile from the accumulators of a cluster's CTAs, each [128] rows of dK | dV in float32 at `stage`: the rows are dealt out
+// over the CTAs, four columns to a thread.
+template <int HD> constexpr int kStagePitch = 2 * HD + 4;
+template <int HD>
+__device__ __noinline__ void sum_parts(const float* stage, const BwdParams& p, int k0, int hk, int b) {
+  const bma_attn_args& a = p.a;
+  const int part = (int)__clusterRelativeBlockRank();
+  constexpr int kPer = 2 * HD / 4;   // groups of four columns of a row
+#pragma unroll 1
+  for (int i = threadIdx.x; i < (BT + p.parts - 1) / p.parts * kPer; i += kConsumers) {
+    const int row = part + p.parts * (i / kPer), c = (i % kPer) * 4;
+    if (row >= BT || k0 + row >= a.L) continue;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int src = 0; src < p.parts; ++src) {
+      const float4 v = cluster_ld4(cluster_addr(stage + row * kStagePitch<HD> + c, (uint32_t)src));
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    const bool is_k = c < HD;
+    const bma_tensor& t = is_k ? a.dk : a.dv;
+    const float f = is_k ? a.scale : 1.f;
+    const int64_t off = (int64_t)b * t.stride_b + (int64_t)(k0 + row) * t.stride_l + (int64_t)hk * t.stride_h + (is_k ? c : c - HD);
+    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(t.ptr) + off) = make_uint2(pack_bf16(s.x * f, s.y * f), pack_bf16(s.z * f, s.w * f));
+  }
+}
+
 template <int HD, bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
-                const __grid_constant__ CUtensorMap map_dk, const __grid_constant__ CUtensorMap map_dv, const BwdParams p) {
+                const __grid_constant__ CUtensorMap map_dk, const __grid_constant__ CUtensorMap map_dv, const __grid_constant__ BwdParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr uint32_t kTileBytes = kTileBytesOf<HD>;
   BwdSmem<HD>& sm = *reinterpret_cast<BwdSmem<HD>*>(smem_raw);
 
   const bma_attn_args& a = p.a;
   int kj, hk, b;   // (under a causal mask kv tile 0 sees the most q tiles)
-  cta_of(p.by_rank, kj, hk, b);
+  cta_of_cluster(p.by_rank, kj, hk, b);
   hk += p.hk0;
   b += p.b0;
   const int G = a.Hq / a.Hkv;
@@ -159,6 +186,12 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int64_t row = ((int64_t)lb * p.l.H + lh) * p.l.NKV + kj;
     total += p.l.full_q_num[row] + p.l.q_num[row];
   }
+  int skip = 0;
+  if (p.parts > 1) {   // this CTA's share of the walk
+    const int part = (int)__clusterRelativeBlockRank(), all = total;
+    skip = all * part / p.parts;
+    total = all * (part + 1) / p.parts - skip;
+  }
   if (warp == kWarpTma) {
     tmem_alloc(&sm.tmem_base, kTmemCols);
     tmem_relinquish();
@@ -178,7 +211,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
         for (int box = 0; box < HD / 64; ++box) tma_load_4d(dst + box * kHalfTile, m, bar, box * 64, head, row0, b);
       };
-      QTileIter loader(p.l, b, hk, G, kj);
+      QTileIter loader(p.l, b, hk, G, kj, skip);
       bool ok = true;
       for (int n = 0; n < total && ok; ++n) {
         int h, qi; bool partial;
@@ -271,7 +304,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (!ok && leader) report_device_error(p.status, 310);
     } else if (warp == kWarpStat && total > 0) {
       // ---------------------------------------------------------------- row statistics of the coming q tiles
-      QTileIter loader(p.l, b, hk, G, kj);
+      QTileIter loader(p.l, b, hk, G, kj, skip);
       bool ok = true;
       for (int n = 0; n < total && ok; ++n) {
         int h, qi; bool partial;
@@ -297,7 +330,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       // ---------------------------------------------------------------- dSt hand-over to the dQ replay kernel
       // BAR_STG says that all consumers have staged (and fenced) the dSt image of tile n in shared memory; one
       // bulk store moves it to its slot, and BAR_DSR tells the consumers that the buffer has been read.
-      QTileIter loader(p.l, b, hk, G, kj);
+      QTileIter loader(p.l, b, hk, G, kj, skip);
       const uint64_t policy = l2_evict_first();
       const int64_t first_head_base = __ldg(p.head_base + (int64_t)p.b0 * a.Hq + (int64_t)p.hk0 * G);
       bool ok = true;
@@ -332,7 +365,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const uint32_t cols = lane_base + part * kCols;   // this thread's query columns of St and dPt
     const int k = k0 + row;
     bool ok = true;
-    QTileIter walker(p.l, b, hk, G, kj);
+    QTileIter walker(p.l, b, hk, G, kj, skip);
     int h = 0, qi = 0;
     bool partial = false;
     float pr[kCols];  // Pt of the current tile (this thread's key row, its query columns)
@@ -446,6 +479,30 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (ok && total == 0) ok = mbar_wait(&sm.bar[BAR_KV], 0);  // the K/V loads must land before their buffers are reused below
     if (!ok) {
       report_device_error(p.status, 320 + warp);
+    } else if (p.parts > 1) {
+      // the accumulators as they are, [128] rows of dK | dV in float32 over all of the tiles; the cluster adds them up below
+      if (p.ds_out != nullptr && total > 0) ok = mbar_wait(&sm.bar[BAR_DSR], (total - 1) & 1);   // the last dSt image has been read
+      if (!ok) report_device_error(p.status, 340 + warp);
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; ok && c < HD / kParts / 16; ++c) {
+        const int col = part * (HD / kParts) + c * 16;
+        uint32_t rk[16], rv[16];
+        if (total > 0) {
+          tmem_ld16(tmem + COL_DK + lane_base + col, rk);
+          tmem_ld16(tmem + COL_DV + lane_base + col, rv);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) { rk[j] = 0u; rv[j] = 0u; }
+        }
+        uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<float*>(smem_raw) + row * kStagePitch<HD> + col);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          dst[u] = make_uint4(rk[u * 4], rk[u * 4 + 1], rk[u * 4 + 2], rk[u * 4 + 3]);
+          dst[HD / 4 + u] = make_uint4(rv[u * 4], rv[u * 4 + 1], rv[u * 4 + 2], rv[u * 4 + 3]);
+        }
+      }
     } else {
       tc_fence_after();
       // dK (scaled) and dV go through shared memory -- the K and V tiles are dead now -- in the 128-byte-swizzled
@@ -499,8 +556,13 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   }
 
   tc_fence_before();
-  __syncthreads();
+  if (p.parts > 1) cluster_sync();
+  else __syncthreads();
   if (warp == kWarpTma) tmem_dealloc(tmem, kTmemCols);
+  if (p.parts > 1) {
+    if (threadIdx.x < kConsumers) sum_parts<HD>(reinterpret_cast<const float*>(smem_raw), p, k0, hk, b);
+    cluster_sync();   // shared memory stays until the others have read it
+  }
 }
 
 bool aligned16(const bma_tensor& t) {
@@ -519,14 +581,22 @@ size_t sm100_bwd_scratch_min_bytes(const bma_attn_args& a, const bma_block_lists
 
 template <typename P>
 static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                       const CUtensorMap& mdk, const CUtensorMap& mdv, P& p, int b0, int nb, int hk0, int nhk, cudaStream_t st) {
+                       const CUtensorMap& mdk, const CUtensorMap& mdv, P& p, const Walks& walks, int b0, int nb, int hk0, int nhk, cudaStream_t st) {
   p.b0 = b0; p.hk0 = hk0; p.nhk = nhk;
   p.by_rank = longest_first(ceil_div(a.L, BT), nhk, nb, (int64_t)4 * a.N * a.d * (a.Hq / a.Hkv));
-  const dim3 grid = cta_grid(p.by_rank, ceil_div(a.L, BT), nhk, nb);
   int rc;
   auto launch = [&](auto kernel, size_t smem) -> int {
+    static ClusterCounts known[2];
+    p.parts = share_walks(walks, 6.0, kMaxParts, [&](int parts) { return clusters_at_once(known[a.d == 128], kernel, kThreads, smem, parts); });
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, kThreads, smem, st>>>(mq, mk, mv, mdo, mdk, mdv, p);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = cta_grid(p.by_rank, ceil_div(a.L, BT), nhk, nb, p.parts);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = cluster_attribute(p.parts);
+    if (p.parts > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
+    BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, mdo, mdk, mdv, static_cast<const BwdParams&>(p)));
     return BMA_OK;
   };
   if (a.d == 128) rc = a.key_bias ? launch(bwd_dkdv_kernel<128, true>, sizeof(BwdSmem<128>)) : launch(bwd_dkdv_kernel<128, false>, sizeof(BwdSmem<128>));
@@ -548,6 +618,29 @@ static int64_t unit_blocks(const bma_attn_args& a, const bma_block_lists& l, con
   for (int g = 0; g < G; ++g) n += head_blocks(a, l, visited, b, hk * G + g);
   return n;
 }
+// The walks of nb x nhk heads' kv tiles, which take 1.7 us a tile; a CTA takes about six tiles more for set-up, drain and the sum over a
+// cluster.  The number of tiles is the caller's count of visited blocks, where there is one; the longest walk of a causal mask is that of
+// the first kv tile, other masks are taken as even.  (G = 8 query heads of 64 on one kv head, 3 x 1920 tokens, causal: 45 CTAs in
+// 3 parts, the call 288 -> 180 us; 1 x 4096, 8/1 heads of 128 562 -> 214; 2 x 4096, 16/4 heads 665 -> 548; host path and launch order included.)
+static Walks dkdv_walks(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& l, const int64_t* visited, int nb, int nhk) {
+  const int64_t ctas = (int64_t)ceil_div(a.L, BT) * nhk * nb;
+  if (ctas > 4 * kSms) return {4 * kSms, 1., 1., true};   // many waves: nothing is shared
+  const int G = a.Hq / a.Hkv, NQ = ceil_div(a.N, BT);
+  const bool causal = (spec.flags & BMA_MASK_CAUSAL) != 0;
+  Walks w{(int)ctas, (double)G * NQ, (double)ctas * G * NQ * (causal ? 0.5 : 1.), !causal};
+  if (visited) {
+    int64_t all = 0;
+    for (int64_t i = 0; i < (int64_t)l.B * l.H; ++i) all += visited[i];
+    w.sum = std::min((double)all / ((double)l.B * l.H) * nb * nhk * G, w.sum);   // (per list head, on average)
+  }
+  const double mean = w.sum / ctas;
+  if (spec.flags & BMA_MASK_BAND) w.longest = std::min(w.longest, G * (((double)spec.band_left + spec.band_right) / BT + 2.));
+  if (spec.flags & kTableTerms) w.longest = std::min(w.longest, 2. * mean + G);
+  if (!causal) w.longest = std::min(w.longest, std::max(mean, 1.));
+  w.longest = std::max(w.longest, 1.);
+  return w;
+}
+
 // tables + one dSt image (32 KB) per visited block of the whole problem
 size_t sm100_bwd_scratch_bytes(const bma_attn_args& a, const bma_block_lists& lists, const int64_t* visited_host) {
   if (lists.NKV > 1024 || lists.NQ <= 0 || lists.B <= 0 || lists.H <= 0) return 0;
@@ -602,7 +695,7 @@ int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
     for (int hk = 0; hk < a.Hkv; ++hk) largest = std::max(largest, unit_blocks(a, lists, visited_host, b, hk));
   const bool hand_over = capacity >= 1 && largest <= capacity;
   if (!hand_over) {
-    rc = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, 0, a.B, 0, a.Hkv, st);
+    rc = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, dkdv_walks(a, spec, lists, visited_host, a.B, a.Hkv), 0, a.B, 0, a.Hkv, st);
     if (rc) return rc;
     if (mark) BMA_CUDA_TRY(cudaEventRecord(mark, st));
     return sm100_bwd_dq(a, spec, lists, st);
@@ -613,7 +706,7 @@ int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   p.capacity = capacity;
   bool first = true;
   auto run_range = [&](int b0, int nb, int hk0, int nhk, bool whole) -> int {
-    int r = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, b0, nb, hk0, nhk, st);
+    int r = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, dkdv_walks(a, spec, lists, visited_host, nb, nhk), b0, nb, hk0, nhk, st);
     if (r) return r;
     if (mark && first && whole) BMA_CUDA_TRY(cudaEventRecord(mark, st));   // one boundary only when one range covers everything
     first = false;

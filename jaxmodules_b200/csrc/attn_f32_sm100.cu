@@ -34,8 +34,6 @@
 // Tensor memory columns hold the accumulators of a tile and then, over the columns that the reading thread has just
 // consumed, the three planes of P or dS as A operands (per 16 keys: 8 columns hi, 8 mid, and 8 lo in the other half).
 // Every mbarrier wait is bounded; on a timeout the thread records an error code and unwinds.
-#include <algorithm>
-#include <atomic>
 
 #include "common.cuh"
 #include "ptx_sm100.cuh"
@@ -1923,36 +1921,11 @@ cudaLaunchConfig_t f32_fwd_config(int tiles, int parts, size_t smem, cudaStream_
   cfg.stream = st;
   return cfg;
 }
-cudaLaunchAttribute row_cluster(int n) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = n; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  return attr;
-}
 // Clusters of `parts` CTAs of the forward kernel that the device runs at the same time.
-constexpr int kMaxParts = 8;
 int f32_fwd_clusters(int dp, int parts) {
-  if (parts == 1) return kSms;
-  static std::atomic<int> known[2][kMaxParts + 1];   // that, plus one
-  std::atomic<int>& k = known[dp == 128][parts];
-  int n = k.load(std::memory_order_relaxed);
-  if (!n) {
-    auto ask = [&](auto kernel, size_t smem) {
-      cudaLaunchConfig_t cfg = f32_fwd_config(kSms, parts, smem, nullptr);
-      cudaLaunchAttribute attr = row_cluster(parts);
-      cfg.attrs = &attr; cfg.numAttrs = 1;
-      int most = 0;
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-          cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();
-        most = 0;
-      }
-      return most;
-    };
-    n = 1 + (dp == 128 ? ask(f32_fwd_kernel<128, false>, sizeof(FwdSmem<128>)) : ask(f32_fwd_kernel<64, false>, sizeof(FwdSmem<64>)));
-    k.store(n, std::memory_order_relaxed);
-  }
-  return n - 1;
+  static ClusterCounts narrow, wide;
+  return dp == 128 ? clusters_at_once(wide, f32_fwd_kernel<128, false>, kThreads, sizeof(FwdSmem<128>), parts)
+                   : clusters_at_once(narrow, f32_fwd_kernel<64, false>, kThreads, sizeof(FwdSmem<64>), parts);
 }
 
 // How many CTAs share a tile's key list: `parts` in one launch of all tiles, or, where every tile takes as long, 1 for whole waves of
@@ -1989,13 +1962,8 @@ FwdShare f32_fwd_share(const bma_attn_args& a, const bma_mask_spec& spec, int dp
     longest = w;
   }
   auto even = [&](int count, int parts, int clusters) { return (double)ceil_div(count, clusters) * (longest / parts + o); };
-  double cost = 1e30;
-  for (int parts = 1; parts <= std::min(kMaxParts, NKV); ++parts) {
-    const int clusters = f32_fwd_clusters(dp, parts);
-    if (clusters < 1) continue;
-    const double c = causal ? std::max(longest / parts + o, (sum / parts + tiles * o) / clusters * 1.05) : even(tiles, parts, clusters);
-    if (c < 0.95 * cost) { cost = c; best = {parts, 0, 1}; }
-  }
+  best.parts = share_walks({tiles, longest, sum, !causal}, o, NKV, [&](int parts) { return f32_fwd_clusters(dp, parts); });
+  double cost = even(tiles, best.parts, f32_fwd_clusters(dp, best.parts));
   const int last = tiles % kSms;
   if (!causal && tiles > kSms && last > 0)
     for (int parts = 2; parts <= std::min(kMaxParts, NKV); ++parts) {
@@ -2032,7 +2000,7 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     const int items = (int)launch_ctas(p.order);
     auto run = [&](int first, int count, int parts) -> int {
       cudaLaunchConfig_t cfg = f32_fwd_config(count, parts, smem, st);
-      cudaLaunchAttribute attr = row_cluster(parts);
+      cudaLaunchAttribute attr = cluster_attribute(parts);
       if (parts > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
       BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p, parts, first));
       count_launches(1);

@@ -6,6 +6,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "../../include/bma.h"
 
 namespace bma {
@@ -51,12 +54,77 @@ constexpr int64_t kStreamInL2 = 64 << 20;   // of 126 MB, of which a line may ta
 inline bool longest_first(int64_t tiles, int64_t heads, int64_t batches, int64_t stream_bytes_per_head) {
   return tiles * heads * batches <= 4 * kSms && heads <= 65535 && heads * batches * stream_bytes_per_head <= kStreamInL2;
 }
-inline dim3 cta_grid(bool by_rank, int tiles, int heads, int batches) { return by_rank ? dim3(heads, batches, tiles) : dim3(tiles, heads, batches); }
+// With `parts` CTAs to a (tile, head, batch), which are a cluster.
+inline dim3 cta_grid(bool by_rank, int tiles, int heads, int batches, int parts = 1) {
+  return by_rank ? dim3(heads * parts, batches, tiles) : dim3(tiles * parts, heads, batches);
+}
+inline cudaLaunchAttribute cluster_attribute(int parts) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  return attr;
+}
+constexpr int kMaxParts = 8;
+// How many clusters of `parts` CTAs of a kernel the device runs at the same time (0 where it runs none); `known` keeps the answers of a
+// kernel.
+struct ClusterCounts {
+  std::atomic<int> plus_one[kMaxParts + 1];
+};
+template <typename K>
+int clusters_at_once(ClusterCounts& known, K kernel, int threads, size_t smem, int parts) {
+  if (parts == 1) return kSms;
+  std::atomic<int>& k = known.plus_one[parts];
+  int n = k.load(std::memory_order_relaxed);
+  if (!n) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kSms * parts);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr = cluster_attribute(parts);
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int most = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      most = 0;
+    }
+    n = 1 + most;
+    k.store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+// Walks of a launch: its CTAs, the longest and all of them together, in tiles.
+struct Walks {
+  int ctas;
+  double longest, sum;
+  bool even;      // all about as long as the longest
+};
+// The number of CTAs that share a walk, for the shortest time of the launch.  With n clusters at once a launch takes the longest of: waves of
+// walks of one length, or else the longest walk, or the even share of all; each CTA `extra` tiles besides its own.
+template <typename N>
+int share_walks(const Walks& w, double extra, int most_parts, N clusters) {
+  int best = 1;
+  double cost = 1e30;
+  for (int parts = 1; parts <= most_parts && parts <= kMaxParts; ++parts) {
+    const int n = clusters(parts);
+    if (n < 1) continue;
+    const double c = w.even ? (double)((w.ctas + n - 1) / n) * (w.longest / parts + extra)
+                            : std::max(w.longest / parts + extra, (w.sum / parts + w.ctas * extra) / n * 1.05);
+    if (c < 0.95 * cost) { cost = c; best = parts; }
+  }
+  return best;
+}
 // rank: 0 for the first tile to start of its head
 __device__ __forceinline__ void cta_of(bool by_rank, int& rank, int& head, int& batch) {
   rank = by_rank ? blockIdx.z : blockIdx.x;
   head = by_rank ? blockIdx.x : blockIdx.y;
   batch = by_rank ? blockIdx.y : blockIdx.z;
+}
+__device__ __forceinline__ void cta_of_cluster(bool by_rank, int& rank, int& head, int& batch) {   // the same for a launch in clusters (or not)
+  const dim3 id = __clusterIdx();
+  rank = by_rank ? id.z : id.x;
+  head = by_rank ? id.x : id.y;
+  batch = by_rank ? id.y : id.z;
 }
 // The same in groups, for the float32 kernels, which run 6 - 12 times as long on a byte, so that no launch is too long for it:
 // one-dimensional grid, rank 0 of every head of a group, then rank 1, and so on; `head` counts the (batch, head) pairs.
@@ -337,14 +405,21 @@ __device__ __forceinline__ int interval_class(const bma_mask_spec& s, int qi, in
   return all ? 2 : any ? 1 : 0;
 }
 
-struct QTileIter {  // flattened walk over (group head, listed q tile)
+struct QTileIter {  // flattened walk over (group head, listed q tile), from its entry `skip` on
   const bma_block_lists& l;
   int b, hk, G, kj;
   int g, it, nfull, npart;
   const int32_t* full_idx;
   const int32_t* part_idx;
-  __device__ QTileIter(const bma_block_lists& l_, int b_, int hk_, int G_, int kj_)
-      : l(l_), b(b_), hk(hk_), G(G_), kj(kj_), g(-1), it(0), nfull(0), npart(0), full_idx(nullptr), part_idx(nullptr) {}
+  __device__ QTileIter(const bma_block_lists& l_, int b_, int hk_, int G_, int kj_, int skip = 0)
+      : l(l_), b(b_), hk(hk_), G(G_), kj(kj_), g(-1), it(0), nfull(0), npart(0), full_idx(nullptr), part_idx(nullptr) {
+    while (skip > 0) {   // (fewer entries than that is a caller's error: the walk then ends at once)
+      if (++g >= G) { it = nfull + npart; return; }
+      load_head();
+      it = min(skip, nfull + npart);
+      skip -= it;
+    }
+  }
   __device__ void load_head() {
     const int h = hk * G + g;
     const int lb = l.B == 1 ? 0 : b, lh = l.H == 1 ? 0 : h;
@@ -357,6 +432,7 @@ struct QTileIter {  // flattened walk over (group head, listed q tile)
   }
   __device__ bool next(int& h, int& qi, bool& partial) {
     if (g < 0) { g = 0; load_head(); }
+    if (g >= G) return false;
     while (it >= nfull + npart) {
       if (++g >= G) return false;
       load_head();

@@ -1,6 +1,6 @@
 """The order in which CTAs start (csrc/common.cuh, longest_first and LaunchOrder).  Every (tile, head, batch) has to be done exactly once
-in either order, and in groups of heads that do and do not divide them: a call over all heads equals (bfloat16: bit for bit) calls over
-one head at a time."""
+in either order, and in groups of heads that do and do not divide them: a call over all heads equals calls over one head at a
+time (O and dQ in bfloat16 bit for bit)."""
 import numpy as np
 import pytest
 import torch
@@ -51,9 +51,10 @@ def test_all_heads_equal_one_head_at_a_time(dtype, B, L, Hq, Hkv, d, recompute):
                 one = call(q[b:b + 1, :, s], k[b:b + 1, :, hk:hk + 1], v[b:b + 1, :, hk:hk + 1], do[b:b + 1, :, s], ids[b:b + 1])
                 for name, x, y in zip(("O", "dQ", "dK", "dV"), whole, one):
                     part = x[b:b + 1, :, s] if name in ("O", "dQ") else x[b:b + 1, :, hk:hk + 1]
-                    # (a float32 forward pass over few tiles shares their keys out over CTAs: each evaluation is within 2e-6 of the
-                    # exact result in the 2-norm, tests/test_gpu_f32.py)
-                    assert torch.equal(part, y) or (dtype == torch.float32 and (part.double() - y.double()).norm() <= 4e-6 * y.double().norm()), (name, b, hk)
+                    # (launches of few CTAs share walks out over clusters: float32 evaluations are within 2e-6 each of the exact result
+                    # in the 2-norm, tests/test_gpu_f32.py; dK and dV in bfloat16 are rounded from sums of another order, which moves few values by a unit)
+                    tol = 4e-6 if dtype == torch.float32 else 1e-3 if name in ("dK", "dV") else 0.0
+                    assert (part.double() - y.double()).norm() <= tol * y.double().norm(), (name, b, hk)
     finally:
         A.set_backward_scratch_limit(limit)
     assert A.device_status() == 0
