@@ -136,7 +136,8 @@ __device__ __noinline__ void sum_parts(const float* stage, const BwdParams& p, i
   }
 }
 
-template <int HD, bool KB>
+// SHARED: the CTAs of a cluster share a kv tile's walk.
+template <int HD, bool KB, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -147,7 +148,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   const bma_attn_args& a = p.a;
   int kj, hk, b;   // (under a causal mask kv tile 0 sees the most q tiles)
-  cta_of_cluster(p.by_rank, kj, hk, b);
+  if constexpr (SHARED) cta_of_cluster(p.by_rank, kj, hk, b);
+  else cta_of(p.by_rank, kj, hk, b);
   hk += p.hk0;
   b += p.b0;
   const int G = a.Hq / a.Hkv;
@@ -187,7 +189,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     total += p.l.full_q_num[row] + p.l.q_num[row];
   }
   int skip = 0;
-  if (p.parts > 1) {   // this CTA's share of the walk
+  if constexpr (SHARED) {   // this CTA's share of the walk
     const int part = (int)__clusterRelativeBlockRank(), all = total;
     skip = all * part / p.parts;
     total = all * (part + 1) / p.parts - skip;
@@ -479,7 +481,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (ok && total == 0) ok = mbar_wait(&sm.bar[BAR_KV], 0);  // the K/V loads must land before their buffers are reused below
     if (!ok) {
       report_device_error(p.status, 320 + warp);
-    } else if (p.parts > 1) {
+    } else if constexpr (SHARED) {
       // the accumulators as they are, [128] rows of dK | dV in float32 over all of the tiles; the cluster adds them up below
       if (p.ds_out != nullptr && total > 0) ok = mbar_wait(&sm.bar[BAR_DSR], (total - 1) & 1);   // the last dSt image has been read
       if (!ok) report_device_error(p.status, 340 + warp);
@@ -556,10 +558,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   }
 
   tc_fence_before();
-  if (p.parts > 1) cluster_sync();
+  if constexpr (SHARED) cluster_sync();
   else __syncthreads();
   if (warp == kWarpTma) tmem_dealloc(tmem, kTmemCols);
-  if (p.parts > 1) {
+  if constexpr (SHARED) {
     if (threadIdx.x < kConsumers) sum_parts<HD>(reinterpret_cast<const float*>(smem_raw), p, k0, hk, b);
     cluster_sync();   // shared memory stays until the others have read it
   }
@@ -585,9 +587,10 @@ static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUte
   p.b0 = b0; p.hk0 = hk0; p.nhk = nhk;
   p.by_rank = longest_first(ceil_div(a.L, BT), nhk, nb, (int64_t)4 * a.N * a.d * (a.Hq / a.Hkv));
   int rc;
-  auto launch = [&](auto kernel, size_t smem) -> int {
+  auto launch = [&](auto kernel, auto shared, size_t smem) -> int {
     static ClusterCounts known[2];
-    p.parts = share_walks(walks, 6.0, kMaxParts, [&](int parts) { return clusters_at_once(known[a.d == 128], kernel, kThreads, smem, parts); });
+    p.parts = share_walks(walks, 6.0, kMaxParts, [&](int parts) { return clusters_at_once(known[a.d == 128], shared, kThreads, smem, parts); });
+    if (p.parts > 1) kernel = shared;
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = cta_grid(p.by_rank, ceil_div(a.L, BT), nhk, nb, p.parts);
@@ -599,8 +602,10 @@ static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUte
     BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, mdo, mdk, mdv, static_cast<const BwdParams&>(p)));
     return BMA_OK;
   };
-  if (a.d == 128) rc = a.key_bias ? launch(bwd_dkdv_kernel<128, true>, sizeof(BwdSmem<128>)) : launch(bwd_dkdv_kernel<128, false>, sizeof(BwdSmem<128>));
-  else rc = a.key_bias ? launch(bwd_dkdv_kernel<64, true>, sizeof(BwdSmem<64>)) : launch(bwd_dkdv_kernel<64, false>, sizeof(BwdSmem<64>));
+  if (a.d == 128) rc = a.key_bias ? launch(bwd_dkdv_kernel<128, true, false>, bwd_dkdv_kernel<128, true, true>, sizeof(BwdSmem<128>))
+                                  : launch(bwd_dkdv_kernel<128, false, false>, bwd_dkdv_kernel<128, false, true>, sizeof(BwdSmem<128>));
+  else rc = a.key_bias ? launch(bwd_dkdv_kernel<64, true, false>, bwd_dkdv_kernel<64, true, true>, sizeof(BwdSmem<64>))
+                       : launch(bwd_dkdv_kernel<64, false, false>, bwd_dkdv_kernel<64, false, true>, sizeof(BwdSmem<64>));
   if (rc) return rc;
   count_launches(1);
   BMA_CUDA_TRY(cudaGetLastError());

@@ -239,6 +239,7 @@ struct F32Params {
   float scale_log2;
   int* status;
   LaunchOrder order;
+  int parts;       // CTAs of a cluster that share a walk (dK / dV and dQ)
 };
 
 // ---- results that are not finite ----------------------------------------------------------------------------------
@@ -360,6 +361,36 @@ __device__ __forceinline__ void store_rows(const float* stage, int pitch, const 
       else static_cast<__nv_bfloat16*>(t.ptr)[off] = __float2bfloat16_rn(stage[r * pitch + c]);
     }
   }
+}
+
+// Rows of a gradient whose tile's walk is shared out over the CTAs of a cluster: the sum of the partials that each has staged at `stage`, the rows
+// dealt out over the CTAs, four columns to one of the 256 row threads; a result that is not finite is noted in the first CTA.
+template <int COLS>
+__device__ __noinline__ void sum_rows(const float* stage, int pitch, const bma_tensor& t, int b, int l0, int lmax, int h, int d, int parts, int part, int* not_finite) {
+  const bool vec = (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && ((t.stride_b | t.stride_l | t.stride_h) & 3) == 0 && (d & 3) == 0;
+  float z = 0.f;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < (BM + parts - 1) / parts * (COLS / 4); i += 256) {
+    const int row = part + parts * (i / (COLS / 4)), c = (i % (COLS / 4)) * 4;
+    if (row >= BM || l0 + row >= lmax || c >= d) continue;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int src = 0; src < parts; ++src) {
+      const float4 v = cluster_ld4(cluster_addr(stage + row * pitch + c, (uint32_t)src));
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    note_finite(z, (s.x + s.y) + (s.z + s.w));
+    float* dst = static_cast<float*>(t.ptr) + (int64_t)b * t.stride_b + (int64_t)(l0 + row) * t.stride_l + (int64_t)h * t.stride_h + c;
+    if (vec) {
+      *reinterpret_cast<float4*>(dst) = s;
+    } else {
+      const float e4[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (c + e < d) dst[e] = e4[e];
+    }
+  }
+  if (!(z == 0.f)) cluster_st(cluster_addr(not_finite, 0), 1);
 }
 
 // Rows of a tile whose key list is shared out over the CTAs of a cluster: the weighted sum of their partials (two per CTA: [2][BM] rows
@@ -761,31 +792,37 @@ enum {
   KB_Q_FULL, KB_Q_FREE = KB_Q_FULL + 2, KB_DO_FULL = KB_Q_FREE + 2, KB_DO_FREE = KB_DO_FULL + 2, KB_STAT = KB_DO_FREE + 2,
   KB_NUM = KB_STAT + 2
 };
+struct WalkShare { int g, it, tiles; };   // the part of a walk that a CTA of a cluster takes: its first head and entry, its number of tiles
 struct __align__(1024) DkdvSmem {
   uint8_t k[3][kRowBox];
   uint8_t v[3][kRowBox];
   uint8_t q[2][3][kHalfBox];
   uint8_t d_o[2][3][kHalfBox];
-  float nlse2[2][BH], ndelta[2][BH];   // minus the log-sum-exp (log2 units) and delta
+  alignas(16) float nlse2[2][BH], ndelta[2][BH];   // minus the log-sum-exp (log2 units) and delta
   uint64_t bar[KB_NUM];
   uint32_t tmem_base;
+  WalkShare share;
   int not_finite;
 };
 static_assert(dkdv_smem<4>() <= sizeof(DkdvSmem), "a tile is done again in the same shared memory");
 constexpr uint32_t COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
 
 // flattened walk over (group head, listed q tile, half tile); a half tile past the end of the queries is left out
+template <bool SHARED>   // a part of the walk
 struct HalfIter {
   QTileIter it;
-  int N, h, qi;
+  int N, h, qi, left;
   bool partial, second;
-  __device__ HalfIter(const bma_block_lists& l, int b, int hk, int G, int kj, int N_) : it(l, b, hk, G, kj), N(N_), h(0), qi(0), partial(false), second(false) {}
+  __device__ HalfIter(const bma_block_lists& l, int b, int hk, int G, int kj, int N_, const WalkShare& w)
+      : it(l, b, hk, G, kj), N(N_), h(0), qi(0), left(SHARED ? w.tiles : 0), partial(false), second(false) {
+    if (SHARED && left > 0) it.start(w.g, w.it);
+  }
   __device__ bool next(int& h_, int& q0_, bool& partial_) {
     if (second) {
       second = false;
       q0_ = qi * 128 + BH;
     } else {
-      if (!it.next(h, qi, partial)) return false;
+      if ((SHARED && --left < 0) || !it.next(h, qi, partial)) return false;
       q0_ = qi * 128;
       second = q0_ + BH < N;
     }
@@ -795,15 +832,35 @@ struct HalfIter {
   }
 };
 
-template <bool KB>
+// (one thread)
+__device__ __noinline__ WalkShare walk_share(const F32Params& p, int b, int hk, int G, int kj) {
+  WalkShare w{0, 0, 0};
+  auto entries = [&](int g) {
+    const int64_t row = ((int64_t)(p.l.B == 1 ? 0 : b) * p.l.H + (p.l.H == 1 ? 0 : hk * G + g)) * p.l.NKV + kj;
+    return p.l.full_q_num[row] + p.l.q_num[row];
+  };
+  int all = 0;
+  for (int g = 0; g < G; ++g) all += entries(g);
+  const int part = (int)blockIdx.x % p.parts, skip = all * part / p.parts;
+  w.tiles = all * (part + 1) / p.parts - skip;
+  for (w.it = skip; w.g < G - 1; ++w.g) {
+    const int n = entries(w.g);
+    if (w.it < n) break;
+    w.it -= n;
+  }
+  return w;
+}
+
+template <bool KB, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                 const __grid_constant__ CUtensorMap map_qh, const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DkdvSmem& sm = *reinterpret_cast<DkdvSmem*>(smem_raw);
   const bma_attn_args& a = p.a;
+  const int parts = SHARED ? p.parts : 1;
   int kj, hk;
-  cta_of(p.order, (int)blockIdx.x, kj, hk);
+  cta_of(p.order, (int)blockIdx.x / parts, kj, hk);
   const int b = hk / a.Hkv, G = a.Hq / a.Hkv;
   hk -= b * a.Hkv;
   const int k0 = kj * BM;
@@ -829,6 +886,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
       tma_load_4d(sm.k[pl], &map_k, &sm.bar[KB_KV], 0, hk, k0, b + pl * a.B);
       tma_load_4d(sm.v[pl], &map_v, &sm.bar[KB_KV], 0, hk, k0, b + pl * a.B);
     }
+    if constexpr (SHARED) sm.share = walk_share(p, b, hk, G, kj);
   }
   if (warp == 8) {
     tmem_alloc(&sm.tmem_base, kTmemCols);
@@ -841,7 +899,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
 
   if (warp >= 8) {
     setmaxnreg_dec_80();
-    HalfIter walk(p.l, b, hk, G, kj, a.N);
+    HalfIter<SHARED> walk(p.l, b, hk, G, kj, a.N, sm.share);
     int h, q0;
     bool partial, ok = true;
     if (warp == 8 || warp == 11) {
@@ -949,7 +1007,7 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
       mbar_arrive(acc_free);
       return true;
     };
-    HalfIter walk(p.l, b, hk, G, kj, a.N);
+    HalfIter<SHARED> walk(p.l, b, hk, G, kj, a.N, sm.share);
     int h, q0, n = 0;
     bool partial;
     for (; ok && walk.next(h, q0, partial); ++n) {
@@ -1025,18 +1083,29 @@ f32_dkdv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
       note_finite(z, acc[j].x);
       note_finite(z, acc[j].y);
     }
-    if (z != 0.f) sm.not_finite = 1;
+    if (z != 0.f && parts == 1) sm.not_finite = 1;
 #pragma unroll
     for (int j = 0; j < 64; j += 4)
       if (ok) *reinterpret_cast<float4*>(stage + row * kPitch + j) = make_float4(acc[j / 2].x, acc[j / 2].y, acc[j / 2 + 1].x, acc[j / 2 + 1].y);
     mbar_arrive(&sm.bar[KB_EPI0 + w]);
     ok = mbar_wait(&sm.bar[KB_EPI0 + w], 0) && ok;
-    if (ok) store_rows<128>(stage, kPitch, w == 0 ? a.dv : a.dk, b, k0, a.L, hk, a.d, row);
-    else report_device_error(p.status, 730 + warp);
+    if (!ok) report_device_error(p.status, 730 + warp);
+    else if (parts == 1) store_rows<128>(stage, kPitch, w == 0 ? a.dv : a.dk, b, k0, a.L, hk, a.d, row);
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (SHARED) cluster_sync();
+  else __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if constexpr (SHARED) {
+    const int part = (int)blockIdx.x % parts;
+    if (warp < 8) {
+#pragma unroll 1
+      for (int i = 0; i < 2; ++i)
+        sum_rows<64>(reinterpret_cast<const float*>(i ? sm.k[0] : sm.v[0]), 68, i ? a.dk : a.dv, b, k0, a.L, hk, a.d, parts, part, &sm.not_finite);
+    }
+    cluster_sync();   // shared memory stays until the others have read it
+    if (part > 0) return;
+  }
   if (warp < 8 && sm.not_finite) redo_row<REDO_DKDV, 4>(reinterpret_cast<float*>(smem_raw), p, kj, hk, b);
 }
 
@@ -1063,15 +1132,16 @@ struct __align__(1024) DqSmem {
 static_assert(dq_smem<4>() <= sizeof(DqSmem), "as above");
 constexpr uint32_t COL_S2 = 0, COL_DP2 = 256, COL_DQ2 = 384;   // S: two buffers of 128 columns
 
-template <bool KB>
+template <bool KB, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kh,
               const __grid_constant__ CUtensorMap map_vh, const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DqSmem& sm = *reinterpret_cast<DqSmem*>(smem_raw);
   const bma_attn_args& a = p.a;
+  const int parts = SHARED ? p.parts : 1;
   int qi, h;
-  cta_of(p.order, (int)blockIdx.x, qi, h);
+  cta_of(p.order, (int)blockIdx.x / parts, qi, h);
   qi = p.order.tiles - 1 - qi;
   const int b = h / a.Hq;
   h -= b * a.Hq;
@@ -1099,11 +1169,13 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     tmem_relinquish();
   }
   tc_fence_before();
-  const int T = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
+  const int listed = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
+  const int part = (int)blockIdx.x % parts, t0 = listed * part / parts, T = listed * (part + 1) / parts - t0;   // this CTA's part of the list
+  const uint16_t* entry = sm.list.entry + t0;
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   // half tiles in all; the second half of the last tile may lie past the end of the keys
-  const int total = T == 0 ? 0 : 2 * T - ((int)(sm.list.entry[T - 1] & 0x7fff) * 128 + BH >= a.L ? 1 : 0);
+  const int total = T == 0 ? 0 : 2 * T - ((int)(entry[T - 1] & 0x7fff) * 128 + BH >= a.L ? 1 : 0);
 
   if (warp >= 8) {
     setmaxnreg_dec_80();
@@ -1117,7 +1189,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         uint64_t* full = &sm.bar[(is_k ? QB_K_FULL : QB_V_FULL) + st];
         if (n >= stages) ok = mbar_wait(&sm.bar[(is_k ? QB_K_FREE : QB_V_FREE) + st], (n / stages - 1) & 1);
         if (!ok) break;
-        const int row = (int)(sm.list.entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
+        const int row = (int)(entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
         mbar_expect_tx(full, 3 * kHalfBox);
 #pragma unroll
         for (int pl = 0; pl < 3; ++pl) tma_load_4d(is_k ? sm.k[st][pl] : sm.v[st][pl], is_k ? &map_kh : &map_vh, full, 0, hk, row, b + pl * a.B);
@@ -1188,7 +1260,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       return true;
     };
     for (int n = 0; n < total && ok; ++n) {
-      const uint32_t e = sm.list.entry[n >> 1];
+      const uint32_t e = entry[n >> 1];
       const int k0 = (int)(e & 0x7fff) * 128 + (n & 1) * BH;
       uint32_t bits = 0xffffffffu;
       if (e & 0x8000u) {
@@ -1241,7 +1313,7 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       note_finite(z, acc[j].x);
       note_finite(z, acc[j].y);
     }
-    if (z != 0.f) sm.not_finite = 1;
+    if (z != 0.f && parts == 1) sm.not_finite = 1;
     constexpr int kPitch = 68;
     float* stage = reinterpret_cast<float*>(&sm.q[0][0]);   // every MMA that read the Q planes has completed
     if (ok) {
@@ -1251,12 +1323,18 @@ f32_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
     mbar_arrive(&sm.bar[QB_EPI]);
     ok = mbar_wait(&sm.bar[QB_EPI], 0) && ok;
-    if (ok) store_rows<256>(stage, kPitch, a.dq, b, q0, a.N, h, a.d, threadIdx.x);
-    else report_device_error(p.status, 830 + warp);
+    if (!ok) report_device_error(p.status, 830 + warp);
+    else if (parts == 1) store_rows<256>(stage, kPitch, a.dq, b, q0, a.N, h, a.d, threadIdx.x);
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (SHARED) cluster_sync();
+  else __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if constexpr (SHARED) {
+    if (warp < 8) sum_rows<64>(reinterpret_cast<const float*>(&sm.q[0][0]), 68, a.dq, b, q0, a.N, h, a.d, parts, part, &sm.not_finite);
+    cluster_sync();   // shared memory stays until the others have read it
+    if (part > 0) return;
+  }
   if (warp < 8 && sm.not_finite) redo_row<REDO_DQ, 4>(reinterpret_cast<float*>(smem_raw), p, qi, h, b);
 }
 
@@ -1340,16 +1418,17 @@ struct __align__(1024) DkdvWideSmem {
   uint8_t k[3][2][kRowBox];
   uint8_t q[3][kBoxPlanes];
   uint8_t d_o[2][kBoxPlanes];
-  float nlse2[2][BH], ndelta[2][BH];   // minus the log-sum-exp (log2 units) and delta
+  alignas(16) float nlse2[2][BH], ndelta[2][BH];   // minus the log-sum-exp (log2 units) and delta
   uint64_t bar[XB_NUM];
   uint32_t tmem_base;
+  WalkShare share;
   int not_finite;
 };
 static_assert(dkdv_smem<8>() <= sizeof(DkdvWideSmem), "as above");
 constexpr int kWidePitch = 132;
 static_assert(2 * BM * kWidePitch * sizeof(float) <= sizeof(uint8_t[3][2][kRowBox]) + 3 * kBoxPlanes, "dV and dK are staged over K and Q");
 
-template <bool KB>
+template <bool KB, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_qh,
                      const __grid_constant__ CUtensorMap map_do, const __grid_constant__ F32WideParams wp) {
@@ -1357,8 +1436,9 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   DkdvWideSmem& sm = *reinterpret_cast<DkdvWideSmem*>(smem_raw);
   const F32Params& p = wp.f;
   const bma_attn_args& a = p.a;
+  const int parts = SHARED ? p.parts : 1;
   int kj, hk;
-  cta_of(p.order, (int)blockIdx.x, kj, hk);
+  cta_of(p.order, (int)blockIdx.x / parts, kj, hk);
   const int b = hk / a.Hkv, G = a.Hq / a.Hkv;
   hk -= b * a.Hkv;
   const int k0 = kj * BM;
@@ -1382,6 +1462,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     for (int pl = 0; pl < 3; ++pl)
 #pragma unroll
       for (int box = 0; box < 2; ++box) tma_load_4d(sm.k[pl][box], &map_k, &sm.bar[XB_K], box * 64, hk, k0, b + pl * a.B);
+    if constexpr (SHARED) sm.share = walk_share(p, b, hk, G, kj);
   }
   if (warp == 8) {
     tmem_alloc(&sm.tmem_base, kTmemCols);
@@ -1394,7 +1475,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
 
   if (warp >= 8) {
     setmaxnreg_dec_80();
-    HalfIter walk(p.l, b, hk, G, kj, a.N);
+    HalfIter<SHARED> walk(p.l, b, hk, G, kj, a.N, sm.share);
     int h, q0;
     bool partial, ok = true;
     if (warp == 8 || warp == 11) {
@@ -1502,7 +1583,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
 #pragma unroll
       for (int j = 0; j < 16; ++j) acc[c][j] = both(0.f);
     bool ok = true;
-    HalfIter walk(p.l, b, hk, G, kj, a.N);
+    HalfIter<SHARED> walk(p.l, b, hk, G, kj, a.N, sm.share);
     int h, q0, n = 0;
     bool partial;
     for (; ok && walk.next(h, q0, partial); ++n) {
@@ -1581,7 +1662,7 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         note_finite(z, acc[c][j].x);
         note_finite(z, acc[c][j].y);
       }
-    if (z != 0.f) sm.not_finite = 1;
+    if (z != 0.f && parts == 1) sm.not_finite = 1;
     // ---- epilogue: every MMA has completed; dV and dK are staged over the K planes and the Q ring
     mbar_arrive(&sm.bar[XB_EPI]);
     ok = mbar_wait(&sm.bar[XB_EPI], 0) && ok;
@@ -1597,16 +1678,28 @@ f32_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     }
     mbar_arrive(&sm.bar[XB_EPI]);
     ok = mbar_wait(&sm.bar[XB_EPI], 1) && ok;
-    if (ok) {
+    if (!ok) {
+      report_device_error(p.status, 780 + warp);
+    } else if (parts == 1) {
       store_rows<256>(stage, kWidePitch, a.dv, b, k0, a.L, hk, a.d, threadIdx.x);
       store_rows<256>(stage + BM * kWidePitch, kWidePitch, a.dk, b, k0, a.L, hk, a.d, threadIdx.x);
-    } else {
-      report_device_error(p.status, 780 + warp);
     }
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (SHARED) cluster_sync();
+  else __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if constexpr (SHARED) {
+    const int part = (int)blockIdx.x % parts;
+    if (warp < 8) {
+      const float* stage = reinterpret_cast<const float*>(smem_raw);
+#pragma unroll 1
+      for (int i = 0; i < 2; ++i)
+        sum_rows<128>(stage + i * BM * kWidePitch, kWidePitch, i ? a.dk : a.dv, b, k0, a.L, hk, a.d, parts, part, &sm.not_finite);
+    }
+    cluster_sync();   // shared memory stays until the others have read it
+    if (part > 0) return;
+  }
   if (warp < 8 && sm.not_finite) redo_row<REDO_DKDV, 8>(reinterpret_cast<float*>(smem_raw), p, kj, hk, b);
 }
 
@@ -1626,7 +1719,7 @@ struct __align__(1024) DqWideSmem {
 
 static_assert(dq_smem<8>() <= sizeof(DqWideSmem), "as above");
 
-template <bool KB>
+template <bool KB, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kh,
                    const __grid_constant__ CUtensorMap map_vh, const __grid_constant__ F32WideParams wp) {
@@ -1634,8 +1727,9 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   DqWideSmem& sm = *reinterpret_cast<DqWideSmem*>(smem_raw);
   const F32Params& p = wp.f;
   const bma_attn_args& a = p.a;
+  const int parts = SHARED ? p.parts : 1;
   int qi, h;
-  cta_of(p.order, (int)blockIdx.x, qi, h);
+  cta_of(p.order, (int)blockIdx.x / parts, qi, h);
   qi = p.order.tiles - 1 - qi;
   const int b = h / a.Hq;
   h -= b * a.Hq;
@@ -1662,11 +1756,13 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     tmem_relinquish();
   }
   tc_fence_before();
-  const int T = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
+  const int listed = build_kv_list(sm.list, p.l, p.spec, b, h, qi);
+  const int part = (int)blockIdx.x % parts, t0 = listed * part / parts, T = listed * (part + 1) / parts - t0;   // this CTA's part of the list
+  const uint16_t* entry = sm.list.entry + t0;
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   // half tiles in all; the second half of the last tile may lie past the end of the keys
-  const int total = T == 0 ? 0 : 2 * T - ((int)(sm.list.entry[T - 1] & 0x7fff) * 128 + BH >= a.L ? 1 : 0);
+  const int total = T == 0 ? 0 : 2 * T - ((int)(entry[T - 1] & 0x7fff) * 128 + BH >= a.L ? 1 : 0);
 
   if (warp >= 8) {
     setmaxnreg_dec_80();
@@ -1677,7 +1773,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const int slot = i % 3, n = i >> 1;
         if (i >= 3) ok = mbar_wait(&sm.bar[YB_K_FREE + slot], (i / 3 - 1) & 1);
         if (!ok) break;
-        const int r0 = (int)(sm.list.entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
+        const int r0 = (int)(entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
         mbar_expect_tx(&sm.bar[YB_K_FULL + slot], kBoxPlanes);
 #pragma unroll
         for (int pl = 0; pl < 3; ++pl)
@@ -1689,7 +1785,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       for (int n = 0; n < total && ok; ++n) {
         if (n >= 1) ok = mbar_wait(&sm.bar[YB_V_FREE], (n - 1) & 1);
         if (!ok) break;
-        const int r0 = (int)(sm.list.entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
+        const int r0 = (int)(entry[n >> 1] & 0x7fff) * 128 + (n & 1) * BH;
         mbar_expect_tx(&sm.bar[YB_V_FULL], 2 * kBoxPlanes);
 #pragma unroll
         for (int box = 0; box < 2; ++box)
@@ -1756,7 +1852,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       for (int j = 0; j < 16; ++j) acc[c][j] = both(0.f);
     bool ok = true;
     for (int n = 0; n < total && ok; ++n) {
-      const uint32_t e = sm.list.entry[n >> 1];
+      const uint32_t e = entry[n >> 1];
       const int k0 = (int)(e & 0x7fff) * 128 + (n & 1) * BH;
       uint32_t bits = 0xffffffffu;
       if (e & 0x8000u) {
@@ -1822,7 +1918,7 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         note_finite(z, acc[c][j].x);
         note_finite(z, acc[c][j].y);
       }
-    if (z != 0.f) sm.not_finite = 1;
+    if (z != 0.f && parts == 1) sm.not_finite = 1;
     // every thread has seen the last chunk, so every MMA that read the Q planes has completed
     mbar_arrive(&sm.bar[YB_EPI]);
     ok = mbar_wait(&sm.bar[YB_EPI], 0) && ok;
@@ -1837,12 +1933,18 @@ f32_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     }
     mbar_arrive(&sm.bar[YB_EPI]);
     ok = mbar_wait(&sm.bar[YB_EPI], 1) && ok;
-    if (ok) store_rows<256>(stage, kWidePitch, a.dq, b, q0, a.N, h, a.d, threadIdx.x);
-    else report_device_error(p.status, 880 + warp);
+    if (!ok) report_device_error(p.status, 880 + warp);
+    else if (parts == 1) store_rows<256>(stage, kWidePitch, a.dq, b, q0, a.N, h, a.d, threadIdx.x);
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (SHARED) cluster_sync();
+  else __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
+  if constexpr (SHARED) {
+    if (warp < 8) sum_rows<128>(reinterpret_cast<const float*>(&sm.q[0][0][0]), kWidePitch, a.dq, b, q0, a.N, h, a.d, parts, part, &sm.not_finite);
+    cluster_sync();   // shared memory stays until the others have read it
+    if (part > 0) return;
+  }
   if (warp < 8 && sm.not_finite) redo_row<REDO_DQ, 8>(reinterpret_cast<float*>(smem_raw), p, qi, h, b);
 }
 
@@ -1938,34 +2040,54 @@ int f32_fwd_clusters(int dp, int parts) {
 struct FwdShare {
   int parts, last, last_parts;
 };
-FwdShare f32_fwd_share(const bma_attn_args& a, const bma_mask_spec& spec, int dp, int NQ, int NKV) {
-  FwdShare best{1, 0, 1};
+// Walks of the query tiles over key tiles, of the key tiles over a head group's query tiles.  (Of other masks than causal ones and bands
+// nothing is known here: as if they were full.)
+Walks q_walks(const bma_attn_args& a, const bma_mask_spec& spec, int NQ, int NKV) {
   const int heads = a.B * a.Hq;
-  const int64_t tiles64 = (int64_t)NQ * heads;
-  if (tiles64 > 4 * kSms || NKV < 2) return best;
-  const int tiles = (int)tiles64;
-  const double o = 3.;
-  double longest = NKV, sum = (double)tiles * NKV;
-  const bool causal = (spec.flags & BMA_MASK_CAUSAL) != 0;
-  if (causal) {
-    longest = sum = 0.;
+  Walks w{NQ * heads, (double)NKV, (double)NQ * heads * NKV, true};
+  if (spec.flags & BMA_MASK_CAUSAL) {
+    w = {NQ * heads, 0., 0., false};
     for (int qi = 0; qi < NQ; ++qi) {
       const int64_t keys = std::min<int64_t>((int64_t)(qi + 1) * BM, a.N) + spec.q_offset - spec.k_offset;
-      const double w = (double)std::min<int64_t>(std::max<int64_t>((keys + BM - 1) / BM, 0), NKV);
-      longest = std::max(longest, w);
-      sum += w * heads;
+      const double t = (double)std::min<int64_t>(std::max<int64_t>((keys + BM - 1) / BM, 0), NKV);
+      w.longest = std::max(w.longest, t);
+      w.sum += t * heads;
     }
   }
-  if (spec.flags & BMA_MASK_BAND) {   // the walks of a band are about as long as it is wide
-    const double w = std::min(longest, ((double)spec.band_left + spec.band_right) / BM + 2.);
-    sum = std::min(sum, w * tiles);
-    longest = w;
+  if (spec.flags & BMA_MASK_BAND) {
+    w.longest = std::min(w.longest, ((double)spec.band_left + spec.band_right) / BM + 2.);
+    w.sum = std::min(w.sum, w.longest * w.ctas);
   }
+  return w;
+}
+Walks k_walks(const bma_attn_args& a, const bma_mask_spec& spec, int NQ, int NKV) {
+  const int G = a.Hq / a.Hkv;
+  const Walks q = q_walks(a, spec, NQ, NKV);
+  Walks w{NKV * a.B * a.Hkv, (double)G * NQ, q.sum, q.even};
+  if (spec.flags & BMA_MASK_BAND) w.longest = std::min(w.longest, G * q.longest);
+  return w;
+}
+// CTAs that share a walk of a backward pass, likewise, with float32 accumulators to add up.  (Calls, forward and backward, causal: 1 x 1423, 4/1
+// heads of 128 750 -> 195 us, 1 x 4096, 8/2 heads of 128 2220 -> 805, 1 x 4096, 4 heads of 64 404 -> 280, 1 x 3000, 16/4 heads of 64 823 -> 538;
+// forward, host path and launch order included.  The shared kernels are instances of their own: the part of a walk costs the plain dK / dV
+// kernel 7 % in registers, 173 -> 186 us on 2 x 2048 tokens of 16 heads of 64.)
+template <typename K>
+int f32_bwd_parts(const Walks& w, int64_t ctas, ClusterCounts& known, K kernel, size_t smem) {
+  if (ctas > 4 * kSms) return 1;
+  return share_walks(w, 3.0, (int)std::max(1.0, w.longest), [&](int parts) { return clusters_at_once(known, kernel, kThreads, smem, parts); });
+}
+
+FwdShare f32_fwd_share(const bma_attn_args& a, const bma_mask_spec& spec, int dp, int NQ, int NKV) {
+  FwdShare best{1, 0, 1};
+  if ((int64_t)NQ * a.B * a.Hq > 4 * kSms || NKV < 2) return best;
+  const Walks w = q_walks(a, spec, NQ, NKV);
+  const int tiles = w.ctas;
+  const double o = 3., longest = w.longest;
   auto even = [&](int count, int parts, int clusters) { return (double)ceil_div(count, clusters) * (longest / parts + o); };
-  best.parts = share_walks({tiles, longest, sum, !causal}, o, NKV, [&](int parts) { return f32_fwd_clusters(dp, parts); });
+  best.parts = share_walks(w, o, NKV, [&](int parts) { return f32_fwd_clusters(dp, parts); });
   double cost = even(tiles, best.parts, f32_fwd_clusters(dp, best.parts));
   const int last = tiles % kSms;
-  if (!causal && tiles > kSms && last > 0)
+  if (w.even && tiles > kSms && last > 0)
     for (int parts = 2; parts <= std::min(kMaxParts, NKV); ++parts) {
       const int clusters = f32_fwd_clusters(dp, parts);
       if (clusters < last) continue;
@@ -2024,41 +2146,56 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   int rc;
   if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, spec, lists, pl, w, true, st))) return rc;
   CUtensorMap mq, mk, mv, mdo, mqh, mkh, mvh, mdoh;
+  static ClusterCounts known[4];
+  const int64_t k_ctas = (int64_t)lists.NKV * a.B * a.Hkv, q_ctas = (int64_t)lists.NQ * a.B * a.Hq;
+  const bool few = std::min(k_ctas, q_ctas) <= 4 * kSms;
+  const Walks kw = few ? k_walks(a, spec, lists.NQ, lists.NKV) : Walks{}, qw = few ? q_walks(a, spec, lists.NQ, lists.NKV) : Walks{};
+  auto launch = [&](auto kernel, const LaunchOrder& order, int parts, size_t smem, auto... args) -> int {
+    BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(launch_ctas(order) * parts);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = cluster_attribute(parts);
+    if (parts > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
+    BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+    count_launches(1);
+    return BMA_OK;
+  };
   if (a.d > 64) {
     if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, 128, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, 128, BM)) ||
         (rc = plane_map(&mqh, w + pl.q, a.B, a.N, a.Hq, 128, BH)) || (rc = plane_map(&mkh, w + pl.k, a.B, a.L, a.Hkv, 128, BH)) ||
         (rc = plane_map(&mvh, w + pl.v, a.B, a.L, a.Hkv, 128, BH)) || (rc = plane_map(&mdoh, w + pl.d_o, a.B, a.N, a.Hq, 128, BH)))
       return rc;
-    auto dkdv = a.key_bias ? f32_dkdv_wide_kernel<true> : f32_dkdv_wide_kernel<false>;
-    auto dq = a.key_bias ? f32_dq_wide_kernel<true> : f32_dq_wide_kernel<false>;
-    BMA_CUDA_TRY(cudaFuncSetAttribute(dkdv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvWideSmem)));
-    BMA_CUDA_TRY(cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqWideSmem)));
+    auto dkdv = a.key_bias ? f32_dkdv_wide_kernel<true, false> : f32_dkdv_wide_kernel<false, false>;
+    auto dkdv_shared = a.key_bias ? f32_dkdv_wide_kernel<true, true> : f32_dkdv_wide_kernel<false, true>;
+    auto dq = a.key_bias ? f32_dq_wide_kernel<true, false> : f32_dq_wide_kernel<false, false>;
+    auto dq_shared = a.key_bias ? f32_dq_wide_kernel<true, true> : f32_dq_wide_kernel<false, true>;
     F32WideParams wp{p, w + pl.v};
     wp.f.order = k_order(a, 128);
-    dkdv<<<launch_ctas(wp.f.order), kThreads, sizeof(DkdvWideSmem), st>>>(mk, mqh, mdoh, wp);
+    wp.f.parts = f32_bwd_parts(kw, k_ctas, known[0], dkdv_shared, sizeof(DkdvWideSmem));
+    if ((rc = launch(wp.f.parts > 1 ? dkdv_shared : dkdv, wp.f.order, wp.f.parts, sizeof(DkdvWideSmem), mk, mqh, mdoh, wp))) return rc;
     wp.a_planes = w + pl.d_o;
     wp.f.order = q_order(a, 128);
-    dq<<<launch_ctas(wp.f.order), kThreads, sizeof(DqWideSmem), st>>>(mq, mkh, mvh, wp);
-    count_launches(2);
-    BMA_CUDA_TRY(cudaGetLastError());
-    return BMA_OK;
+    wp.f.parts = f32_bwd_parts(qw, q_ctas, known[1], dq_shared, sizeof(DqWideSmem));
+    return launch(wp.f.parts > 1 ? dq_shared : dq, wp.f.order, wp.f.parts, sizeof(DqWideSmem), mq, mkh, mvh, wp);
   }
   if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, 64, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, 64, BM)) ||
       (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, 64, BM)) || (rc = plane_map(&mdo, w + pl.d_o, a.B, a.N, a.Hq, 64, BM)) ||
       (rc = plane_map(&mqh, w + pl.q, a.B, a.N, a.Hq, 64, BH)) || (rc = plane_map(&mkh, w + pl.k, a.B, a.L, a.Hkv, 64, BH)) ||
       (rc = plane_map(&mvh, w + pl.v, a.B, a.L, a.Hkv, 64, BH)) || (rc = plane_map(&mdoh, w + pl.d_o, a.B, a.N, a.Hq, 64, BH)))
     return rc;
-  auto dkdv = a.key_bias ? f32_dkdv_kernel<true> : f32_dkdv_kernel<false>;
-  auto dq = a.key_bias ? f32_dq_kernel<true> : f32_dq_kernel<false>;
-  BMA_CUDA_TRY(cudaFuncSetAttribute(dkdv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DkdvSmem)));
-  BMA_CUDA_TRY(cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DqSmem)));
+  auto dkdv = a.key_bias ? f32_dkdv_kernel<true, false> : f32_dkdv_kernel<false, false>;
+  auto dkdv_shared = a.key_bias ? f32_dkdv_kernel<true, true> : f32_dkdv_kernel<false, true>;
+  auto dq = a.key_bias ? f32_dq_kernel<true, false> : f32_dq_kernel<false, false>;
+  auto dq_shared = a.key_bias ? f32_dq_kernel<true, true> : f32_dq_kernel<false, true>;
   p.order = k_order(a, 64);
-  dkdv<<<launch_ctas(p.order), kThreads, sizeof(DkdvSmem), st>>>(mk, mv, mqh, mdoh, p);
+  p.parts = f32_bwd_parts(kw, k_ctas, known[2], dkdv_shared, sizeof(DkdvSmem));
+  if ((rc = launch(p.parts > 1 ? dkdv_shared : dkdv, p.order, p.parts, sizeof(DkdvSmem), mk, mv, mqh, mdoh, p))) return rc;
   p.order = q_order(a, 64);
-  dq<<<launch_ctas(p.order), kThreads, sizeof(DqSmem), st>>>(mq, mkh, mvh, mdo, p);
-  count_launches(2);
-  BMA_CUDA_TRY(cudaGetLastError());
-  return BMA_OK;
+  p.parts = f32_bwd_parts(qw, q_ctas, known[3], dq_shared, sizeof(DqSmem));
+  return launch(p.parts > 1 ? dq_shared : dq, p.order, p.parts, sizeof(DqSmem), mq, mkh, mvh, mdo, p);
 }
 
 }  // namespace bma

@@ -430,6 +430,11 @@ struct QTileIter {  // flattened walk over (group head, listed q tile), from its
     part_idx = l.q_idx + row * l.NQ;
     it = 0;
   }
+  __device__ void start(int g_, int it_) {   // from entry it_ of head g_ on
+    g = g_;
+    load_head();
+    it = it_;
+  }
   __device__ bool next(int& h, int& qi, bool& partial) {
     if (g < 0) { g = 0; load_head(); }
     if (g >= G) return false;
