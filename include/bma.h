@@ -293,6 +293,12 @@ int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const
 int bma_attn_bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
                      void* workspace, size_t workspace_bytes, bma_stream_t stream);
 
+/* The same without bma_attn_bwd_preprocess before it: delta is taken from args->o and args->d_o on the way through dO and written to
+ * args->delta.  With the full workspace both accept lists without arrays (all eight NULL, B = H = 1) for a mask of interval terms only,
+ * and write them into the workspace in the same launch. */
+int bma_attn_bwd_f32_o(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
+                       void* workspace, size_t workspace_bytes, bma_stream_t stream);
+
 /* Backward preprocess: delta = rowsum(dO * O); when d_o_bf16 is non-NULL also writes a
  * bf16 copy of dO there (and takes delta from that rounded copy, the values the backward's
  * dO V^T product sees, so that dP - delta cancels exactly where it should) as a DENSE

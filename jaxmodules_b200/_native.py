@@ -113,6 +113,7 @@ SIGNATURES = {
     "bma_attn_f32_workspace_bytes": (C.c_size_t, [C.POINTER(AttnArgs), C.c_int32]),
     "bma_attn_fwd_f32": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t, C.c_void_p]),
     "bma_attn_bwd_f32": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t, C.c_void_p]),
+    "bma_attn_bwd_f32_o": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t, C.c_void_p]),
     "bma_attn_bwd_preprocess": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.c_void_p]),
     "bma_attn_bwd_workspace_bytes": (C.c_size_t, [C.POINTER(AttnArgs)]),
     "bma_block_lists_visited": (C.c_int, [C.POINTER(BlockLists), C.c_void_p, C.c_void_p]),

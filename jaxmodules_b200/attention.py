@@ -82,6 +82,7 @@ def kernel_log_affine(kernel_fn: Callable, d: int) -> Tuple[float, float]:
     return float(a), float(b)
 
 
+_TABLE_TERMS = nat.BMA_MASK_SEGMENT | nat.BMA_MASK_BITMAP | nat.BMA_MASK_TILES    # terms that are looked up, not known from the indices
 _DTYPES = {torch.float32: nat.BMA_DTYPE_F32, torch.bfloat16: nat.BMA_DTYPE_BF16}
 
 
@@ -247,7 +248,7 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
             ready = lists_fn(tq, tk, both_sides) if lists_fn is not None else None
             if ready is not None:
                 lists, lt = ready
-            elif not both_sides and host.implies_lists(Q, K, V, key_bias, scale, backend, C.addressof(dmask.spec)):
+            elif (not both_sides or f32_bytes) and host.implies_lists(Q, K, V, key_bias, scale, backend, C.addressof(dmask.spec)):
                 lists, lt = nat.BlockLists(1, 1, -(-N // tq), -(-L // tk), tq, tk), None     # no arrays: the kernels know the blocks
             else:
                 lists, lt = compile_block_lists(dmask, B, Hq, N, L, tq, tk, dev, q_side=both_sides, stream=st, conservative=True, views=False)
@@ -257,7 +258,7 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
                                   _DTYPES[out_dtype] == nat.BMA_DTYPE_BF16, st)
         _maybe_check_status(dev, "bma_attn_fwd")
     ctx = dict(dmask=dmask, lists=lists, list_tensors=lt, backend=be, scale=scale, lists_fn=lists_fn,
-               lists_tile=(tq, tk), lists_have_q_side=both_sides, key_bias=key_bias)
+               lists_tile=(tq, tk), lists_have_q_side=both_sides and lt is not None, key_bias=key_bias)
     return O, lse, ctx
 
 
@@ -272,8 +273,11 @@ def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
         st = nat.stream(dev)
         be, tq, tk, f32_bytes = host.routes(Q, K, V, key_bias, scale, backend, False, True)[1]
         lists_fn = ctx.get("lists_fn")
+        planes = _float32_planes(dev, f32_bytes) if f32_bytes else None
         with _span("mask_compile_bwd", dev):
-            if ctx.get("lists_have_q_side") and ctx.get("lists_tile") == (tq, tk):
+            if planes is not None and lists_fn is None and not ctx["dmask"].spec.flags & _TABLE_TERMS and not ctx.get("lists_have_q_side"):
+                lists, lt = nat.BlockLists(1, 1, -(-N // tq), -(-L // tk), tq, tk), None     # no arrays: written by the pass itself
+            elif ctx.get("lists_have_q_side") and ctx.get("lists_tile") == (tq, tk):
                 lists, lt = ctx["lists"], ctx["list_tensors"]      # built by the forward pass
             else:
                 ready = lists_fn(tq, tk, True) if lists_fn is not None else None
@@ -284,7 +288,10 @@ def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
             dO = dO.contiguous()
         bf16_copy = be == nat.BMA_BACKEND_TCGEN05 and dO.dtype != torch.bfloat16
         reuse = ctx.get("reuse")       # a dict the caller keeps for one (O, dO): delta and the bf16 cotangent are taken once
-        if reuse is not None and "delta" in reuse and (not bf16_copy or reuse["do_bf16"] is not None):
+        do_bf16 = None
+        if f32_bytes and reuse is None:
+            delta = None               # taken by the pass itself
+        elif reuse is not None and "delta" in reuse and (not bf16_copy or reuse["do_bf16"] is not None):
             delta, do_bf16 = reuse["delta"], (reuse["do_bf16"] if bf16_copy else None)
         else:
             with _span("bwd_preprocess", dev):
@@ -294,7 +301,6 @@ def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
         if do_bf16 is not None:
             dO = do_bf16
         if f32_bytes:
-            planes = _float32_planes(dev, f32_bytes)
             with _span("bwd", dev):
                 grads = host.backward(Q, K, V, O, lse, dO, delta, key_bias, scale, backend, spec_at, lists_at, f32_bytes, planes, 0, 0, 0, st)
             _maybe_check_status(dev, "bma_attn_bwd_f32")

@@ -146,6 +146,11 @@ struct SplitJob {
 struct SplitParams {
   SplitJob job[4];
   int B, d;
+  bma_tensor o;          // backward: with `delta`, delta = rowsum(dO * O) on the way through dO (job 3)
+  float* delta;          // null: the caller's
+  int jobs;              // blockIdx.y == jobs: the block lists of a mask of interval terms, both sides, where the caller has none
+  bma_block_lists lists;
+  bma_mask_spec spec;
   const uint8_t* used;   // null, or one byte per kv block [used_B, NKV] (jobs 1 and 2, K and V): 0 = no list names it
   int used_B, NKV;
 };
@@ -166,19 +171,52 @@ __global__ void __launch_bounds__(256) used_blocks_kernel(bma_block_lists l, bma
     for (int i = lane; i < nfull; i += 32) mark[l.full_kv_idx[row * l.NKV + i]] = 1;
     for (int i = lane; i < npart; i += 32) mark[l.kv_idx[row * l.NKV + i]] = 1;
   }
-  if (backward)
+  if (backward && l.q_num)
     for (int i = threadIdx.x; i < l.H * l.NKV; i += 256)
       if (l.q_num[(int64_t)blockIdx.x * l.H * l.NKV + i] + l.full_q_num[(int64_t)blockIdx.x * l.H * l.NKV + i] > 0) mark[i % l.NKV] = 1;
   __syncthreads();
   for (int i = threadIdx.x; i < l.NKV; i += 256) used[(int64_t)blockIdx.x * l.NKV + i] = mark[i];
 }
 
-// One thread per 8 columns: 32 bytes in, three 16-byte lines out.  Bound by HBM (4 bytes read, 6 written per element), or
+// Block lists of a mask of interval terms: a warp per row of either side.
+__device__ __forceinline__ void write_lists(const bma_block_lists& l, const bma_mask_spec& spec) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1;
+  for (int r = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5); r < l.NQ + l.NKV; r += (int)gridDim.x * 8) {
+    const bool q_side = r >= l.NQ;
+    const int row = q_side ? r - l.NQ : r, width = q_side ? l.NQ : l.NKV;
+    int32_t* full = (q_side ? l.full_q_idx : l.full_kv_idx) + (int64_t)row * width;
+    int32_t* part = (q_side ? l.q_idx : l.kv_idx) + (int64_t)row * width;
+    int nfull = 0, npart = 0;
+    for (int base = 0; base < width; base += 32) {
+      const int j = base + lane;
+      const int c = j >= width ? 0 : q_side ? interval_class(spec, j, row, BM, BM) : interval_class(spec, row, j, BM, BM);
+      const unsigned mf = __ballot_sync(0xffffffffu, c == 2), mp = __ballot_sync(0xffffffffu, c == 1);
+      if (c == 2) full[nfull + __popc(mf & below)] = j;
+      if (c == 1) part[npart + __popc(mp & below)] = j;
+      nfull += __popc(mf);
+      npart += __popc(mp);
+    }
+    if (lane == 0) {
+      (q_side ? l.full_q_num : l.full_kv_num)[row] = nfull;
+      (q_side ? l.q_num : l.kv_num)[row] = npart;
+    }
+  }
+}
+
+// One thread per 8 columns: 32 bytes in, three 16-byte lines out.  Backward the same launch takes delta = rowsum(dO * O) and writes the
+// block lists that the caller left to it: launches of their own, 2.6 and 3 us of the device and 8 - 10 of the host each (2 x 128 tokens, 8 heads,
+// forward and backward: the call 154 -> 143 us; 2 x 2048, 16 heads, where O and dO were read in a pass of their own: 533 -> 526).  Bound by HBM (4 bytes read, 6 written per element), or
 // by launch latency where the tensors are small.
 template <int DP>
 __global__ void __launch_bounds__(256) split_kernel(const SplitParams p) {
+  if ((int)blockIdx.y == p.jobs) {
+    write_lists(p.lists, p.spec);
+    return;
+  }
   const SplitJob& job = p.job[blockIdx.y];
   constexpr int kChunks = DP / 8;
+  const bool take_delta = blockIdx.y == 3 && p.delta != nullptr, o_f32 = p.o.dtype == BMA_DTYPE_F32;
   const int64_t n = (int64_t)p.B * job.L * job.H * kChunks;
   const bool f32 = job.t.dtype == BMA_DTYPE_F32;
   const bool vec = f32 && (reinterpret_cast<uintptr_t>(job.t.ptr) & 15) == 0 && ((job.t.stride_b | job.t.stride_l | job.t.stride_h) & 3) == 0;
@@ -208,6 +246,33 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitParams p) {
     for (int e = 0; e < 4; ++e) split3(make_float2(v[2 * e], v[2 * e + 1]), w[0][e], w[1][e], w[2][e]);
 #pragma unroll
     for (int q = 0; q < 3; ++q) out[q * n + i] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+    if (take_delta) {
+      // Sums in the order of bwd_preprocess_rows4_kernel (four columns, then a tree over the columns' highest bits first), bit for bit: next to a
+      // huge key, dS is the rounding of delta alone, and what a tile that is done again makes of it is that of the FP32 tile kernels.
+      const int64_t at = (int64_t)b * p.o.stride_b + (int64_t)l * p.o.stride_l + (int64_t)h * p.o.stride_h + c;
+      float s[2] = {0.f, 0.f};
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (c + 4 * u >= p.d) continue;
+        float o4[4];
+        if (o_f32) {
+          const float4 x = *reinterpret_cast<const float4*>(static_cast<const float*>(p.o.ptr) + at + 4 * u);
+          o4[0] = x.x; o4[1] = x.y; o4[2] = x.z; o4[3] = x.w;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o4[e] = to_float(static_cast<const __nv_bfloat16*>(p.o.ptr)[at + 4 * u + e]);
+        }
+        s[u] = fmaf(v[4 * u], o4[0], fmaf(v[4 * u + 1], o4[1], fmaf(v[4 * u + 2], o4[2], v[4 * u + 3] * o4[3])));
+      }
+      const int lane = threadIdx.x & 31;   // (the kChunks lanes of a row are all here or all past the end)
+      const unsigned group = ((1u << kChunks) - 1) << (lane & ~(kChunks - 1));
+#pragma unroll
+      for (int off = kChunks / 2; off; off /= 2) {
+        s[0] += __shfl_xor_sync(group, s[0], off);
+        s[1] += __shfl_xor_sync(group, s[1], off);
+      }
+      if ((lane & (kChunks - 1)) == 0) p.delta[((int64_t)b * job.H + h) * job.L + l] = s[0] + s[1];
+    }
   };
   if (!p.used || blockIdx.y == 0 || blockIdx.y == 3) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) split8(i);
@@ -1954,7 +2019,7 @@ size_t plane_bytes(int B, int L, int H, int dp) { return (size_t)3 * B * L * H *
 size_t align_up(size_t x) { return (x + 1023) / 1024 * 1024; }
 
 struct Planes {
-  size_t q, k, v, d_o, used, total;   // offsets in the workspace
+  size_t q, k, v, d_o, used, lists, total;   // offsets in the workspace: planes, marks of listed blocks, block lists (backward)
 };
 // Few queries against many keys may see a small part of them: then only the planes of listed kv blocks are made.  (What the
 // other blocks' planes hold is read by the dK / dV kernel alone, as the resident operand of a CTA that has no query tile.)
@@ -1972,12 +2037,31 @@ Planes planes_layout(const bma_attn_args& a, bool backward) {
   p.v = p.k + align_up(plane_bytes(a.B, a.L, a.Hkv, dp));
   p.d_o = p.v + align_up(plane_bytes(a.B, a.L, a.Hkv, dp));
   p.used = p.d_o + (backward ? align_up(plane_bytes(a.B, a.N, a.Hq, dp)) : 0);
-  p.total = p.used + (used_blocks(a) ? align_up((size_t)a.B * ceil_div(a.L, BM)) : 0);
+  p.lists = p.used + (used_blocks(a) ? align_up((size_t)a.B * ceil_div(a.L, BM)) : 0);
+  const size_t NQ = ceil_div(a.N, BM), NKV = ceil_div(a.L, BM);
+  p.total = p.lists + (backward ? align_up(sizeof(int32_t) * (2 * (NQ + NKV) + 4 * NQ * NKV)) : 0);
   return p;
 }
+// The arrays of lists that the pass writes itself
+bma_block_lists own_lists(const bma_block_lists& sizes, uint8_t* at) {
+  bma_block_lists l = sizes;
+  int32_t* p = reinterpret_cast<int32_t*>(at);
+  auto take = [&](int64_t n) { int32_t* r = p; p += n; return r; };
+  const int64_t cells = (int64_t)l.NQ * l.NKV;
+  l.kv_num = take(l.NQ); l.full_kv_num = take(l.NQ); l.q_num = take(l.NKV); l.full_q_num = take(l.NKV);
+  l.kv_idx = take(cells); l.full_kv_idx = take(cells); l.q_idx = take(cells); l.full_q_idx = take(cells);
+  return l;
+}
 
-int launch_split(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& l, const Planes& pl, uint8_t* ws, bool backward, cudaStream_t st) {
+int launch_split(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& l, const Planes& pl, uint8_t* ws, bool backward, bool own_delta,
+                 cudaStream_t st) {
   SplitParams sp;
+  const bool lists_wanted = backward && !l.kv_num;
+  sp.o = a.o;
+  sp.delta = own_delta ? a.delta : nullptr;
+  sp.jobs = backward ? 4 : 3;
+  sp.lists = lists_wanted ? own_lists(l, ws + pl.lists) : l;
+  sp.spec = spec;
   sp.B = a.B; sp.d = a.d;
   sp.used = nullptr; sp.used_B = l.B; sp.NKV = l.NKV;
   if (used_blocks(a)) {
@@ -1991,7 +2075,7 @@ int launch_split(const bma_attn_args& a, const bma_mask_spec& spec, const bma_bl
   sp.job[3] = {a.d_o, ws + pl.d_o, a.N, a.Hq};
   const int dp = padded_d(a);
   const int64_t most = std::max((int64_t)a.B * a.N * a.Hq, (int64_t)a.B * a.L * a.Hkv) * (dp / 8);
-  const dim3 grid((unsigned)std::min<int64_t>((most + 255) / 256, 148 * 8), backward ? 4 : 3);
+  const dim3 grid((unsigned)std::min<int64_t>((most + 255) / 256, 148 * 8), sp.jobs + (lists_wanted ? 1 : 0));
   if (dp == 64) split_kernel<64><<<grid, 256, 0, st>>>(sp);
   else split_kernel<128><<<grid, 256, 0, st>>>(sp);
   count_launches(1);
@@ -2111,7 +2195,7 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   const int dp = padded_d(a);
   F32Params p;
   int rc;
-  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, spec, lists, pl, w, false, st))) return rc;
+  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, spec, lists, pl, w, false, false, st))) return rc;
   CUtensorMap mq, mk, mv;
   if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, dp, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, dp, BH)) ||
       (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, dp, BH)))
@@ -2139,12 +2223,13 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   return BMA_OK;
 }
 
-int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, cudaStream_t st) {
+int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& given, void* ws, bool own_delta, cudaStream_t st) {
   const Planes pl = planes_layout(a, true);
   uint8_t* w = static_cast<uint8_t*>(ws);
+  const bma_block_lists lists = given.kv_num ? given : own_lists(given, w + pl.lists);
   F32Params p;
   int rc;
-  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, spec, lists, pl, w, true, st))) return rc;
+  if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, spec, given, pl, w, true, own_delta, st))) return rc;
   CUtensorMap mq, mk, mv, mdo, mqh, mkh, mvh, mdoh;
   static ClusterCounts known[4];
   const int64_t k_ctas = (int64_t)lists.NKV * a.B * a.Hkv, q_ctas = (int64_t)lists.NQ * a.B * a.Hq;

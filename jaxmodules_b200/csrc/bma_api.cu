@@ -232,12 +232,13 @@ int validate_common(const bma_attn_args* a) {
   return BMA_OK;
 }
 
-// `implied`: the mask if the pass knows the blocks of interval terms by itself, so that all four arrays of the kv side may be NULL
+// `implied`: the mask if the pass knows the blocks of interval terms by itself, so that the arrays may all be NULL
 int validate_lists(const bma_attn_args* a, const bma_block_lists* l, int tile, bool need_q_side, const bma_mask_spec* implied = nullptr) {
   BMA_REQUIRE(l != nullptr, BMA_ERR_ARG);
-  const bool none = !l->kv_num && !l->kv_idx && !l->full_kv_num && !l->full_kv_idx;
+  const bool none = !l->kv_num && !l->kv_idx && !l->full_kv_num && !l->full_kv_idx &&
+                    (!need_q_side || (!l->q_num && !l->q_idx && !l->full_q_num && !l->full_q_idx && l->B == 1 && l->H == 1));
   BMA_REQUIRE((l->kv_num && l->kv_idx && l->full_kv_num && l->full_kv_idx) || (none && implied && !(implied->flags & kTableTerms)), BMA_ERR_ARG);
-  BMA_REQUIRE(!need_q_side || (l->q_num && l->q_idx && l->full_q_num && l->full_q_idx), BMA_ERR_ARG);
+  BMA_REQUIRE(!need_q_side || none || (l->q_num && l->q_idx && l->full_q_num && l->full_q_idx), BMA_ERR_ARG);
   BMA_REQUIRE(l->q_block == tile && l->kv_block == tile, BMA_ERR_ARG);
   BMA_REQUIRE(l->NQ == ceil_div(a->N, tile) && l->NKV == ceil_div(a->L, tile), BMA_ERR_ARG);
   BMA_REQUIRE((l->B == 1 || l->B == a->B) && (l->H == 1 || l->H == a->Hq), BMA_ERR_ARG);
@@ -391,8 +392,12 @@ int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const
   return f32_fwd(*args, *spec, *lists, workspace, static_cast<cudaStream_t>(stream));
 }
 
-int bma_attn_bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
-                     size_t workspace_bytes, bma_stream_t stream) {
+static bool rows_of_16_bytes(const bma_tensor& t) {
+  return (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && t.stride_b % 4 == 0 && t.stride_l % 4 == 0 && t.stride_h % 4 == 0;
+}
+
+static int bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+                   size_t workspace_bytes, bool own_delta, bma_stream_t stream) {
   const size_t need = bma_attn_f32_workspace_bytes(args, 1);
   BMA_REQUIRE(need > 0, BMA_ERR_UNSUPPORTED);
   BMA_REQUIRE(spec != nullptr && args->lse && args->delta, BMA_ERR_ARG);
@@ -402,13 +407,30 @@ int bma_attn_bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const
       (rc = validate_tensor(args->dq, true)) || (rc = validate_tensor(args->dk, true)) ||
       (rc = validate_tensor(args->dv, true)))
     return rc;
+  if (own_delta && (rc = validate_tensor(args->o, true))) return rc;
   BMA_REQUIRE(args->dq.dtype == args->q.dtype && args->dk.dtype == args->q.dtype && args->dv.dtype == args->q.dtype,
               BMA_ERR_UNSUPPORTED);
-  if ((rc = validate_lists(args, lists, kSm100Tile, true))) return rc;
+  const bool room = workspace && workspace_bytes >= need;
+  if ((rc = validate_lists(args, lists, kSm100Tile, true, room ? spec : nullptr))) return rc;   // (without room for them lists are needed)
   BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
-  if (!workspace || workspace_bytes < need) return simt_wide_bwd(*args, *spec, *lists, static_cast<cudaStream_t>(stream));
-  BMA_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15) == 0, BMA_ERR_WORKSPACE);
-  return f32_bwd(*args, *spec, *lists, workspace, static_cast<cudaStream_t>(stream));
+  BMA_REQUIRE(!room || (reinterpret_cast<uintptr_t>(workspace) & 15) == 0, BMA_ERR_WORKSPACE);
+  // delta on the way through dO only where bwd_preprocess_rows4_kernel would take it, whose sums the split kernel repeats
+  if (own_delta && !(room && args->d % 4 == 0 && rows_of_16_bytes(args->o) && rows_of_16_bytes(args->d_o))) {
+    own_delta = false;
+    if ((rc = bma_attn_bwd_preprocess(args, nullptr, stream))) return rc;
+  }
+  if (!room) return simt_wide_bwd(*args, *spec, *lists, static_cast<cudaStream_t>(stream));
+  return f32_bwd(*args, *spec, *lists, workspace, own_delta, static_cast<cudaStream_t>(stream));
+}
+
+int bma_attn_bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+                     size_t workspace_bytes, bma_stream_t stream) {
+  return bwd_f32(args, spec, lists, workspace, workspace_bytes, false, stream);
+}
+
+int bma_attn_bwd_f32_o(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+                       size_t workspace_bytes, bma_stream_t stream) {
+  return bwd_f32(args, spec, lists, workspace, workspace_bytes, true, stream);
 }
 
 int bma_attn_bwd_preprocess(const bma_attn_args* args, void* d_o_bf16, bma_stream_t stream) {
@@ -421,10 +443,7 @@ int bma_attn_bwd_preprocess(const bma_attn_args* args, void* d_o_bf16, bma_strea
   const int grid = (int)std::min<int64_t>((rows + 7) / 8, (int64_t)sm_count() * 16);
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(d_o_bf16);
   const bool of = args->o.dtype == BMA_DTYPE_F32, gf = args->d_o.dtype == BMA_DTYPE_F32;
-  auto vec_ok = [&](const bma_tensor& t) {
-    return (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && t.stride_b % 4 == 0 && t.stride_l % 4 == 0 && t.stride_h % 4 == 0;
-  };
-  const bool vec = args->d % 4 == 0 && vec_ok(args->o) && vec_ok(args->d_o) && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+  const bool vec = args->d % 4 == 0 && rows_of_16_bytes(args->o) && rows_of_16_bytes(args->d_o) && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
   const int64_t units4 = (int64_t)args->B * args->Hq * ((args->N + 3) / 4);
   const int grid4 = (int)std::min<int64_t>((units4 + 7) / 8, (int64_t)sm_count() * 32);
 #define BMA_PRE(TO, TDO)                                                                   \

@@ -480,7 +480,8 @@ size_t sm100_bwd_scratch_min_bytes(const bma_attn_args& a, const bma_block_lists
 // float32 on the tensor core (attn_f32_sm100.cu): 0 where the path does not take the request
 size_t f32_workspace_bytes(const bma_attn_args& a, bool backward);
 int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, cudaStream_t st);
-int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, cudaStream_t st);
+// own_delta: a.delta is written, from a.o and a.d_o.  Lists without arrays: the mask has interval terms only, and the pass writes them itself.
+int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, bool own_delta, cudaStream_t st);
 bool sm100_device();
 bool sm100_supported(const bma_attn_args& a);
 bool sm100_bwd_supported(const bma_attn_args& a);
