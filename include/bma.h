@@ -358,6 +358,12 @@ int bma_attn_bwd(const bma_attn_args* args, const bma_mask_spec* spec,
  * usable; bma_device_status then returns BMA_ERR_DEVICE_CHECK with *detail == code. */
 int bma_debug_expire_wait(uint64_t limit_ns, int32_t code, bma_stream_t stream);
 
+/* bma_attn_bwd_preprocess followed by bma_attn_bwd, with fewer launches: args->o and args->d_o are those of the preprocess, args->delta is
+ * written, and d_o_bf16 (or NULL where the cotangent is bf16 already) receives the dense bf16 copy that the pass then reads. */
+int bma_attn_bwd_o(const bma_attn_args* args, void* d_o_bf16, const bma_mask_spec* spec, const bma_block_lists* lists,
+                   void* workspace, size_t workspace_bytes, const int64_t* visited_host, void* mid_event,
+                   bma_stream_t stream);
+
 /* Merge of two partial attention results over disjoint key sets (sequence-sharded
  * execution; no counterpart in the reference, which is single-device):
  *   lse = log(exp(lse_a) + exp(lse_b)),  o = exp(lse_a - lse) o_a + exp(lse_b - lse) o_b,

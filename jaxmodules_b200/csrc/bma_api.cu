@@ -6,6 +6,7 @@
 #include <atomic>
 #include <mutex>
 
+#include "bwd_preprocess.cuh"
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 
@@ -51,79 +52,9 @@ int* device_status_ptr() {
 namespace {
 
 // ---- backward preprocess: delta = rowsum(dO * O), optional bf16 copy of dO ---------------
-__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
-  const float4 x = *reinterpret_cast<const float4*>(p);
-  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-}
-__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
-  const uint2 x = *reinterpret_cast<const uint2*>(p);
-  v[0] = __uint_as_float(x.x << 16); v[1] = __uint_as_float(x.x & 0xffff0000u);
-  v[2] = __uint_as_float(x.y << 16); v[3] = __uint_as_float(x.y & 0xffff0000u);
-}
-
-// Streaming form for d <= 128 with vector accesses: one warp takes FOUR consecutive queries of one
-// (batch, head), issues all eight 16-byte loads per lane before it uses any of them, and writes the four
-// delta values as one 16-byte line, so that the [B, Hq, N] delta array is written in whole sectors
-// (one warp per row wrote 4 bytes per 32-byte sector).  Bound by HBM: reads |O| + |dO|, writes the bf16
-// copy of dO and delta.
 template <typename TO, typename TDO>
-__global__ void __launch_bounds__(256) bwd_preprocess_rows4_kernel(bma_attn_args a, __nv_bfloat16* __restrict__ do_bf16) {
-  const int lane = threadIdx.x & 31;
-  const int warps = (blockDim.x >> 5);
-  const int64_t nq4 = (a.N + 3) / 4;
-  const int64_t units = (int64_t)a.B * a.Hq * nq4;
-  const int c = lane * 4;
-  const bool act = c < a.d;
-  for (int64_t u = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); u < units; u += (int64_t)gridDim.x * warps) {
-    const int q0 = (int)(u % nq4) * 4;
-    const int h = (int)((u / nq4) % a.Hq);
-    const int b = (int)(u / (nq4 * a.Hq));
-    float gv[4][4], ov[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int q = q0 + i;
-      if (act && q < a.N) {
-        load4(static_cast<const TDO*>(a.d_o.ptr) + (int64_t)b * a.d_o.stride_b + (int64_t)q * a.d_o.stride_l + (int64_t)h * a.d_o.stride_h + c, gv[i]);
-        load4(static_cast<const TO*>(a.o.ptr) + (int64_t)b * a.o.stride_b + (int64_t)q * a.o.stride_l + (int64_t)h * a.o.stride_h + c, ov[i]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { gv[i][e] = 0.f; ov[i][e] = 0.f; }
-      }
-    }
-    // With a bf16 copy, delta is taken from the ROUNDED cotangent -- the values the dP = dO V^T product of the backward
-    // kernels sees -- so that dP - delta cancels where it should (a row that attends one key has dS = 0 exactly; with
-    // the float32 cotangent in delta and the bf16 one in dP the difference of the two roundings would survive).
-    float acc[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int q = q0 + i;
-      if (do_bf16) {
-        __nv_bfloat162 lo = __floats2bfloat162_rn(gv[i][0], gv[i][1]), hi = __floats2bfloat162_rn(gv[i][2], gv[i][3]);
-        uint2 w;
-        w.x = *reinterpret_cast<uint32_t*>(&lo);
-        w.y = *reinterpret_cast<uint32_t*>(&hi);
-        gv[i][0] = __uint_as_float(w.x << 16); gv[i][1] = __uint_as_float(w.x & 0xffff0000u);
-        gv[i][2] = __uint_as_float(w.y << 16); gv[i][3] = __uint_as_float(w.y & 0xffff0000u);
-        if (act && q < a.N) *reinterpret_cast<uint2*>(do_bf16 + (((int64_t)b * a.N + q) * a.Hq + h) * a.d + c) = w;
-      }
-      acc[i] = fmaf(gv[i][0], ov[i][0], fmaf(gv[i][1], ov[i][1], fmaf(gv[i][2], ov[i][2], gv[i][3] * ov[i][3])));
-    }
-#pragma unroll
-    for (int off = 16; off; off >>= 1) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
-    }
-    float* dst = a.delta + ((int64_t)b * a.Hq + h) * a.N + q0;
-    if (lane == 0) {
-      if (q0 + 3 < a.N && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        *reinterpret_cast<float4*>(dst) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (q0 + i < a.N) dst[i] = acc[i];
-      }
-    }
-  }
+__global__ void __launch_bounds__(256) bwd_preprocess_rows4_kernel(const bma_attn_args a, __nv_bfloat16* __restrict__ do_bf16) {
+  preprocess_rows4<TO, TDO>(a, do_bf16, blockIdx.x, gridDim.x);
 }
 
 // One warp per (b, q, h) row.  VEC: 4-element vector accesses (d % 4 == 0, 16-byte aligned rows).
@@ -392,10 +323,6 @@ int bma_attn_fwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const
   return f32_fwd(*args, *spec, *lists, workspace, static_cast<cudaStream_t>(stream));
 }
 
-static bool rows_of_16_bytes(const bma_tensor& t) {
-  return (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && t.stride_b % 4 == 0 && t.stride_l % 4 == 0 && t.stride_h % 4 == 0;
-}
-
 static int bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
                    size_t workspace_bytes, bool own_delta, bma_stream_t stream) {
   const size_t need = bma_attn_f32_workspace_bytes(args, 1);
@@ -415,7 +342,7 @@ static int bwd_f32(const bma_attn_args* args, const bma_mask_spec* spec, const b
   BMA_REQUIRE(spec->q_valid <= args->N && spec->k_valid <= args->L, BMA_ERR_ARG);
   BMA_REQUIRE(!room || (reinterpret_cast<uintptr_t>(workspace) & 15) == 0, BMA_ERR_WORKSPACE);
   // delta on the way through dO only where bwd_preprocess_rows4_kernel would take it, whose sums the split kernel repeats
-  if (own_delta && !(room && args->d % 4 == 0 && rows_of_16_bytes(args->o) && rows_of_16_bytes(args->d_o))) {
+  if (own_delta && !(room && preprocess_vectors(*args, nullptr))) {
     own_delta = false;
     if ((rc = bma_attn_bwd_preprocess(args, nullptr, stream))) return rc;
   }
@@ -443,12 +370,10 @@ int bma_attn_bwd_preprocess(const bma_attn_args* args, void* d_o_bf16, bma_strea
   const int grid = (int)std::min<int64_t>((rows + 7) / 8, (int64_t)sm_count() * 16);
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(d_o_bf16);
   const bool of = args->o.dtype == BMA_DTYPE_F32, gf = args->d_o.dtype == BMA_DTYPE_F32;
-  const bool vec = args->d % 4 == 0 && rows_of_16_bytes(args->o) && rows_of_16_bytes(args->d_o) && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
-  const int64_t units4 = (int64_t)args->B * args->Hq * ((args->N + 3) / 4);
-  const int grid4 = (int)std::min<int64_t>((units4 + 7) / 8, (int64_t)sm_count() * 32);
+  const bool vec = preprocess_vectors(*args, out);
 #define BMA_PRE(TO, TDO)                                                                   \
   do {                                                                                     \
-    if (vec && args->d <= 128) bwd_preprocess_rows4_kernel<TO, TDO><<<grid4, 256, 0, st>>>(*args, out); \
+    if (vec && args->d <= 128) bwd_preprocess_rows4_kernel<TO, TDO><<<preprocess_rows4_ctas(*args), 256, 0, st>>>(*args, out); \
     else if (vec) bwd_preprocess_kernel<TO, TDO, true><<<grid, 256, 0, st>>>(*args, out);  \
     else bwd_preprocess_kernel<TO, TDO, false><<<grid, 256, 0, st>>>(*args, out);          \
   } while (0)
@@ -493,8 +418,8 @@ int bma_debug_expire_wait(uint64_t limit_ns, int32_t code, bma_stream_t stream) 
   return BMA_OK;
 }
 
-int bma_attn_bwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
-                 size_t workspace_bytes, const int64_t* visited_host, void* mid_event, bma_stream_t stream) {
+static int bwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+               size_t workspace_bytes, const int64_t* visited_host, void* mid_event, const BwdPreprocess* pre, bma_stream_t stream) {
   cudaEvent_t mark = static_cast<cudaEvent_t>(mid_event);
   int rc = validate_common(args);
   if (rc != BMA_OK) return rc;
@@ -517,9 +442,31 @@ int bma_attn_bwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma
   if (be == BMA_BACKEND_TCGEN05) {
     const size_t need = sm100_bwd_workspace_bytes(*args);
     BMA_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), BMA_ERR_WORKSPACE);
-    return sm100_bwd(*args, *spec, *lists, workspace, workspace_bytes, visited_host, mark, st);
+    return sm100_bwd(*args, *spec, *lists, workspace, workspace_bytes, visited_host, mark, pre, st);
   }
+  if (pre && (rc = bma_attn_bwd_preprocess(&pre->a, pre->out, stream))) return rc;
   return simt_bwd(*args, *spec, *lists, st);
+}
+
+int bma_attn_bwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+                 size_t workspace_bytes, const int64_t* visited_host, void* mid_event, bma_stream_t stream) {
+  return bwd(args, spec, lists, workspace, workspace_bytes, visited_host, mid_event, nullptr, stream);
+}
+
+int bma_attn_bwd_o(const bma_attn_args* args, void* d_o_bf16, const bma_mask_spec* spec, const bma_block_lists* lists, void* workspace,
+                   size_t workspace_bytes, const int64_t* visited_host, void* mid_event, bma_stream_t stream) {
+  int rc = validate_common(args);
+  if (rc != BMA_OK) return rc;
+  if ((rc = validate_tensor(args->o, true)) || (rc = validate_tensor(args->d_o, true))) return rc;
+  BMA_REQUIRE(args->delta != nullptr, BMA_ERR_ARG);
+  BwdPreprocess pre{*args, static_cast<__nv_bfloat16*>(d_o_bf16)};
+  bma_attn_args a = *args;
+  if (d_o_bf16) {   // the dense copy that the pass then reads
+    a.d_o.ptr = d_o_bf16;
+    a.d_o.dtype = BMA_DTYPE_BF16;
+    a.d_o.stride_h = a.d; a.d_o.stride_l = (int64_t)a.Hq * a.d; a.d_o.stride_b = (int64_t)a.N * a.Hq * a.d;
+  }
+  return bwd(&a, spec, lists, workspace, workspace_bytes, visited_host, mid_event, &pre, stream);
 }
 
 int bma_attn_merge(const bma_attn_args* args, bma_stream_t stream) {

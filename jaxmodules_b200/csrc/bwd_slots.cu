@@ -12,6 +12,7 @@
 // One small launch per backward call (two with many list heads) builds the tables from the kv-side lists into the front of the caller's workspace.
 #include <algorithm>
 
+#include "bwd_preprocess.cuh"
 #include "common.cuh"
 
 namespace bma {
@@ -46,14 +47,14 @@ __device__ __forceinline__ long long block_sum256(long long v, long long* part) 
 //   the last CTA: head_base[i], i in [0, B * Hq] = exclusive prefix over (b, h) of the list heads' totals.
 // (A row base counts list entries; a block listed twice leaves an unused slot behind.)
 enum SlotPhase { ALL, ROWS, HEADS };
-__global__ void __launch_bounds__(256) slot_tables_kernel(SlotPhase phase, bma_block_lists l, int B, int Hq, int32_t* __restrict__ rank,
-                                                          int32_t* __restrict__ row_base, int64_t* __restrict__ head_total,
-                                                          int64_t* __restrict__ head_base) {
+__device__ __forceinline__ void slot_tables(SlotPhase phase, const bma_block_lists& l, int B, int Hq, int32_t* __restrict__ rank,
+                                            int32_t* __restrict__ row_base, int64_t* __restrict__ head_total,
+                                            int64_t* __restrict__ head_base, int cta, int ctas) {
   __shared__ uint32_t bits[8][kMaxKvTilesBwd / 32];
   __shared__ long long part[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int groups = (l.NQ + 7) / 8;
-  if (phase == HEADS || (phase == ALL && blockIdx.x == gridDim.x - 1)) {
+  if (phase == HEADS || (phase == ALL && cta == ctas - 1)) {
     const int LHEADS = phase == HEADS ? 0 : l.B * l.H;
     for (int i = w; i < LHEADS; i += 8) {   // one warp per list head
       long long s = 0;
@@ -91,8 +92,8 @@ __global__ void __launch_bounds__(256) slot_tables_kernel(SlotPhase phase, bma_b
     if (threadIdx.x == 0) head_base[n] = carry;
     return;
   }
-  const int64_t head_row = (int64_t)(blockIdx.x / groups) * l.NQ;
-  const int first = (int)(blockIdx.x % groups) * 8;
+  const int64_t head_row = (int64_t)(cta / groups) * l.NQ;
+  const int first = (cta % groups) * 8;
   long long s = 0;
   for (int r = threadIdx.x; r < first; r += 256) s += row_visits(l, head_row + r);
   const int before = (int)block_sum256(s, part);
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(256) slot_tables_kernel(SlotPhase phase, bma_b
     int mine = before;
     for (int i = first; i < r; ++i) mine += row_visits(l, head_row + i);
     row_base[row] = mine;
-    if (phase == ROWS && r == l.NQ - 1) head_total[blockIdx.x / groups] = mine + row_visits(l, row);
+    if (phase == ROWS && r == l.NQ - 1) head_total[cta / groups] = mine + row_visits(l, row);
   }
   const int words = (l.NKV + 31) / 32;
   bits[w][lane] = 0u;
@@ -135,6 +136,18 @@ __global__ void __launch_bounds__(256) slot_tables_kernel(SlotPhase phase, bma_b
     const int j = word * 32 + lane;
     if (j < l.NKV) out[j] = (bw >> lane) & 1u ? start + __popc(bw & ((1u << lane) - 1u)) : -1;
   }
+}
+
+__global__ void __launch_bounds__(256) slot_tables_kernel(SlotPhase phase, const bma_block_lists l, int B, int Hq, const SlotTables t) {
+  slot_tables(phase, l, B, Hq, t.rank, t.row_base, t.head_total, t.head_base, blockIdx.x, gridDim.x);
+}
+// The tables by the first `ctas` CTAs, delta and the bf16 copy of the cotangent by the others: both come before the dK/dV kernel and neither
+// needs the other.  A launch less: 4.6 us of the host and 4 of the device (2 x 1000 tokens, lambda window, 16/4 heads: the call 161 -> 154 us).
+template <typename TO, typename TDO>
+__global__ void __launch_bounds__(256) slots_and_preprocess_kernel(const bma_block_lists l, int B, int Hq, const SlotTables t, int ctas,
+                                                                   const bma_attn_args a, __nv_bfloat16* __restrict__ do_bf16) {
+  if ((int)blockIdx.x < ctas) slot_tables(ALL, l, B, Hq, t.rank, t.row_base, t.head_total, t.head_base, blockIdx.x, ctas);
+  else preprocess_rows4<TO, TDO>(a, do_bf16, (int)blockIdx.x - ctas, (int)gridDim.x - ctas);
 }
 
 // visited[b', h'] = sum over the rows of a list head of (kv_num + full_kv_num)
@@ -174,13 +187,29 @@ SlotTables slot_tables_layout(const bma_attn_args& a, const bma_block_lists& l, 
   return t;
 }
 
-int slot_tables_build(const bma_attn_args& a, const bma_block_lists& l, const SlotTables& t, cudaStream_t st) {
+int slot_tables_build(const bma_attn_args& a, const bma_block_lists& l, const SlotTables& t, const BwdPreprocess* pre, cudaStream_t st) {
   BMA_REQUIRE(l.NKV <= kMaxKvTilesBwd, BMA_ERR_LIMIT);
   const int64_t ctas = (int64_t)l.B * l.H * ((l.NQ + 7) / 8) + 1;
   BMA_REQUIRE(ctas <= INT32_MAX, BMA_ERR_LIMIT);
   const bool one = (int64_t)l.B * l.H <= kHeadsInOneLaunch;
-  slot_tables_kernel<<<(unsigned)(one ? ctas : ctas - 1), 256, 0, st>>>(one ? ALL : ROWS, l, a.B, a.Hq, t.rank, t.row_base, t.head_total, t.head_base);
-  if (!one) slot_tables_kernel<<<1, 256, 0, st>>>(HEADS, l, a.B, a.Hq, t.rank, t.row_base, t.head_total, t.head_base);
+  if (pre && one && a.d <= 128 && preprocess_vectors(pre->a, pre->out)) {
+    const unsigned grid = (unsigned)(ctas + preprocess_rows4_ctas(pre->a));
+    const bool of = pre->a.o.dtype == BMA_DTYPE_F32, gf = pre->a.d_o.dtype == BMA_DTYPE_F32;
+    auto launch = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(l, a.B, a.Hq, t, (int)ctas, pre->a, pre->out); };
+    if (of && gf) launch(slots_and_preprocess_kernel<float, float>);
+    else if (of) launch(slots_and_preprocess_kernel<float, __nv_bfloat16>);
+    else if (gf) launch(slots_and_preprocess_kernel<__nv_bfloat16, float>);
+    else launch(slots_and_preprocess_kernel<__nv_bfloat16, __nv_bfloat16>);
+    count_launches(1);
+    BMA_CUDA_TRY(cudaGetLastError());
+    return BMA_OK;
+  }
+  if (pre) {
+    const int rc = bma_attn_bwd_preprocess(&pre->a, pre->out, st);
+    if (rc) return rc;
+  }
+  slot_tables_kernel<<<(unsigned)(one ? ctas : ctas - 1), 256, 0, st>>>(one ? ALL : ROWS, l, a.B, a.Hq, t);
+  if (!one) slot_tables_kernel<<<1, 256, 0, st>>>(HEADS, l, a.B, a.Hq, t);
   count_launches(one ? 1 : 2);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;

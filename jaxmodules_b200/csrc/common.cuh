@@ -472,8 +472,9 @@ int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
               cudaStream_t st);
 size_t sm100_fwd_workspace_bytes(const bma_attn_args& a, const bma_block_lists& lists);
 bool sm100_fwd_wants_lists(const bma_attn_args& a, const bma_mask_spec& spec);
+struct BwdPreprocess;
 int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws,
-              size_t ws_bytes, const int64_t* visited_host, cudaEvent_t mark, cudaStream_t st);
+              size_t ws_bytes, const int64_t* visited_host, cudaEvent_t mark, const BwdPreprocess* pre, cudaStream_t st);
 size_t sm100_bwd_workspace_bytes(const bma_attn_args& a);
 size_t sm100_bwd_scratch_bytes(const bma_attn_args& a, const bma_block_lists& lists, const int64_t* visited_host);
 size_t sm100_bwd_scratch_min_bytes(const bma_attn_args& a, const bma_block_lists& lists, const int64_t* visited_host);
@@ -487,6 +488,11 @@ bool sm100_supported(const bma_attn_args& a);
 bool sm100_bwd_supported(const bma_attn_args& a);
 
 // Compact slot addressing of the backward scratch (bwd_slots.cu): tables at the front of the workspace.
+// The preprocess that a backward pass has still to run: the arguments with the cotangent as it came, and the bf16 copy to write (or null)
+struct BwdPreprocess {
+  bma_attn_args a;
+  __nv_bfloat16* out;
+};
 struct SlotTables {
   int64_t* head_base;   // [B*Hq + 1] exclusive prefix of visited blocks over (b, h), row-major
   int64_t* head_total;  // [lists.B * lists.H]
@@ -495,7 +501,8 @@ struct SlotTables {
   size_t bytes;         // size of the tables (a multiple of 1024); the slots follow
 };
 SlotTables slot_tables_layout(const bma_attn_args& a, const bma_block_lists& l, void* ws);
-int slot_tables_build(const bma_attn_args& a, const bma_block_lists& l, const SlotTables& t, cudaStream_t st);
+// With `pre`: the preprocess too, in the same launch where that can be.
+int slot_tables_build(const bma_attn_args& a, const bma_block_lists& l, const SlotTables& t, const BwdPreprocess* pre, cudaStream_t st);
 int block_lists_visited(const bma_block_lists& l, int64_t* visited, cudaStream_t st);
 
 constexpr int kSimtTile = 64;

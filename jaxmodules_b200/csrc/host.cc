@@ -28,7 +28,7 @@ using OptTensor = std::optional<Tensor>;
 #define BMA_FUNCTIONS(X)                                                                                                      \
   X(bma_mask_compile_workspace_bytes) X(bma_mask_compile) X(bma_attn_plan) X(bma_attn_bwd_plan) X(bma_attn_fwd_implies_lists) X(bma_attn_fwd_workspace_bytes) \
   X(bma_attn_fwd_ws) X(bma_attn_f32_workspace_bytes) X(bma_attn_fwd_f32) X(bma_attn_bwd_f32) X(bma_attn_bwd_f32_o) X(bma_attn_bwd_preprocess)       \
-  X(bma_attn_bwd_workspace_bytes) X(bma_attn_bwd_scratch_bytes) X(bma_attn_bwd_scratch_min_bytes) X(bma_attn_bwd)
+  X(bma_attn_bwd_workspace_bytes) X(bma_attn_bwd_scratch_bytes) X(bma_attn_bwd_scratch_min_bytes) X(bma_attn_bwd) X(bma_attn_bwd_o)
 struct Library {
 #define X(name) decltype(&::name) name = nullptr;
   BMA_FUNCTIONS(X)
@@ -228,7 +228,7 @@ std::tuple<size_t, size_t, size_t> backward_bytes(const Tensor& q, const Tensor&
           counts ? lib.bma_attn_bwd_scratch_min_bytes(&a, lists, counts) : 0};
 }
 
-// `delta` may be left out where the float32 kernels run: they take it themselves.
+// Where `delta` is left out the pass takes it itself, from `d_o` as it came.
 std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o,
                                             OptTensor delta, const OptTensor& key_bias, std::optional<double> scale, int backend, uintptr_t spec_at,
                                             uintptr_t lists_at, size_t f32_bytes, const OptTensor& workspace, size_t ws_bytes, uintptr_t visited,
@@ -238,7 +238,9 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q, const Tensor& k, co
   const bma_block_lists* lists = at_address<bma_block_lists>(lists_at);
   Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
   a.o = describe(o); a.d_o = describe(d_o);
-  const bool own_delta = f32_bytes && !delta;
+  const bool own_delta = !delta;
+  Tensor copy;
+  if (own_delta && !f32_bytes && d_o.scalar_type() != at::kBFloat16) copy = at::empty({a.B, a.N, a.Hq, a.d}, q.options().dtype(at::kBFloat16).requires_grad(false));
   if (own_delta) delta = at::empty({a.B, a.Hq, a.N}, q.options().dtype(at::kFloat).requires_grad(false));
   a.lse = lse.data_ptr<float>(); a.delta = delta->data_ptr<float>();
   a.dq = describe(dq); a.dk = describe(dk); a.dv = describe(dv);
@@ -253,6 +255,8 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q, const Tensor& k, co
     Group group("bma.bwd");
     const bma_stream_t st = reinterpret_cast<bma_stream_t>(stream);
     if (f32_bytes) rc = (own_delta ? lib.bma_attn_bwd_f32_o : lib.bma_attn_bwd_f32)(&a, spec, lists, ws, ws ? f32_bytes : 0, st);
+    else if (own_delta)
+      rc = lib.bma_attn_bwd_o(&a, copy.defined() ? copy.data_ptr() : nullptr, spec, lists, ws, ws_bytes, at_address<const int64_t>(visited), at_address<void>(mid_event), st);
     else rc = lib.bma_attn_bwd(&a, spec, lists, ws, ws_bytes, at_address<const int64_t>(visited), at_address<void>(mid_event), st);
   }
   check(rc, f32_bytes ? "bma_attn_bwd_f32" : "bma_attn_bwd");
