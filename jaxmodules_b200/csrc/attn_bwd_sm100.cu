@@ -136,8 +136,8 @@ __device__ __noinline__ void sum_parts(const float* stage, const BwdParams& p, i
   }
 }
 
-// SHARED: the CTAs of a cluster share a kv tile's walk.
-template <int HD, bool KB, bool SHARED>
+// SHARED: the CTAs of a cluster share a kv tile's walk.  BY_RANK: order of the CTAs of the others, see longest_first.
+template <int HD, bool KB, bool SHARED, bool BY_RANK = false>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -149,7 +149,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const bma_attn_args& a = p.a;
   int kj, hk, b;   // (under a causal mask kv tile 0 sees the most q tiles)
   if constexpr (SHARED) cta_of_cluster(p.by_rank, kj, hk, b);
-  else cta_of(p.by_rank, kj, hk, b);
+  else cta_of<BY_RANK>(kj, hk, b);
   hk += p.hk0;
   b += p.b0;
   const int G = a.Hq / a.Hkv;
@@ -587,10 +587,10 @@ static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUte
   p.b0 = b0; p.hk0 = hk0; p.nhk = nhk;
   p.by_rank = longest_first(ceil_div(a.L, BT), nhk, nb, (int64_t)4 * a.N * a.d * (a.Hq / a.Hkv));
   int rc;
-  auto launch = [&](auto kernel, auto shared, size_t smem) -> int {
+  auto launch = [&](auto by_head, auto by_rank, auto shared, size_t smem) -> int {
     static ClusterCounts known[2];
     p.parts = share_walks(walks, 6.0, kMaxParts, [&](int parts) { return clusters_at_once(known[a.d == 128], shared, kThreads, smem, parts); });
-    if (p.parts > 1) kernel = shared;
+    const auto kernel = p.parts > 1 ? shared : p.by_rank ? by_rank : by_head;
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = cta_grid(p.by_rank, ceil_div(a.L, BT), nhk, nb, p.parts);
@@ -602,10 +602,10 @@ static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUte
     BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, mdo, mdk, mdv, static_cast<const BwdParams&>(p)));
     return BMA_OK;
   };
-  if (a.d == 128) rc = a.key_bias ? launch(bwd_dkdv_kernel<128, true, false>, bwd_dkdv_kernel<128, true, true>, sizeof(BwdSmem<128>))
-                                  : launch(bwd_dkdv_kernel<128, false, false>, bwd_dkdv_kernel<128, false, true>, sizeof(BwdSmem<128>));
-  else rc = a.key_bias ? launch(bwd_dkdv_kernel<64, true, false>, bwd_dkdv_kernel<64, true, true>, sizeof(BwdSmem<64>))
-                       : launch(bwd_dkdv_kernel<64, false, false>, bwd_dkdv_kernel<64, false, true>, sizeof(BwdSmem<64>));
+  if (a.d == 128) rc = a.key_bias ? launch(bwd_dkdv_kernel<128, true, false>, bwd_dkdv_kernel<128, true, false, true>, bwd_dkdv_kernel<128, true, true>, sizeof(BwdSmem<128>))
+                                  : launch(bwd_dkdv_kernel<128, false, false>, bwd_dkdv_kernel<128, false, false, true>, bwd_dkdv_kernel<128, false, true>, sizeof(BwdSmem<128>));
+  else rc = a.key_bias ? launch(bwd_dkdv_kernel<64, true, false>, bwd_dkdv_kernel<64, true, false, true>, bwd_dkdv_kernel<64, true, true>, sizeof(BwdSmem<64>))
+                       : launch(bwd_dkdv_kernel<64, false, false>, bwd_dkdv_kernel<64, false, false, true>, bwd_dkdv_kernel<64, false, true>, sizeof(BwdSmem<64>));
   if (rc) return rc;
   count_launches(1);
   BMA_CUDA_TRY(cudaGetLastError());

@@ -78,7 +78,6 @@ struct FwdParams {
   bma_mask_spec spec;
   bma_block_lists l;
   int pairs;       // ceil(query tiles / 2), one CTA each
-  bool by_rank;    // order of the CTAs, see cta_of
   float scale_log2;
   int* status;
 };
@@ -172,17 +171,24 @@ __device__ __forceinline__ float exp_part(const float* s, float sc, float m_sub,
 // into the scores BEFORE the running maximum is taken.  Compiled in only where it is needed: a key bias, or a
 // negative scale, for which max(raw score) * scale is the MINIMUM of the scaled scores and the exponentials
 // taken against it would overflow.
-template <int HD, bool KB>
+// The classes of a q tile's blocks where a call has no lists.  A function of its own: inlined, it costs the loop of the d = 64 kernel
+// registers (444 us, against 433, of B=4 L=4096 H=32/8 causal with lists).
+__device__ __noinline__ void implied_classes(const bma_mask_spec& spec, int qi, int n, uint8_t* cls) {
+  for (int i = threadIdx.x; i < n; i += kThreads) cls[i] = (uint8_t)interval_class(spec, qi, i, BM, BN);
+}
+
+// BY_RANK: order of the CTAs, see longest_first.
+template <int HD, bool KB, bool BY_RANK>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-           const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, const FwdParams p) {
+           const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, const __grid_constant__ FwdParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr uint32_t kTileBytes = kTileBytesOf<HD>;
   FwdSmem<HD>& sm = *reinterpret_cast<FwdSmem<HD>*>(smem_raw);
 
   const bma_attn_args& a = p.a;
   int pair, h, b;
-  cta_of(p.by_rank, pair, h, b);
+  cta_of<BY_RANK>(pair, h, b);
   pair = p.pairs - 1 - pair;   // the last pair of a causal mask has the longest walk
   const int hk = h / (a.Hq / a.Hkv);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // provably warp-uniform
@@ -219,7 +225,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     const int qi = pair * 2 + x;
     if (qi >= NQ) break;
     if (!p.l.kv_num) {   // no lists: a mask of interval terms, whose blocks are known from the indices
-      for (int i = threadIdx.x; i < NKV; i += kThreads) sm.cls[x][i] = (uint8_t)interval_class(p.spec, qi, i, BM, BN);
+      implied_classes(p.spec, qi, NKV, sm.cls[x]);
       continue;
     }
     const int64_t lrow = ((int64_t)lb * p.l.H + lh) * NQ + qi;
@@ -1761,15 +1767,16 @@ int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
     return BMA_OK;
   }
   p.pairs = ceil_div(ceil_div(a.N, BM), 2);
-  p.by_rank = longest_first(p.pairs, a.Hq, a.B, (int64_t)4 * a.L * a.d * a.Hkv / a.Hq);
-  const dim3 grid = cta_grid(p.by_rank, p.pairs, a.Hq, a.B);
-  auto launch = [&](auto kernel, size_t smem) -> int {
+  const bool by_rank = longest_first(p.pairs, a.Hq, a.B, (int64_t)4 * a.L * a.d * a.Hkv / a.Hq);
+  const dim3 grid = cta_grid(by_rank, p.pairs, a.Hq, a.B);
+  auto launch = [&](auto by_head, auto ranked, size_t smem) -> int {
+    const auto kernel = by_rank ? ranked : by_head;
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<grid, kThreads, smem, st>>>(mq, mk, mv, mo, p);
     return BMA_OK;
   };
-  if (a.d == 128) rc = kb ? launch(fwd_kernel<128, true>, sizeof(FwdSmem<128>)) : launch(fwd_kernel<128, false>, sizeof(FwdSmem<128>));
-  else rc = kb ? launch(fwd_kernel<64, true>, sizeof(FwdSmem<64>)) : launch(fwd_kernel<64, false>, sizeof(FwdSmem<64>));
+  if (a.d == 128) rc = kb ? launch(fwd_kernel<128, true, false>, fwd_kernel<128, true, true>, sizeof(FwdSmem<128>)) : launch(fwd_kernel<128, false, false>, fwd_kernel<128, false, true>, sizeof(FwdSmem<128>));
+  else rc = kb ? launch(fwd_kernel<64, true, false>, fwd_kernel<64, true, true>, sizeof(FwdSmem<64>)) : launch(fwd_kernel<64, false, false>, fwd_kernel<64, false, true>, sizeof(FwdSmem<64>));
   if (rc) return rc;
   count_launches(1);
   BMA_CUDA_TRY(cudaGetLastError());

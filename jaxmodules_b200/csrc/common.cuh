@@ -120,6 +120,14 @@ __device__ __forceinline__ void cta_of(bool by_rank, int& rank, int& head, int& 
   head = by_rank ? blockIdx.x : blockIdx.y;
   batch = by_rank ? blockIdx.y : blockIdx.z;
 }
+// With the order known to the compiler: the selects above cost the loops of the d = 64 kernels registers, 1.5 and 3.5 % (B=4 L=4096 H=32/8
+// causal, dK/dV 825 -> 838 us, forward 433 -> 448).
+template <bool BY_RANK>
+__device__ __forceinline__ void cta_of(int& rank, int& head, int& batch) {
+  rank = BY_RANK ? blockIdx.z : blockIdx.x;
+  head = BY_RANK ? blockIdx.x : blockIdx.y;
+  batch = BY_RANK ? blockIdx.y : blockIdx.z;
+}
 __device__ __forceinline__ void cta_of_cluster(bool by_rank, int& rank, int& head, int& batch) {   // the same for a launch in clusters (or not)
   const dim3 id = __clusterIdx();
   rank = by_rank ? id.z : id.x;
