@@ -12,7 +12,7 @@
 // dQ, dK and dV are summed over the tiles in registers, with rounded FP32 adds.  Against float64 the 2-norm error is 1.4e-7 - 3.5e-7 (causal, B=2 L=2048 H=16 d=64; the FP32 tile
 // kernels: 4.1e-7 - 8.5e-7).
 //
-// Measured there: forward 134 us (tile kernels 861), dK/dV 218 (1383), dQ 158 (1357), the two splits 21 each; forward with
+// Measured there: forward 110 us (tile kernels 861), dK/dV 171 (1383), dQ 133 (1357), the two splits 21 each; forward with
 // d=128, N=L=1500, 16 heads: 134 us (1139).
 //
 // One split kernel writes the planes of Q, K, V (and dO) into the caller's workspace as [3, B, L, H, DP] bf16, DP = 64 or
