@@ -380,7 +380,7 @@ def _float32_planes(dev: torch.device, nbytes: int) -> Optional[torch.Tensor]:
 
 def _backward_scratch(dev: torch.device, nbytes: int) -> torch.Tensor:
     # keyed by stream too: two backward passes in flight on different streams must not share slots
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(), nat.stream(dev))
+    key = (nat.device_index(dev), nat.stream(dev))
     buf = _scratch_buffers.get(key)
     if buf is None or buf.numel() < nbytes:
         _scratch_buffers.pop(key, None)   # drop the old buffer before asking for the larger one

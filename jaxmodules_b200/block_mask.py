@@ -255,11 +255,12 @@ def compile_block_lists(dmask: "_masks.DeviceMask", B: int, H: int, N: int, L: i
     LB = out_B if out_B is not None else (B if dmask.depends_b else 1)
     LH = out_H if out_H is not None else (H if dmask.depends_h else 1)
     device = torch.device(device)
+    index = nat.device_index(device)
     lists = nat.BlockLists(LB, LH, NQ, NKV, q_block, kv_block)
     arrays = nat.host().compile_lists(
         C.addressof(dmask.spec), C.addressof(lists), B, H, q_side, views, nat.BMA_MASK_COMPILE_CONSERVATIVE if conservative else 0,
         NQ * q_block if floor_blocks else _ANY, NKV * kv_block if floor_blocks else _ANY,
-        torch.cuda.current_device() if device.index is None else device.index, nat.stream(device) if stream is None else stream)
+        index, nat.stream(device) if stream is None else stream)
     if not views:
         return lists, dict(_buffer=arrays[0])
     if not q_side:
