@@ -168,7 +168,8 @@ int validate_lists(const bma_attn_args* a, const bma_block_lists* l, int tile, b
   BMA_REQUIRE(l != nullptr, BMA_ERR_ARG);
   const bool none = !l->kv_num && !l->kv_idx && !l->full_kv_num && !l->full_kv_idx &&
                     (!need_q_side || (!l->q_num && !l->q_idx && !l->full_q_num && !l->full_q_idx && l->B == 1 && l->H == 1));
-  BMA_REQUIRE((l->kv_num && l->kv_idx && l->full_kv_num && l->full_kv_idx) || (none && implied && !(implied->flags & kTableTerms)), BMA_ERR_ARG);
+  BMA_REQUIRE((l->kv_num && l->kv_idx && l->full_kv_num && l->full_kv_idx) || (none && implied && !(implied->flags & kTableTerms) && interval_terms_valid(*implied)),
+              BMA_ERR_ARG);
   BMA_REQUIRE(!need_q_side || none || (l->q_num && l->q_idx && l->full_q_num && l->full_q_idx), BMA_ERR_ARG);
   BMA_REQUIRE(l->q_block == tile && l->kv_block == tile, BMA_ERR_ARG);
   BMA_REQUIRE(l->NQ == ceil_div(a->N, tile) && l->NKV == ceil_div(a->L, tile), BMA_ERR_ARG);
@@ -273,7 +274,7 @@ size_t bma_attn_fwd_workspace_bytes(const bma_attn_args* args, const bma_block_l
 }
 
 int32_t bma_attn_fwd_implies_lists(const bma_attn_args* args, const bma_mask_spec* spec) {
-  if (validate_common(args) != BMA_OK || !spec || (spec->flags & kTableTerms)) return 0;
+  if (validate_common(args) != BMA_OK || !spec || (spec->flags & kTableTerms) || !interval_terms_valid(*spec)) return 0;
   if (bma_attn_f32_workspace_bytes(args, 0)) return 1;
   return pick_backend(args) == BMA_BACKEND_TCGEN05 && !sm100_fwd_wants_lists(*args, *spec);
 }

@@ -156,6 +156,13 @@ inline unsigned launch_ctas(const LaunchOrder& o) { return (unsigned)(o.tiles * 
 // Terms of the mask that are looked up (segment ids, bit table, tile bits) rather than computed from the indices.
 constexpr int kTableTerms = BMA_MASK_SEGMENT | BMA_MASK_BITMAP | BMA_MASK_TILES;
 
+// What the interval terms of a mask have to satisfy, for lists to be compiled from them or for a pass to know its blocks without lists.
+inline bool interval_terms_valid(const bma_mask_spec& s) {
+  if (s.q_valid < 0 || s.k_valid < 0) return false;
+  if ((s.flags & BMA_MASK_BLOCK_WINDOW) && !(s.win_block > 0 && s.win_left >= 0 && s.win_right >= 0 && (int64_t)s.win_left + s.win_right <= s.win_nblk)) return false;
+  return !(s.flags & BMA_MASK_BAND) || (s.band_left >= 0 && s.band_right >= 0);
+}
+
 // ---- mask predicate --------------------------------------------------------------------
 // Device copy of bma_mask_spec with the per-(b,h) row pointers resolved once per CTA.
 struct MaskView {

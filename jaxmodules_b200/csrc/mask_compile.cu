@@ -383,7 +383,7 @@ int mask_compile_validate(const bma_mask_spec& s, int B, int H, const bma_block_
   const bool all_q = l.q_num && l.q_idx && l.full_q_num && l.full_q_idx;
   BMA_REQUIRE(!any_q || all_q, BMA_ERR_ARG);
   BMA_REQUIRE((l.B == B || (l.B == 1 && !depends_on_b(s))) && (l.H == H || (l.H == 1 && !depends_on_h(s))), BMA_ERR_ARG);
-  BMA_REQUIRE(s.q_valid >= 0 && s.k_valid >= 0, BMA_ERR_ARG);
+  BMA_REQUIRE(interval_terms_valid(s), BMA_ERR_ARG);
   BMA_REQUIRE((int64_t)l.NQ * l.q_block >= s.q_valid && (int64_t)l.NKV * l.kv_block >= s.k_valid, BMA_ERR_ARG);
   if (s.flags & BMA_MASK_SEGMENT) BMA_REQUIRE(s.seg_q && s.seg_k, BMA_ERR_ARG);
   if (s.flags & BMA_MASK_BITMAP)
@@ -393,10 +393,6 @@ int mask_compile_validate(const bma_mask_spec& s, int B, int H, const bma_block_
     BMA_REQUIRE((int64_t)s.tiles_q * 128 >= (int64_t)s.q_valid + s.q_offset && (int64_t)s.tiles_k * 128 >= (int64_t)s.k_valid + s.k_offset,
                 BMA_ERR_ARG);
   }
-  if (s.flags & BMA_MASK_BLOCK_WINDOW)
-    BMA_REQUIRE(s.win_block > 0 && s.win_left >= 0 && s.win_right >= 0 && s.win_left + s.win_right <= s.win_nblk,
-                BMA_ERR_ARG);
-  if (s.flags & BMA_MASK_BAND) BMA_REQUIRE(s.band_left >= 0 && s.band_right >= 0, BMA_ERR_ARG);
   BMA_REQUIRE(l.NQ <= kMaxRowWidth && l.NKV <= kMaxRowWidth, BMA_ERR_LIMIT);
   return BMA_OK;
 }
