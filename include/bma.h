@@ -268,6 +268,10 @@ int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec,
  * are accepted for every such mask on the tensor-core kernels. */
 int32_t bma_attn_fwd_implies_lists(const bma_attn_args* args, const bma_mask_spec* spec);
 
+/* What passes given lists without arrays take block (qi, kj) of q_block x kv_block elements for: 0 empty, 1 partial, 2 full, by its elements, as
+ * in the lists that bma_mask_compile makes of the mask; -1 where the mask has other than interval terms or is not valid.  Runs on the host. */
+int32_t bma_mask_block_class(const bma_mask_spec* spec, int32_t q_block, int32_t kv_block, int32_t qi, int32_t kj);
+
 /* The same with a workspace (16-byte aligned), which lets few queries against many keys spread over the whole chip: partial
  * results of runs of keys are combined through it.  bma_attn_fwd_workspace_bytes is 0 where none is used; with less than
  * that bma_attn_fwd_ws runs as bma_attn_fwd does.  (Up to eight runs meet in the shared memory of a cluster of CTAs instead, on

@@ -107,6 +107,7 @@ SIGNATURES = {
     "bma_attn_plan": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "bma_attn_bwd_plan": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "bma_attn_fwd_implies_lists": (C.c_int32, [C.POINTER(AttnArgs), C.POINTER(MaskSpec)]),
+    "bma_mask_block_class": (C.c_int32, [C.POINTER(MaskSpec), C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "bma_attn_fwd": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p]),
     "bma_attn_fwd_workspace_bytes": (C.c_size_t, [C.POINTER(AttnArgs), C.POINTER(BlockLists)]),
     "bma_attn_fwd_ws": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t, C.c_void_p]),

@@ -279,6 +279,11 @@ int32_t bma_attn_fwd_implies_lists(const bma_attn_args* args, const bma_mask_spe
   return pick_backend(args) == BMA_BACKEND_TCGEN05 && !sm100_fwd_wants_lists(*args, *spec);
 }
 
+int32_t bma_mask_block_class(const bma_mask_spec* spec, int32_t q_block, int32_t kv_block, int32_t qi, int32_t kj) {
+  if (!spec || (spec->flags & kTableTerms) || !interval_terms_valid(*spec) || q_block <= 0 || kv_block <= 0 || qi < 0 || kj < 0) return -1;
+  return interval_class(*spec, qi, kj, q_block, kv_block);
+}
+
 int bma_attn_fwd(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
                  bma_stream_t stream) {
   return bma_attn_fwd_ws(args, spec, lists, nullptr, 0, stream);
