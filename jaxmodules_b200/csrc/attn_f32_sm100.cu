@@ -553,7 +553,8 @@ struct __align__(1024) FwdSmem {
 
 static_assert(fwd_smem<4>() <= sizeof(FwdSmem<64>) && fwd_smem<8>() <= sizeof(FwdSmem<128>), "a tile is done again in the same shared memory");
 
-// KB: with a key bias, or a negative scale (for which the maximum of the scores is not that of the scaled ones).
+// KB: with a key bias, or a scale that is not positive: for a negative one the maximum of the scores is not that of the scaled ones, and a scale of 0
+// would make a NaN of a score that the mask has set to -inf before it is scaled (its tile would be done again with FP32 arithmetic).
 template <int DP, bool KB>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -2216,7 +2217,7 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     const int r = run(0, items - share.last, share.parts);
     return r || !share.last ? r : run(items - share.last, share.last, share.last_parts);
   };
-  if (a.key_bias || a.scale < 0.f) rc = dp == 64 ? launch(f32_fwd_kernel<64, true>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, true>, sizeof(FwdSmem<128>));
+  if (a.key_bias || !(a.scale > 0.f)) rc = dp == 64 ? launch(f32_fwd_kernel<64, true>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, true>, sizeof(FwdSmem<128>));
   else rc = dp == 64 ? launch(f32_fwd_kernel<64, false>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, false>, sizeof(FwdSmem<128>));
   if (rc) return rc;
   BMA_CUDA_TRY(cudaGetLastError());
