@@ -167,16 +167,16 @@ __device__ __forceinline__ float exp_part(const float* s, float sc, float m_sub,
 #endif
 }
 
-// KB: the variant that folds the scale (and the per-head key bias, bma_attn_args.key_bias, when there is one)
-// into the scores BEFORE the running maximum is taken.  Compiled in only where it is needed: a key bias, or a
-// negative scale, for which max(raw score) * scale is the MINIMUM of the scaled scores and the exponentials
-// taken against it would overflow.
 // The classes of a q tile's blocks where a call has no lists.  A function of its own: inlined, it costs the loop of the d = 64 kernel
 // registers (444 us, against 433, of B=4 L=4096 H=32/8 causal with lists).
 __device__ __noinline__ void implied_classes(const bma_mask_spec& spec, int qi, int n, uint8_t* cls) {
   for (int i = threadIdx.x; i < n; i += kThreads) cls[i] = (uint8_t)interval_class(spec, qi, i, BM, BN);
 }
 
+// KB: the variant that folds the scale (and the per-head key bias, bma_attn_args.key_bias, when there is one)
+// into the scores BEFORE the running maximum is taken.  Compiled in only where it is needed: a key bias, a
+// negative scale, for which max(raw score) * scale is the MINIMUM of the scaled scores and the exponentials
+// taken against it would overflow, or a scale of 0, which would make NaN of the masked scores (-inf).
 // BY_RANK: order of the CTAs, see longest_first.
 template <int HD, bool KB, bool BY_RANK>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -1735,7 +1735,7 @@ int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   p.scale_log2 = a.scale * kLog2e;
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
-  const bool kb = a.key_bias != nullptr || a.scale < 0.f;
+  const bool kb = a.key_bias != nullptr || !(a.scale > 0.f);
   const SplitPlan split = split_plan(a, lists);
   if (split.splits == 1 || split_cluster(a.d, split) > 1 || (split.splits > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_bytes >= sm100_fwd_workspace_bytes(a, lists)))
     return sm100_fwd_split(a, p, split, mk, mv, ws, kb, st);

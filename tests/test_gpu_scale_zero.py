@@ -12,7 +12,7 @@ TERMS = {"causal": M.MaskTerms(causal=True), "band": M.MaskTerms(band=(100, 30))
 
 
 @pytest.mark.parametrize("mask", TERMS)
-@pytest.mark.parametrize("dtype", [torch.float32])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("N,d", [(300, 64), (300, 128), (16, 64)])
 def test_scale_zero(N, d, dtype, mask):
     L = 400
