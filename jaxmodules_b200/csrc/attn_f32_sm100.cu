@@ -304,7 +304,8 @@ struct F32Params {
   float scale_log2;
   int* status;
   LaunchOrder order;
-  int parts;       // CTAs of a cluster that share a walk (dK / dV and dQ)
+  int parts;       // CTAs of a cluster that share a walk
+  int first;       // forward: number of tiles, in launch order, that an earlier launch has done
 };
 
 // ---- results that are not finite ----------------------------------------------------------------------------------
@@ -555,17 +556,20 @@ static_assert(fwd_smem<4>() <= sizeof(FwdSmem<64>) && fwd_smem<8>() <= sizeof(Fw
 
 // KB: with a key bias, or a scale that is not positive: for a negative one the maximum of the scores is not that of the scaled ones, and a scale of 0
 // would make a NaN of a score that the mask has set to -inf before it is scaled (its tile would be done again with FP32 arithmetic).
-template <int DP, bool KB>
+// SHARED: the CTAs of a cluster share a tile's keys; an instance of its own, since the part costs the plain kernel registers (4 x 4096 tokens,
+// 16 heads, causal: the call 1 437 us with it, 1 408 without at 128 head columns, 765 and 757 at 64).
+template <int DP, bool KB, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1)
 f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ F32Params p, const int parts, const int first) {
+               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ F32Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using Smem = FwdSmem<DP>;
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   constexpr int kBoxes = Smem::kBoxes, kStages = Smem::kStages;
   const bma_attn_args& a = p.a;
+  const int parts = SHARED ? p.parts : 1;
   int qi, h;
-  cta_of(p.order, first + (int)blockIdx.x / parts, qi, h);
+  cta_of(p.order, (SHARED ? p.first : 0) + (int)blockIdx.x / parts, qi, h);
   qi = p.order.tiles - 1 - qi;
   const int b = h / a.Hq;
   h -= b * a.Hq;
@@ -799,46 +803,46 @@ f32_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ++syncs;
     };
     rendezvous();
-    if (parts > 1) {   // both partial results as they are; the cluster adds them up below
+    if constexpr (SHARED) {   // both partial results as they are; the cluster adds them up below
       float* stage = reinterpret_cast<float*>(sm.q) + (x * BM + row) * (DP + 4);
 #pragma unroll
       for (int j = 0; j < DP; j += 4) *reinterpret_cast<float4*>(stage + j) = make_float4(o[j / 2].x, o[j / 2].y, o[j / 2 + 1].x, o[j / 2 + 1].y);
       if (!ok) report_device_error(p.status, 630 + warp);
     } else {
-    const float mo = sm.ml[x ^ 1][0][row], lo = sm.ml[x ^ 1][1][row];
-    const float mt = fmaxf(m, mo), ms = (mt == -INFINITY) ? 0.f : mt;
-    const float fx = ex2(m - ms), fo = ex2(mo - ms);
-    const float lt = l * fx + lo * fo;
-    const float mine = lt > 0.f ? fx / lt : 0.f;
-    constexpr int kPitch = DP + 4;
-    float* stage = reinterpret_cast<float*>(sm.q) + row * kPitch;
-    if (x == 0) {
+      const float mo = sm.ml[x ^ 1][0][row], lo = sm.ml[x ^ 1][1][row];
+      const float mt = fmaxf(m, mo), ms = (mt == -INFINITY) ? 0.f : mt;
+      const float fx = ex2(m - ms), fo = ex2(mo - ms);
+      const float lt = l * fx + lo * fo;
+      const float mine = lt > 0.f ? fx / lt : 0.f;
+      constexpr int kPitch = DP + 4;
+      float* stage = reinterpret_cast<float*>(sm.q) + row * kPitch;
+      if (x == 0) {
 #pragma unroll
-      for (int j = 0; j < DP; j += 4) *reinterpret_cast<float4*>(stage + j) = make_float4(o[j / 2].x * mine, o[j / 2].y * mine, o[j / 2 + 1].x * mine, o[j / 2 + 1].y * mine);
-    }
-    rendezvous();
-    if (x == 1) {
-      float z = 0.f;
-#pragma unroll
-      for (int j = 0; j < DP; j += 4) {
-        float4 v = *reinterpret_cast<float4*>(stage + j);
-        v.x = fmaf(o[j / 2].x, mine, v.x); v.y = fmaf(o[j / 2].y, mine, v.y); v.z = fmaf(o[j / 2 + 1].x, mine, v.z); v.w = fmaf(o[j / 2 + 1].y, mine, v.w);
-        *reinterpret_cast<float4*>(stage + j) = v;
-        note_finite(z, (v.x + v.y) + (v.z + v.w));
+        for (int j = 0; j < DP; j += 4) *reinterpret_cast<float4*>(stage + j) = make_float4(o[j / 2].x * mine, o[j / 2].y * mine, o[j / 2 + 1].x * mine, o[j / 2 + 1].y * mine);
       }
-      if (z != 0.f) sm.not_finite = 1;
-      if (q < a.N && a.lse) a.lse[((int64_t)b * a.Hq + h) * a.N + q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
-    }
-    rendezvous();
-    if (ok) store_rows<256>(reinterpret_cast<const float*>(sm.q), kPitch, a.o, b, q0, a.N, h, a.d, threadIdx.x);
-    else report_device_error(p.status, 630 + warp);
+      rendezvous();
+      if (x == 1) {
+        float z = 0.f;
+#pragma unroll
+        for (int j = 0; j < DP; j += 4) {
+          float4 v = *reinterpret_cast<float4*>(stage + j);
+          v.x = fmaf(o[j / 2].x, mine, v.x); v.y = fmaf(o[j / 2].y, mine, v.y); v.z = fmaf(o[j / 2 + 1].x, mine, v.z); v.w = fmaf(o[j / 2 + 1].y, mine, v.w);
+          *reinterpret_cast<float4*>(stage + j) = v;
+          note_finite(z, (v.x + v.y) + (v.z + v.w));
+        }
+        if (z != 0.f) sm.not_finite = 1;
+        if (q < a.N && a.lse) a.lse[((int64_t)b * a.Hq + h) * a.N + q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
+      }
+      rendezvous();
+      if (ok) store_rows<256>(reinterpret_cast<const float*>(sm.q), kPitch, a.o, b, q0, a.N, h, a.d, threadIdx.x);
+      else report_device_error(p.status, 630 + warp);
     }
   }
   tc_fence_before();
-  if (parts > 1) cluster_sync();
+  if constexpr (SHARED) cluster_sync();
   else __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
-  if (parts > 1) {
+  if constexpr (SHARED) {
     if (warp < 8) sum_parts<DP>(reinterpret_cast<const float*>(sm.q), &sm.ml[0][0][0], &sm.not_finite, p, parts, part, q0, h, b);
     cluster_sync();   // shared memory stays until the others have read it
     if (part > 0) return;
@@ -2094,6 +2098,7 @@ LaunchOrder k_order(const bma_attn_args& a, int dp) { return launch_order(ceil_d
 
 int make_params(F32Params& p, const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists) {
   p.a = a; p.spec = spec; p.l = lists;
+  p.parts = 1; p.first = 0;
   p.scale_log2 = a.scale * kLog2e;
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
@@ -2111,8 +2116,8 @@ cudaLaunchConfig_t f32_fwd_config(int tiles, int parts, size_t smem, cudaStream_
 // Clusters of `parts` CTAs of the forward kernel that the device runs at the same time.
 int f32_fwd_clusters(int dp, int parts) {
   static ClusterCounts narrow, wide;
-  return dp == 128 ? clusters_at_once(wide, f32_fwd_kernel<128, false>, kThreads, sizeof(FwdSmem<128>), parts)
-                   : clusters_at_once(narrow, f32_fwd_kernel<64, false>, kThreads, sizeof(FwdSmem<64>), parts);
+  return dp == 128 ? clusters_at_once(wide, f32_fwd_kernel<128, false, true>, kThreads, sizeof(FwdSmem<128>), parts)
+                   : clusters_at_once(narrow, f32_fwd_kernel<64, false, true>, kThreads, sizeof(FwdSmem<64>), parts);
 }
 
 // How many CTAs share a tile's key list: `parts` in one launch of all tiles, or, where every tile takes as long, 1 for whole waves of
@@ -2202,14 +2207,16 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
       (rc = plane_map(&mv, w + pl.v, a.B, a.L, a.Hkv, dp, BH)))
     return rc;
   p.order = q_order(a, dp);
-  auto launch = [&](auto kernel, size_t smem) -> int {
-    BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto launch = [&](auto plain, auto shared, size_t smem) -> int {
     const int items = (int)launch_ctas(p.order);
     auto run = [&](int first, int count, int parts) -> int {
+      const auto kernel = parts > 1 ? shared : plain;
+      BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      p.parts = parts; p.first = first;
       cudaLaunchConfig_t cfg = f32_fwd_config(count, parts, smem, st);
       cudaLaunchAttribute attr = cluster_attribute(parts);
       if (parts > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
-      BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p, parts, first));
+      BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p));
       count_launches(1);
       return BMA_OK;
     };
@@ -2217,8 +2224,10 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     const int r = run(0, items - share.last, share.parts);
     return r || !share.last ? r : run(items - share.last, share.last, share.last_parts);
   };
-  if (a.key_bias || !(a.scale > 0.f)) rc = dp == 64 ? launch(f32_fwd_kernel<64, true>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, true>, sizeof(FwdSmem<128>));
-  else rc = dp == 64 ? launch(f32_fwd_kernel<64, false>, sizeof(FwdSmem<64>)) : launch(f32_fwd_kernel<128, false>, sizeof(FwdSmem<128>));
+  if (a.key_bias || !(a.scale > 0.f)) rc = dp == 64 ? launch(f32_fwd_kernel<64, true, false>, f32_fwd_kernel<64, true, true>, sizeof(FwdSmem<64>))
+                                                   : launch(f32_fwd_kernel<128, true, false>, f32_fwd_kernel<128, true, true>, sizeof(FwdSmem<128>));
+  else rc = dp == 64 ? launch(f32_fwd_kernel<64, false, false>, f32_fwd_kernel<64, false, true>, sizeof(FwdSmem<64>))
+                     : launch(f32_fwd_kernel<128, false, false>, f32_fwd_kernel<128, false, true>, sizeof(FwdSmem<128>));
   if (rc) return rc;
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
