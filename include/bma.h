@@ -153,6 +153,8 @@ int bma_version(void);
 /* Number of CUDA kernels this library has launched in the calling process (diagnostics for
  * benchmarks; no counterpart in the reference). */
 unsigned long long bma_launch_count(void);
+/* Of those, the launches in clusters of `ctas` CTAs (2 - 8) that share the work of a tile; 0 for other sizes. */
+unsigned long long bma_cluster_launch_count(int32_t ctas);
 
 /* Static text for a status code; for BMA_ERR_CUDA the text of the last CUDA error seen by
  * the calling thread is appended. */

@@ -94,6 +94,7 @@ class AttnArgs(C.Structure):
 SIGNATURES = {
     "bma_version": (C.c_int, []),
     "bma_launch_count": (C.c_ulonglong, []),
+    "bma_cluster_launch_count": (C.c_ulonglong, [C.c_int32]),
     "bma_error_string": (C.c_char_p, [C.c_int]),
     "bma_mask_compile_workspace_bytes": (C.c_size_t, [C.POINTER(MaskSpec), C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "bma_mask_compile": (C.c_int, [C.POINTER(MaskSpec), C.c_int32, C.c_int32, C.POINTER(BlockLists), C.c_void_p,

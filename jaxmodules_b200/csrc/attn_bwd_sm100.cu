@@ -607,7 +607,7 @@ static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUte
   else rc = a.key_bias ? launch(bwd_dkdv_kernel<64, true, false>, bwd_dkdv_kernel<64, true, false, true>, bwd_dkdv_kernel<64, true, true>, sizeof(BwdSmem<64>))
                        : launch(bwd_dkdv_kernel<64, false, false>, bwd_dkdv_kernel<64, false, false, true>, bwd_dkdv_kernel<64, false, true>, sizeof(BwdSmem<64>));
   if (rc) return rc;
-  count_launches(1);
+  count_launches(1, p.parts);
   BMA_CUDA_TRY(cudaGetLastError());
   return BMA_OK;
 }

@@ -2217,7 +2217,7 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
       cudaLaunchAttribute attr = cluster_attribute(parts);
       if (parts > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
       BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p));
-      count_launches(1);
+      count_launches(1, parts);
       return BMA_OK;
     };
     const FwdShare share = f32_fwd_share(a, spec, dp, lists.NQ, lists.NKV);
@@ -2255,7 +2255,7 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     cudaLaunchAttribute attr = cluster_attribute(parts);
     if (parts > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
     BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
-    count_launches(1);
+    count_launches(1, parts);
     return BMA_OK;
   };
   if (a.d > 64) {

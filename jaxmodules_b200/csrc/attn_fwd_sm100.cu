@@ -1701,7 +1701,7 @@ static int sm100_fwd_split(const bma_attn_args& a, const FwdParams& f, const Spl
   if (a.d == 128) rc = kb ? launch(fwd_split_kernel<128, true>, sizeof(FwdSplitSmem<128>)) : launch(fwd_split_kernel<128, false>, sizeof(FwdSplitSmem<128>));
   else rc = kb ? launch(fwd_split_kernel<64, true>, sizeof(FwdSplitSmem<64>)) : launch(fwd_split_kernel<64, false>, sizeof(FwdSplitSmem<64>));
   if (rc) return rc;
-  count_launches(1);
+  count_launches(1, p.cluster);
   if (plan.splits > p.cluster) {
     const int64_t rows = (int64_t)plan.units * plan.heads * plan.tile_queries;
     const unsigned grid = (unsigned)((rows + 7) / 8);

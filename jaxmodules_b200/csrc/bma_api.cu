@@ -27,9 +27,13 @@ constexpr int kMaxDevices = 64;
 int* g_status_ptr[kMaxDevices] = {};
 std::mutex g_status_mutex;
 std::atomic<unsigned long long> g_launches{0};
+std::atomic<unsigned long long> g_cluster_launches[kMaxParts + 1] = {};
 }  // namespace
 
-void count_launches(int n) { g_launches.fetch_add((unsigned long long)n, std::memory_order_relaxed); }
+void count_launches(int n, int cluster) {
+  g_launches.fetch_add((unsigned long long)n, std::memory_order_relaxed);
+  if (cluster > 1 && cluster <= kMaxParts) g_cluster_launches[cluster].fetch_add((unsigned long long)n, std::memory_order_relaxed);
+}
 
 void set_last_cuda_error(cudaError_t e, const char* where) {
   std::snprintf(g_err_text, sizeof(g_err_text), "CUDA error %d (%s) at %s", (int)e, cudaGetErrorString(e), where);
@@ -207,6 +211,10 @@ extern "C" {
 int bma_version(void) { return 1000; }
 
 unsigned long long bma_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
+
+unsigned long long bma_cluster_launch_count(int32_t ctas) {
+  return ctas > 1 && ctas <= kMaxParts ? g_cluster_launches[ctas].load(std::memory_order_relaxed) : 0;
+}
 
 const char* bma_error_string(int status) {
   switch (status) {

@@ -36,7 +36,8 @@ void set_last_cuda_error(cudaError_t e, const char* where);
 int* device_status_ptr();
 
 // Host-side count of kernels launched by this library in this process (diagnostics).
-void count_launches(int n);
+constexpr int kMaxParts = 8;   // CTAs of a cluster
+void count_launches(int n, int cluster = 1);
 
 __device__ __forceinline__ void report_device_error(int* status, int code) { atomicCAS(status, 0, code); }
 
@@ -64,7 +65,6 @@ inline cudaLaunchAttribute cluster_attribute(int parts) {
   attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
   return attr;
 }
-constexpr int kMaxParts = 8;
 // How many clusters of `parts` CTAs of a kernel the device runs at the same time (0 where it runs none); `known` keeps the answers of a
 // kernel.
 struct ClusterCounts {
