@@ -629,17 +629,17 @@ static int64_t unit_blocks(const bma_attn_args& a, const bma_block_lists& l, con
 // 3 parts, the call 288 -> 180 us; 1 x 4096, 8/1 heads of 128 562 -> 214; 2 x 4096, 16/4 heads 665 -> 548; host path and launch order included.)
 static Walks dkdv_walks(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& l, const int64_t* visited, int nb, int nhk) {
   const int64_t ctas = (int64_t)ceil_div(a.L, BT) * nhk * nb;
-  if (ctas > 4 * kSms) return {4 * kSms, 1., 1., true};   // many waves: nothing is shared
+  if (ctas > 4 * kSms) return {4 * kSms, 1., 1., true, true};   // many waves: nothing is shared
   const int G = a.Hq / a.Hkv, NQ = ceil_div(a.N, BT);
   const bool causal = (spec.flags & BMA_MASK_CAUSAL) != 0;
-  Walks w{(int)ctas, (double)G * NQ, (double)ctas * G * NQ * (causal ? 0.5 : 1.), !causal};
+  Walks w{(int)ctas, (double)G * NQ, (double)ctas * G * NQ * (causal ? 0.5 : 1.), !causal, visited || !(spec.flags & kTableTerms)};
   if (visited) {
     int64_t all = 0;
     for (int64_t i = 0; i < (int64_t)l.B * l.H; ++i) all += visited[i];
     w.sum = std::min((double)all / ((double)l.B * l.H) * nb * nhk * G, w.sum);   // (per list head, on average)
   }
   const double mean = w.sum / ctas;
-  if (spec.flags & BMA_MASK_BAND) w.longest = std::min(w.longest, G * (((double)spec.band_left + spec.band_right) / BT + 2.));
+  bound_walks(w, spec, G);
   if (spec.flags & kTableTerms) w.longest = std::min(w.longest, 2. * mean + G);
   if (!causal) w.longest = std::min(w.longest, std::max(mean, 1.));
   w.longest = std::max(w.longest, 1.);

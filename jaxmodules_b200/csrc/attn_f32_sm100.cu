@@ -2121,7 +2121,7 @@ int f32_fwd_clusters(int dp, int parts) {
 }
 
 // How many CTAs share a tile's key list: `parts` in one launch of all tiles, or, where every tile takes as long, 1 for whole waves of
-// tiles and `last_parts` for the `last` ones, in a launch of their own.  Launches of up to four waves leave SMs without work: too
+// tiles and `last_parts` for the `last` ones, in a launch of their own (which costs short walks more than it gives).  Launches of up to four waves leave SMs without work: too
 // few tiles, a last wave of a few, or a causal mask whose longest walk takes longer than the average SM's share.  The model counts key tiles:
 // a walk of w tiles takes w / parts + 3, the three for set-up, merge and the partials' way through shared memory (a CTA takes 8 - 14 us
 // besides its tiles of 3.1 us at 64 head columns, 4.8 at 128).  Calls: 1 x 1500 tokens, 16/4 heads of 128, no mask, 148 + 44 tiles in 3
@@ -2130,13 +2130,14 @@ int f32_fwd_clusters(int dp, int parts) {
 struct FwdShare {
   int parts, last, last_parts;
 };
-// Walks of the query tiles over key tiles, of the key tiles over a head group's query tiles.  (Of other masks than causal ones and bands
-// nothing is known here: as if they were full.)
+// Walks of the query tiles over key tiles, of the key tiles over a head group's query tiles.  (Of terms that are looked up nothing
+// is known here.)
 Walks q_walks(const bma_attn_args& a, const bma_mask_spec& spec, int NQ, int NKV) {
   const int heads = a.B * a.Hq;
-  Walks w{NQ * heads, (double)NKV, (double)NQ * heads * NKV, true};
+  const bool known = !(spec.flags & kTableTerms);
+  Walks w{NQ * heads, (double)NKV, (double)NQ * heads * NKV, true, known};
   if (spec.flags & BMA_MASK_CAUSAL) {
-    w = {NQ * heads, 0., 0., false};
+    w = {NQ * heads, 0., 0., false, known};
     for (int qi = 0; qi < NQ; ++qi) {
       const int64_t keys = std::min<int64_t>((int64_t)(qi + 1) * BM, a.N) + spec.q_offset - spec.k_offset;
       const double t = (double)std::min<int64_t>(std::max<int64_t>((keys + BM - 1) / BM, 0), NKV);
@@ -2144,17 +2145,14 @@ Walks q_walks(const bma_attn_args& a, const bma_mask_spec& spec, int NQ, int NKV
       w.sum += t * heads;
     }
   }
-  if (spec.flags & BMA_MASK_BAND) {
-    w.longest = std::min(w.longest, ((double)spec.band_left + spec.band_right) / BM + 2.);
-    w.sum = std::min(w.sum, w.longest * w.ctas);
-  }
+  bound_walks(w, spec, 1);
   return w;
 }
 Walks k_walks(const bma_attn_args& a, const bma_mask_spec& spec, int NQ, int NKV) {
   const int G = a.Hq / a.Hkv;
   const Walks q = q_walks(a, spec, NQ, NKV);
-  Walks w{NKV * a.B * a.Hkv, (double)G * NQ, q.sum, q.even};
-  if (spec.flags & BMA_MASK_BAND) w.longest = std::min(w.longest, G * q.longest);
+  Walks w{NKV * a.B * a.Hkv, (double)G * NQ, q.sum, q.even, q.known};
+  bound_walks(w, spec, G);
   return w;
 }
 // CTAs that share a walk of a backward pass, likewise, with float32 accumulators to add up.  (Calls, forward and backward, causal: 1 x 1423, 4/1
@@ -2177,7 +2175,7 @@ FwdShare f32_fwd_share(const bma_attn_args& a, const bma_mask_spec& spec, int dp
   best.parts = share_walks(w, o, NKV, [&](int parts) { return f32_fwd_clusters(dp, parts); });
   double cost = even(tiles, best.parts, f32_fwd_clusters(dp, best.parts));
   const int last = tiles % kSms;
-  if (w.even && tiles > kSms && last > 0)
+  if (w.even && w.known && tiles > kSms && last > 0)
     for (int parts = 2; parts <= std::min(kMaxParts, NKV); ++parts) {
       const int clusters = f32_fwd_clusters(dp, parts);
       if (clusters < last) continue;

@@ -98,9 +98,20 @@ struct Walks {
   int ctas;
   double longest, sum;
   bool even;      // all about as long as the longest
+  bool known;     // false: as if terms of the mask that are looked up allowed everything
 };
+// Bands and block windows bound a walk by the 128-tiles that they are wide, and the two that they cut; `heads` such walks make one.
+inline void bound_walks(Walks& w, const bma_mask_spec& s, int heads) {
+  double width = 1e30;
+  if (s.flags & BMA_MASK_BAND) width = (double)s.band_left + s.band_right;
+  if (s.flags & BMA_MASK_BLOCK_WINDOW) width = std::min(width, ((double)s.win_left + s.win_right) * s.win_block);
+  w.longest = std::min(w.longest, heads * (width / 128 + 2.));
+  w.sum = std::min(w.sum, w.longest * w.ctas);
+}
 // The number of CTAs that share a walk, for the shortest time of the launch.  With n clusters at once a launch takes the longest of: waves of
-// walks of one length, or else the longest walk, or the even share of all; each CTA `extra` tiles besides its own.
+// walks of one length, or else the longest walk, or the even share of all; each CTA `extra` tiles besides its own.  Where the walks may be much
+// shorter than they are taken to be, more CTAs than run at once cost more than they give, and have to promise a third less time (float32,
+// documents of 300 of 4096 tokens, one head of 64, forward: 4 CTAs to a walk, all of them at once, 40 us, as unshared; 8 in two waves 54).
 template <typename N>
 int share_walks(const Walks& w, double extra, int most_parts, N clusters) {
   int best = 1;
@@ -110,7 +121,7 @@ int share_walks(const Walks& w, double extra, int most_parts, N clusters) {
     if (n < 1) continue;
     const double c = w.even ? (double)((w.ctas + n - 1) / n) * (w.longest / parts + extra)
                             : std::max(w.longest / parts + extra, (w.sum / parts + w.ctas * extra) / n * 1.05);
-    if (c < 0.95 * cost) { cost = c; best = parts; }
+    if (c < (w.known || n >= w.ctas ? 0.95 : 0.7) * cost) { cost = c; best = parts; }
   }
   return best;
 }

@@ -108,3 +108,26 @@ def test_not_finite_while_shared(d, operand, value):
         assert torch.equal(torch.isinf(x), inf) and torch.equal(x[inf], w[inf]), name
         fin = torch.isfinite(w)
         assert fin.any() and (x[fin].double() - w[fin].double()).abs().max() <= 2e-5 * max(1.0, float(w[fin].abs().max())), name
+
+
+def _sizes(dtype, N, H, d, **kw):
+    q, k, v, do = _inputs(1, N, N, H, H, d, dtype)
+    q, k, v = (t.requires_grad_(True) for t in (q, k, v))
+    return launches(lambda: torch.autograd.grad(jm.masked_attention_via_map(q, k, v, **kw), (q, k, v), do.float()))[2]
+
+
+def test_windows_make_walks_short():
+    """512 tiles whose walks a block window keeps to six tiles: no more to share than with a band (the last of the forward's four waves at most)."""
+    window = _sizes(torch.float32, 16384, 4, 64, block_size=64, window_size=(256, 256))
+    assert window == _sizes(torch.float32, 16384, 4, 64, mask_fn=M.sliding_window_mask(256, 256)) and len(window) <= 1
+
+
+def test_walks_of_unknown_length():
+    """Documents may make walks short: no more CTAs share one than run at once."""
+    ids = torch.arange(4096, dtype=torch.int32)[None] // 300
+    sizes = _sizes(torch.float32, 4096, 1, 64, mask_fn=M.document_mask(ids.numpy(), causal=True))
+    assert len(sizes) == 3 and max(sizes) * 32 <= 148        # (forward, dK / dV and dQ of 32 tiles each)
+    ids = torch.arange(1500, dtype=torch.int32)[None] // 128
+    q, k, v, _ = _inputs(1, 1500, 1500, 16, 4, 128)
+    _, n, clusters = launches(lambda: jm.masked_attention_via_map(q, k, v, mask_fn=M.document_mask(ids.numpy())))
+    assert clusters == []                                    # the last tiles have no launch of their own
