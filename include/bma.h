@@ -258,6 +258,11 @@ int bma_mask_tiles_build(const bma_mask_program* program, int32_t B, int32_t H, 
 int bma_attn_plan(const bma_attn_args* args, int32_t* backend, int32_t* q_tile, int32_t* kv_tile);
 int bma_attn_bwd_plan(const bma_attn_args* args, int32_t* backend, int32_t* q_tile, int32_t* kv_tile);
 
+/* Order of sums, of the passes below: where a call has too few tiles for the chip, the CTAs of a cluster share the walk of a
+ * tile, and how many do depends on the sizes of the call (B, heads, lengths), the interval terms of the mask and the device.  So repeated calls
+ * give the same bits, and so they are with any workspace and any lists of the same blocks; but some batches or heads alone need not give the
+ * bits that they have in the whole call (float32 forward and backward, dK and dV of the tensor-core backward, few queries). */
+
 /* Forward: O = softmax_masked(Q K^T * scale) V and lse, visiting only listed blocks and
  * applying the element predicate only on partial ones.  Replaces the lax.map/lax.scan
  * nest of jaxmodules/attention.py:52-177, 219-241. */
@@ -339,8 +344,8 @@ int bma_block_lists_visited(const bma_block_lists* lists, int64_t* visited, bma_
  * and a block that only one side names is reported through the status word, never written.
  * A workspace that holds the tables plus at least the largest (batch, kv head) unit still takes this
  * path: the backward then runs as consecutive launches over ranges of units that reuse the slots.
- * With a smaller or NULL workspace the dQ kernel recomputes S and dP; results agree to the bf16
- * rounding of dS either way.  The workspace must be 256-byte aligned. */
+ * With a smaller or NULL workspace the dQ kernel recomputes S and dP; dQ agrees to the bf16
+ * rounding of dS either way, dK and dV are the same bits.  The workspace must be 256-byte aligned. */
 size_t bma_attn_bwd_scratch_bytes(const bma_attn_args* args, const bma_block_lists* lists,
                                   const int64_t* visited_host);
 /* The smallest workspace that still takes the hand-over path: the tables plus the largest unit. */

@@ -349,7 +349,8 @@ last_backward_info = {}    # sizes of the most recent backward call (diagnostics
 def set_backward_scratch_limit(nbytes: int, fraction: float = 1.0) -> None:
     """Upper bound in bytes of the backward scratch buffer; 0 switches the dS hand-over off.  Buffers above the new
     limit are freed at once.  ``fraction`` < 1 additionally caps every call at that share of what it would need,
-    which forces the backward to run in ranges (a knob for tests and for measuring what ranges cost)."""
+    which forces the backward to run in ranges (a knob for tests and for measuring what ranges cost).  dK and dV are the same bits under any
+    limit; dQ differs by the rounding of dS where the hand-over is off."""
     global _scratch_limit, _scratch_fraction
     _scratch_limit, _scratch_fraction = int(nbytes), float(fraction)
     for key in [k for k, t in _scratch_buffers.items() if t.numel() > _scratch_limit]:
@@ -440,6 +441,9 @@ def masked_attention_via_map(
 
     float32 inputs keep float32 accuracy (2e-6 in the 2-norm) and the effect that infinities and NaN have in float32
     arithmetic, block-sparse: what lies in a key block that a query block does not visit does not reach it.
+
+    Repeated calls give the same bits.  A slice of the batch or of the heads alone need not give those it has in the whole call: where a
+    call has too few tiles for the chip, several CTAs share one and add up, and how many depends on the sizes of the call.
 
     Extras (keyword-only, defaulting to the reference's behaviour): ``out_dtype`` — the
     reference returns float32 for every input dtype, pass ``torch.bfloat16`` to halve the

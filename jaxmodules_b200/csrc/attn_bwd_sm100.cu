@@ -581,6 +581,9 @@ size_t sm100_bwd_workspace_bytes(const bma_attn_args&) { return 0; }
 // tables + the largest (batch, kv head) unit: the smallest workspace that still takes the hand-over path
 size_t sm100_bwd_scratch_min_bytes(const bma_attn_args& a, const bma_block_lists& lists, const int64_t* visited_host);
 
+// A tile of a walk takes 1.7 us; a CTA takes about six tiles more for set-up, drain and the sum over a cluster.  The walks are those of the whole
+// call, also in a launch of some of its heads.  (G = 8 query heads of 64 on one kv head, 3 x 1920 tokens, causal: 45 CTAs in 3 parts, the
+// call 288 -> 180 us; 1 x 4096, 8/1 heads of 128 562 -> 214; 2 x 4096, 16/4 heads 665 -> 548; host path and launch order included.)
 template <typename P>
 static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
                        const CUtensorMap& mdk, const CUtensorMap& mdv, P& p, const Walks& walks, int b0, int nb, int hk0, int nhk, cudaStream_t st) {
@@ -589,7 +592,7 @@ static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUte
   int rc;
   auto launch = [&](auto by_head, auto by_rank, auto shared, size_t smem) -> int {
     static ClusterCounts known[2];
-    p.parts = share_walks(walks, 6.0, kMaxParts, [&](int parts) { return clusters_at_once(known[a.d == 128], shared, kThreads, smem, parts); });
+    p.parts = walks.ctas > 4 * kSms ? 1 : share_walks(walks, 6.0, kMaxParts, [&](int parts) { return clusters_at_once(known[a.d == 128], shared, kThreads, smem, parts); });
     const auto kernel = p.parts > 1 ? shared : p.by_rank ? by_rank : by_head;
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg{};
@@ -623,29 +626,6 @@ static int64_t unit_blocks(const bma_attn_args& a, const bma_block_lists& l, con
   for (int g = 0; g < G; ++g) n += head_blocks(a, l, visited, b, hk * G + g);
   return n;
 }
-// The walks of nb x nhk heads' kv tiles, which take 1.7 us a tile; a CTA takes about six tiles more for set-up, drain and the sum over a
-// cluster.  The number of tiles is the caller's count of visited blocks, where there is one; the longest walk of a causal mask is that of
-// the first kv tile, other masks are taken as even.  (G = 8 query heads of 64 on one kv head, 3 x 1920 tokens, causal: 45 CTAs in
-// 3 parts, the call 288 -> 180 us; 1 x 4096, 8/1 heads of 128 562 -> 214; 2 x 4096, 16/4 heads 665 -> 548; host path and launch order included.)
-static Walks dkdv_walks(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& l, const int64_t* visited, int nb, int nhk) {
-  const int64_t ctas = (int64_t)ceil_div(a.L, BT) * nhk * nb;
-  if (ctas > 4 * kSms) return {4 * kSms, 1., 1., true, true};   // many waves: nothing is shared
-  const int G = a.Hq / a.Hkv, NQ = ceil_div(a.N, BT);
-  const bool causal = (spec.flags & BMA_MASK_CAUSAL) != 0;
-  Walks w{(int)ctas, (double)G * NQ, (double)ctas * G * NQ * (causal ? 0.5 : 1.), !causal, visited || !(spec.flags & kTableTerms)};
-  if (visited) {
-    int64_t all = 0;
-    for (int64_t i = 0; i < (int64_t)l.B * l.H; ++i) all += visited[i];
-    w.sum = std::min((double)all / ((double)l.B * l.H) * nb * nhk * G, w.sum);   // (per list head, on average)
-  }
-  const double mean = w.sum / ctas;
-  bound_walks(w, spec, G);
-  if (spec.flags & kTableTerms) w.longest = std::min(w.longest, 2. * mean + G);
-  if (!causal) w.longest = std::min(w.longest, std::max(mean, 1.));
-  w.longest = std::max(w.longest, 1.);
-  return w;
-}
-
 // tables + one dSt image (32 KB) per visited block of the whole problem
 size_t sm100_bwd_scratch_bytes(const bma_attn_args& a, const bma_block_lists& lists, const int64_t* visited_host) {
   if (lists.NKV > 1024 || lists.NQ <= 0 || lists.B <= 0 || lists.H <= 0) return 0;
@@ -699,9 +679,11 @@ int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   for (int b = 0; b < a.B; ++b)
     for (int hk = 0; hk < a.Hkv; ++hk) largest = std::max(largest, unit_blocks(a, lists, visited_host, b, hk));
   const bool hand_over = capacity >= 1 && largest <= capacity;
+  const bool many = (int64_t)ceil_div(a.L, BT) * a.Hkv * a.B > 4 * kSms;   // waves: nothing is shared
+  const Walks walks = many ? Walks{4 * kSms + 1} : k_walks(a, spec);
   if (!hand_over) {
     if (pre && (rc = bma_attn_bwd_preprocess(&pre->a, pre->out, st))) return rc;
-    rc = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, dkdv_walks(a, spec, lists, visited_host, a.B, a.Hkv), 0, a.B, 0, a.Hkv, st);
+    rc = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, walks, 0, a.B, 0, a.Hkv, st);
     if (rc) return rc;
     if (mark) BMA_CUDA_TRY(cudaEventRecord(mark, st));
     return sm100_bwd_dq(a, spec, lists, st);
@@ -712,7 +694,7 @@ int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   p.capacity = capacity;
   bool first = true;
   auto run_range = [&](int b0, int nb, int hk0, int nhk, bool whole) -> int {
-    int r = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, dkdv_walks(a, spec, lists, visited_host, nb, nhk), b0, nb, hk0, nhk, st);
+    int r = launch_dkdv(a, mq, mk, mv, mdo, mdk, mdv, p, walks, b0, nb, hk0, nhk, st);
     if (r) return r;
     if (mark && first && whole) BMA_CUDA_TRY(cudaEventRecord(mark, st));   // one boundary only when one range covers everything
     first = false;

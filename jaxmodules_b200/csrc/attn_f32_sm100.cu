@@ -2130,31 +2130,6 @@ int f32_fwd_clusters(int dp, int parts) {
 struct FwdShare {
   int parts, last, last_parts;
 };
-// Walks of the query tiles over key tiles, of the key tiles over a head group's query tiles.  (Of terms that are looked up nothing
-// is known here.)
-Walks q_walks(const bma_attn_args& a, const bma_mask_spec& spec, int NQ, int NKV) {
-  const int heads = a.B * a.Hq;
-  const bool known = !(spec.flags & kTableTerms);
-  Walks w{NQ * heads, (double)NKV, (double)NQ * heads * NKV, true, known};
-  if (spec.flags & BMA_MASK_CAUSAL) {
-    w = {NQ * heads, 0., 0., false, known};
-    for (int qi = 0; qi < NQ; ++qi) {
-      const int64_t keys = std::min<int64_t>((int64_t)(qi + 1) * BM, a.N) + spec.q_offset - spec.k_offset;
-      const double t = (double)std::min<int64_t>(std::max<int64_t>((keys + BM - 1) / BM, 0), NKV);
-      w.longest = std::max(w.longest, t);
-      w.sum += t * heads;
-    }
-  }
-  bound_walks(w, spec, 1);
-  return w;
-}
-Walks k_walks(const bma_attn_args& a, const bma_mask_spec& spec, int NQ, int NKV) {
-  const int G = a.Hq / a.Hkv;
-  const Walks q = q_walks(a, spec, NQ, NKV);
-  Walks w{NKV * a.B * a.Hkv, (double)G * NQ, q.sum, q.even, q.known};
-  bound_walks(w, spec, G);
-  return w;
-}
 // CTAs that share a walk of a backward pass, likewise, with float32 accumulators to add up.  (Calls, forward and backward, causal: 1 x 1423, 4/1
 // heads of 128 750 -> 195 us, 1 x 4096, 8/2 heads of 128 2220 -> 805, 1 x 4096, 4 heads of 64 404 -> 280, 1 x 3000, 16/4 heads of 64 823 -> 538;
 // forward, host path and launch order included.  The shared kernels are instances of their own: the part of a walk costs the plain dK / dV
@@ -2168,7 +2143,7 @@ int f32_bwd_parts(const Walks& w, int64_t ctas, ClusterCounts& known, K kernel, 
 FwdShare f32_fwd_share(const bma_attn_args& a, const bma_mask_spec& spec, int dp, int NQ, int NKV) {
   FwdShare best{1, 0, 1};
   if ((int64_t)NQ * a.B * a.Hq > 4 * kSms || NKV < 2) return best;
-  const Walks w = q_walks(a, spec, NQ, NKV);
+  const Walks w = q_walks(a, spec);
   const int tiles = w.ctas;
   const double o = 3., longest = w.longest;
   auto even = [&](int count, int parts, int clusters) { return (double)ceil_div(count, clusters) * (longest / parts + o); };
@@ -2242,7 +2217,7 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   static ClusterCounts known[4];
   const int64_t k_ctas = (int64_t)lists.NKV * a.B * a.Hkv, q_ctas = (int64_t)lists.NQ * a.B * a.Hq;
   const bool few = std::min(k_ctas, q_ctas) <= 4 * kSms;
-  const Walks kw = few ? k_walks(a, spec, lists.NQ, lists.NKV) : Walks{}, qw = few ? q_walks(a, spec, lists.NQ, lists.NKV) : Walks{};
+  const Walks kw = few ? k_walks(a, spec) : Walks{}, qw = few ? q_walks(a, spec) : Walks{};
   auto launch = [&](auto kernel, const LaunchOrder& order, int parts, size_t smem, auto... args) -> int {
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg{};

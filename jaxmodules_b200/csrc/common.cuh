@@ -41,6 +41,9 @@ void count_launches(int n, int cluster = 1);
 
 __device__ __forceinline__ void report_device_error(int* status, int code) { atomicCAS(status, 0, code); }
 
+// Terms of the mask that are looked up (segment ids, bit table, tile bits) rather than computed from the indices.
+constexpr int kTableTerms = BMA_MASK_SEGMENT | BMA_MASK_BITMAP | BMA_MASK_TILES;
+
 // ---- order of a launch's CTAs -------------------------------------------------------------
 // One CTA per (tile, head, batch).  CTAs start in the order of their linear index: one head after another, the longest walk of each
 // (under a causal mask) first, or the longest walks of all heads first.  In the first order a launch ends with the longest walks of its last
@@ -108,6 +111,31 @@ inline void bound_walks(Walks& w, const bma_mask_spec& s, int heads) {
   w.longest = std::min(w.longest, heads * (width / 128 + 2.));
   w.sum = std::min(w.sum, w.longest * w.ctas);
 }
+// Walks of the 128-query tiles over key tiles, of the key tiles over a head group's query tiles, as the arguments and the mask say and nothing else:
+// the order of a sum does not depend on the workspace of a call or on the ranges it is run in.  (Of terms that are looked up nothing is known here.)
+inline Walks q_walks(const bma_attn_args& a, const bma_mask_spec& spec) {
+  const int heads = a.B * a.Hq, NQ = (a.N + 127) / 128, NKV = (a.L + 127) / 128;
+  const bool known = !(spec.flags & kTableTerms);
+  Walks w{NQ * heads, (double)NKV, (double)NQ * heads * NKV, true, known};
+  if (spec.flags & BMA_MASK_CAUSAL) {
+    w = {NQ * heads, 0., 0., false, known};
+    for (int qi = 0; qi < NQ; ++qi) {
+      const int64_t keys = std::min<int64_t>((int64_t)(qi + 1) * 128, a.N) + spec.q_offset - spec.k_offset;
+      const double t = (double)std::min<int64_t>(std::max<int64_t>((keys + 127) / 128, 0), NKV);
+      w.longest = std::max(w.longest, t);
+      w.sum += t * heads;
+    }
+  }
+  bound_walks(w, spec, 1);
+  return w;
+}
+inline Walks k_walks(const bma_attn_args& a, const bma_mask_spec& spec) {
+  const int G = a.Hq / a.Hkv, NQ = (a.N + 127) / 128, NKV = (a.L + 127) / 128;
+  const Walks q = q_walks(a, spec);
+  Walks w{NKV * a.B * a.Hkv, (double)G * NQ, q.sum, q.even, q.known};
+  bound_walks(w, spec, G);
+  return w;
+}
 // The number of CTAs that share a walk, for the shortest time of the launch.  With n clusters at once a launch takes the longest of: waves of
 // walks of one length, or else the longest walk, or the even share of all; each CTA `extra` tiles besides its own.  Where the walks may be much
 // shorter than they are taken to be, more CTAs than run at once cost more than they give, and have to promise a third less time (float32,
@@ -163,9 +191,6 @@ inline LaunchOrder launch_order(int tiles, int64_t heads, int64_t stream_bytes_p
   return {tiles, (int)heads, (int)((heads + groups - 1) / groups)};   // groups of one size: a small last one would end the launch alone
 }
 inline unsigned launch_ctas(const LaunchOrder& o) { return (unsigned)(o.tiles * o.heads); }
-
-// Terms of the mask that are looked up (segment ids, bit table, tile bits) rather than computed from the indices.
-constexpr int kTableTerms = BMA_MASK_SEGMENT | BMA_MASK_BITMAP | BMA_MASK_TILES;
 
 // What the interval terms of a mask have to satisfy, for lists to be compiled from them or for a pass to know its blocks without lists.
 inline bool interval_terms_valid(const bma_mask_spec& s) {

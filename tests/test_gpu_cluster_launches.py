@@ -131,3 +131,35 @@ def test_walks_of_unknown_length():
     q, k, v, _ = _inputs(1, 1500, 1500, 16, 4, 128)
     _, n, clusters = launches(lambda: jm.masked_attention_via_map(q, k, v, mask_fn=M.document_mask(ids.numpy())))
     assert clusters == []                                    # the last tiles have no launch of their own
+
+
+SCRATCH = {
+    "causal": lambda B, N: dict(is_causal=True),
+    "documents": lambda B, N: dict(mask_fn=M.document_mask((torch.arange(N, dtype=torch.int32) // 130)[None].repeat(B, 1).numpy(), causal=True)),
+    "table": lambda B, N: dict(mask_fn=lambda b, h, q, k: (k <= q) & (q - k < 200) & ((q + k) % 7 != 0)),
+    "window": lambda B, N: dict(block_size=50, window_size=(100, 50)),
+}
+
+
+@pytest.mark.parametrize("mask", SCRATCH)
+@pytest.mark.parametrize("B,N,Hq,Hkv,d", [(3, 700, 8, 2, 64), (2, 500, 12, 4, 128), (4, 300, 16, 1, 128)])
+def test_scratch_does_not_change_the_sums(B, N, Hq, Hkv, d, mask):
+    """The CTAs that share a walk are chosen for the whole call: with all dS tiles handed over, in ranges of heads through a small buffer and without
+    the hand-over dK and dV are the same bits, and so is dQ where it is read from the same tiles."""
+    q, k, v, do = _inputs(B, N, N, Hq, Hkv, d, torch.bfloat16)
+    q, k, v = (t.requires_grad_(True) for t in (q, k, v))
+    limit, grads, kernels = A._scratch_limit, [], []
+    try:
+        for share in ((limit, 1.0), (limit, 0.5), (0, 1.0)):
+            A.set_backward_scratch_limit(*share)
+            O = jm.masked_attention_via_map(q, k, v, **SCRATCH[mask](B, N))
+            g, _, clusters = launches(lambda: torch.autograd.grad(O, (q, k, v), do.float()))
+            grads.append(g)
+            kernels.append(clusters)
+    finally:
+        A.set_backward_scratch_limit(limit)
+    whole, ranges, recomputed = kernels
+    assert len(whole) == 1 and recomputed == whole and len(ranges) > 1 and set(ranges) == set(whole)
+    for name, x, y, z in zip(("dQ", "dK", "dV"), *grads):
+        assert torch.equal(x, y), name
+        assert name == "dQ" or torch.equal(x, z), name
