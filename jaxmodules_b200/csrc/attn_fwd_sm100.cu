@@ -1140,7 +1140,10 @@ __device__ __forceinline__ SplitRow split_row(const FwdSplitParams& p, int unit,
   return r;
 }
 
-template <int HD, bool KB>
+// CLUSTER: the runs of a unit are a cluster and meet in shared memory.  Else a CTA writes O or, of several runs, its partial itself, and merges its two
+// warpgroups in registers on the way: half the shared memory traffic, and no sums by rows (64 x 16 queries on 2048 keys, 32 heads of 128: the call
+// 427 us by rows, 406 so; 27 queries on 18680 keys, 2 x 42 heads of 64, seven runs, 138 and 129).
+template <int HD, bool KB, bool CLUSTER>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const FwdSplitParams sp) {
@@ -1351,42 +1354,102 @@ fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     tc_fence_after();
     if (m_ref == -INFINITY) l = 0.f;            // no allowed key (the polynomial exponential of a masked score is 2^-126, not 0)
 
-    // ---- the partial results of the two warpgroups to shared memory (after the rendezvous no MMA reads K or V any more)
     sm.ml[x][0][row] = m_ref;
     sm.ml[x][1][row] = l;
-    mbar_arrive(&sm.bar[SB_SYNC]);
-    ok = mbar_wait(&sm.bar[SB_SYNC], 0) && ok;
-    if (!ok) {
-      report_device_error(p.status, 170 + warp);
-    } else if (__any_sync(0xffffffffu, r.valid)) {
-      float* stage = reinterpret_cast<float*>(sm.k[0]) + (x * BM + row) * kPitch;
+    uint32_t syncs = 0;
+    auto rendezvous = [&]() {   // (after the first one no MMA reads K or V any more)
+      mbar_arrive(&sm.bar[SB_SYNC]);
+      ok = mbar_wait(&sm.bar[SB_SYNC], syncs & 1) && ok;
+      ++syncs;
+    };
+    rendezvous();
+    if constexpr (CLUSTER) {   // both partial results as they are; the cluster adds them up below
+      if (!ok) {
+        report_device_error(p.status, 170 + warp);
+      } else if (__any_sync(0xffffffffu, r.valid)) {
+        float* stage = reinterpret_cast<float*>(sm.k[0]) + (x * BM + row) * kPitch;
 #pragma unroll
-      for (int c = 0; c < HD / 32; ++c) {
-        uint32_t v[32];
-        if (cnt > 0) {
-          tmem_ld32(tmem_o + c * 32, v);
-          tmem_wait_ld();
-        } else {
+        for (int c = 0; c < HD / 32; ++c) {
+          uint32_t v[32];
+          if (cnt > 0) {
+            tmem_ld32(tmem_o + c * 32, v);
+            tmem_wait_ld();
+          } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = 0u;
+            for (int j = 0; j < 32; ++j) v[j] = 0u;
+          }
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(stage + c * 32 + j) =
+                make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
         }
+      }
+    } else {
+      // ---- merge of the two warpgroups through shared memory
+      const float mo = sm.ml[x ^ 1][0][row], lo = sm.ml[x ^ 1][1][row];
+      const float mt = fmaxf(m_ref, mo), ms = (mt == -INFINITY) ? 0.f : mt;
+      const float fx = ex2(m_ref - ms), lt = l * fx + lo * ex2(mo - ms);
+      // with several splits the partial stays unnormalised, relative to its own maximum
+      const float mine = cnt > 0 && l > 0.f ? (sp.splits == 1 ? fx / lt : fx) : 0.f;
+      float* stage = reinterpret_cast<float*>(sm.k[0]) + row * kPitch;
+      for (int turn = 0; turn < 2; ++turn) {
+        if (turn == x) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(stage + c * 32 + j) =
-              make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+          for (int c = 0; c < HD / 32; ++c) {
+            uint32_t v[32];
+            if (cnt > 0) {
+              tmem_ld32(tmem_o + c * 32, v);
+              tmem_wait_ld();
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              float4 o4 = turn == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<float4*>(stage + c * 32 + j);
+              o4.x = fmaf(__uint_as_float(v[j]), mine, o4.x); o4.y = fmaf(__uint_as_float(v[j + 1]), mine, o4.y);
+              o4.z = fmaf(__uint_as_float(v[j + 2]), mine, o4.z); o4.w = fmaf(__uint_as_float(v[j + 3]), mine, o4.w);
+              *reinterpret_cast<float4*>(stage + c * 32 + j) = o4;
+            }
+          }
+        }
+        rendezvous();
+      }
+      if (!ok) {
+        report_device_error(p.status, 170 + warp);
+      } else {
+        if (x == 0 && r.valid) {
+          if (sp.splits > 1) sp.part_ml[((int64_t)unit * sp.splits + split) * BM + row] = make_float2(mt, lt);
+          else if (a.lse) a.lse[((int64_t)b * a.Hq + r.h) * a.N + r.q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
+        }
+        // a warp per row: whole lines of O or of the partial
+        for (int i = warp; i < BM; i += 8) {
+          const SplitRow ri = split_row(sp, unit, i);
+          if (!ri.valid) continue;
+          const float* src = reinterpret_cast<const float*>(sm.k[0]) + i * kPitch;
+          if (sp.splits > 1) {
+            float* dst = sp.part_o + (((int64_t)unit * sp.splits + split) * BM + i) * HD;
+            if (lane < HD / 4) reinterpret_cast<float4*>(dst)[lane] = reinterpret_cast<const float4*>(src)[lane];
+          } else if (lane < HD / 4) {
+            const float4 o4 = reinterpret_cast<const float4*>(src)[lane];
+            const int64_t off = (int64_t)b * a.o.stride_b + (int64_t)ri.q * a.o.stride_l + (int64_t)ri.h * a.o.stride_h + lane * 4;
+            if (a.o.dtype == BMA_DTYPE_F32) *reinterpret_cast<float4*>(static_cast<float*>(a.o.ptr) + off) = o4;
+            else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.o.ptr) + off) = make_uint2(pack_bf16(o4.x, o4.y), pack_bf16(o4.z, o4.w));
+          }
+        }
       }
     }
   }
   tc_fence_before();
-  if (sp.cluster > 1) cluster_sync();
+  if constexpr (CLUSTER) cluster_sync();
   else __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, kTmemCols);
 
   // ---- every row: the weighted sum of its partials (two per CTA), relative to their common maximum; half a warp per row, the rows dealt
   // out over the CTAs of the cluster.  (A round of loads from another CTA takes 0.5 us: all rows go through the three rounds
   // at once.  The code is short rather than unrolled: it runs once, from a cold instruction cache.)
-  if (warp < 8) {
-    const int rows = sp.heads * sp.tile_queries, sources = 2 * sp.cluster, rank = sp.cluster > 1 ? (int)cluster_rank() : 0;
+  if (CLUSTER && warp < 8) {
+    const int rows = sp.heads * sp.tile_queries, sources = 2 * sp.cluster, rank = (int)cluster_rank();
     const int c = lane & 15;
 #pragma unroll 1
     for (int i0 = warp * 2; i0 * sp.cluster < rows; i0 += 16) {
@@ -1421,13 +1484,6 @@ fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         }
       }
       if (!valid) continue;
-      if (sp.splits > sp.cluster) {   // the runs meet in the workspace: unnormalised, relative to the maximum of this one
-        const int64_t at = ((int64_t)unit * sp.splits + split) * BM + i;
-        if (c == 0) sp.part_ml[at] = make_float2(mt, lt);
-#pragma unroll
-        for (int u = 0; u < HD / 64; ++u) reinterpret_cast<float4*>(sp.part_o + at * HD)[u * 16 + c] = acc[u];
-        continue;
-      }
       if (c == 0 && a.lse) a.lse[((int64_t)b * a.Hq + h) * a.N + q] = lt > 0.f ? (mt + log2f(lt)) * kLn2 : -INFINITY;
       const float inv = lt > 0.f ? 1.f / lt : 0.f;
 #pragma unroll
@@ -1439,7 +1495,7 @@ fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       }
     }
   }
-  if (sp.cluster > 1) cluster_sync();   // shared memory stays until the others have read it
+  if constexpr (CLUSTER) cluster_sync();   // shared memory stays until the others have read it
 }
 
 // One warp per (unit, row): O = sum over the splits of 2^(m_s - m) O_s / sum of 2^(m_s - m) l_s, and the log-sum-exp.
@@ -1672,7 +1728,7 @@ static int split_cluster(int d, const SplitPlan& plan) {
       }
       return most;
     };
-    n = 1 + (d == 128 ? ask(fwd_split_kernel<128, false>, sizeof(FwdSplitSmem<128>)) : ask(fwd_split_kernel<64, false>, sizeof(FwdSplitSmem<64>)));
+    n = 1 + (d == 128 ? ask(fwd_split_kernel<128, false, true>, sizeof(FwdSplitSmem<128>)) : ask(fwd_split_kernel<64, false, true>, sizeof(FwdSplitSmem<64>)));
     known.store(n, std::memory_order_relaxed);
   }
   const int clusters = n - 1;
@@ -1690,7 +1746,8 @@ static int sm100_fwd_split(const bma_attn_args& a, const FwdParams& f, const Spl
   p.part_o = static_cast<float*>(ws);
   p.part_ml = reinterpret_cast<float2*>(p.part_o + (size_t)plan.units * plan.splits * BM * a.d);
   p.cluster = split_cluster(a.d, plan);
-  auto launch = [&](auto kernel, size_t smem) -> int {
+  auto launch = [&](auto alone, auto in_cluster, size_t smem) -> int {
+    const auto kernel = p.cluster > 1 ? in_cluster : alone;
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = split_config(plan, smem, st);
     cudaLaunchAttribute attr = cluster_of(p.cluster);
@@ -1698,8 +1755,10 @@ static int sm100_fwd_split(const bma_attn_args& a, const FwdParams& f, const Spl
     BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p));
     return BMA_OK;
   };
-  if (a.d == 128) rc = kb ? launch(fwd_split_kernel<128, true>, sizeof(FwdSplitSmem<128>)) : launch(fwd_split_kernel<128, false>, sizeof(FwdSplitSmem<128>));
-  else rc = kb ? launch(fwd_split_kernel<64, true>, sizeof(FwdSplitSmem<64>)) : launch(fwd_split_kernel<64, false>, sizeof(FwdSplitSmem<64>));
+  if (a.d == 128) rc = kb ? launch(fwd_split_kernel<128, true, false>, fwd_split_kernel<128, true, true>, sizeof(FwdSplitSmem<128>))
+                          : launch(fwd_split_kernel<128, false, false>, fwd_split_kernel<128, false, true>, sizeof(FwdSplitSmem<128>));
+  else rc = kb ? launch(fwd_split_kernel<64, true, false>, fwd_split_kernel<64, true, true>, sizeof(FwdSplitSmem<64>))
+               : launch(fwd_split_kernel<64, false, false>, fwd_split_kernel<64, false, true>, sizeof(FwdSplitSmem<64>));
   if (rc) return rc;
   count_launches(1, p.cluster);
   if (plan.splits > p.cluster) {
