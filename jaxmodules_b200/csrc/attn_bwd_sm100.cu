@@ -591,8 +591,8 @@ static int launch_dkdv(const bma_attn_args& a, const CUtensorMap& mq, const CUte
   p.by_rank = longest_first(ceil_div(a.L, BT), nhk, nb, (int64_t)4 * a.N * a.d * (a.Hq / a.Hkv));
   int rc;
   auto launch = [&](auto by_head, auto by_rank, auto shared, size_t smem) -> int {
-    static ClusterCounts known[2];
-    p.parts = walks.ctas > 4 * kSms ? 1 : share_walks(walks, 6.0, kMaxParts, [&](int parts) { return clusters_at_once(known[a.d == 128], shared, kThreads, smem, parts); });
+    static ClusterCounts known[2][2];
+    p.parts = walks.ctas > 4 * kSms ? 1 : share_walks(walks, 6.0, kMaxParts, [&](int parts) { return clusters_at_once(known[a.d == 128][a.key_bias != nullptr], shared, kThreads, smem, parts); });
     const auto kernel = p.parts > 1 ? shared : p.by_rank ? by_rank : by_head;
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg{};

@@ -2114,10 +2114,13 @@ cudaLaunchConfig_t f32_fwd_config(int tiles, int parts, size_t smem, cudaStream_
   return cfg;
 }
 // Clusters of `parts` CTAs of the forward kernel that the device runs at the same time.
-int f32_fwd_clusters(int dp, int parts) {
-  static ClusterCounts narrow, wide;
-  return dp == 128 ? clusters_at_once(wide, f32_fwd_kernel<128, false, true>, kThreads, sizeof(FwdSmem<128>), parts)
-                   : clusters_at_once(narrow, f32_fwd_kernel<64, false, true>, kThreads, sizeof(FwdSmem<64>), parts);
+bool f32_fwd_kb(const bma_attn_args& a) { return a.key_bias || !(a.scale > 0.f); }
+int f32_fwd_clusters(const bma_attn_args& a, int dp, int parts) {
+  static ClusterCounts known[2][2];
+  const bool kb = f32_fwd_kb(a);
+  ClusterCounts& k = known[dp == 128][kb];
+  if (dp == 128) return clusters_at_once(k, kb ? f32_fwd_kernel<128, true, true> : f32_fwd_kernel<128, false, true>, kThreads, sizeof(FwdSmem<128>), parts);
+  return clusters_at_once(k, kb ? f32_fwd_kernel<64, true, true> : f32_fwd_kernel<64, false, true>, kThreads, sizeof(FwdSmem<64>), parts);
 }
 
 // How many CTAs share a tile's key list: `parts` in one launch of all tiles, or, where every tile takes as long, 1 for whole waves of
@@ -2147,14 +2150,14 @@ FwdShare f32_fwd_share(const bma_attn_args& a, const bma_mask_spec& spec, int dp
   const int tiles = w.ctas;
   const double o = 3., longest = w.longest;
   auto even = [&](int count, int parts, int clusters) { return (double)ceil_div(count, clusters) * (longest / parts + o); };
-  best.parts = share_walks(w, o, NKV, [&](int parts) { return f32_fwd_clusters(dp, parts); });
-  double cost = even(tiles, best.parts, f32_fwd_clusters(dp, best.parts));
-  const int last = tiles % kSms;
-  if (w.even && w.known && tiles > kSms && last > 0)
+  best.parts = share_walks(w, o, NKV, [&](int parts) { return f32_fwd_clusters(a, dp, parts); });
+  double cost = even(tiles, best.parts, f32_fwd_clusters(a, dp, best.parts));
+  const int sms = device_sms(current_device()), last = tiles % sms;
+  if (w.even && w.known && tiles > sms && last > 0)
     for (int parts = 2; parts <= std::min(kMaxParts, NKV); ++parts) {
-      const int clusters = f32_fwd_clusters(dp, parts);
+      const int clusters = f32_fwd_clusters(a, dp, parts);
       if (clusters < last) continue;
-      const double c = even(tiles - last, 1, kSms) + even(last, parts, clusters);
+      const double c = even(tiles - last, 1, sms) + even(last, parts, clusters);
       if (c < 0.95 * cost) { cost = c; best = {1, last, parts}; }
     }
   return best;
@@ -2197,7 +2200,7 @@ int f32_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     const int r = run(0, items - share.last, share.parts);
     return r || !share.last ? r : run(items - share.last, share.last, share.last_parts);
   };
-  if (a.key_bias || !(a.scale > 0.f)) rc = dp == 64 ? launch(f32_fwd_kernel<64, true, false>, f32_fwd_kernel<64, true, true>, sizeof(FwdSmem<64>))
+  if (f32_fwd_kb(a)) rc = dp == 64 ? launch(f32_fwd_kernel<64, true, false>, f32_fwd_kernel<64, true, true>, sizeof(FwdSmem<64>))
                                                    : launch(f32_fwd_kernel<128, true, false>, f32_fwd_kernel<128, true, true>, sizeof(FwdSmem<128>));
   else rc = dp == 64 ? launch(f32_fwd_kernel<64, false, false>, f32_fwd_kernel<64, false, true>, sizeof(FwdSmem<64>))
                      : launch(f32_fwd_kernel<128, false, false>, f32_fwd_kernel<128, false, true>, sizeof(FwdSmem<128>));
@@ -2214,7 +2217,8 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   int rc;
   if ((rc = make_params(p, a, spec, lists)) || (rc = launch_split(a, spec, given, pl, w, true, own_delta, st))) return rc;
   CUtensorMap mq, mk, mv, mdo, mqh, mkh, mvh, mdoh;
-  static ClusterCounts known[4];
+  static ClusterCounts known[4][2];
+  const int kb = a.key_bias != nullptr;
   const int64_t k_ctas = (int64_t)lists.NKV * a.B * a.Hkv, q_ctas = (int64_t)lists.NQ * a.B * a.Hq;
   const bool few = std::min(k_ctas, q_ctas) <= 4 * kSms;
   const Walks kw = few ? k_walks(a, spec) : Walks{}, qw = few ? q_walks(a, spec) : Walks{};
@@ -2242,11 +2246,11 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
     auto dq_shared = a.key_bias ? f32_dq_wide_kernel<true, true> : f32_dq_wide_kernel<false, true>;
     F32WideParams wp{p, w + pl.v};
     wp.f.order = k_order(a, 128);
-    wp.f.parts = f32_bwd_parts(kw, k_ctas, known[0], dkdv_shared, sizeof(DkdvWideSmem));
+    wp.f.parts = f32_bwd_parts(kw, k_ctas, known[0][kb], dkdv_shared, sizeof(DkdvWideSmem));
     if ((rc = launch(wp.f.parts > 1 ? dkdv_shared : dkdv, wp.f.order, wp.f.parts, sizeof(DkdvWideSmem), mk, mqh, mdoh, wp))) return rc;
     wp.a_planes = w + pl.d_o;
     wp.f.order = q_order(a, 128);
-    wp.f.parts = f32_bwd_parts(qw, q_ctas, known[1], dq_shared, sizeof(DqWideSmem));
+    wp.f.parts = f32_bwd_parts(qw, q_ctas, known[1][kb], dq_shared, sizeof(DqWideSmem));
     return launch(wp.f.parts > 1 ? dq_shared : dq, wp.f.order, wp.f.parts, sizeof(DqWideSmem), mq, mkh, mvh, wp);
   }
   if ((rc = plane_map(&mq, w + pl.q, a.B, a.N, a.Hq, 64, BM)) || (rc = plane_map(&mk, w + pl.k, a.B, a.L, a.Hkv, 64, BM)) ||
@@ -2259,10 +2263,10 @@ int f32_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_l
   auto dq = a.key_bias ? f32_dq_kernel<true, false> : f32_dq_kernel<false, false>;
   auto dq_shared = a.key_bias ? f32_dq_kernel<true, true> : f32_dq_kernel<false, true>;
   p.order = k_order(a, 64);
-  p.parts = f32_bwd_parts(kw, k_ctas, known[2], dkdv_shared, sizeof(DkdvSmem));
+  p.parts = f32_bwd_parts(kw, k_ctas, known[2][kb], dkdv_shared, sizeof(DkdvSmem));
   if ((rc = launch(p.parts > 1 ? dkdv_shared : dkdv, p.order, p.parts, sizeof(DkdvSmem), mk, mv, mqh, mdoh, p))) return rc;
   p.order = q_order(a, 64);
-  p.parts = f32_bwd_parts(qw, q_ctas, known[3], dq_shared, sizeof(DqSmem));
+  p.parts = f32_bwd_parts(qw, q_ctas, known[3][kb], dq_shared, sizeof(DqSmem));
   return launch(p.parts > 1 ? dq_shared : dq, p.order, p.parts, sizeof(DqSmem), mq, mkh, mvh, mdo, p);
 }
 

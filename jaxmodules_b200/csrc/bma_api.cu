@@ -23,7 +23,6 @@ int mask_compile_static(const bma_mask_spec& spec, int B, int H, const bma_block
 namespace {
 thread_local char g_err_text[512] = "";
 __device__ int g_device_status_word = 0;
-constexpr int kMaxDevices = 64;
 int* g_status_ptr[kMaxDevices] = {};
 std::mutex g_status_mutex;
 std::atomic<unsigned long long> g_launches{0};

@@ -68,33 +68,49 @@ inline cudaLaunchAttribute cluster_attribute(int parts) {
   attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
   return attr;
 }
-// How many clusters of `parts` CTAs of a kernel the device runs at the same time (0 where it runs none); `known` keeps the answers of a
-// kernel.
+// The current device, and its number of SMs (asked once per device).
+constexpr int kMaxDevices = 64;
+inline int current_device() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices ? dev : 0;
+}
+inline int device_sms(int dev) {
+  static std::atomic<int> known[kMaxDevices];
+  int n = known[dev].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
+    (void)cudaGetLastError();
+    return kSms;
+  }
+  known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+// How many clusters of `parts` CTAs of a kernel the current device runs at the same time (0 where it runs none).  `known` keeps the answers for one
+// instance of a kernel, by device; a question that fails is asked again by the next call.
 struct ClusterCounts {
-  std::atomic<int> plus_one[kMaxParts + 1];
+  std::atomic<int> plus_one[kMaxDevices][kMaxParts + 1];
 };
 template <typename K>
 int clusters_at_once(ClusterCounts& known, K kernel, int threads, size_t smem, int parts) {
-  if (parts == 1) return kSms;
-  std::atomic<int>& k = known.plus_one[parts];
-  int n = k.load(std::memory_order_relaxed);
-  if (!n) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kSms * parts);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr = cluster_attribute(parts);
-    cfg.attrs = &attr; cfg.numAttrs = 1;
-    int most = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
-      (void)cudaGetLastError();
-      most = 0;
-    }
-    n = 1 + most;
-    k.store(n, std::memory_order_relaxed);
+  const int dev = current_device();
+  if (parts == 1) return device_sms(dev);
+  std::atomic<int>& k = known.plus_one[dev][parts];
+  const int n = k.load(std::memory_order_relaxed);
+  if (n) return n - 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kSms * parts);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr = cluster_attribute(parts);
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  int most = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
   }
-  return n - 1;
+  k.store(1 + most, std::memory_order_relaxed);
+  return most;
 }
 // Walks of a launch: its CTAs, the longest and all of them together, in tiles.
 struct Walks {
