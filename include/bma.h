@@ -279,11 +279,12 @@ int32_t bma_attn_fwd_implies_lists(const bma_attn_args* args, const bma_mask_spe
  * in the lists that bma_mask_compile makes of the mask; -1 where the mask has other than interval terms or is not valid.  Runs on the host. */
 int32_t bma_mask_block_class(const bma_mask_spec* spec, int32_t q_block, int32_t kv_block, int32_t qi, int32_t kj);
 
-/* The same with a workspace (16-byte aligned), which lets few queries against many keys spread over the whole chip: partial
+/* bma_attn_fwd with a workspace (16-byte aligned), which lets few queries against many keys spread over the whole chip: partial
  * results of runs of keys are combined through it.  bma_attn_fwd_workspace_bytes is 0 where none is used; with less than
- * that bma_attn_fwd_ws runs as bma_attn_fwd does.  (Up to eight runs meet in the shared memory of a cluster of CTAs instead, on
- * a device that has room for the clusters.) */
+ * that bma_attn_fwd_ws runs as bma_attn_fwd does.  Up to eight runs meet in the shared memory of a cluster of CTAs instead, on
+ * a device that has room for the clusters: bma_attn_fwd_uses_workspace is 0 there (and where there are no runs), and none need be given. */
 size_t bma_attn_fwd_workspace_bytes(const bma_attn_args* args, const bma_block_lists* lists);
+int32_t bma_attn_fwd_uses_workspace(const bma_attn_args* args, const bma_block_lists* lists);
 int bma_attn_fwd_ws(const bma_attn_args* args, const bma_mask_spec* spec, const bma_block_lists* lists,
                     void* workspace, size_t workspace_bytes, bma_stream_t stream);
 

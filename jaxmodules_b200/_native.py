@@ -111,6 +111,7 @@ SIGNATURES = {
     "bma_mask_block_class": (C.c_int32, [C.POINTER(MaskSpec), C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "bma_attn_fwd": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p]),
     "bma_attn_fwd_workspace_bytes": (C.c_size_t, [C.POINTER(AttnArgs), C.POINTER(BlockLists)]),
+    "bma_attn_fwd_uses_workspace": (C.c_int32, [C.POINTER(AttnArgs), C.POINTER(BlockLists)]),
     "bma_attn_fwd_ws": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t, C.c_void_p]),
     "bma_attn_f32_workspace_bytes": (C.c_size_t, [C.POINTER(AttnArgs), C.c_int32]),
     "bma_attn_fwd_f32": (C.c_int, [C.POINTER(AttnArgs), C.POINTER(MaskSpec), C.POINTER(BlockLists), C.c_void_p, C.c_size_t, C.c_void_p]),

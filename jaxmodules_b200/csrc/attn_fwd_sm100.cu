@@ -20,7 +20,6 @@
 // S_x (overwrites it) needs no extra barrier.  Every mbarrier wait is bounded; on a timeout the
 // thread records an error code and unwinds to the common exit where TMEM is released.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -1100,7 +1099,6 @@ enum {
   SB_V_FREE = SB_V_FULL + 2, SB_NUM = SB_V_FREE + 2
 };
 constexpr int kSplitKStages = 3, kSplitVStages = 2;
-constexpr int kMaxCluster = 8;   // runs that meet in shared memory
 
 template <int HD>
 struct __align__(1024) FwdSplitSmem {
@@ -1667,10 +1665,7 @@ static SplitPlan split_plan(const bma_attn_args& a, const bma_block_lists& l) {
   const int64_t units = (int64_t)a.B * (a.Hq / p.heads) * p.q_tiles;
   if (units > (1 << 20)) return p;
   p.units = (int)units;
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? std::max(n, 1) : 148;
-  }();
+  const int sms = device_sms(current_device());
   double best = 1e30;
   for (int s = 1; s <= std::min(l.NKV / 2, sms); ++s) {
     if (s > 1 && units * s > (int64_t)kMaxSplitWaves * sms) break;
@@ -1688,51 +1683,27 @@ bool sm100_fwd_wants_lists(const bma_attn_args& a, const bma_mask_spec& spec) {
   return split_plan(a, one).splits == 0 && fwd_persistent_enabled(spec);
 }
 
+// CTAs of a cluster: the runs of a unit, where up to eight of them run at the same time on the SMs of a GPC without making more waves
+// of the launch; else 1, and the runs meet in the workspace.  (4 runs of 32 units, 16 queries on 8192 keys: 32 us against
+// 33 + 4 in two launches.)
+static bool needs_kb(const bma_attn_args& a) { return a.key_bias != nullptr || !(a.scale > 0.f); }
+static int split_cluster(const bma_attn_args& a, const SplitPlan& plan) {
+  if (plan.splits < 2 || plan.splits > kMaxParts) return 1;
+  static ClusterCounts known[2][2];
+  const bool kb = needs_kb(a);
+  ClusterCounts& k = known[a.d == 128][kb];
+  const int clusters = a.d == 128 ? clusters_at_once(k, kb ? fwd_split_kernel<128, true, true> : fwd_split_kernel<128, false, true>, kThreads, sizeof(FwdSplitSmem<128>), plan.splits)
+                                  : clusters_at_once(k, kb ? fwd_split_kernel<64, true, true> : fwd_split_kernel<64, false, true>, kThreads, sizeof(FwdSplitSmem<64>), plan.splits);
+  return clusters > 0 && ceil_div(plan.units, clusters) <= ceil_div(plan.units * plan.splits, device_sms(current_device())) ? plan.splits : 1;
+}
+
 size_t sm100_fwd_workspace_bytes(const bma_attn_args& a, const bma_block_lists& lists) {
   const SplitPlan p = split_plan(a, lists);
   return p.splits > 1 ? (size_t)p.units * p.splits * BM * (a.d + 2) * sizeof(float) : 0;
 }
-
-// CTAs of a cluster: the runs of a unit, where up to eight of them run at the same time on the SMs of a GPC without making more waves
-// of the launch; else 1, and the runs meet in the workspace.  (4 runs of 32 units, 16 queries on 8192 keys: 32 us against
-// 33 + 4 in two launches.)
-static cudaLaunchAttribute cluster_of(int n) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 1; attr.val.clusterDim.y = n; attr.val.clusterDim.z = 1;
-  return attr;
-}
-static cudaLaunchConfig_t split_config(const SplitPlan& plan, size_t smem, cudaStream_t st) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(plan.units, plan.splits);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  return cfg;
-}
-static int split_cluster(int d, const SplitPlan& plan) {
-  if (plan.splits < 2 || plan.splits > kMaxCluster) return 1;
-  static std::atomic<int> at_once[2][kMaxCluster + 1];   // clusters of a size that the device runs at the same time, plus one
-  std::atomic<int>& known = at_once[d == 128][plan.splits];
-  int n = known.load(std::memory_order_relaxed);
-  if (!n) {
-    auto ask = [&](auto kernel, size_t smem) {
-      cudaLaunchConfig_t cfg = split_config(plan, smem, nullptr);
-      cudaLaunchAttribute attr = cluster_of(plan.splits);
-      cfg.attrs = &attr; cfg.numAttrs = 1;
-      int most = 0;
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-          cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();
-        most = 0;
-      }
-      return most;
-    };
-    n = 1 + (d == 128 ? ask(fwd_split_kernel<128, false, true>, sizeof(FwdSplitSmem<128>)) : ask(fwd_split_kernel<64, false, true>, sizeof(FwdSplitSmem<64>)));
-    known.store(n, std::memory_order_relaxed);
-  }
-  const int clusters = n - 1;
-  return clusters > 0 && ceil_div(plan.units, clusters) <= ceil_div(plan.units * plan.splits, kSms) ? plan.splits : 1;
+bool sm100_fwd_uses_workspace(const bma_attn_args& a, const bma_block_lists& lists) {
+  const SplitPlan p = split_plan(a, lists);
+  return p.splits > split_cluster(a, p);
 }
 
 static int sm100_fwd_split(const bma_attn_args& a, const FwdParams& f, const SplitPlan& plan, const CUtensorMap& mk, const CUtensorMap& mv,
@@ -1745,12 +1716,16 @@ static int sm100_fwd_split(const bma_attn_args& a, const FwdParams& f, const Spl
   p.heads = plan.heads; p.tile_queries = plan.tile_queries; p.q_tiles = plan.q_tiles; p.splits = plan.splits;
   p.part_o = static_cast<float*>(ws);
   p.part_ml = reinterpret_cast<float2*>(p.part_o + (size_t)plan.units * plan.splits * BM * a.d);
-  p.cluster = split_cluster(a.d, plan);
+  p.cluster = split_cluster(a, plan);
   auto launch = [&](auto alone, auto in_cluster, size_t smem) -> int {
     const auto kernel = p.cluster > 1 ? in_cluster : alone;
     BMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cudaLaunchConfig_t cfg = split_config(plan, smem, st);
-    cudaLaunchAttribute attr = cluster_of(p.cluster);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(plan.units, plan.splits);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = cluster_attribute(1, p.cluster);
     if (p.cluster > 1) { cfg.attrs = &attr; cfg.numAttrs = 1; }
     BMA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p));
     return BMA_OK;
@@ -1794,9 +1769,9 @@ int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block
   p.scale_log2 = a.scale * kLog2e;
   p.status = device_status_ptr();
   BMA_REQUIRE(p.status != nullptr, BMA_ERR_CUDA);
-  const bool kb = a.key_bias != nullptr || !(a.scale > 0.f);
+  const bool kb = needs_kb(a);
   const SplitPlan split = split_plan(a, lists);
-  if (split.splits == 1 || split_cluster(a.d, split) > 1 || (split.splits > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_bytes >= sm100_fwd_workspace_bytes(a, lists)))
+  if (split.splits > 0 && (split.splits <= split_cluster(a, split) || (ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_bytes >= sm100_fwd_workspace_bytes(a, lists))))
     return sm100_fwd_split(a, p, split, mk, mv, ws, kb, st);
   if (lists.kv_num && fwd_persistent_enabled(spec)) {
     // One CTA per SM for the whole launch; items are drawn from a counter that is zeroed on the stream first.

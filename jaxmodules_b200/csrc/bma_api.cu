@@ -280,6 +280,10 @@ size_t bma_attn_fwd_workspace_bytes(const bma_attn_args* args, const bma_block_l
   return sm100_fwd_workspace_bytes(*args, *lists);
 }
 
+int32_t bma_attn_fwd_uses_workspace(const bma_attn_args* args, const bma_block_lists* lists) {
+  return validate_common(args) == BMA_OK && lists && pick_backend(args) == BMA_BACKEND_TCGEN05 && sm100_fwd_uses_workspace(*args, *lists);
+}
+
 int32_t bma_attn_fwd_implies_lists(const bma_attn_args* args, const bma_mask_spec* spec) {
   if (validate_common(args) != BMA_OK || !spec || (spec->flags & kTableTerms) || !interval_terms_valid(*spec)) return 0;
   if (bma_attn_f32_workspace_bytes(args, 0)) return 1;

@@ -62,10 +62,10 @@ inline bool longest_first(int64_t tiles, int64_t heads, int64_t batches, int64_t
 inline dim3 cta_grid(bool by_rank, int tiles, int heads, int batches, int parts = 1) {
   return by_rank ? dim3(heads * parts, batches, tiles) : dim3(tiles * parts, heads, batches);
 }
-inline cudaLaunchAttribute cluster_attribute(int parts) {
+inline cudaLaunchAttribute cluster_attribute(int x, int y = 1) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  attr.val.clusterDim.x = x; attr.val.clusterDim.y = y; attr.val.clusterDim.z = 1;
   return attr;
 }
 // The current device, and its number of SMs (asked once per device).
@@ -574,6 +574,7 @@ int simt_wide_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_b
 int sm100_fwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws, size_t ws_bytes,
               cudaStream_t st);
 size_t sm100_fwd_workspace_bytes(const bma_attn_args& a, const bma_block_lists& lists);
+bool sm100_fwd_uses_workspace(const bma_attn_args& a, const bma_block_lists& lists);
 bool sm100_fwd_wants_lists(const bma_attn_args& a, const bma_mask_spec& spec);
 struct BwdPreprocess;
 int sm100_bwd(const bma_attn_args& a, const bma_mask_spec& spec, const bma_block_lists& lists, void* ws,

@@ -27,7 +27,7 @@ using OptTensor = std::optional<Tensor>;
 // ---- the library ------------------------------------------------------------------------------------------------
 #define BMA_FUNCTIONS(X)                                                                                                      \
   X(bma_mask_compile_workspace_bytes) X(bma_mask_compile) X(bma_attn_plan) X(bma_attn_bwd_plan) X(bma_attn_fwd_implies_lists) X(bma_attn_fwd_workspace_bytes) \
-  X(bma_attn_fwd_ws) X(bma_attn_f32_workspace_bytes) X(bma_attn_fwd_f32) X(bma_attn_bwd_f32) X(bma_attn_bwd_f32_o) X(bma_attn_bwd_preprocess)       \
+  X(bma_attn_fwd_uses_workspace) X(bma_attn_fwd_ws) X(bma_attn_f32_workspace_bytes) X(bma_attn_fwd_f32) X(bma_attn_bwd_f32) X(bma_attn_bwd_f32_o) X(bma_attn_bwd_preprocess)       \
   X(bma_attn_bwd_workspace_bytes) X(bma_attn_bwd_scratch_bytes) X(bma_attn_bwd_scratch_min_bytes) X(bma_attn_bwd) X(bma_attn_bwd_o)
 struct Library {
 #define X(name) decltype(&::name) name = nullptr;
@@ -185,7 +185,7 @@ std::tuple<Tensor, Tensor> forward(const Tensor& q, const Tensor& k, const Tenso
   a.o = describe(o);
   a.lse = lse.data_ptr<float>();
   size_t ws_bytes = 0;
-  if (!f32_bytes && (ws_bytes = lib.bma_attn_fwd_workspace_bytes(&a, lists))) ws = bytes_on(q, ws_bytes);
+  if (!f32_bytes && lib.bma_attn_fwd_uses_workspace(&a, lists)) ws = bytes_on(q, ws_bytes = lib.bma_attn_fwd_workspace_bytes(&a, lists));
   int rc;
   {
     Group group("bma.fwd");

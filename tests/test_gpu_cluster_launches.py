@@ -1,6 +1,7 @@
 """That the CTAs of a cluster do share walks and runs where the tests of tests/test_gpu_shared_walks.py, tests/test_gpu_f32_shared_rows.py and
 tests/test_gpu_implied_lists.py mean them to (bma_cluster_launch_count), and the kernels with a key bias and with results that are not finite
 while they share."""
+import ctypes as C
 import math
 
 import pytest
@@ -64,6 +65,8 @@ def test_few_queries(B, N, L, Hq, Hkv, d, clusters):
     q, k, v, _ = _inputs(B, N, L, Hq, Hkv, d, torch.bfloat16)
     _, n, sizes = launches(lambda: jm.masked_attention_via_map(q, k, v, block_size=N + 1))
     assert len(sizes) == clusters and n == 2 - clusters
+    args, lists = A._make_args(q, k, v), nat.BlockLists(1, 1, 1, -(-L // 128), 128, 128)
+    assert nat.lib().bma_attn_fwd_uses_workspace(C.byref(args), C.byref(lists)) == 1 - clusters      # (and none is allocated where it is not)
 
 
 @pytest.mark.parametrize("dtype,d", [(torch.float32, 64), (torch.float32, 128), (torch.bfloat16, 64), (torch.bfloat16, 128)])
