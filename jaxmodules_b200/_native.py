@@ -172,7 +172,7 @@ _host = None
 
 
 def host():
-    """The extension module _host.so (csrc/host.cc), bound to the loaded library; raises if it was not built."""
+    """The extension module _host.so (csrc/host.cc), bound to the loaded library; raises if it was not built, or built for another torch."""
     global _host
     if _host is None:
         handle = lib()
@@ -180,6 +180,9 @@ def host():
             from . import _host as module
         except ImportError as e:
             raise RuntimeError(f"jaxmodules_b200/_host.so cannot be loaded ({e}): build it with `python -m jaxmodules_b200.build`") from e
+        if module.torch_version != torch.__version__:
+            raise RuntimeError(f"jaxmodules_b200/_host.so was built for torch {module.torch_version}, this is {torch.__version__}: build it again with "
+                               "`python -m jaxmodules_b200.build`")
         module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in SIGNATURES}, BmaError)
         _host = module
     return _host

@@ -1,4 +1,5 @@
-"""Builds libbma.so (the C-ABI library with every CUDA kernel) in-tree with nvcc for sm_100a, and _host.so (the host side of a call, csrc/host.cc).
+"""Builds libbma.so (the C-ABI library with every CUDA kernel) in-tree with nvcc for sm_100a, and, where torch is installed, _host.so (the host
+side of a call, csrc/host.cc) with the host compiler, for that torch.  The library needs neither.
 
     python -m jaxmodules_b200.build [--force] [--verbose]
 
@@ -62,7 +63,6 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     with ThreadPoolExecutor(max_workers=min(8, len(SOURCES)) + 1) as ex:
         host = ex.submit(_build_host, force)
         results = list(ex.map(compile_one, SOURCES))
-        host.result()
     objs = [str(o) for o, _ in results]
     if verbose:
         for _, log in results:
@@ -73,26 +73,36 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    host.result()
     _build_jax_adapter(force)
     return LIB
 
 
 def _build_host(force: bool) -> None:
-    """_host.so: the extension module between torch tensors and the entry points of the library."""
-    src = CSRC / "host.cc"
-    if not force and not _stale(HOST, [src, PKG.parent / "include" / "bma.h", Path(__file__)]):
-        return
+    """_host.so: the extension module between torch tensors and the entry points of the library.  It is built again for another torch, Python or
+    compiler: what it was built with lies beside the objects."""
+    import importlib.metadata
     import sysconfig
+    try:
+        importlib.metadata.version("torch")
+    except importlib.metadata.PackageNotFoundError:
+        return
+    src, cxx, stamp = CSRC / "host.cc", os.environ.get("CXX", "g++"), OBJ / "host.with"
+    made_with = f"torch {importlib.metadata.version('torch')}, {sysconfig.get_config_var('SOABI')}, {cxx}"
+    if not force and not _stale(HOST, [src, PKG.parent / "include" / "bma.h", Path(__file__)]) and stamp.exists() and stamp.read_text() == made_with:
+        return
     import torch
     inc = Path(torch.__file__).parent / "include"
     dirs = [sysconfig.get_paths()["include"], inc, inc / "torch" / "csrc" / "api" / "include", Path(_nvcc()).resolve().parent.parent / "include"]
-    cmd = [os.environ.get("CXX", "g++"), "-shared", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    cmd = [cxx, "-shared", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f'-DBMA_TORCH_VERSION="{torch.__version__}"']
     for d in dirs:
         cmd += ["-isystem", str(d)]
     cmd += [str(src), "-o", str(HOST), "-L", str(Path(torch.__file__).parent / "lib"), "-lc10", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-ldl"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"building the host module failed:\n{r.stdout}\n{r.stderr}")
+    stamp.write_text(made_with)
 
 
 def _build_jax_adapter(force: bool) -> None:

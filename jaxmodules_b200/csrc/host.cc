@@ -266,6 +266,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q, const Tensor& k, co
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
+  m.attr("torch_version") = BMA_TORCH_VERSION;   // the one whose headers this was built with
   m.def("bind", &bind);
   m.def("routes", torch::wrap_pybind_function(routes));
   m.def("implies_lists", torch::wrap_pybind_function(implies_lists));
