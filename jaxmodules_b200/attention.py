@@ -147,20 +147,6 @@ def plan(Q, K, V, backend=nat.BMA_BACKEND_AUTO, backward: bool = False, key_bias
     return be.value, tq.value, tk.value
 
 
-def _route(a: nat.AttnArgs, backward: bool):
-    """(backend, q_tile, kv_tile, workspace bytes) of one pass for an argument structure; the workspace is that of the float32
-    tensor-core kernels (``bma_attn_fwd_f32`` / ``bma_attn_bwd_f32``) and 0 where ``plan``'s kernels run."""
-    lib = nat.lib()
-    if a.q.dtype == nat.BMA_DTYPE_F32:
-        nbytes = lib.bma_attn_f32_workspace_bytes(C.byref(a), int(backward))
-        if nbytes:
-            return nat.BMA_BACKEND_SIMT, nat.F32_TILE, nat.F32_TILE, nbytes
-    be, tq, tk = C.c_int32(), C.c_int32(), C.c_int32()
-    fn = lib.bma_attn_bwd_plan if backward else lib.bma_attn_plan
-    nat.check(fn(C.byref(a), C.byref(be), C.byref(tq), C.byref(tk)), "bma_attn_plan")
-    return be.value, tq.value, tk.value, 0
-
-
 def tiles(Q, K, V, backend=nat.BMA_BACKEND_AUTO, backward: bool = False, key_bias=None, scale=None):
     """(q_tile, kv_tile) of the block lists that ``attention_forward`` / ``attention_backward`` consume.  They are
     ``plan``'s, except for float32 inputs on the tensor core, whose lists have 128-blocks."""

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 import jaxmodules_b200 as jm
-from jaxmodules_b200 import attention as A
+from jaxmodules_b200 import _native as nat, attention as A
 from jaxmodules_b200 import masks as M
 
 pytestmark = pytest.mark.gpu
@@ -43,8 +43,7 @@ def test_without_planes(monkeypatch, refuse, N, L, d, kw):
                 raise torch.OutOfMemoryError("no room")
             return empty(*a, **k)
 
-        args = A._make_args(t[0], t[1], t[2])
-        sizes = {A._route(args, b)[3] for b in (False, True)}
+        sizes = {route[3] for route in nat.host().routes(*t[:3], None, None, nat.BMA_BACKEND_AUTO, True, True)}
         monkeypatch.setattr(torch, "empty", no_planes)
     got = _call(t, kw)
     monkeypatch.undo()
