@@ -206,7 +206,8 @@ def _maybe_check_status(dev, where):
 
 def set_profile_sink(sink):
     """Install (or remove with None) a dict that collects (start, end) CUDA event pairs per
-    launch group: 'mask_compile', 'fwd', 'bwd_preprocess', 'bwd'."""
+    launch group: 'mask_compile', 'fwd', 'bwd_preprocess', 'bwd'.  So that it can be timed by itself, the preprocess of a bfloat16
+    backward pass is then a launch of its own; without a sink it shares the launch of the slot tables."""
     global _profile_sink
     _profile_sink = sink
 
@@ -249,7 +250,9 @@ def attention_forward(Q, K, V, terms: _masks.MaskTerms, *, out_dtype=torch.float
 
 
 def attention_backward(Q, K, V, O, lse, dO, ctx, backend=nat.BMA_BACKEND_AUTO):
-    """dQ, dK, dV through ``bma_attn_bwd_preprocess`` + ``bma_attn_bwd``."""
+    """dQ, dK, dV through ``bma_attn_bwd_f32_o`` or ``bma_attn_bwd_o``, which take delta themselves; where the caller keeps delta for several
+    calls (``ctx["reuse"]``), where the FP32 tile kernels run and under a profile sink through ``bma_attn_bwd_preprocess`` and
+    ``bma_attn_bwd_f32`` or ``bma_attn_bwd``."""
     host = nat.host()
     dev = Q.device
     B, N, Hq, _ = Q.shape

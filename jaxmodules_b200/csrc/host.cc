@@ -1,9 +1,8 @@
 // The host side of one attention or mask call: arguments, allocations, launches, one call per step from Python.
 //
 // A small call is bound by its host path: the passes of 2 x 128 float32 tokens of 8 heads take 43 us of the device, and took 200 us
-// of the host with the argument structures filled in, and the tensors allocated, from Python (144 us now; 16 queries against 8192 keys
-// 62 -> 45 us, 39 of them on the device; create_block_mask of 16 x 16 blocks 48 -> 22).  Everything is built for one call and
-// dropped with it; the library's entry points are those of include/bma.h, handed over as addresses by jaxmodules_b200/_native.py,
+// of the host with the argument structures filled in, and the tensors allocated, from Python (136 - 147 us now; create_block_mask of
+// 16 x 16 blocks 48 -> 22).  Everything is built for one call and dropped with it; the library's entry points are those of include/bma.h, handed over as addresses by jaxmodules_b200/_native.py,
 // so that both sides use the one library that is loaded.
 #include <cuda_runtime_api.h>
 #include <nvtx3/nvToolsExt.h>
