@@ -154,7 +154,7 @@ inline Walks k_walks(const bma_attn_args& a, const bma_mask_spec& spec) {
 }
 // The number of CTAs that share a walk, for the shortest time of the launch.  With n clusters at once a launch takes the longest of: waves of
 // walks of one length, or else the longest walk, or the even share of all; each CTA `extra` tiles besides its own.  Where the walks may be much
-// shorter than they are taken to be, more CTAs than run at once cost more than they give, and have to promise a third less time (float32,
+// shorter than they are taken to be, more CTAs than run at once cost more than they give, and have to promise a quarter less time (float32,
 // documents of 300 of 4096 tokens, one head of 64, forward: 4 CTAs to a walk, all of them at once, 40 us, as unshared; 8 in two waves 54).
 template <typename N>
 int share_walks(const Walks& w, double extra, int most_parts, N clusters) {
@@ -165,7 +165,7 @@ int share_walks(const Walks& w, double extra, int most_parts, N clusters) {
     if (n < 1) continue;
     const double c = w.even ? (double)((w.ctas + n - 1) / n) * (w.longest / parts + extra)
                             : std::max(w.longest / parts + extra, (w.sum / parts + w.ctas * extra) / n * 1.05);
-    if (c < (w.known || n >= w.ctas ? 0.95 : 0.7) * cost) { cost = c; best = parts; }
+    if (c < (w.known || n >= w.ctas ? 0.95 : 0.75) * cost) { cost = c; best = parts; }
   }
   return best;
 }
